@@ -5,7 +5,23 @@
 // The reference multiplies one weight matrix by all B activation rows in one pass over the
 // weights (crates/vipera-backend-cpu/src/model.rs:1005-1025) and promises that a row's
 // result does not depend on its neighbours in the batch (model.rs:881-882); here every output
-// element sums over K in the same fixed order whatever M is.
+// element sums over K in an order that is fixed for its class of row counts: up to eight rows, or more.
+//
+// Up to eight rows the stream of W bounds the product (gemv_rows_kernel): a warp reads eight rows of W
+// through a ring of its own, 512 neighbouring bytes of a row at a time, a lane's four values against all
+// rows of A, and adds its lanes' sums at the end.
+// More rows (gemm_simt_kernel): the multiply-add units and the reads of shared memory that feed them.  K is
+// cut into eight slabs (of whole chunks of 32), a slab's even and odd places are two chains of fused
+// multiply-adds (the two halves of a packed 32-bit pair) whose ends are added, and the slabs are added in
+// their order.  A block takes a tile of rows and columns through a ring of cp.async
+// stages (rows of 32 values, 16 bytes of padding so that neighbouring rows' 16-byte reads meet no bank
+// twice), and where the tiles are too few to fill the chip the eight slabs of a tile go to the eight
+// blocks of a cluster, which add their parts through distributed shared memory: one launch and no
+// scratch either way.
+//
+// Measured (B200; a 64 x 64 tile staged value by value before): 8 rows, W 17,920 x 1,536: 166 -> 30 us (3.7 TB/s);
+// 8 rows, W 1,536 x 1,536 and 1,536 x 8,960: 461 -> 16 us on average; 1,024 rows, W 9,728 x 896: 758 -> 535 us
+// (33 TFLOP/s).  Sums in parts are also closer to 64-bit ones: 8e-7 instead of 3e-6 on a decode step's logits.
 //
 // Epilogues:
 //   STORE     out[m, n] = acc (+ bias[n]), stored as float or bfloat16
@@ -15,123 +31,395 @@
 //             out[m, f] = (up + bias) * act(gate + bias), act = silu, silu(z) = z/(1+exp(-z))
 //             (model.rs:4368-4374), or the tanh form of gelu,
 //             0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))
-#include "common.cuh"
+#include "simt.cuh"
 
 enum GemmEpilogue { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU = 2 };
 
-constexpr int BM = 64, BN = 64, BK = 16, PAD = 4;
+constexpr int kSlabs = 8;          // parts of K with sums of their own
+constexpr int kChunk = 32;         // values of K a stage holds
+constexpr int kPitch = kChunk + 4; // floats per staged row
 
-template <typename TA, typename TW, typename TO, int EPI>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, int M, int N, int K,
-                 const float* __restrict__ bias, TO* __restrict__ out, float* __restrict__ resid, int activation) {
-  __shared__ float As[BK][BM + PAD];
-  __shared__ float Ws[BK][BN + PAD];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int load_row = tid >> 2, load_k = (tid & 3) * 4;
+// The tiles.  A warp's lanes are LM x LN; a thread owns TM x TN outputs, LM rows and LN columns apart.
+template <int BM_, int BN_, int WM_, int WN_, int LM_, int LN_, int TM_, int TN_, int STAGES_>
+struct Tile {
+  static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, LM = LM_, LN = LN_, TM = TM_, TN = TN_, STAGES = STAGES_;
+  static constexpr int kThreads = WM * WN * 32;
+  static constexpr int kSumPitch = BN + 8;
+  static constexpr int kStageFloats = (BM + BN) * kPitch;
+  static constexpr int kSharedBytes = (STAGES * kStageFloats + BM * kSumPitch) * 4;
+  static_assert(LM * LN == 32 && WM * LM * TM == BM && WN * LN * TN == BN, "the tile is covered once");
+};
+using TileSome = Tile<32, 128, 4, 1, 1, 32, 8, 4, 3>;
+using TileMid = Tile<64, 128, 2, 2, 4, 8, 8, 8, 3>;
+using TileMany = Tile<128, 128, 4, 2, 4, 8, 8, 8, 3>;
 
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+struct GemmArgs {
+  const void* A;
+  const void* W;
+  int M, N, K, slab;   // slab: values of K per slab, a multiple of kChunk
+  const float* bias;
+  void* out;
+  float* resid;
+  int activation, epilogue, out_bf16;
+};
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    {
-      const int m = m0 + load_row;
-      const TA* src = A + static_cast<size_t>(m) * K + k0 + load_k;
+// `rows` rows of [extent, K] from row0 on, values k0 .. k0 + kChunk - 1, into shared memory as floats; zeros outside.
+// DIRECT: 32-bit rows of whole 16-byte pieces, copied without passing through registers.
+template <typename T, bool DIRECT, int ROWS, int THREADS>
+__device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src, int row0, int extent, int k0, int k_end, int K) {
+  if (DIRECT) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        As[load_k + e][load_row] = (m < M && k0 + load_k + e < K) ? to_float<TA>(src[e]) : 0.0f;
-      const int n = n0 + load_row;
-      const TW* wsrc = W + static_cast<size_t>(n) * K + k0 + load_k;
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        Ws[load_k + e][load_row] = (n < N && k0 + load_k + e < K) ? to_float<TW>(wsrc[e]) : 0.0f;
+    for (int i = threadIdx.x; i < ROWS * (kChunk / 4); i += THREADS) {
+      const int r = i / (kChunk / 4), piece = (i % (kChunk / 4)) * 4;
+      const bool valid = row0 + r < extent && k0 + piece < k_end;
+      copy_16(shared_address(dst + r * kPitch + piece),
+              reinterpret_cast<const float*>(src) + (valid ? static_cast<size_t>(row0 + r) * K + k0 + piece : 0), valid);
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[4], w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+  } else {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < ROWS * kChunk; i += THREADS) {
+      const int r = i / kChunk, k = i % kChunk;
+      const bool valid = row0 + r < extent && k0 + k < k_end;
+      dst[r * kPitch + k] = valid ? to_float<T>(src[static_cast<size_t>(row0 + r) * K + k0 + k]) : 0.0f;
     }
-    __syncthreads();
   }
+}
 
+template <typename TA, typename TW, typename T, bool DIRECT, bool CLUSTER>
+__global__ void __launch_bounds__(T::kThreads)
+gemm_simt_kernel(const GemmArgs p) {
+  extern __shared__ __align__(16) float gemm_shared[];
+  float* sums = gemm_shared + T::STAGES * T::kStageFloats;   // [BM][kSumPitch]
+  const TA* A = static_cast<const TA*>(p.A);
+  const TW* W = static_cast<const TW*>(p.W);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile_n = CLUSTER ? blockIdx.x / kSlabs : blockIdx.x;
+  const int own_slab = CLUSTER ? blockIdx.x % kSlabs : 0;
+  const int m0 = blockIdx.y * T::BM, n0 = tile_n * T::BN;
+  const int first_m = (warp / T::WN) * (T::LM * T::TM) + lane / T::LN;
+  const int first_n = (warp % T::WN) * (T::LN * T::TN) + lane % T::LN;
+  const int begin = own_slab * p.slab, end = CLUSTER ? min(p.K, begin + p.slab) : p.K;
+  const int chunks = end > begin ? (end - begin + kChunk - 1) / kChunk : 0;   // (slabs are whole chunks)
+  const int slab_chunks = p.slab / kChunk;
+
+  auto stage_w = [&](int chunk) {
+    if (chunk < chunks)
+      stage_rows<TW, DIRECT, T::BN, T::kThreads>(gemm_shared + (chunk % T::STAGES) * T::kStageFloats + T::BM * kPitch, W, n0, p.N,
+                                                 begin + chunk * kChunk, end, p.K);
+  };
+  auto stage_a = [&](int chunk) {
+    if (chunk < chunks)
+      stage_rows<TA, DIRECT, T::BM, T::kThreads>(gemm_shared + (chunk % T::STAGES) * T::kStageFloats, A, m0, p.M,
+                                                 begin + chunk * kChunk, end, p.K);
+    copy_commit();
+  };
+  pdl_launch_dependents();
+  // the weights of the first stages are asked for before the kernel ahead has ended
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-    if (EPI == EPI_SWIGLU) {
-      // columns tx, tx+16 are gate and up of feature (n0/2 + tx); tx+32, tx+48 of (n0/2 + 16 + tx)
+  for (int c = 0; c < T::STAGES - 1; ++c) stage_w(c);
+  pdl_wait();
 #pragma unroll
-      for (int pair = 0; pair < 2; ++pair) {
-        const int n_gate = n0 + tx + 32 * pair;
-        if (n_gate + 16 >= N) continue;
-        const int feature = n0 / 2 + 16 * pair + tx;
-        float gate = acc[i][2 * pair], up = acc[i][2 * pair + 1];
-        if (bias) {
-          gate += bias[n_gate];
-          up += bias[n_gate + 16];
+  for (int c = 0; c < T::STAGES - 1; ++c) stage_a(c);
+
+  unsigned long long acc[T::TM][T::TN];   // (sum over even places, sum over odd places)
+#pragma unroll
+  for (int i = 0; i < T::TM; ++i)
+#pragma unroll
+    for (int j = 0; j < T::TN; ++j) acc[i][j] = 0ull;
+
+  int in_slab = 0;
+  bool summed = false;
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    copy_wait<T::STAGES - 2>();
+    __syncthreads();   // this chunk has landed for every thread, and the one before is read out
+    stage_w(chunk + T::STAGES - 1);
+    stage_a(chunk + T::STAGES - 1);
+    const float* a_s = gemm_shared + (chunk % T::STAGES) * T::kStageFloats + first_m * kPitch;
+    const float* w_s = gemm_shared + (chunk % T::STAGES) * T::kStageFloats + (T::BM + first_n) * kPitch;
+#pragma unroll
+    for (int k = 0; k < kChunk; k += 4) {
+      ulonglong2 a[T::TM];
+#pragma unroll
+      for (int i = 0; i < T::TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * T::LM * kPitch + k);
+#pragma unroll
+      for (int j = 0; j < T::TN; ++j) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(w_s + j * T::LN * kPitch + k);
+#pragma unroll
+        for (int i = 0; i < T::TM; ++i) {
+          fma_pair(acc[i][j], a[i].x, w.x);
+          fma_pair(acc[i][j], a[i].y, w.y);
         }
-        const float value = up * gate_activation(gate, activation);
-        out[static_cast<size_t>(m) * (N / 2) + feature] = from_float<TO>(value);
       }
+    }
+    if (++in_slab == slab_chunks || chunk + 1 == chunks) {
+      // a slab's end: its sums join the tile's (a thread's own places)
+#pragma unroll
+      for (int i = 0; i < T::TM; ++i)
+#pragma unroll
+        for (int j = 0; j < T::TN; ++j) {
+          float* at = sums + (first_m + i * T::LM) * T::kSumPitch + first_n + j * T::LN;
+          const float slab_sum = sum_of_pair(acc[i][j]);
+          *at = summed ? *at + slab_sum : slab_sum;
+          acc[i][j] = 0ull;
+        }
+      in_slab = 0;
+      summed = true;
+    }
+  }
+  if (CLUSTER) cluster_sync();
+  else __syncthreads();
+
+  // The ending.  In a cluster each block finishes every eighth row of the tile.
+  const int used_slabs = CLUSTER ? (p.K + p.slab - 1) / p.slab : 1;
+  auto total = [&](int m, int n) {
+    if (!CLUSTER) return sums[m * T::kSumPitch + n];
+    const uint32_t at = shared_address(sums + m * T::kSumPitch + n);
+    float part[kSlabs];   // (what a block without values of K holds is not used)
+#pragma unroll
+    for (int s = 0; s < kSlabs; ++s) part[s] = remote_float(at, s);
+    float sum = part[0];
+#pragma unroll
+    for (int s = 1; s < kSlabs; ++s) sum = s < used_slabs ? sum + part[s] : sum;
+    return sum;
+  };
+  const bool gated = p.epilogue == EPI_SWIGLU;
+  const int columns = gated ? T::BN / 2 : T::BN;   // (powers of two)
+  const int column_bits = 31 - __clz(columns), blocks = CLUSTER ? kSlabs : 1;
+  auto store = [&](size_t at, float value) {
+    if (p.out_bf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value);
+    else static_cast<float*>(p.out)[at] = value;
+  };
+  for (int i = threadIdx.x; i < T::BM / blocks * columns; i += T::kThreads) {
+    const int m = (i >> column_bits) * blocks + own_slab, c = i & (columns - 1);
+    if (m0 + m >= p.M) continue;
+    if (gated) {
+      const int n = (c / 16) * 32 + c % 16;   // the gate's column; the feature's up value is 16 further
+      if (n0 + n + 16 >= p.N) continue;
+      float gate = total(m, n), up = total(m, n + 16);
+      if (p.bias) {
+        gate += p.bias[n0 + n];
+        up += p.bias[n0 + n + 16];
+      }
+      store(static_cast<size_t>(m0 + m) * (p.N / 2) + n0 / 2 + c, up * gate_activation(gate, p.activation));
     } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = n0 + tx + 16 * j;
-        if (n >= N) continue;
-        float value = acc[i][j];
-        if (EPI == EPI_STORE) {
-          if (bias) value += bias[n];
-          out[static_cast<size_t>(m) * N + n] = from_float<TO>(value);
-        } else {
-          if (bias) value += bias[n];
-          resid[static_cast<size_t>(m) * N + n] += value;
-        }
-      }
+      if (n0 + c >= p.N) continue;
+      float value = total(m, c);
+      if (p.bias) value += p.bias[n0 + c];
+      const size_t at = static_cast<size_t>(m0 + m) * p.N + n0 + c;
+      if (p.epilogue == EPI_STORE) store(at, value);
+      else p.resid[at] += value;
     }
   }
+  if (CLUSTER) cluster_sync();   // no block leaves while another reads its part
+}
+
+// ---------------------------------------------------------------------------------------
+// Up to eight rows.  A group of `warps` warps (1, 2, 4 or 8, as many as it takes to give every
+// multiprocessor a dozen) shares eight rows of W, each warp every `warps`-th run of 128 values of K.  Two
+// runs are in flight while one is used, the first two before the kernel ahead has ended.  MR: rows of A
+// computed (1, 2, 4 or 8; the sums' order does not depend on it).
+// ---------------------------------------------------------------------------------------
+constexpr int kFewRows = 8;     // rows of A, and rows of W a warp holds
+constexpr int kFewWarps = 8;    // of a block
+constexpr int kFewStages = 3;   // runs of a warp's ring
+
+template <int MR>
+__global__ void __launch_bounds__(kFewWarps * 32, 2)
+gemv_rows_kernel(const GemmArgs p, int warps) {
+  __shared__ float parts[kFewWarps][kFewRows * MR];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = (blockIdx.x * kFewWarps + warp) / warps, member = warp % warps;
+  const float* A = static_cast<const float*>(p.A);
+  const float* W = static_cast<const float*>(p.W);
+  const bool gated = p.epilogue == EPI_SWIGLU;
+  // the group's rows: eight neighbours, or the gates and the ups of four neighbouring features
+  auto row_of = [&](int r) {
+    if (!gated) return group * kFewRows + r;
+    const int feature = group * (kFewRows / 2) + r % (kFewRows / 2);
+    return feature / 16 * 32 + feature % 16 + (r >= kFewRows / 2 ? 16 : 0);
+  };
+  // A lane copies the 16 bytes of each row that it will use itself, so a wait for its own copies is all it needs.
+  extern __shared__ __align__(16) float few_shared[];
+  float* ring = few_shared + (warp * kFewStages * kFewRows * 32 + lane) * 4;
+  const float* rows[kFewRows];
+  bool live[kFewRows];
+#pragma unroll
+  for (int r = 0; r < kFewRows; ++r) {
+    const int n = row_of(r);
+    live[r] = n < p.N;
+    rows[r] = W + (live[r] ? static_cast<size_t>(n) * p.K : 0);
+  }
+  const int step = warps * 128;
+  auto ask = [&](int stage, int k) {
+#pragma unroll
+    for (int r = 0; r < kFewRows; ++r) {
+      const bool valid = live[r] && k < p.K;
+      copy_16(shared_address(ring + (stage * kFewRows + r) * 128), rows[r] + (valid ? k : 0), valid);
+    }
+    copy_commit();
+  };
+  int k = member * 128 + lane * 4;
+  pdl_launch_dependents();
+#pragma unroll
+  for (int stage = 0; stage < kFewStages - 1; ++stage) ask(stage, k + stage * step);
+  pdl_wait();
+  float acc[kFewRows * MR];
+#pragma unroll
+  for (int i = 0; i < kFewRows * MR; ++i) acc[i] = 0.0f;
+  int stage = 0;
+  for (int k0 = member * 128; k0 < p.K; k0 += step, k += step) {
+    float4 a[MR];
+#pragma unroll
+    for (int m = 0; m < MR; ++m)
+      a[m] = k < p.K && m < p.M ? *reinterpret_cast<const float4*>(A + static_cast<size_t>(m) * p.K + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    copy_wait<kFewStages - 2>();
+    const int last = stage == 0 ? kFewStages - 1 : stage - 1;
+    ask(last, k + (kFewStages - 1) * step);   // (the stage read out in the pass before)
+#pragma unroll
+    for (int r = 0; r < kFewRows; ++r) {
+      const float4 w = *reinterpret_cast<const float4*>(ring + (stage * kFewRows + r) * 128);
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        float& sum = acc[m * kFewRows + r];
+        sum = fmaf(a[m].x, w.x, sum);
+        sum = fmaf(a[m].y, w.y, sum);
+        sum = fmaf(a[m].z, w.z, sum);
+        sum = fmaf(a[m].w, w.w, sum);
+      }
+    }
+    stage = stage == kFewStages - 1 ? 0 : stage + 1;
+  }
+  // The lanes' sums: at each step a lane keeps one half of the values it holds and hands over the other, until
+  // it holds one or two; then every lane holds the same value's.
+  int held = kFewRows * MR, first = 0;
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1) {
+    const bool upper = (lane & offset) != 0;
+    if (held > 1) {
+      held >>= 1;
+#pragma unroll
+      for (int i = 0; i < kFewRows * MR / 2; ++i) {
+        if (i < held) {
+          const float keep = upper ? acc[i + held] : acc[i], give = upper ? acc[i] : acc[i + held];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, offset);
+        }
+      }
+      if (upper) first += held;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], offset);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kFewRows * MR / 2; ++i)
+    if (i < held) parts[warp][first + i] = acc[i];
+  __syncthreads();
+  auto total = [&](int own, int i) {   // value i of the block's group `own`, its warps in their order
+    float sum = parts[own * warps][i];
+    for (int o = 1; o < warps; ++o) sum += parts[own * warps + o][i];
+    return sum;
+  };
+  auto store = [&](size_t at, float value) {
+    if (p.out_bf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value);
+    else static_cast<float*>(p.out)[at] = value;
+  };
+  const int per_group = (gated ? kFewRows / 2 : kFewRows) * MR;
+  for (int i = threadIdx.x; i < kFewWarps / warps * per_group; i += kFewWarps * 32) {
+    const int own = i / per_group, item = i % per_group;
+    const int r = item % (per_group / MR), m = item / (per_group / MR);
+    const int first_row = (blockIdx.x * (kFewWarps / warps) + own) * kFewRows;
+    if (m >= p.M) continue;
+    if (gated) {
+      const int feature = first_row / 2 + r, n = feature / 16 * 32 + feature % 16;
+      if (n + 16 >= p.N) continue;
+      float gate = total(own, m * kFewRows + r), up = total(own, m * kFewRows + r + kFewRows / 2);
+      if (p.bias) {
+        gate += p.bias[n];
+        up += p.bias[n + 16];
+      }
+      store(static_cast<size_t>(m) * (p.N / 2) + feature, up * gate_activation(gate, p.activation));
+    } else {
+      const int n = first_row + r;
+      if (n >= p.N) continue;
+      float value = total(own, m * kFewRows + r);
+      if (p.bias) value += p.bias[n];
+      const size_t at = static_cast<size_t>(m) * p.N + n;
+      if (p.epilogue == EPI_STORE) store(at, value);
+      else p.resid[at] += value;
+    }
+  }
+}
+
+template <int MR>
+static int launch_few_rows(const GemmArgs& p, int warps, dim3 grid, dim3 block, cudaStream_t s) {
+  constexpr int kBytes = kFewWarps * kFewStages * kFewRows * 32 * 16;
+  static SharedMemoryOptIn opt_in;
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(gemv_rows_kernel<MR>), kBytes);
+  return opted ? opted : vipera_launch(gemv_rows_kernel<MR>, grid, block, kBytes, s, p, warps);
+}
+
+static int launch_few(const GemmArgs& p, cudaStream_t s) {
+  constexpr int kWarpsWanted = 148 * 12;
+  const long long groups = (p.N + kFewRows - 1) / kFewRows;
+  int warps = 1;
+  while (warps < kFewWarps && groups * warps < kWarpsWanted) warps *= 2;
+  const dim3 grid(static_cast<unsigned>((groups * warps + kFewWarps - 1) / kFewWarps)), block(kFewWarps * 32);
+  if (p.M == 1) return launch_few_rows<1>(p, warps, grid, block, s);
+  if (p.M == 2) return launch_few_rows<2>(p, warps, grid, block, s);
+  if (p.M <= 4) return launch_few_rows<4>(p, warps, grid, block, s);
+  return launch_few_rows<8>(p, warps, grid, block, s);
+}
+
+template <typename TA, typename TW, typename T, bool DIRECT, bool CLUSTER>
+static int launch_form(const GemmArgs& p, cudaStream_t s) {
+  auto kernel = gemm_simt_kernel<TA, TW, T, DIRECT, CLUSTER>;
+  static SharedMemoryOptIn opt_in;   // one per form of the kernel
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(kernel), T::kSharedBytes);
+  if (opted) return opted;
+  const unsigned tiles_n = (p.N + T::BN - 1) / T::BN, tiles_m = (p.M + T::BM - 1) / T::BM;
+  if (tiles_m > 65535u) return VIPERA_BAD_SHAPE;
+  return launch_in_clusters(kernel, CLUSTER ? kSlabs : 1, dim3(CLUSTER ? tiles_n * kSlabs : tiles_n, tiles_m), dim3(T::kThreads),
+                            T::kSharedBytes, s, p);
+}
+
+// A tile's slabs go to a cluster where whole tiles would leave much of the chip idle: fewer small tiles
+// than multiprocessors, or a last wave that is mostly empty for the large ones (a block a multiprocessor).
+template <typename TA, typename TW, typename T, bool DIRECT>
+static int launch_tile(const GemmArgs& p, cudaStream_t s) {
+  constexpr long long kSms = 148;
+  const long long tiles = static_cast<long long>((p.N + T::BN - 1) / T::BN) * ((p.M + T::BM - 1) / T::BM);
+  bool cluster;
+  if (T::BM <= 32) cluster = tiles < kSms;
+  else cluster = tiles * 5 < (tiles + kSms - 1) / kSms * kSms * 4;
+  // a slab of less than three chunks is all start and ending
+  if (cluster && p.slab >= 3 * kChunk) return launch_form<TA, TW, T, DIRECT, true>(p, s);
+  return launch_form<TA, TW, T, DIRECT, false>(p, s);
+}
+
+template <typename TA, typename TW>
+static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
+  constexpr bool kBothFloat = sizeof(TA) == 4 && sizeof(TW) == 4;
+  if constexpr (kBothFloat) {
+    if (p.K % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.W)) & 15) == 0) {
+      if (p.M <= kFewRows) return launch_few(p, s);
+      if (p.M <= TileSome::BM) return launch_tile<TA, TW, TileSome, true>(p, s);
+      if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileMid, true>(p, s);
+      return launch_tile<TA, TW, TileMany, true>(p, s);
+    }
+  }
+  // rows that do not start on 16 bytes, or values that are widened on the way
+  return launch_tile<TA, TW, TileSome, false>(p, s);
 }
 
 template <typename TA, typename TW>
 static int launch_typed(const TA* A, const TW* W, int M, int N, int K, int epilogue, const float* bias,
                         void* out, int out_dtype, float* resid, int activation, cudaStream_t s) {
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (epilogue == EPI_RESIDUAL) {
-    if (!resid) return VIPERA_BAD_ARGUMENT;
-    gemm_simt_kernel<TA, TW, float, EPI_RESIDUAL><<<grid, 256, 0, s>>>(A, W, M, N, K, bias, nullptr, resid, activation);
-  } else if (epilogue == EPI_STORE) {
-    if (!out) return VIPERA_BAD_ARGUMENT;
-    if (out_dtype == VIPERA_F32)
-      gemm_simt_kernel<TA, TW, float, EPI_STORE><<<grid, 256, 0, s>>>(A, W, M, N, K, bias, static_cast<float*>(out), nullptr, activation);
-    else if (out_dtype == VIPERA_BF16)
-      gemm_simt_kernel<TA, TW, __nv_bfloat16, EPI_STORE><<<grid, 256, 0, s>>>(A, W, M, N, K, bias, static_cast<__nv_bfloat16*>(out), nullptr, activation);
-    else
-      return VIPERA_BAD_DTYPE;
-  } else if (epilogue == EPI_SWIGLU) {
-    if (!out) return VIPERA_BAD_ARGUMENT;
-    if (N % 32 != 0) return VIPERA_BAD_SHAPE;  // gate/up groups of 16 must pair up
-    if (out_dtype == VIPERA_F32)
-      gemm_simt_kernel<TA, TW, float, EPI_SWIGLU><<<grid, 256, 0, s>>>(A, W, M, N, K, bias, static_cast<float*>(out), nullptr, activation);
-    else if (out_dtype == VIPERA_BF16)
-      gemm_simt_kernel<TA, TW, __nv_bfloat16, EPI_SWIGLU><<<grid, 256, 0, s>>>(A, W, M, N, K, bias, static_cast<__nv_bfloat16*>(out), nullptr, activation);
-    else
-      return VIPERA_BAD_DTYPE;
-  } else {
-    return VIPERA_BAD_ARGUMENT;
-  }
-  return vipera_launch_status();
+  const int slab = ((K + kSlabs - 1) / kSlabs + kChunk - 1) / kChunk * kChunk;
+  if (epilogue != EPI_STORE && epilogue != EPI_RESIDUAL && epilogue != EPI_SWIGLU) return VIPERA_BAD_ARGUMENT;
+  if (epilogue == EPI_RESIDUAL ? !resid : !out) return VIPERA_BAD_ARGUMENT;
+  if (epilogue == EPI_SWIGLU && N % 32 != 0) return VIPERA_BAD_SHAPE;  // gate/up groups of 16 must pair up
+  if (epilogue != EPI_RESIDUAL && out_dtype != VIPERA_F32 && out_dtype != VIPERA_BF16) return VIPERA_BAD_DTYPE;
+  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16};
+  return launch_sizes<TA, TW>(p, s);
 }
 
 // A is [M, K] and W is [N, K], both row-major and contiguous.  For SWIGLU, N counts the
