@@ -39,3 +39,66 @@ def test_product_tiles_and_slabs(m, n, k, types):
     last = torch.empty(beside, n, device=DEV)
     ops.gemm_simt(a[-beside:].contiguous(), w, epilogue=ops.EPI_STORE, bias=bias, out=last)
     assert torch.equal(last[-1], out[-1])
+
+
+def _attention_want(q, keys, values, entry, position, heads, kv_heads, scale, mask, sink, chunk, window, keep_first, gate):
+    out = torch.zeros(len(q), heads, values[0].shape[-1], dtype=torch.float64)
+    for t in range(len(q)):
+        e, p = int(entry[t]), int(position[t])
+        j = torch.arange(p + 1)
+        first = p // chunk * chunk if chunk else (max(0, p - window + 1) if window else 0)
+        seen = (j >= first) | ((j < keep_first) if window else (j < 0))
+        for h in range(heads):
+            k, v = keys[e][: p + 1, h // (heads // kv_heads)][seen], values[e][: p + 1, h // (heads // kv_heads)][seen]
+            score = (k.double() @ q[t, h].double()) * scale
+            if sink is not None:
+                score = torch.cat([score, sink[h:h + 1].double()])
+            out[t, h] = torch.softmax(score, 0)[: len(k)] @ v.double()
+    return out * torch.sigmoid(gate.double()).view(len(q), heads, 1)
+
+
+# counts of tokens at the borders of the two forms (64) and of a tile (64 rows, several requests in one), head sizes of
+# every instance, rows that are not whole 16-byte pieces, every mask; a value nobody may see yet is infinite
+@pytest.mark.parametrize("counts,firsts", [([1], [0]), ([1, 1, 1], [5, 130, 700]), ([64], [3]), ([65], [0]), ([1, 70, 130, 1], [90, 0, 65, 200])])
+@pytest.mark.parametrize("d,dv,heads,kv_heads", [(64, 64, 7, 1), (128, 96, 4, 2), (80, 256, 12, 1), (30, 18, 2, 2)])
+@pytest.mark.parametrize("mask", ["all", "window", "chunk"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_forms(counts, firsts, d, dv, heads, kv_heads, mask, dtype):
+    ops = _ops()
+    torch.manual_seed(sum(counts) + d + dv)
+    page, entries = 16, len(counts)
+    longest = max(c + f for c, f in zip(counts, firsts))
+    width = -(-longest // page)
+    table = torch.randperm(entries * width).view(entries, width).to(torch.int32)
+    k_pool = torch.full((entries * width, page, kv_heads, d), float("nan")).to(dtype)
+    v_pool = torch.full((entries * width, page, kv_heads, dv), float("nan")).to(dtype)
+    keys, values = [], []
+    for e, (c, f) in enumerate(zip(counts, firsts)):
+        k, v = torch.randn(c + f, kv_heads, d).to(dtype), torch.randn(c + f, kv_heads, dv).to(dtype)
+        if c > 1:
+            v[-1] = float("inf")
+        at = torch.arange(c + f)
+        k_pool[table[e].long()[at // page], at % page], v_pool[table[e].long()[at // page], at % page] = k, v
+        keys.append(k)
+        values.append(v)
+    entry = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])
+    position = torch.cat([torch.arange(f, f + c, dtype=torch.int32) for c, f in zip(counts, firsts)])
+    tokens, scale = sum(counts), d ** -0.5
+    q = torch.randn(tokens, heads, d).to(dtype)
+    sink, gate = torch.randn(heads), torch.randn(tokens, heads)
+    options = {"all": dict(window=0, keep_first=0, chunk=0), "window": dict(window=50, keep_first=3, chunk=0),
+               "chunk": dict(window=0, keep_first=0, chunk=48)}[mask]
+    learned = sink if mask != "chunk" else None
+    want = _attention_want(q, keys, values, entry, position, heads, kv_heads, scale, mask, learned, gate=gate, **options)
+    out = torch.full((tokens, heads * dv), float("nan"), device=DEV, dtype=dtype)
+    ops.attention(q.view(tokens, -1).to(DEV), out, k_pool.to(DEV), v_pool.to(DEV), token_seq=entry.to(DEV), positions=position.to(DEV),
+                  block_table=table.to(DEV), num_heads=heads, num_kv_heads=kv_heads, head_dim=d, scale=scale, value_dim=dv,
+                  sink_values=None if learned is None else learned.to(DEV), gate=gate.to(DEV), gate_per_head=True, **options)
+    got = out.double().cpu().view(tokens, heads, dv)
+    last = torch.zeros(tokens, dtype=torch.bool)
+    for e, c in enumerate(counts):
+        last |= (entry == e) & (position == firsts[e] + c - 1) & (c > 1)
+    assert torch.isinf(got[last]).all() and torch.isfinite(got[~last]).all()
+    # 32-bit: a few roundings of 2^-24 per term, bfloat16: the output's own rounding
+    if (~last).any():
+        assert _rel(got[~last], want[~last]) < (2e-6 if dtype == torch.float32 else 4e-3)

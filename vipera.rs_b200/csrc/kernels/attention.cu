@@ -4,9 +4,10 @@
 // Definition (crates/vipera-backend-cpu/src/model.rs:1804-1859): query head h reads KV head
 // h / group; s_j = (q . k_j) * scale; a query at position p sees keys 0..p (with a window w,
 // keys p-w+1..p); weights exp(s_j - max) over their sum; output = weighted sum of v_j.
-// Traversal: one warp per (token, query head) folds the keys 32 at a time with a running
-// (max, sum, output), the online form of the reference's chunk fold (model.rs:2752-2857) and
-// of its device kernels' partials (crates/vipera-backend-gpu/src/layer.cu:307-467).
+// Traversal: a block folds the keys 64 at a time with a running (max, sum, output) per row, the online
+// form of the reference's chunk fold (model.rs:2752-2857) and of its device kernels' partials
+// (crates/vipera-backend-gpu/src/layer.cu:307-467); few tokens split their keys between the blocks of a
+// cluster, more share what they read in tiles (see the two kernels).
 // Keys are found through the block table: position j lives in page table[j / page], slot
 // j % page (model.rs:1507-1542).
 //
@@ -20,148 +21,526 @@
 // the output may be gated: out[t, h, e] *= sigmoid(gate[t * gate_stride + h * value_dim + e]), the gate
 // a 32-bit pre-activation (`gate_per_head`: one per head, gate[t * gate_stride + h]).
 //
-// This kernel is the attention of the 32-bit path and takes every head size that is a
-// up to 256 (keys and values each; sizes that are not a multiple of 8 are read value by value), any number of heads and groups, any page size.
-#include "common.cuh"
+// This is the attention of the 32-bit path and of bfloat16 head sizes without tensor-core kernels.  It takes
+// every head size up to 256 (keys and values each; rows that are not whole 16-byte pieces are read value by
+// value), any number of heads and groups, any page size.
+#include "simt.cuh"
 
-constexpr int kWarpsPerBlock = 4;
 constexpr int kMaxHeadDim = 256;
+constexpr int kTileKeys = 64;       // keys a block holds at a time
+constexpr int kAttentionThreads = 128;
 
-template <typename T>
-__device__ __forceinline__ float dot_row(const float* __restrict__ q, const T* __restrict__ row, int d);
+struct AttentionParams {
+  const void* q;
+  void* out;
+  const void* k_pool;
+  const void* v_pool;
+  const int* token_seq;
+  const int* positions;
+  const int* block_table;
+  int table_width, page_size, num_tokens, num_heads, num_kv_heads, head_dim, value_dim;
+  float scale;
+  int window, keep_first, sink, chunk;
+  float out_scale;
+  const float* sink_values;
+  const float* gate;
+  long long gate_stride;
+  int gate_per_head;
+};
 
-template <>
-__device__ __forceinline__ float dot_row<float>(const float* __restrict__ q, const float* __restrict__ row, int d) {
-  float sum = 0.0f;
-  if (d & 3) {   // rows of such a size do not start on 16 bytes
-    for (int i = 0; i < d; ++i) sum = fmaf(q[i], row[i], sum);
-    return sum;
-  }
-  const float4* r4 = reinterpret_cast<const float4*>(row);
-  for (int i = 0; i < d / 4; ++i) {
-    const float4 v = r4[i];
-    sum = fmaf(q[4 * i + 0], v.x, sum);
-    sum = fmaf(q[4 * i + 1], v.y, sum);
-    sum = fmaf(q[4 * i + 2], v.z, sum);
-    sum = fmaf(q[4 * i + 3], v.w, sum);
-  }
-  return sum;
-}
-
-template <>
-__device__ __forceinline__ float dot_row<__nv_bfloat16>(const float* __restrict__ q, const __nv_bfloat16* __restrict__ row, int d) {
-  float sum = 0.0f;
-  if (d & 7) {
-    for (int i = 0; i < d; ++i) sum = fmaf(q[i], __bfloat162float(row[i]), sum);
-    return sum;
-  }
-  const uint4* r8 = reinterpret_cast<const uint4*>(row);
-  for (int i = 0; i < d / 8; ++i) {
-    const uint4 raw = r8[i];
-    const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __bfloat1622float2(pairs[e]);
-      sum = fmaf(q[8 * i + 2 * e], f.x, sum);
-      sum = fmaf(q[8 * i + 2 * e + 1], f.y, sum);
-    }
-  }
-  return sum;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-attention_kernel(const T* __restrict__ q, T* __restrict__ out, const T* __restrict__ k_pool,
-                 const T* __restrict__ v_pool, const int* __restrict__ token_seq,
-                 const int* __restrict__ positions, const int* __restrict__ block_table, int table_width,
-                 int page_size, int num_heads, int num_kv_heads, int head_dim, int value_dim, float scale,
-                 int window, int keep_first, int sink, int chunk, float out_scale,
-                 const float* __restrict__ sink_values, const float* __restrict__ gate, long long gate_stride,
-                 int gate_per_head) {
-  __shared__ float q_shared[kWarpsPerBlock][kMaxHeadDim];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x;
-  const int h = blockIdx.y * kWarpsPerBlock + warp;
-  if (h >= num_heads) return;
-  const int group = num_heads / num_kv_heads;
-  const int kv_head = h / group;
-  const int position = positions[t];
-  const int* table = block_table + static_cast<size_t>(token_seq[t]) * table_width;
+// What a query at `position` sees: keys 0 .. kept - 1 and first .. position.
+__device__ __forceinline__ void visible_keys(const AttentionParams& p, int position, int* kept, int* first) {
   // a mask of chunks: a query sees the keys of its own chunk of `chunk` positions, counted from 0
-  const int first = chunk > 0 ? position / chunk * chunk : (window > 0 ? max(0, position - window + 1) : 0);
+  *first = p.chunk > 0 ? position / p.chunk * p.chunk : (p.window > 0 ? max(0, position - p.window + 1) : 0);
+  *kept = p.window > 0 ? min(p.keep_first, *first) : 0;
+}
 
-  const T* q_row = q + (static_cast<size_t>(t) * num_heads + h) * head_dim;
-  float* qs = q_shared[warp];
-  for (int i = lane; i < head_dim; i += 32) qs[i] = to_float<T>(q_row[i]);
-  __syncwarp();
-
-  float acc[kMaxHeadDim / 32];
+// Rows of a pool (row r's place in place[r], -1: zeros) into shared memory as floats, `pitch` apart.  VEC: rows of
+// whole 16-byte pieces on 16-byte boundaries (32-bit ones are copied asynchronously: the caller waits).
+template <typename T, bool VEC>
+__device__ __forceinline__ void stage_keys(float* dst, int pitch, const T* __restrict__ pool, size_t row_stride, int size,
+                                           const int* place, int rows) {
+  constexpr int kPiece = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;
+  const int pieces = size / kPiece;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < rows * pieces; i += kAttentionThreads) {
+    const int r = i / pieces, c = (i - r * pieces) * kPiece;
+    const int at = place[r];
+    const T* src = pool + (at >= 0 ? static_cast<size_t>(at) * row_stride + c : 0);
+    float* to = dst + r * pitch + c;
+    if constexpr (!VEC) {
+      *to = at >= 0 ? to_float<T>(*src) : 0.0f;
+    } else if constexpr (sizeof(T) == 4) {
+      copy_16(shared_address(to), src, at >= 0);
+    } else {
+      const uint4 raw = at >= 0 ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);
+      const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-  for (int i = 0; i < kMaxHeadDim / 32; ++i) acc[i] = 0.0f;
-  float running_max = -INFINITY, running_sum = 0.0f;
-  const size_t row_stride = static_cast<size_t>(num_kv_heads) * head_dim;
-  const size_t v_stride = static_cast<size_t>(num_kv_heads) * value_dim;
-  // two runs of keys: the kept first ones that the window has left behind, then the window
-  const int kept_end = window > 0 ? min(keep_first, first) : 0;
-
-  for (int run = 0; run < 2; ++run) {
-  const int run_first = run == 0 ? 0 : first;
-  const int run_last = run == 0 ? kept_end - 1 : position;
-  for (int base = run_first; base <= run_last; base += 32) {
-    const int j = base + lane;
-    const bool valid = j <= run_last;
-    float score = -INFINITY;
-    if (valid) {
-      const int page = table[j / page_size];
-      const T* k_row = k_pool + (static_cast<size_t>(page) * page_size + j % page_size) * row_stride +
-                       static_cast<size_t>(kv_head) * head_dim;
-      score = dot_row<T>(qs, k_row, head_dim) * scale;
+      for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(to + 2 * e) = __bfloat1622float2(pairs[e]);
     }
-    const float new_max = fmaxf(running_max, warp_max(score));
-    const float alpha = expf(running_max - new_max);  // 0 on the first tile
-    const float weight = valid ? expf(score - new_max) : 0.0f;
-    running_sum = running_sum * alpha + warp_sum(weight);
-    running_max = new_max;
+  }
+}
+
+// The output gate's factor for (token, head, value e).
+__device__ __forceinline__ float gate_factor(const AttentionParams& p, int t, int h, int e) {
+  if (!p.gate) return 1.0f;
+  const float* row = p.gate + static_cast<size_t>(t) * p.gate_stride;
+  return 1.0f / (1.0f + expf(-(p.gate_per_head ? row[h] : row[static_cast<size_t>(h) * p.value_dim + e])));
+}
+// Folds the sink (a key of score 0, or of a learned one, whose value is zero) into (max, sum); returns the factor
+// of the accumulated output, 1 / sum and out_scale included.
+__device__ __forceinline__ float ending_factor(const AttentionParams& p, int h, float row_max, float row_sum) {
+  if (p.sink || p.sink_values) {
+    const float sink_score = p.sink_values ? p.sink_values[h] : 0.0f;
+    const float top = fmaxf(row_max, sink_score);
+    const float alpha = row_max == top ? 1.0f : expf(row_max - top);
+    return alpha * (p.out_scale / (row_sum * alpha + expf(sink_score - top)));
+  }
+  return p.out_scale / row_sum;
+}
+
+// ---------------------------------------------------------------------------------------
+// Steps of few tokens: a cluster of eight blocks per (token, up to eight query heads of one KV head), an eighth of
+// the visible keys each, joined through distributed shared memory.  A tile of 64 keys and their values is
+// staged; a thread scores one key against four heads (packed multiply-adds), a warp takes the softmax of two heads,
+// a thread then owns value columns of all eight heads.  DP: head and value sizes up to 64, 128 or 256.
+// What bounds it is the trips to memory of a block's few tiles, so the keys of a (token, KV head) are read once
+// for its heads and by eight multiprocessors.  8 tokens, 12 heads of 128 on 2, 1,000 keys, 32-bit: 23 us (a warp
+// per (token, head): 1,117 us).
+// ---------------------------------------------------------------------------------------
+constexpr int kSplits = 8, kRows = 8, kScorePitch = 12;
+
+template <int DP>
+struct SplitShared {
+  float q[kRows][DP];
+  float k[kTileKeys][DP + 4];
+  float v[kTileKeys][DP];
+  float score[kTileKeys][kScorePitch];   // [key][head]
+  float out[kRows][DP];
+  float top[kRows], sum[kRows], alpha[kRows];
+  int place[kTileKeys];
+};
+
+template <typename T, int DP, bool VEC>
+__global__ void __launch_bounds__(kAttentionThreads)
+attention_split_kernel(const AttentionParams p) {
+  extern __shared__ __align__(16) unsigned char split_raw[];
+  SplitShared<DP>& s = *reinterpret_cast<SplitShared<DP>*>(split_raw);
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int split = blockIdx.x, t = blockIdx.z;
+  const int group = p.num_heads / p.num_kv_heads, parts = (group + kRows - 1) / kRows;
+  const int kv_head = blockIdx.y / parts, h0 = kv_head * group + (blockIdx.y % parts) * kRows;
+  const int heads = min(kRows, (kv_head + 1) * group - h0);
+  const int d = p.head_dim, dv = p.value_dim;
+  // columns that no row of a pool fills are read with the others: zeros
+  for (int i = tid; i < kTileKeys * (DP + 4 - d); i += kAttentionThreads) s.k[i / (DP + 4 - d)][d + i % (DP + 4 - d)] = 0.0f;
+  pdl_wait();
+  const int position = p.positions[t];
+  const int* table = p.block_table + static_cast<size_t>(p.token_seq[t]) * p.table_width;
+  int kept, first;
+  visible_keys(p, position, &kept, &first);
+  const int keys = kept + max(position - first + 1, 0);
+  const int share = (keys + kSplits - 1) / kSplits;
+  const int begin = min(split * share, keys), end = min(begin + share, keys);
+  auto look_up = [&](int base) {   // where the key of this thread lies in the tile from `base` on
+    const int index = min(base + (tid & (kTileKeys - 1)), end - 1);
+    const int key = index < kept ? index : first + index - kept;
+    return table[key / p.page_size] * p.page_size + key % p.page_size;
+  };
+  int ahead = begin < end ? look_up(begin) : 0;
+  for (int i = tid; i < kRows * DP; i += kAttentionThreads) {
+    const int r = i / DP, c = i % DP;
+    s.q[r][c] = r < heads && c < d ? to_float<T>(static_cast<const T*>(p.q)[(static_cast<size_t>(t) * p.num_heads + h0 + r) * d + c]) : 0.0f;
+  }
+  if (tid < kRows) {
+    s.top[tid] = -INFINITY;
+    s.sum[tid] = 0.0f;
+  }
+  constexpr int kColumns = (DP + kAttentionThreads - 1) / kAttentionThreads;
+  float acc[kRows][kColumns];
 #pragma unroll
-    for (int i = 0; i < kMaxHeadDim / 32; ++i) acc[i] *= alpha;
-    const int count = min(32, run_last - base + 1);
-    for (int jj = 0; jj < count; ++jj) {
-      const float w = __shfl_sync(0xffffffffu, weight, jj);
-      const int key = base + jj;
-      const int page = table[key / page_size];
-      const T* v_row = v_pool + (static_cast<size_t>(page) * page_size + key % page_size) * v_stride +
-                       static_cast<size_t>(kv_head) * value_dim;
+  for (int r = 0; r < kRows; ++r)
 #pragma unroll
-      for (int i = 0; i < kMaxHeadDim / 32; ++i) {
-        const int e = lane + 32 * i;
-        if (e < value_dim) acc[i] = fmaf(w, to_float<T>(v_row[e]), acc[i]);
+    for (int j = 0; j < kColumns; ++j) acc[r][j] = 0.0f;
+
+  for (int base = begin; base < end; base += kTileKeys) {
+    const int count = min(kTileKeys, end - base);
+    __syncthreads();   // the tile before is read out
+    if (tid < kTileKeys) s.place[tid] = ahead;
+    __syncthreads();
+    stage_keys<T, VEC>(&s.k[0][0], DP + 4, static_cast<const T*>(p.k_pool) + static_cast<size_t>(kv_head) * d,
+                       static_cast<size_t>(p.num_kv_heads) * d, d, s.place, count);
+    stage_keys<T, VEC>(&s.v[0][0], DP, static_cast<const T*>(p.v_pool) + static_cast<size_t>(kv_head) * dv,
+                       static_cast<size_t>(p.num_kv_heads) * dv, dv, s.place, count);
+    copy_commit();
+    if (base + kTileKeys < end) ahead = look_up(base + kTileKeys);
+    copy_wait<0>();
+    __syncthreads();
+    {
+      const int key = tid & (kTileKeys - 1), r0 = (tid / kTileKeys) * 4;
+      unsigned long long dot[4] = {0ull, 0ull, 0ull, 0ull};
+      if (key < count) {
+#pragma unroll 8
+        for (int c = 0; c < DP; c += 4) {
+          const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(&s.k[key][c]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&s.q[r0 + r][c]);
+            fma_pair(dot[r], qq.x, kk.x);
+            fma_pair(dot[r], qq.y, kk.y);
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) s.score[key][r0 + r] = key < count ? sum_of_pair(dot[r]) * p.scale : -INFINITY;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int own = 0; own < 2; ++own) {
+      const int r = 2 * warp + own;
+      const float a = s.score[lane][r], b = s.score[lane + 32][r];
+      const float before = s.top[r], top = fmaxf(before, warp_max(fmaxf(a, b)));
+      const float shift = top == -INFINITY ? 0.0f : top;
+      const float wa = lane < count ? expf(a - shift) : 0.0f, wb = lane + 32 < count ? expf(b - shift) : 0.0f;
+      s.score[lane][r] = wa;
+      s.score[lane + 32][r] = wb;
+      const float sum = warp_sum(wa + wb);
+      if (lane == 0) {
+        const float alpha = before == top ? 1.0f : expf(before - top);
+        s.top[r] = top;
+        s.alpha[r] = alpha;
+        s.sum[r] = s.sum[r] * alpha + sum;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int j = 0; j < kColumns; ++j) acc[r][j] *= s.alpha[r];
+#pragma unroll
+    for (int j = 0; j < kColumns; ++j) {
+      const int c = tid + j * kAttentionThreads;
+      if (c >= dv) continue;
+#pragma unroll 8
+      for (int key = 0; key < count; ++key) {
+        const float v = s.v[key][c];
+        const float4 lo = *reinterpret_cast<const float4*>(&s.score[key][0]), hi = *reinterpret_cast<const float4*>(&s.score[key][4]);
+        acc[0][j] = fmaf(lo.x, v, acc[0][j]);
+        acc[1][j] = fmaf(lo.y, v, acc[1][j]);
+        acc[2][j] = fmaf(lo.z, v, acc[2][j]);
+        acc[3][j] = fmaf(lo.w, v, acc[3][j]);
+        acc[4][j] = fmaf(hi.x, v, acc[4][j]);
+        acc[5][j] = fmaf(hi.y, v, acc[5][j]);
+        acc[6][j] = fmaf(hi.z, v, acc[6][j]);
+        acc[7][j] = fmaf(hi.w, v, acc[7][j]);
       }
     }
   }
-  }
-  if (sink || sink_values) {
-    // the sink's score is 0 (or the head's learned one): fold it in like one more key whose value is zero
-    const float sink_score = sink_values ? sink_values[h] : 0.0f;
-    const float new_max = fmaxf(running_max, sink_score);
-    const float alpha = expf(running_max - new_max);
-    running_sum = running_sum * alpha + expf(sink_score - new_max);
 #pragma unroll
-    for (int i = 0; i < kMaxHeadDim / 32; ++i) acc[i] *= alpha;
-  }
-  const float inverse = out_scale / running_sum;
-  T* out_row = out + (static_cast<size_t>(t) * num_heads + h) * value_dim;
-  const float* gate_row = gate && !gate_per_head ? gate + static_cast<size_t>(t) * gate_stride + static_cast<size_t>(h) * value_dim : nullptr;
-  const float head_gate = gate && gate_per_head ? 1.0f / (1.0f + expf(-gate[static_cast<size_t>(t) * gate_stride + h])) : 1.0f;
+  for (int j = 0; j < kColumns; ++j) {
+    const int c = tid + j * kAttentionThreads;
+    if (c < DP) {
 #pragma unroll
-  for (int i = 0; i < kMaxHeadDim / 32; ++i) {
-    const int e = lane + 32 * i;
-    if (e < value_dim) {
-      float value = acc[i] * inverse;
-      if (gate_row) value *= 1.0f / (1.0f + expf(-gate_row[e]));
-      else value *= head_gate;
-      out_row[e] = from_float<T>(value);
+      for (int r = 0; r < kRows; ++r) s.out[r][c] = acc[r][j];
     }
   }
+  cluster_sync();
+  // block r of the cluster joins head r
+  if (split < heads) {
+    const int h = h0 + split;
+    float tops[kSplits], sums[kSplits], top = -INFINITY;
+#pragma unroll
+    for (int b = 0; b < kSplits; ++b) {
+      tops[b] = remote_float(shared_address(&s.top[split]), b);
+      sums[b] = remote_float(shared_address(&s.sum[split]), b);
+      top = fmaxf(top, tops[b]);
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int b = 0; b < kSplits; ++b) {
+      tops[b] = tops[b] == top ? 1.0f : expf(tops[b] - top);   // (0 where a block saw no key)
+      sum += sums[b] * tops[b];
+    }
+    const float factor = ending_factor(p, h, top, sum);
+    for (int c = tid; c < dv; c += kAttentionThreads) {
+      float part[kSplits], value = 0.0f;
+#pragma unroll
+      for (int b = 0; b < kSplits; ++b) part[b] = remote_float(shared_address(&s.out[split][c]), b);
+#pragma unroll
+      for (int b = 0; b < kSplits; ++b) value = fmaf(part[b], tops[b], value);
+      static_cast<T*>(p.out)[(static_cast<size_t>(t) * p.num_heads + h) * dv + c] = from_float<T>(value * factor * gate_factor(p, t, h, c));
+    }
+  }
+  cluster_sync();   // no block leaves while another reads its part
+}
+
+// ---------------------------------------------------------------------------------------
+// Steps of more tokens: a block takes 64 neighbouring tokens and one head and walks the keys 64 at a time.  A
+// thread owns 8 rows x 4 keys of the scores (packed multiply-adds) and 8 rows x DP / 16 values of the output;
+// sixteen lanes share a row, a warp sixteen rows, so that a row's weights pass through shared memory
+// within its warp.  Tokens of several requests in one tile are folded one request after another, the
+// others' rows masked.  Bound by the multiply-adds and the reads of shared memory that feed them: 64 x 64 tiles
+// read a key 64 times less often than a warp per row.  1,024 tokens of three requests (700, 1 and 323, histories
+// 0, 900, 40), 14 heads of 64 on 2, 32-bit: 269 us (a warp per (token, head): 1,146 us).
+// ---------------------------------------------------------------------------------------
+constexpr int kTileRows = 64;
+
+template <int DP>
+struct TileShared {
+  float q[kTileRows][DP + 4];
+  float k[kTileKeys][DP + 4];   // then the tile's weights, [row][kTileKeys + 4]
+  float v[kTileKeys][DP];
+  int place[kTileKeys];
+  int seq[kTileRows], last[kTileRows], first[kTileRows], kept[kTileRows];
+};
+
+template <typename T, int DP, bool VEC>
+__global__ void __launch_bounds__(kAttentionThreads)
+attention_tile_kernel(const AttentionParams p) {
+  extern __shared__ __align__(16) unsigned char tile_raw[];
+  TileShared<DP>& s = *reinterpret_cast<TileShared<DP>*>(tile_raw);
+  constexpr int kWeightPitch = kTileKeys + 4;
+  static_assert(kTileRows * kWeightPitch <= kTileKeys * (DP + 4), "the weights take the keys' place");
+  float* weights = &s.k[0][0];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.x, kv_head = h / (p.num_heads / p.num_kv_heads);
+  const int t0 = (gridDim.y - 1 - blockIdx.y) * kTileRows;   // the longest histories of a prompt first
+  const int rows = min(kTileRows, p.num_tokens - t0);
+  const int d = p.head_dim, dv = p.value_dim;
+  pdl_wait();
+  if (tid < kTileRows) {
+    const bool valid = tid < rows;
+    s.seq[tid] = valid ? p.token_seq[t0 + tid] : -1;
+    s.last[tid] = valid ? p.positions[t0 + tid] : -1;
+    s.first[tid] = 0;
+    s.kept[tid] = 0;
+    if (valid) visible_keys(p, s.last[tid], &s.kept[tid], &s.first[tid]);
+  }
+#pragma unroll 4
+  for (int i = tid; i < kTileRows * d; i += kAttentionThreads) {
+    const int r = i / d, c = i - r * d;
+    s.q[r][c] = r < rows ? to_float<T>(static_cast<const T*>(p.q)[(static_cast<size_t>(t0 + r) * p.num_heads + h) * d + c]) : 0.0f;
+  }
+  if (d < DP) {
+    const int spare = DP - d;
+    for (int i = tid; i < kTileRows * spare; i += kAttentionThreads) s.q[i / spare][d + i % spare] = 0.0f;
+  }
+  if (dv < DP) {
+    const int spare = DP - dv;
+    for (int i = tid; i < kTileKeys * spare; i += kAttentionThreads) s.v[i / spare][dv + i % spare] = 0.0f;
+  }
+  __syncthreads();
+
+  const int row0 = warp * 16 + (lane >> 4), column0 = lane & 15;   // rows row0 + 2 i; keys column0 + 16 j; values 4 column0 + 64 j
+  constexpr int kGroups = DP / 64;
+  float out[8][kGroups][4];
+  float row_max[8], row_sum[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    row_max[i] = -INFINITY;
+    row_sum[i] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kGroups; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) out[i][j][e] = 0.0f;
+  }
+
+  for (int seg = 0; seg < rows;) {
+    // the rows of one request that follow one another, and the keys any of them sees
+    const int seq = s.seq[seg];
+    int seg_end = seg, low = 0x7fffffff, high = -1, most_kept = 0;
+    while (seg_end < rows && s.seq[seg_end] == seq) {
+      low = min(low, s.first[seg_end]);
+      high = max(high, s.last[seg_end]);
+      most_kept = max(most_kept, s.kept[seg_end]);
+      ++seg_end;
+    }
+    const int* table = p.block_table + static_cast<size_t>(seq) * p.table_width;
+    for (int run = 0; run < 2; ++run) {
+      const int run_first = run == 0 ? 0 : low, run_end = run == 0 ? most_kept : high + 1;
+      auto look_up = [&](int base) {   // where the key of this thread lies in the tile from `base` on, -1: nowhere
+        const int key = base + (tid & (kTileKeys - 1));
+        if (key >= run_end) return -1;
+        const int page = table[key / p.page_size];   // (a page that no row sees may be gone)
+        return page >= 0 ? page * p.page_size + key % p.page_size : -1;
+      };
+      int ahead = run_first < run_end ? look_up(run_first) : -1;
+      for (int base = run_first; base < run_end; base += kTileKeys) {
+        const int count = min(kTileKeys, run_end - base);
+        __syncthreads();   // the tile before is read out
+        if (tid < kTileKeys) s.place[tid] = ahead;
+        if (d < DP) {   // the weights were here
+          const int spare = DP - d;
+          for (int i = tid; i < kTileKeys * spare; i += kAttentionThreads) s.k[i / spare][d + i % spare] = 0.0f;
+        }
+        __syncthreads();
+        stage_keys<T, VEC>(&s.k[0][0], DP + 4, static_cast<const T*>(p.k_pool) + static_cast<size_t>(kv_head) * d,
+                           static_cast<size_t>(p.num_kv_heads) * d, d, s.place, kTileKeys);
+        copy_commit();
+        stage_keys<T, VEC>(&s.v[0][0], DP, static_cast<const T*>(p.v_pool) + static_cast<size_t>(kv_head) * dv,
+                           static_cast<size_t>(p.num_kv_heads) * dv, dv, s.place, kTileKeys);
+        copy_commit();
+        if (base + kTileKeys < run_end) ahead = look_up(base + kTileKeys);
+        copy_wait<1>();
+        __syncthreads();
+        unsigned long long dot[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dot[i][j] = 0ull;
+#pragma unroll 2
+        for (int c = 0; c < DP; c += 4) {
+          ulonglong2 kk[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const ulonglong2*>(&s.k[column0 + 16 * j][c]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&s.q[row0 + 2 * i][c]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              fma_pair(dot[i][j], qq.x, kk[j].x);
+              fma_pair(dot[i][j], qq.y, kk[j].y);
+            }
+          }
+        }
+        copy_wait<0>();
+        __syncthreads();   // the keys are read out (the weights take their place), and the values are there
+        bool some_hidden = false;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = row0 + 2 * i;
+          const int from = run == 0 ? 0 : s.first[row], to = run == 0 ? s.kept[row] : s.last[row] + 1;
+          const bool mine = row >= seg && row < seg_end;
+          float score[4];
+          bool seen[4];
+          float top = row_max[i];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int key = base + column0 + 16 * j;
+            seen[j] = mine && key >= from && key < to;
+            some_hidden |= !seen[j];
+            score[j] = sum_of_pair(dot[i][j]) * p.scale;
+            if (seen[j]) top = fmaxf(top, score[j]);
+          }
+#pragma unroll
+          for (int offset = 8; offset > 0; offset >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, offset));
+          const float shift = top == -INFINITY ? 0.0f : top;
+          float sum = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float w = expf(score[j] - shift);
+            if (seen[j]) sum += w;
+            weights[row * kWeightPitch + column0 + 16 * j] = seen[j] ? w : -1.0f;   // below 0: not seen at all
+          }
+#pragma unroll
+          for (int offset = 8; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+          const float alpha = row_max[i] == top ? 1.0f : expf(row_max[i] - top);
+          row_max[i] = top;
+          row_sum[i] = row_sum[i] * alpha + sum;
+#pragma unroll
+          for (int j = 0; j < kGroups; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) out[i][j][e] *= alpha;
+        }
+        const bool edge = __any_sync(0xffffffffu, some_hidden);
+        __syncwarp();   // a warp's rows and their weights are its own
+        if (!edge) {
+#pragma unroll 2
+          for (int key = 0; key < kTileKeys; key += 2) {
+            float2 w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = *reinterpret_cast<const float2*>(weights + (row0 + 2 * i) * kWeightPitch + key);
+#pragma unroll
+            for (int j = 0; j < kGroups; ++j) {
+              const float4 a = *reinterpret_cast<const float4*>(&s.v[key][4 * column0 + 64 * j]);
+              const float4 b = *reinterpret_cast<const float4*>(&s.v[key + 1][4 * column0 + 64 * j]);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                out[i][j][0] = fmaf(w[i].y, b.x, fmaf(w[i].x, a.x, out[i][j][0]));
+                out[i][j][1] = fmaf(w[i].y, b.y, fmaf(w[i].x, a.y, out[i][j][1]));
+                out[i][j][2] = fmaf(w[i].y, b.z, fmaf(w[i].x, a.z, out[i][j][2]));
+                out[i][j][3] = fmaf(w[i].y, b.w, fmaf(w[i].x, a.w, out[i][j][3]));
+              }
+            }
+          }
+        } else {
+          // a value a row does not see is left out, whatever it holds (0 times infinity is not 0)
+#pragma unroll 2
+          for (int key = 0; key < count; ++key) {
+            float w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = weights[(row0 + 2 * i) * kWeightPitch + key];
+#pragma unroll
+            for (int j = 0; j < kGroups; ++j) {
+              const float4 a = *reinterpret_cast<const float4*>(&s.v[key][4 * column0 + 64 * j]);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                if (!(w[i] < 0.0f)) {
+                  out[i][j][0] = fmaf(w[i], a.x, out[i][j][0]);
+                  out[i][j][1] = fmaf(w[i], a.y, out[i][j][1]);
+                  out[i][j][2] = fmaf(w[i], a.z, out[i][j][2]);
+                  out[i][j][3] = fmaf(w[i], a.w, out[i][j][3]);
+                }
+              }
+            }
+          }
+        }
+      }
+    }
+    seg = seg_end;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = row0 + 2 * i;
+    if (row >= rows) continue;
+    const int t = t0 + row;
+    const float factor = ending_factor(p, h, row_max[i], row_sum[i]);
+    T* out_row = static_cast<T*>(p.out) + (static_cast<size_t>(t) * p.num_heads + h) * dv;
+#pragma unroll
+    for (int j = 0; j < kGroups; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = 4 * column0 + 64 * j + e;
+        if (c < dv) out_row[c] = from_float<T>(out[i][j][e] * factor * gate_factor(p, t, h, c));
+      }
+  }
+}
+
+// Up to this many tokens (a tile's rows) a step's keys are split between blocks: a single tile per head would leave
+// the chip idle.  With more, tiles of 64 tokens share what they read.
+constexpr int kSplitTokens = 64;
+
+template <typename T, int DP, bool VEC>
+static int launch_attention(const AttentionParams& p, cudaStream_t s) {
+  if (p.num_tokens <= kSplitTokens) {
+    static SharedMemoryOptIn opt_in;
+    constexpr int kBytes = static_cast<int>(sizeof(SplitShared<DP>));
+    const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_split_kernel<T, DP, VEC>), kBytes);
+    if (opted) return opted;
+    const int group = p.num_heads / p.num_kv_heads;
+    return launch_in_clusters(attention_split_kernel<T, DP, VEC>, kSplits,
+                              dim3(kSplits, p.num_kv_heads * ((group + kRows - 1) / kRows), p.num_tokens), dim3(kAttentionThreads),
+                              kBytes, s, p);
+  }
+  static SharedMemoryOptIn opt_in;
+  constexpr int kBytes = static_cast<int>(sizeof(TileShared<DP>));
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_tile_kernel<T, DP, VEC>), kBytes);
+  if (opted) return opted;
+  return vipera_launch(attention_tile_kernel<T, DP, VEC>, dim3(p.num_heads, (p.num_tokens + kTileRows - 1) / kTileRows),
+                       dim3(kAttentionThreads), kBytes, s, p);
+}
+
+template <typename T>
+static int launch_sizes(const AttentionParams& p, cudaStream_t s) {
+  constexpr int kPiece = 16 / static_cast<int>(sizeof(T));
+  const bool vec = p.head_dim % kPiece == 0 && p.value_dim % kPiece == 0 &&
+                   ((reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool)) & 15) == 0;
+  const int largest = p.head_dim > p.value_dim ? p.head_dim : p.value_dim;
+  if (largest <= 64) return vec ? launch_attention<T, 64, true>(p, s) : launch_attention<T, 64, false>(p, s);
+  if (largest <= 128) return vec ? launch_attention<T, 128, true>(p, s) : launch_attention<T, 128, false>(p, s);
+  return vec ? launch_attention<T, 256, true>(p, s) : launch_attention<T, 256, false>(p, s);
 }
 
 // q is [tokens, heads, d] and out [tokens, heads, value_dim]; the key pool is
@@ -185,23 +564,14 @@ VIPERA_API int vipera_attention_gated(const void* q, void* out, int dtype, const
   if (value_dim <= 0 || value_dim > kMaxHeadDim || keep_first < 0) return VIPERA_BAD_SHAPE;
   if (num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads != 0) return VIPERA_BAD_SHAPE;
   if (page_size <= 0 || table_width <= 0 || window < 0) return VIPERA_BAD_ARGUMENT;
+  if (num_heads > 65535) return VIPERA_BAD_SHAPE;
+  const AttentionParams p{q, out, k_pool, v_pool, token_seq, positions, block_table, table_width, page_size, num_tokens, num_heads,
+                          num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink, chunk, out_scale, sink_values, gate,
+                          gate_stride, gate_per_head};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  dim3 grid(num_tokens, (num_heads + kWarpsPerBlock - 1) / kWarpsPerBlock);
-  if (dtype == VIPERA_F32)
-    attention_kernel<float><<<grid, kWarpsPerBlock * 32, 0, s>>>(
-        static_cast<const float*>(q), static_cast<float*>(out), static_cast<const float*>(k_pool),
-        static_cast<const float*>(v_pool), token_seq, positions, block_table, table_width, page_size,
-        num_heads, num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink, chunk, out_scale, sink_values,
-        gate, gate_stride, gate_per_head);
-  else if (dtype == VIPERA_BF16)
-    attention_kernel<__nv_bfloat16><<<grid, kWarpsPerBlock * 32, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(out),
-        static_cast<const __nv_bfloat16*>(k_pool), static_cast<const __nv_bfloat16*>(v_pool), token_seq,
-        positions, block_table, table_width, page_size, num_heads, num_kv_heads, head_dim, value_dim, scale, window,
-        keep_first, sink, chunk, out_scale, sink_values, gate, gate_stride, gate_per_head);
-  else
-    return VIPERA_BAD_DTYPE;
-  return vipera_launch_status();
+  if (dtype == VIPERA_F32) return launch_sizes<float>(p, s);
+  if (dtype == VIPERA_BF16) return launch_sizes<__nv_bfloat16>(p, s);
+  return VIPERA_BAD_DTYPE;
 }
 
 VIPERA_API int vipera_attention(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,
