@@ -1,5 +1,5 @@
 // Sampling on the device: penalties, greedy argmax, and temperature sampling with top-k,
-// top-p and min-p, one block per row of logits.
+// top-p and min-p, a cluster of blocks per row of logits.
 //
 // Semantics are those of the reference's sampler crate.  Greedy: the best finite logit,
 // ties to the lowest id (crates/vipera-sampler/src/lib.rs:135-156).  Temperature: the k best
@@ -14,11 +14,10 @@
 // With top_k = 0 the reference keeps a head of 4096 and sorts the whole vocabulary only if
 // top-p reaches past it (lib.rs:437, 206-216); this kernel reports that case in `status`
 // (SAMPLE_NEEDS_HOST) and the caller draws that row with the host sampler.
-#include "common.cuh"
+#include "simt.cuh"
 
 enum SampleStatus { SAMPLE_OK = 0, SAMPLE_NO_FINITE = 1, SAMPLE_NO_MASS = 2, SAMPLE_NEEDS_HOST = 3 };
 
-constexpr int kSampleThreads = 1024;
 constexpr int kMaxCandidates = 4096;
 
 __device__ __forceinline__ uint32_t ordered_key(float v) {
@@ -196,188 +195,434 @@ VIPERA_API int vipera_argmax(const float* logits, int rows, int vocab, int* toke
 
 // ---------------------------------------------------------------------------------------
 // temperature sampling
+//
+// A cluster of eight blocks takes a row.  Block b keeps the logits whose index modulo 1024 is in [128 b, 128 b + 128)
+// in shared memory (one trip to memory for the whole draw), so that each of 1024 chains of the softmax sum lies in one
+// block.  Then a histogram over 2,048 equal steps below the best value (few ids meet in a bin, unlike the leading
+// bits of the values) tells the first block how far down it has to go: to the bound-th largest, or to where the
+// weights' sum is past top-p with a margin.  If what lies above is at most 4,096 ids, it goes to the first block,
+// which sorts it and draws; the others leave.  Otherwise the bound-th largest (value, lowest id first) is found
+// digit by digit.  The weights' sum that top-p cuts and the mass are added in order, best first, by one thread from
+// weights in shared memory.
+// What bounds it: the chain of these steps, some 50 us a row, 33 rows at once.  64 rows of 151,936 (a quarter each
+// top-k 50, top-p alone, min-p, greedy): 104 us; with one block a row and a pass over memory per step 440 us.
 // ---------------------------------------------------------------------------------------
+constexpr int kSampleBlocks = 8, kSampleThreads = 512;
+constexpr int kChains = 1024, kOwnChains = kChains / kSampleBlocks;
+constexpr int kBins = 2048;
+constexpr int kMostKept = 200 * 1024;   // bytes of logits a block keeps; longer rows are read again for each step
+
+struct SampleShared {
+  unsigned int histogram[kBins];
+  int ids[kMaxCandidates];              // the first block's candidates, then its weights
+  Best best[kSampleThreads / 32];
+  float least[kSampleThreads / 32];
+  Best row_best;
+  float row_min;
+  float scan_float[kSampleThreads / 32];
+  float chain_sums[kOwnChains / 32];
+  unsigned int finite_count, count, bin, seen;
+  unsigned int scan[kSampleThreads / 32];
+  double scan_double[kSampleThreads / 32];
+  int cut, chosen, last;
+  float mass;
+};
+
+__device__ __forceinline__ uint32_t cluster_address(const void* p, uint32_t block) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(shared_address(p)), "r"(block));
+  return r;
+}
+__device__ __forceinline__ unsigned int remote_word(const void* p, uint32_t block) {
+  unsigned int v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_address(p, block)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void remote_add(const void* p, uint32_t block, unsigned int value) {
+  asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(cluster_address(p, block)), "r"(value) : "memory");
+}
+__device__ __forceinline__ unsigned int remote_fetch_add(const void* p, uint32_t block, unsigned int value) {
+  unsigned int v;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(v) : "r"(cluster_address(p, block)), "r"(value) : "memory");
+  return v;
+}
+__device__ __forceinline__ void remote_store(const void* p, uint32_t block, unsigned int value) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_address(p, block)), "r"(value) : "memory");
+}
+
+// (value, id) as one number: larger is better, equal values best by the lowest id
+__device__ __forceinline__ unsigned long long ranked(float v, int id) {
+  return (static_cast<unsigned long long>(ordered_key(v)) << 32) | (0xffffffffu - static_cast<unsigned int>(id));
+}
+
+template <bool KEPT>
 __global__ void __launch_bounds__(kSampleThreads)
 sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
               const double* __restrict__ uniform, int* __restrict__ tokens, int* __restrict__ status) {
-  __shared__ Best best_scratch[32];
-  __shared__ float sum_scratch[32];
-  __shared__ unsigned int histogram[256];
-  __shared__ unsigned long long candidates[kMaxCandidates];
-  __shared__ unsigned int shared_prefix, shared_remaining, shared_count, shared_equal_taken;
-  __shared__ unsigned int scan_scratch[32];
-
-  const int r = blockIdx.x;
+  extern __shared__ __align__(16) unsigned char sample_raw[];
+  SampleShared& s = *reinterpret_cast<SampleShared*>(sample_raw);
+  float* kept = reinterpret_cast<float*>(sample_raw + (sizeof(SampleShared) + 15) / 16 * 16);   // [runs][kOwnChains]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int own = blockIdx.x, r = blockIdx.y;
   const float* row = logits + static_cast<size_t>(r) * vocab;
-  const int tid = threadIdx.x;
+  const int runs = (vocab + kChains - 1) / kChains, items = runs * kOwnChains;
+  auto id_of = [&](int item) { return item / kOwnChains * kChains + own * kOwnChains + item % kOwnChains; };
+  auto value_of = [&](int item) {
+    if (KEPT) return kept[item];
+    const int id = id_of(item);
+    return id < vocab ? row[id] : NAN;
+  };
+  for (int i = tid; i < kBins; i += kSampleThreads) s.histogram[i] = 0;
+  if (tid == 0) s.finite_count = s.count = 0;
+  pdl_wait();
+  if (KEPT) {
+    if ((vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
+#pragma unroll 4
+      for (int i = tid * 4; i < items; i += kSampleThreads * 4) {
+        const int id = id_of(i);
+        if (id < vocab) copy_16(shared_address(kept + i), row + id, true);
+        else kept[i] = kept[i + 1] = kept[i + 2] = kept[i + 3] = NAN;
+      }
+      copy_commit();
+      copy_wait<0>();
+    } else {
+#pragma unroll 4
+      for (int i = tid; i < items; i += kSampleThreads) kept[i] = id_of(i) < vocab ? row[id_of(i)] : NAN;
+    }
+  }
+  __syncthreads();
 
-  const Best best = block_argmax(row, vocab, best_scratch);
-  if (best.id < 0) {
-    if (tid == 0) { tokens[r] = 0; status[r] = SAMPLE_NO_FINITE; }
-    return;
+  // the best finite logit of the row, ties to the lowest id, and how many are finite
+  {
+    Best best{0.0f, -1};
+    unsigned int own_finite = 0;
+    float least = INFINITY;
+#pragma unroll 4
+    for (int i = tid; i < items; i += kSampleThreads) {
+      const float v = value_of(i);
+      if (finite(v)) {
+        best = better_of(best, Best{v, id_of(i)});
+        least = fminf(least, v);
+        ++own_finite;
+      }
+    }
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+      Best other;
+      other.value = __shfl_xor_sync(0xffffffffu, best.value, offset);
+      other.id = __shfl_xor_sync(0xffffffffu, best.id, offset);
+      best = better_of(best, other);
+      own_finite += __shfl_xor_sync(0xffffffffu, own_finite, offset);
+      least = fminf(least, __shfl_xor_sync(0xffffffffu, least, offset));
+    }
+    if (lane == 0) {
+      s.best[warp] = best;
+      s.least[warp] = least;
+      atomicAdd(&s.finite_count, own_finite);
+    }
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kSampleThreads / 32; ++w) {
+        best = better_of(best, s.best[w]);
+        least = fminf(least, s.least[w]);
+      }
+      s.row_best = best;
+      s.row_min = least;
+    }
+  }
+  cluster_sync();
+  Best best{0.0f, -1};
+  unsigned int finite_total = 0;
+  float least = INFINITY;
+#pragma unroll
+  for (int b = 0; b < kSampleBlocks; ++b) {
+    least = fminf(least, __uint_as_float(remote_word(&s.row_min, b)));
+    best = better_of(best, Best{__uint_as_float(remote_word(&s.row_best.value, b)), static_cast<int>(remote_word(&s.row_best.id, b))});
+    finite_total += remote_word(&s.finite_count, b);
   }
   const float temp = temperature[r];
-  if (temp == 0.0f) {
-    if (tid == 0) { tokens[r] = best.id; status[r] = SAMPLE_OK; }
+  if (best.id < 0 || temp == 0.0f) {
+    if (own == 0 && tid == 0) {
+      tokens[r] = best.id < 0 ? 0 : best.id;
+      status[r] = best.id < 0 ? SAMPLE_NO_FINITE : SAMPLE_OK;
+    }
+    cluster_sync();   // the others have read this block's best
     return;
   }
   const float scale = 1.0f / temp;
   const float peak = best.value * scale;
 
-  // softmax mass over every finite logit, and how many there are
-  float partial = 0.0f;
-  unsigned int finite_count = 0;
-  for (int i = tid; i < vocab; i += kSampleThreads) {
-    const float v = row[i];
-    if (finite(v)) { partial += expf(v * scale - peak); ++finite_count; }
+  // softmax mass over every finite logit: chain t adds the weights of ids t, t + 1024, ... in order
+  if (tid < kOwnChains) {
+    float partial = 0.0f;
+#pragma unroll 8
+    for (int run = 0; run < runs; ++run) {
+      const float v = value_of(run * kOwnChains + tid);
+      if (finite(v)) partial += expf(v * scale - peak);
+    }
+    partial = warp_sum(partial);
+    if (lane == 0) s.chain_sums[warp] = partial;
   }
-  const float total = block_sum(partial, sum_scratch);
-  const unsigned int finite_total = __float2uint_rn(block_sum(static_cast<float>(finite_count), sum_scratch));
-  if (!(total > 0.0f) || !finite(total)) {
-    if (tid == 0) { tokens[r] = 0; status[r] = SAMPLE_NO_MASS; }
-    return;
-  }
-
+  cluster_sync();
+  const int per_block = kOwnChains / 32;
+  const float total = warp_sum(__uint_as_float(remote_word(&s.chain_sums[lane % per_block], lane / per_block)));
   const int requested = top_k[r];
   const bool uncut = requested == 0;
-  if (requested > kMaxCandidates) {
-    if (tid == 0) { tokens[r] = 0; status[r] = SAMPLE_NEEDS_HOST; }
+  if (!(total > 0.0f) || !finite(total) || requested > kMaxCandidates) {
+    if (own == 0 && tid == 0) {
+      tokens[r] = 0;
+      status[r] = !(total > 0.0f) || !finite(total) ? SAMPLE_NO_MASS : SAMPLE_NEEDS_HOST;
+    }
+    cluster_sync();   // the others have read this block's sums
     return;
   }
-  unsigned int bound = uncut ? kMaxCandidates : static_cast<unsigned int>(requested);
-  if (bound > finite_total) bound = finite_total;
+  const unsigned int bound = min(min(uncut ? static_cast<unsigned int>(kMaxCandidates) : static_cast<unsigned int>(requested),
+                                     static_cast<unsigned int>(kMaxCandidates)), finite_total);
 
-  // radix select: the key of the bound-th largest finite logit
-  unsigned int prefix = 0, prefix_mask = 0, remaining = bound;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = tid; i < 256; i += kSampleThreads) histogram[i] = 0;
-    __syncthreads();
-    for (int i = tid; i < vocab; i += kSampleThreads) {
-      const float v = row[i];
-      if (!finite(v)) continue;
-      const uint32_t key = ordered_key(v);
-      if ((key & prefix_mask) == prefix) atomicAdd(&histogram[(key >> shift) & 255u], 1u);
+  // Bins of equal steps below the best value, and how many of them are needed.
+  const float step = (best.value - least) / (kBins - 0.5f), per_step = 1.0f / step;
+  const bool spread = step > 0.0f && finite(step) && finite(per_step);
+  auto bin_of = [&](float v) { return min(static_cast<int>((best.value - v) * per_step), kBins - 1); };
+  int last_bin = -1;   // ids up to this bin go to the first block; below 0: bins cannot tell
+  if (spread) {
+#pragma unroll 4
+    for (int i = tid; i < items; i += kSampleThreads) {
+      const float v = value_of(i);
+      if (finite(v)) atomicAdd(&s.histogram[bin_of(v)], 1u);
     }
-    __syncthreads();
-    if (tid == 0) {
-      unsigned int seen = 0;
-      int bin = 255;
-      for (; bin > 0; --bin) {
-        if (seen + histogram[bin] >= remaining) break;
-        seen += histogram[bin];
+    if (tid == 0) s.bin = kBins;
+    cluster_sync();
+    if (own == 0) {
+      constexpr int kPer = kBins / kSampleThreads;
+      static_assert(kPer == 4, "a thread's bins are one 16-byte read");
+      uint4 n = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int b = 0; b < kSampleBlocks; ++b) {
+        uint4 other;
+        asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(other.x), "=r"(other.y), "=r"(other.z), "=r"(other.w) : "r"(cluster_address(&s.histogram[tid * kPer], b)) : "memory");
+        n.x += other.x, n.y += other.y, n.z += other.z, n.w += other.w;
       }
-      shared_prefix = prefix | (static_cast<unsigned int>(bin) << shift);
-      shared_remaining = remaining - seen;
+      const unsigned int mine[kPer] = {n.x, n.y, n.z, n.w};
+      // what the bins hold at least: their count times the weight a little below their lower end
+      const float top_weight = fmaf(best.value, scale, -peak);   // (0 but for the peak's rounding)
+      unsigned int number = 0;
+      float weight = 0.0f, lower[kPer];
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        lower[j] = static_cast<float>(mine[j]) * expf(top_weight - (tid * kPer + j + 1.01f) * (step * scale));
+        number += mine[j];
+        weight += lower[j];
+      }
+      unsigned int number_before = number;
+      float weight_before = weight;
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const unsigned int other = __shfl_up_sync(0xffffffffu, number_before, offset);
+        const float other_weight = __shfl_up_sync(0xffffffffu, weight_before, offset);
+        if (lane >= offset) number_before += other, weight_before += other_weight;
+      }
+      if (lane == 31) s.scan[warp] = number_before, s.scan_float[warp] = weight_before;
+      __syncthreads();
+      number_before -= number, weight_before -= weight;
+      for (int w = 0; w < warp; ++w) number_before += s.scan[w], weight_before += s.scan_float[w];
+      // 4,096 roundings of 2^-24 and the exponentials' own stay far within a thousandth
+      const float enough = top_p[r] * total * 1.001f;
+      int found = kBins;
+      unsigned int found_number = 0;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        number_before += mine[j], weight_before += lower[j];
+        if (found == kBins && (number_before >= bound || weight_before >= enough)) found = tid * kPer + j, found_number = number_before;
+      }
+      if (found < kBins) atomicMin(&s.bin, static_cast<unsigned int>(found));
+      __syncthreads();
+      if (found < kBins && s.bin == static_cast<unsigned int>(found)) s.seen = found_number;
     }
-    __syncthreads();
-    prefix = shared_prefix;
-    remaining = shared_remaining;
-    prefix_mask |= 255u << shift;
-    __syncthreads();
+    cluster_sync();
+    if (remote_word(&s.seen, 0) <= kMaxCandidates) last_bin = static_cast<int>(remote_word(&s.bin, 0));
+    else {
+      for (int i = tid; i < kBins; i += kSampleThreads) s.histogram[i] = 0;
+      cluster_sync();   // the answer is read and every histogram is empty before anything is added to the first
+    }
   }
-  const uint32_t threshold_key = prefix;    // key of the bound-th largest
-  const unsigned int need_equal = remaining; // how many with exactly that key are taken
 
-  // gather: everything above the threshold, then the lowest ids among the equal ones
-  if (tid == 0) { shared_count = 0; shared_equal_taken = 0; }
-  __syncthreads();
-  for (int i = tid; i < vocab; i += kSampleThreads) {
-    const float v = row[i];
-    if (!finite(v)) continue;
-    const uint32_t key = ordered_key(v);
-    if (key > threshold_key) {
-      const unsigned int slot = atomicAdd(&shared_count, 1u);
-      if (slot < kMaxCandidates)
-        candidates[slot] = (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<unsigned int>(i));
+  // The bound-th largest of (value, id): digits of its number from the highest on.  After each digit, everything
+  // above the digits found is in, and `remaining` of those that share them.
+  unsigned long long prefix = 0;
+  unsigned int remaining = bound;
+  int shift = 64;
+#pragma unroll 1
+  while (last_bin < 0) {
+    const int width = shift == 42 || shift == 10 ? 10 : 11;   // 11, 11, 10 bits of the value, the same of the id
+    const int next = shift - width;
+    for (int i = tid; i < items; i += kSampleThreads) {
+      const float v = value_of(i);
+      if (!finite(v)) continue;
+      const unsigned long long number = ranked(v, id_of(i));
+      if (shift == 64 || (number >> shift) == prefix) atomicAdd(&s.histogram[(number >> next) & (kBins - 1) & ((1u << width) - 1u)], 1u);
     }
+    __syncthreads();
+    if (own != 0)
+      for (int i = tid; i < kBins; i += kSampleThreads)
+        if (const unsigned int n = s.histogram[i]) remote_add(&s.histogram[i], 0, n);
+    cluster_sync();
+    if (own == 0) {
+      // from the highest bin down: a thread's four bins, then the threads before it
+      constexpr int kPer = kBins / kSampleThreads;
+      unsigned int mine[kPer], sum = 0;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) sum += mine[j] = s.histogram[kBins - 1 - (tid * kPer + j)];
+      unsigned int before = sum;
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const unsigned int other = __shfl_up_sync(0xffffffffu, before, offset);
+        if (lane >= offset) before += other;
+      }
+      if (lane == 31) s.scan[warp] = before;
+      __syncthreads();
+      for (int w = 0; w < warp; ++w) before += s.scan[w];
+      before -= sum;
+      if (before < remaining && before + sum >= remaining) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          if (before + mine[j] >= remaining) {
+            s.bin = kBins - 1 - (tid * kPer + j);
+            s.seen = before | (before + mine[j] == remaining ? 0x80000000u : 0u);   // the bin is taken whole
+            break;
+          }
+          before += mine[j];
+        }
+      }
+    }
+    cluster_sync();
+    const unsigned int bin = remote_word(&s.bin, 0), seen = remote_word(&s.seen, 0);
+    prefix = (shift == 64 ? 0ull : prefix << width) | bin;
+    remaining -= seen & 0x7fffffffu;
+    shift = next;
+    if ((seen & 0x80000000u) || shift == 0) break;
+    for (int i = tid; i < kBins; i += kSampleThreads) s.histogram[i] = 0;
+    cluster_sync();   // the answer is read and every histogram is empty before anything is added to the first
   }
-  __syncthreads();
-  // equal keys in ascending id order: a block-wide ordered compaction, chunk by chunk
-  for (int chunk = 0; chunk < vocab; chunk += kSampleThreads) {
-    if (shared_equal_taken >= need_equal) break;
-    const int i = chunk + tid;
-    bool is_equal = false;
-    if (i < vocab) {
-      const float v = row[i];
-      is_equal = finite(v) && ordered_key(v) == threshold_key;
-    }
-    const unsigned int ballot = __ballot_sync(0xffffffffu, is_equal);
-    const int lane = tid & 31, warp = tid >> 5;
-    if (lane == 0) scan_scratch[warp] = __popc(ballot);
-    __syncthreads();
-    unsigned int before = shared_equal_taken;
-    for (int w = 0; w < warp; ++w) before += scan_scratch[w];
-    const unsigned int rank = before + __popc(ballot & ((1u << lane) - 1u));
-    if (is_equal && rank < need_equal) {
-      const unsigned int slot = atomicAdd(&shared_count, 1u);
-      if (slot < kMaxCandidates)
-        candidates[slot] = (static_cast<unsigned long long>(threshold_key) << 32) | (0xffffffffu - static_cast<unsigned int>(i));
-    }
-    __syncthreads();
-    if (tid == 0) {
-      unsigned int all = 0;
-      for (int w = 0; w < kSampleThreads / 32; ++w) all += scan_scratch[w];
-      shared_equal_taken += all;
-    }
-    __syncthreads();
-  }
-  __syncthreads();
-  const unsigned int count = min(shared_count, static_cast<unsigned int>(kMaxCandidates));
 
-  // bitonic sort, descending by (value, then lower id first)
+  // what is good enough goes to the first block
+  {
+    auto taken = [&](float v, int i) { return finite(v) && (last_bin >= 0 ? bin_of(v) <= last_bin : (ranked(v, id_of(i)) >> shift) >= prefix); };
+    unsigned int mine = 0;
+#pragma unroll 4
+    for (int i = tid; i < items; i += kSampleThreads) mine += taken(value_of(i), i);
+    unsigned int upto = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const unsigned int other = __shfl_up_sync(0xffffffffu, upto, offset);
+      if (lane >= offset) upto += other;
+    }
+    unsigned int place = 0;
+    if (lane == 31 && upto) place = remote_fetch_add(&s.count, 0, upto);
+    place = __shfl_sync(0xffffffffu, place, 31) + upto - mine;
+    if (mine) {
+      for (int i = tid; i < items; i += kSampleThreads) {
+        if (taken(value_of(i), i)) {
+          if (place < kMaxCandidates) remote_store(&s.ids[place], 0, static_cast<unsigned int>(id_of(i)));
+          ++place;
+        }
+      }
+    }
+  }
+  cluster_sync();
+  if (own != 0) return;
+
+  const unsigned int gathered = min(s.count, static_cast<unsigned int>(kMaxCandidates)), count = min(gathered, bound);
+  // the candidates' numbers take the place of the logits (and, where those are not kept, room of their own)
+  unsigned long long* candidates = reinterpret_cast<unsigned long long*>(kept);
   unsigned int padded = 1;
-  while (padded < count) padded <<= 1;
-  for (unsigned int i = count + tid; i < padded; i += kSampleThreads) candidates[i] = 0ull;
+  while (padded < gathered) padded <<= 1;
+  for (unsigned int i = tid; i < padded; i += kSampleThreads) candidates[i] = i < gathered ? ranked(row[s.ids[i]], s.ids[i]) : 0ull;
   __syncthreads();
+  // bitonic sort, descending
   for (unsigned int size = 2; size <= padded; size <<= 1) {
     for (unsigned int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (unsigned int i = tid; i < padded; i += kSampleThreads) {
-        const unsigned int partner = i ^ stride;
-        if (partner > i) {
-          const bool descending = (i & size) == 0;
-          const unsigned long long a = candidates[i], b = candidates[partner];
-          if (descending ? a < b : a > b) { candidates[i] = b; candidates[partner] = a; }
-        }
+      for (unsigned int pair = tid; pair < padded / 2; pair += kSampleThreads) {
+        const unsigned int i = 2 * pair - (pair & (stride - 1)), partner = i + stride;
+        const bool descending = (i & size) == 0;
+        const unsigned long long a = candidates[i], b = candidates[partner];
+        if (descending ? a < b : a > b) { candidates[i] = b; candidates[partner] = a; }
       }
       __syncthreads();
     }
   }
-
+  auto id_at = [&](unsigned int i) { return static_cast<int>(0xffffffffu - static_cast<unsigned int>(candidates[i] & 0xffffffffull)); };
+  float* weights = reinterpret_cast<float*>(s.ids);
+  for (unsigned int i = tid; i < kMaxCandidates; i += kSampleThreads)
+    weights[i] = i < count ? expf(key_value(static_cast<uint32_t>(candidates[i] >> 32)) * scale - peak) : 0.0f;
+  __syncthreads();
+  const float best_weight = weights[0], floor_weight = min_p[r] * best_weight;
   if (tid == 0) {
-    // weights, top-p cut, min-p filter and the draw, in order, by one thread
+    // the top-p cut: weights added in order, best first, eight reads at a time
     const float target_mass = top_p[r] * total;
     float cumulative = 0.0f;
     int cut = -1;
-    for (unsigned int i = 0; i < count; ++i) {
-      const float w = expf(key_value(static_cast<uint32_t>(candidates[i] >> 32)) * scale - peak);
-      cumulative += w;
-      if (cumulative >= target_mass) { cut = static_cast<int>(i) + 1; break; }
-    }
-    if (uncut && cut < 0 && count < finite_total) {
-      tokens[r] = 0;
-      status[r] = SAMPLE_NEEDS_HOST;
-      return;
+    for (unsigned int i = 0; i < count && cut < 0; i += 8) {
+      const float4 lo = *reinterpret_cast<const float4*>(weights + i), hi = *reinterpret_cast<const float4*>(weights + i + 4);
+      const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      float upto[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) upto[j] = cumulative = cumulative + w[j];
+#pragma unroll
+      for (int j = 7; j >= 0; --j)
+        if (upto[j] >= target_mass && i + j < count) cut = static_cast<int>(i) + j + 1;
     }
     const unsigned int kept_end = cut >= 0 ? static_cast<unsigned int>(cut) : count;
-    const float best_weight = expf(key_value(static_cast<uint32_t>(candidates[0] >> 32)) * scale - peak);
-    const float floor_weight = min_p[r] * best_weight;
     float mass = 0.0f;
-    for (unsigned int i = 0; i < kept_end; ++i) {
-      const float w = expf(key_value(static_cast<uint32_t>(candidates[i] >> 32)) * scale - peak);
-      if (w >= floor_weight) mass += w;
+    for (unsigned int i = 0; i < kept_end; i += 8) {
+      const float4 lo = *reinterpret_cast<const float4*>(weights + i), hi = *reinterpret_cast<const float4*>(weights + i + 4);
+      const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mass += i + j < kept_end && w[j] >= floor_weight ? w[j] : 0.0f;
     }
-    const double target = uniform[r] * static_cast<double>(mass);
-    double running = 0.0;
-    int chosen = -1, last = -1;
-    for (unsigned int i = 0; i < kept_end; ++i) {
-      const float w = expf(key_value(static_cast<uint32_t>(candidates[i] >> 32)) * scale - peak);
-      if (!(w >= floor_weight)) continue;
-      last = static_cast<int>(0xffffffffu - static_cast<unsigned int>(candidates[i] & 0xffffffffull));
-      running += static_cast<double>(w);
-      if (target < running) { chosen = last; break; }
-    }
-    tokens[r] = chosen >= 0 ? chosen : (last >= 0 ? last : best.id);
+    s.cut = cut;
+    s.mass = mass;
+    s.chosen = kMaxCandidates;
+    s.last = -1;
+  }
+  __syncthreads();
+  if (uncut && s.cut < 0 && count < finite_total) {
+    if (tid == 0) { tokens[r] = 0; status[r] = SAMPLE_NEEDS_HOST; }
+    return;
+  }
+  const unsigned int kept_end = s.cut >= 0 ? static_cast<unsigned int>(s.cut) : count;
+  const double target = uniform[r] * static_cast<double>(s.mass);
+  // the first candidate whose running sum (64-bit) exceeds the target: eight neighbours a thread, then the threads before it
+  constexpr int kPer = kMaxCandidates / kSampleThreads;
+  double running[kPer], sum = 0.0;
+  bool counts[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const unsigned int i = tid * kPer + j;
+    counts[j] = i < kept_end && weights[i] >= floor_weight;
+    if (counts[j]) sum += static_cast<double>(weights[i]);
+    running[j] = sum;
+  }
+  double before = sum;
+#pragma unroll
+  for (int offset = 1; offset < 32; offset <<= 1) {
+    const double other = __shfl_up_sync(0xffffffffu, before, offset);
+    if (lane >= offset) before += other;
+  }
+  if (lane == 31) s.scan_double[warp] = before;
+  __syncthreads();
+  before -= sum;
+  for (int w = 0; w < warp; ++w) before += s.scan_double[w];
+#pragma unroll
+  for (int j = kPer - 1; j >= 0; --j) {
+    if (!counts[j]) continue;
+    if (target < before + running[j]) atomicMin(&s.chosen, tid * kPer + j);
+    atomicMax(&s.last, tid * kPer + j);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    tokens[r] = s.chosen < kMaxCandidates ? id_at(s.chosen) : (s.last >= 0 ? id_at(s.last) : best.id);
     status[r] = SAMPLE_OK;
   }
 }
@@ -390,9 +635,24 @@ VIPERA_API int vipera_sample(const float* logits, int rows, int vocab, const flo
   if (rows <= 0) return VIPERA_OK;
   if (vocab <= 0) return VIPERA_BAD_SHAPE;
   if (!status || !tokens) return VIPERA_BAD_ARGUMENT;
-  sample_kernel<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      logits, vocab, temperature, top_k, top_p, min_p, uniform, tokens, status);
-  return vipera_launch_status();
+  constexpr int kHead = static_cast<int>((sizeof(SampleShared) + 15) / 16 * 16), kRanks = kMaxCandidates * 8;
+  const long long logits_bytes = (static_cast<long long>(vocab) + kChains - 1) / kChains * kOwnChains * 4;
+  const bool keep = logits_bytes <= kMostKept;
+  const int bytes = kHead + static_cast<int>(keep && logits_bytes > kRanks ? logits_bytes : kRanks);
+  static SharedMemoryOptIn opt_in_kept, opt_in_read;
+  const int opted = keep ? opt_in_kept.ask(reinterpret_cast<const void*>(sample_kernel<true>), kHead + kMostKept)
+                         : opt_in_read.ask(reinterpret_cast<const void*>(sample_kernel<false>), kHead + kMostKept);
+  if (opted) return opted;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  for (int first = 0; first < rows; first += 65535) {   // a grid's extent along y
+    const int count = rows - first < 65535 ? rows - first : 65535;
+    const int launched = launch_in_clusters(keep ? sample_kernel<true> : sample_kernel<false>, kSampleBlocks, dim3(kSampleBlocks, count),
+                                            dim3(kSampleThreads), bytes, s, logits + static_cast<size_t>(first) * vocab, vocab,
+                                            temperature + first, top_k + first, top_p + first, min_p + first, uniform + first,
+                                            tokens + first, status + first);
+    if (launched) return launched;
+  }
+  return VIPERA_OK;
 }
 
 // ---------------------------------------------------------------------------------------
