@@ -61,12 +61,27 @@ struct GemmArgs {
   void* out;
   float* resid;
   int activation, epilogue, out_bf16;
+  int wide;            // rows of whole pieces of eight values on 16-byte boundaries
 };
+
+__device__ __forceinline__ void load_eight(const float* src, float (&v)[8]) {
+  const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+  v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+}
+__device__ __forceinline__ void load_eight(const __nv_bfloat16* src, float (&v)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(src);
+  const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __bfloat1622float2(pairs[e]);
+    v[2 * e] = f.x, v[2 * e + 1] = f.y;
+  }
+}
 
 // `rows` rows of [extent, K] from row0 on, values k0 .. k0 + kChunk - 1, into shared memory as floats; zeros outside.
 // DIRECT: 32-bit rows of whole 16-byte pieces, copied without passing through registers.
 template <typename T, bool DIRECT, int ROWS, int THREADS>
-__device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src, int row0, int extent, int k0, int k_end, int K) {
+__device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src, int row0, int extent, int k0, int k_end, int K, bool wide) {
   if (DIRECT) {
 #pragma unroll
     for (int i = threadIdx.x; i < ROWS * (kChunk / 4); i += THREADS) {
@@ -74,6 +89,16 @@ __device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src
       const bool valid = row0 + r < extent && k0 + piece < k_end;
       copy_16(shared_address(dst + r * kPitch + piece),
               reinterpret_cast<const float*>(src) + (valid ? static_cast<size_t>(row0 + r) * K + k0 + piece : 0), valid);
+    }
+  } else if (wide) {
+    // rows of whole pieces of eight values
+#pragma unroll 4
+    for (int i = threadIdx.x; i < ROWS * (kChunk / 8); i += THREADS) {
+      const int r = i / (kChunk / 8), piece = (i % (kChunk / 8)) * 8;
+      float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      if (row0 + r < extent && k0 + piece < k_end) load_eight(src + static_cast<size_t>(row0 + r) * K + k0 + piece, v);
+      *reinterpret_cast<float4*>(dst + r * kPitch + piece) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(dst + r * kPitch + piece + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
   } else {
 #pragma unroll 4
@@ -89,7 +114,8 @@ template <typename TA, typename TW, typename T, bool DIRECT, bool CLUSTER>
 __global__ void __launch_bounds__(T::kThreads)
 gemm_simt_kernel(const GemmArgs p) {
   extern __shared__ __align__(16) float gemm_shared[];
-  float* sums = gemm_shared + T::STAGES * T::kStageFloats;   // [BM][kSumPitch]
+  float* sums = gemm_shared;                                 // [BM][kSumPitch]
+  float* ring = gemm_shared + T::BM * T::kSumPitch;          // as many stages as there are chunks, STAGES at most
   const TA* A = static_cast<const TA*>(p.A);
   const TW* W = static_cast<const TW*>(p.W);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -104,13 +130,13 @@ gemm_simt_kernel(const GemmArgs p) {
 
   auto stage_w = [&](int chunk) {
     if (chunk < chunks)
-      stage_rows<TW, DIRECT, T::BN, T::kThreads>(gemm_shared + (chunk % T::STAGES) * T::kStageFloats + T::BM * kPitch, W, n0, p.N,
-                                                 begin + chunk * kChunk, end, p.K);
+      stage_rows<TW, DIRECT, T::BN, T::kThreads>(ring + (chunk % T::STAGES) * T::kStageFloats + T::BM * kPitch, W, n0, p.N,
+                                                 begin + chunk * kChunk, end, p.K, p.wide != 0);
   };
   auto stage_a = [&](int chunk) {
     if (chunk < chunks)
-      stage_rows<TA, DIRECT, T::BM, T::kThreads>(gemm_shared + (chunk % T::STAGES) * T::kStageFloats, A, m0, p.M,
-                                                 begin + chunk * kChunk, end, p.K);
+      stage_rows<TA, DIRECT, T::BM, T::kThreads>(ring + (chunk % T::STAGES) * T::kStageFloats, A, m0, p.M,
+                                                 begin + chunk * kChunk, end, p.K, p.wide != 0);
     copy_commit();
   };
   pdl_launch_dependents();
@@ -134,8 +160,8 @@ gemm_simt_kernel(const GemmArgs p) {
     __syncthreads();   // this chunk has landed for every thread, and the one before is read out
     stage_w(chunk + T::STAGES - 1);
     stage_a(chunk + T::STAGES - 1);
-    const float* a_s = gemm_shared + (chunk % T::STAGES) * T::kStageFloats + first_m * kPitch;
-    const float* w_s = gemm_shared + (chunk % T::STAGES) * T::kStageFloats + (T::BM + first_n) * kPitch;
+    const float* a_s = ring + (chunk % T::STAGES) * T::kStageFloats + first_m * kPitch;
+    const float* w_s = ring + (chunk % T::STAGES) * T::kStageFloats + (T::BM + first_n) * kPitch;
 #pragma unroll
     for (int k = 0; k < kChunk; k += 4) {
       ulonglong2 a[T::TM];
@@ -189,25 +215,32 @@ gemm_simt_kernel(const GemmArgs p) {
     if (p.out_bf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value);
     else static_cast<float*>(p.out)[at] = value;
   };
-  for (int i = threadIdx.x; i < T::BM / blocks * columns; i += T::kThreads) {
-    const int m = (i >> column_bits) * blocks + own_slab, c = i & (columns - 1);
-    if (m0 + m >= p.M) continue;
-    if (gated) {
-      const int n = (c / 16) * 32 + c % 16;   // the gate's column; the feature's up value is 16 further
-      if (n0 + n + 16 >= p.N) continue;
-      float gate = total(m, n), up = total(m, n + 16);
-      if (p.bias) {
-        gate += p.bias[n0 + n];
-        up += p.bias[n0 + n + 16];
+  // A thread keeps one column (a block has at least as many threads as columns) and takes four rows at a time, whose
+  // reads are all on their way before the first store.
+  static_assert(T::kThreads >= T::BN, "a thread keeps one column");
+  const int c = threadIdx.x & (columns - 1), row_step = T::kThreads >> column_bits;
+  const int n = gated ? (c / 16) * 32 + c % 16 : c;   // gated: the gate's column; the feature's up value is 16 further
+  if (n0 + n + (gated ? 16 : 0) < p.N) {
+    const float bias = p.bias ? p.bias[n0 + n] : 0.0f, up_bias = p.bias && gated ? p.bias[n0 + n + 16] : 0.0f;
+    const int pitch = gated ? p.N / 2 : p.N, column = gated ? n0 / 2 + c : n0 + c;
+    for (int row = threadIdx.x >> column_bits; row < T::BM / blocks; row += 4 * row_step) {
+      float value[4], before[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = (row + i * row_step) * blocks + own_slab;
+        if (row + i * row_step >= T::BM / blocks || m0 + m >= p.M) continue;
+        if (p.epilogue == EPI_RESIDUAL) before[i] = p.resid[static_cast<size_t>(m0 + m) * pitch + column];
+        value[i] = total(m, n) + bias;
+        if (gated) value[i] = (total(m, n + 16) + up_bias) * gate_activation(value[i], p.activation);
       }
-      store(static_cast<size_t>(m0 + m) * (p.N / 2) + n0 / 2 + c, up * gate_activation(gate, p.activation));
-    } else {
-      if (n0 + c >= p.N) continue;
-      float value = total(m, c);
-      if (p.bias) value += p.bias[n0 + c];
-      const size_t at = static_cast<size_t>(m0 + m) * p.N + n0 + c;
-      if (p.epilogue == EPI_STORE) store(at, value);
-      else p.resid[at] += value;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = (row + i * row_step) * blocks + own_slab;
+        if (row + i * row_step >= T::BM / blocks || m0 + m >= p.M) continue;
+        const size_t at = static_cast<size_t>(m0 + m) * pitch + column;
+        if (p.epilogue == EPI_RESIDUAL) p.resid[at] = before[i] + value[i];
+        else store(at, value[i]);
+      }
     }
   }
   if (CLUSTER) cluster_sync();   // no block leaves while another reads its part
@@ -377,8 +410,9 @@ static int launch_form(const GemmArgs& p, cudaStream_t s) {
   if (opted) return opted;
   const unsigned tiles_n = (p.N + T::BN - 1) / T::BN, tiles_m = (p.M + T::BM - 1) / T::BM;
   if (tiles_m > 65535u) return VIPERA_BAD_SHAPE;
-  return launch_in_clusters(kernel, CLUSTER ? kSlabs : 1, dim3(CLUSTER ? tiles_n * kSlabs : tiles_n, tiles_m), dim3(T::kThreads),
-                            T::kSharedBytes, s, p);
+  const int chunks = ((CLUSTER ? p.slab : p.K) + kChunk - 1) / kChunk;
+  const int bytes = T::kSharedBytes - (chunks < T::STAGES ? T::STAGES - chunks : 0) * T::kStageFloats * 4;
+  return launch_in_clusters(kernel, CLUSTER ? kSlabs : 1, dim3(CLUSTER ? tiles_n * kSlabs : tiles_n, tiles_m), dim3(T::kThreads), bytes, s, p);
 }
 
 // A tile's slabs go to a cluster where whole tiles would leave much of the chip idle: fewer small tiles
@@ -407,7 +441,8 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
     }
   }
   // rows that do not start on 16 bytes, or values that are widened on the way
-  return launch_tile<TA, TW, TileSome, false>(p, s);
+  if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileSome, false>(p, s);
+  return launch_tile<TA, TW, TileMid, false>(p, s);
 }
 
 template <typename TA, typename TW>
@@ -418,7 +453,8 @@ static int launch_typed(const TA* A, const TW* W, int M, int N, int K, int epilo
   if (epilogue == EPI_RESIDUAL ? !resid : !out) return VIPERA_BAD_ARGUMENT;
   if (epilogue == EPI_SWIGLU && N % 32 != 0) return VIPERA_BAD_SHAPE;  // gate/up groups of 16 must pair up
   if (epilogue != EPI_RESIDUAL && out_dtype != VIPERA_F32 && out_dtype != VIPERA_BF16) return VIPERA_BAD_DTYPE;
-  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16};
+  const int wide = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
+  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16, wide};
   return launch_sizes<TA, TW>(p, s);
 }
 

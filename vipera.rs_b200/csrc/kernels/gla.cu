@@ -17,13 +17,14 @@
 // part of o to a scratch [row shares][tokens][heads*dv]; gla_finish_kernel adds the shares in a
 // fixed order and applies norm, gate and scale (a warp per (token, head)).
 //
-// Long steps are cut into chunks of kGlaChunk tokens that run side by side, in three launches:
+// Long steps are cut into chunks of kGlaChunk tokens that run side by side, in three launches (as two products a
+// chunk, linear_chunks.cuh; or, for head sizes those do not take, as walks):
 // every chunk from a zero state (its end state E and, per key channel, the sum of its log decays,
 // which gives the chunk's whole decay); per entry the states at the chunks' starts one after
 // another, S <- exp(sum log alpha) S + E, which also leaves the request's new state; every chunk
 // again from its start state, now with outputs.  The recurrence is linear in S, so this only
 // re-associates 32-bit sums.  Chunks are counted from where an entry's tokens start in the step.
-#include "common.cuh"
+#include "linear_chunks.cuh"
 
 #include <algorithm>
 
@@ -187,23 +188,37 @@ __global__ void __launch_bounds__(256) gla_chunk_starts_kernel(const GlaParams p
   const size_t width = static_cast<size_t>(p.heads) * p.dim * p.vdim;
   const size_t item = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
   const int entry = blockIdx.y;
-  if (item >= width) return;
+  if (item >= width) return;   // (width fits 32 bits: a state of 4 G elements a request does not exist)
   const int begin = p.entry_starts[entry], count = p.entry_starts[entry + 1] - begin;
   if (count <= 0) return;
   int job = 0;
   for (int e = 0; e < entry; ++e) job += (p.entry_starts[e + 1] - p.entry_starts[e] + kGlaChunk - 1) / kGlaChunk;
   const int chunks = (count + kGlaChunk - 1) / kGlaChunk;
-  const size_t row = item / p.vdim;   // head * dim + key channel
+  const unsigned row = static_cast<unsigned>(item) / static_cast<unsigned>(p.vdim);   // head * dim + key channel
+  const size_t decays = static_cast<size_t>(p.heads) * p.dim;
   float* state = p.state + static_cast<size_t>(p.state_slots[entry]) * width + item;
   float s = p.fresh[entry] ? 0.0f : *state;
-  for (int k = 0; k < chunks; ++k, ++job) {
-    float* cell = p.chunk_state + static_cast<size_t>(job) * width + item;
-    const float end_state = *cell;
-    *cell = s;
-    s = fmaf(expf(p.chunk_decay[static_cast<size_t>(job) * p.heads * p.dim + row]), s, end_state);
+  // eight chunks at a time: their end states and decays are asked for together, then walked in order (one after
+  // another, the trips to memory of 16 chunks took 275 us; now 21)
+  for (int k0 = 0; k0 < chunks; k0 += 8, job += 8) {
+    float ending[8], decay[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const size_t own = job + min(k, chunks - 1 - k0);
+      ending[k] = p.chunk_state[own * width + item];
+      decay[k] = p.chunk_decay[own * decays + row];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= chunks) break;
+      p.chunk_state[static_cast<size_t>(job + k) * width + item] = s;
+      s = fmaf(expf(decay[k]), s, ending[k]);
+    }
   }
   *state = s;
 }
+
+constexpr int kFinishKept = 8;   // values of a row a lane keeps
 
 template <typename TO>
 __global__ void __launch_bounds__(128) gla_finish_kernel(const GlaParams p) {
@@ -215,7 +230,29 @@ __global__ void __launch_bounds__(128) gla_finish_kernel(const GlaParams p) {
   const int t = item / p.heads, head = item % p.heads;
   const size_t out_width = static_cast<size_t>(p.heads) * p.vdim;
   const size_t base = static_cast<size_t>(t) * out_width + head * p.vdim;
+  const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off + head * p.vdim;
+  TO* out = static_cast<TO*>(p.out) + base;
+  auto ending = [&](float o, float inverse, float g, int e) {
+    out[e] = from_float<TO>(o * inverse * p.norm_weight[e] * (g / (1.0f + expf(-g))) * p.out_scale);
+  };
   float squares = 0.0f;
+  if (p.shares == 1 && p.vdim <= 32 * kFinishKept) {
+    // one share, and a row that fits the warp's registers: read once, all of it at the same time
+    float o[kFinishKept], g[kFinishKept];
+#pragma unroll
+    for (int j = 0; j < kFinishKept; ++j) {
+      const int e = lane + 32 * j;
+      o[j] = e < p.vdim ? p.partial[base + e] : 0.0f;
+      g[j] = e < p.vdim ? gate[e] : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < kFinishKept; ++j) squares = fmaf(o[j], o[j], squares);
+    const float inverse = 1.0f / sqrtf(warp_sum(squares) / static_cast<float>(p.vdim) + p.eps);
+#pragma unroll
+    for (int j = 0; j < kFinishKept; ++j)
+      if (lane + 32 * j < p.vdim) ending(o[j], inverse, g[j], lane + 32 * j);
+    return;
+  }
   for (int e = lane; e < p.vdim; e += 32) {
     float o = 0.0f;
     for (int share = 0; share < p.shares; ++share) o += p.partial[static_cast<size_t>(share) * p.num_tokens * out_width + base + e];
@@ -223,12 +260,7 @@ __global__ void __launch_bounds__(128) gla_finish_kernel(const GlaParams p) {
     squares = fmaf(o, o, squares);
   }
   const float inverse = 1.0f / sqrtf(warp_sum(squares) / static_cast<float>(p.vdim) + p.eps);
-  const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off + head * p.vdim;
-  TO* out = static_cast<TO*>(p.out) + base;
-  for (int e = lane; e < p.vdim; e += 32) {
-    const float g = gate[e];
-    out[e] = from_float<TO>(p.partial[base + e] * inverse * p.norm_weight[e] * (g / (1.0f + expf(-g))) * p.out_scale);
-  }
+  for (int e = lane; e < p.vdim; e += 32) ending(p.partial[base + e], inverse, gate[e], e);
 }
 
 // Rows of the state a warp holds, for a head's key size.
@@ -264,14 +296,22 @@ VIPERA_API int vipera_gla(const GlaParams* params, int out_dtype, void* stream) 
   const size_t decays = static_cast<size_t>(p.num_tokens) * p.heads * p.dim;
   int status = vipera_launch(gla_decay_kernel, dim3(static_cast<unsigned>(std::min<size_t>((decays + 255) / 256, 4096))), 256, 0, s, p);
   if (status) return status;
+  LinearArgs chunks{};
+  if (chunked) {
+    chunks = LinearArgs{p.proj, p.proj_width, p.q_off, p.k_off, p.v_off, p.log_alpha, p.z, nullptr, p.entry_starts, p.chunk_state,
+                        p.chunk_decay, p.partial, p.num_entries, p.heads, p.dim, p.vdim, p.q_scale};
+  }
+  // heads of more than 256 key channels, and rows that are not whole 16-byte pieces, walk their chunks
+  const bool products = chunked && p.num_jobs <= 65535 && linear_chunks_take(chunks);
   if (!chunked) status = pass(0);
   else {
-    status = pass(1);
+    status = products ? launch_linear_ends<true>(chunks, p.num_jobs, s) : pass(1);
     if (!status) {
       const size_t width = static_cast<size_t>(p.heads) * p.dim * p.vdim;
       status = vipera_launch(gla_chunk_starts_kernel, dim3(static_cast<unsigned>((width + 255) / 256), p.num_entries), 256, 0, s, p);
     }
-    if (!status) status = pass(3);
+    if (!status) status = products ? launch_linear_outputs<true>(chunks, p.num_jobs, s) : pass(3);
+    if (products) p.shares = 1;   // the products leave whole outputs
   }
   if (status) return status;
   const int items = p.num_tokens * p.heads;

@@ -19,10 +19,11 @@
 //   ends     a job is a chunk: from zero over the chunk, no outputs, leaving E_c = sum_s
 //            lambda^(len - 1 - s) k_s v_s^T in the chunk's scratch row.
 //   outputs  a job is a chunk: from the state at the chunk's start (the scratch row), with outputs.
+// (The two kinds of chunk jobs run as products, linear_chunks.cuh, where its rows are whole 16-byte pieces.)
 // Between ends and outputs, lightning_carry_kernel walks each entry's chunks: start_c = S;
 // S = lambda^len_c S + E_c; the request's new state is the last S.  Another cut of a prompt only
 // re-associates 32-bit sums.
-#include "common.cuh"
+#include "linear_chunks.cuh"
 
 constexpr int kChunk = 64;
 constexpr int kStage = 16;
@@ -266,6 +267,17 @@ static int launch_scans(const LightningParams& params, bool chunked, cudaStream_
   const int tiles = (p.dv + kColumns - 1) / kColumns;
   if (!chunked)
     return vipera_launch(lightning_scan_kernel<RPT, MODE_WALK>, dim3(tiles, p.heads, p.num_entries), kRowWarps * 32, shared, s, p);
+  // rows that are not whole 16-byte pieces walk their chunks
+  const LinearArgs chunks{p.proj, p.proj_width, p.q_off, p.k_off, p.v_off, nullptr, nullptr, p.decay, p.entry_starts, p.chunk_state,
+                          nullptr, p.raw, p.num_entries, p.heads, p.d, p.dv, 1.0f};
+  const size_t state_floats = static_cast<size_t>(p.heads) * p.d * p.dv;
+  if (linear_chunks_take(chunks)) {
+    int status = launch_linear_ends<false>(chunks, p.num_jobs, s);
+    if (status) return status;
+    status = vipera_launch(lightning_carry_kernel, dim3(static_cast<unsigned>((state_floats + 255) / 256), p.num_entries), 256, 0, s, p);
+    if (status) return status;
+    return launch_linear_outputs<false>(chunks, p.num_jobs, s);
+  }
   p.activated = 1;
   const long long values = static_cast<long long>(p.num_tokens) * p.heads * (2 * p.d + p.dv);
   int status = vipera_launch(lightning_activate_kernel, static_cast<unsigned>((values + 255) / 256), 256, 0, s, p);
