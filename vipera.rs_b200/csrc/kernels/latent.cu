@@ -18,6 +18,8 @@
 // sink per head the softmax's denominator also holds exp(sink_h): a term without a key or a value,
 // which the scale does not touch.
 #include "attention_mma.cuh"
+#include "latent_tc.cuh"
+#include "simt.cuh"
 
 constexpr int kMaxRank = 512;   // latent size
 constexpr int kMaxRot = 128;    // rotated part
@@ -916,6 +918,7 @@ struct LatentParams {
   const float* cq_norm_weight;   // [q_rank]
   void* cq;                      // [tokens, q_rank], the run's type
   int single;              // 1: every request of the step brings one token
+  int* status;             // receives a code where a bounded wait ran out, or null: the fold stays with mma.sync
 };
 
 // How the tensor-core fold cuts a step.  Rows are tokens x heads.  Many rows: two groups of sixteen to a
@@ -984,7 +987,35 @@ static int launch_fold(const LatentFoldParams& f, dim3 grid, size_t shared, cuda
   return vipera_launch(latent_fold_kernel<NR, MT>, grid, kFoldThreads, shared, s, f);
 }
 
+// Rows from which the tcgen05 fold runs a step in the head-major form.  RULE
+constexpr long kTensorRows = 1536;
+
+static bool fold_takes_tensor(const LatentParams& p) {
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool) | reinterpret_cast<uintptr_t>(p.l_heads) |
+                          reinterpret_cast<uintptr_t>(p.qa_heads) | reinterpret_cast<uintptr_t>(p.q_rot);
+  return p.stage == 2 && !p.single && p.status != nullptr && static_cast<long>(p.num_tokens) * p.heads >= kTensorRows &&
+         p.rank % latent_tc::kPart == 0 && p.rot <= latent_tc::kPart && (bases & 15) == 0;
+}
+
+static int launch_fold_tensor(const LatentParams& p, cudaStream_t s) {
+  latent_tc::Params f{};
+  f.qa_heads = p.qa_heads, f.q_rot = p.q_rot;
+  f.k_pool = static_cast<const __nv_bfloat16*>(p.k_pool);
+  f.v_pool = static_cast<const __nv_bfloat16*>(p.v_pool);
+  f.token_entry = p.token_entry, f.positions = p.positions, f.block_table = p.block_table;
+  f.l_heads = static_cast<__nv_bfloat16*>(p.l_heads);
+  f.num_tokens = p.num_tokens, f.heads = p.heads, f.rank = p.rank, f.rot = p.rot;
+  f.table_width = p.table_width, f.page_size = p.page_size, f.padded_tokens = p.padded_tokens, f.window = p.window;
+  f.scale = p.scale, f.sink = p.sink, f.status = p.status;
+  static SharedMemoryOptIn opt_in;
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(latent_tc::latent_fold_tc_kernel), latent_tc::kSharedBytes);
+  if (opted) return opted;
+  const int tiles = (p.num_tokens * p.heads + latent_tc::kRows - 1) / latent_tc::kRows, slices = (p.rank + 255) / 256;
+  return vipera_launch(latent_tc::latent_fold_tc_kernel, dim3(tiles * slices), dim3(latent_tc::kThreads), latent_tc::kSharedBytes, s, f);
+}
+
 static int launch_fold_any(const LatentParams& p, cudaStream_t s) {
+  if (fold_takes_tensor(p)) return launch_fold_tensor(p, s);
   LatentFoldParams f{};
   f.qa = p.qa;
   f.k_pool = static_cast<const __nv_bfloat16*>(p.k_pool);
@@ -1092,6 +1123,9 @@ VIPERA_API int vipera_latent_attention(const LatentParams* params, int dtype, vo
   if (dtype == VIPERA_BF16) return launch_latent<__nv_bfloat16>(p, s);
   return VIPERA_BAD_DTYPE;
 }
+
+// 1 where the fold of these parameters runs on tcgen05 (one launch, whatever the splits), else 0.
+VIPERA_API int vipera_latent_fold_tensor(const LatentParams* params) { return fold_takes_tensor(*params) ? 1 : 0; }
 
 VIPERA_API int vipera_latent_params_size() { return static_cast<int>(sizeof(LatentParams)); }
 VIPERA_API const char* vipera_latent_status_text(int status) { return vipera_status_text(status); }

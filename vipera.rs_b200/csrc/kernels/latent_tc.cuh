@@ -1,0 +1,489 @@
+// The fold over latents on the fifth-generation tensor cores (tcgen05, accumulators in tensor memory), for steps
+// of many (token, head) rows in the head-major form (bfloat16 caches).
+//
+// A block takes 128 rows (numbered token by token, so that a tile's heads share its keys) and a slice of up to
+// 256 of the latent's columns, and walks the keys 64 at a time:
+//
+//   S = Q [c | kr]^T     tcgen05.mma 128 x 64 over rank + rot values, from shared memory, into tensor memory
+//   softmax              a row a thread; weights rounded to bfloat16 go back to tensor memory, where the
+//                        output product takes them from; their sum is that of the rounded weights
+//   O += P C             tcgen05.mma 128 x 64 columns x 64 keys per part of 64 columns, in tensor memory
+//
+// Two score and two weight buffers let the scores of one tile run while the softmax of the one before is
+// computed.  Keys and values are the same rows: a tile comes as parts of [64 keys][64 columns] (8 KB, 128-byte
+// swizzle), read along the columns for the scores and along the keys for the output.  The queries fill 144 KB of
+// shared memory, which leaves ten slots for parts: a ring for those that only the scores read, and one for
+// those the output product reads too (a tile's four and some of the next).  The scores are computed in the block of
+// each slice: with 512 columns of output beside them, tensor memory would not do (512 columns an SM).
+//
+// Roles: warps 0-3 softmax and ending, warp 4 issues the products, then a warp per slot, which brings one part after
+// another through the block table (cp.async; first of all each brings a part of the queries).  A thread that handed
+// over several parts in their order waited for the newest before the oldest could be used: 500 us where a warp per
+// slot takes MEASURED.  Tokens of several requests in a tile are folded one request after another.
+// Every wait is bounded; one that runs out leaves a code in the status word and the rows unwritten.
+#pragma once
+
+#include "common.cuh"
+
+namespace latent_tc {
+
+constexpr int kRows = 128, kKeys = 64, kPart = 64;   // rows, keys of a tile, columns of a part
+constexpr int kPartBytes = kKeys * kPart * 2, kQueryBytes = kRows * kPart * 2;
+constexpr int kScoreSlots = 4, kValueSlots = 6, kSlots = kScoreSlots + kValueSlots;
+constexpr int kMostParts = 9;                        // 512 / 64 and the rotated part
+constexpr int kSoftmaxWarps = 4, kIssuer = 4, kFirstLoader = 5;
+constexpr int kThreads = (kFirstLoader + kSlots) * 32;
+constexpr uint32_t kColsO = 0, kColsS = 256, kColsP = 384, kTmemCols = 512;   // O 256, S 2 x 64, P 2 x 32
+constexpr uint32_t kWaitLimit = 1u << 22;
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kMaxSlack = 8.0f;                    // in powers of two
+enum { WAIT_EXPIRED = 5 };
+static_assert(kSlots >= kMostParts, "a loading warp brings at most one part of the queries");
+
+struct Params {
+  const float* qa_heads;           // [heads, padded_tokens, rank], unscaled
+  const float* q_rot;              // [tokens, heads, rot], scaled
+  const __nv_bfloat16* k_pool;     // latents
+  const __nv_bfloat16* v_pool;     // rotated key parts
+  const int* token_entry;
+  const int* positions;
+  const int* block_table;
+  __nv_bfloat16* l_heads;          // [heads, padded_tokens, rank]
+  int num_tokens, heads, rank, rot, table_width, page_size, padded_tokens, window;
+  float scale;
+  const float* sink;
+  int* status;
+};
+
+struct Shared {
+  uint64_t full[kSlots], empty[kSlots], query[kMostParts], score[2], weight[2], done;
+  uint32_t tmem_base;
+  int abort_flag;
+  int entry[kRows], position[kRows];   // of the tile's tokens
+};
+
+constexpr int kSharedBytes = kMostParts * kQueryBytes + kSlots * kPartBytes + static_cast<int>(sizeof(Shared)) + 1024;
+static_assert(kSharedBytes <= 227 * 1024, "a block's shared memory");
+
+__device__ __forceinline__ uint32_t addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(addr(bar)), "r"(count));
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(addr(bar)) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(addr(bar)), "r"(parity) : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ void bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
+    if (bar_try(bar, parity)) return;
+    if (spin > 8) __nanosleep(32);
+    if ((spin & 1023u) == 1023u && *abort_flag) return;
+  }
+  *abort_flag = 1;
+  atomicExch(status, WAIT_EXPIRED);
+}
+__device__ __forceinline__ void copy_piece(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(addr(bar)) : "memory");
+}
+__device__ __forceinline__ void mma_shared(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_tensor(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+#define LATENT_TC_8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
+__device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : LATENT_TC_8(r, 0), LATENT_TC_8(r, 8), LATENT_TC_8(r, 16), LATENT_TC_8(r, 24)
+      : "r"(taddr));
+}
+#undef LATENT_TC_8
+__device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+#define LATENT_TC_8(r, o) "r"(r[o]), "r"(r[o + 1]), "r"(r[o + 2]), "r"(r[o + 3]), "r"(r[o + 4]), "r"(r[o + 5]), "r"(r[o + 6]), "r"(r[o + 7])
+__device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), LATENT_TC_8(r, 0), LATENT_TC_8(r, 8), LATENT_TC_8(r, 16), LATENT_TC_8(r, 24)
+      : "memory");
+}
+#undef LATENT_TC_8
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// 2^x with the hardware's approximation (the weights are rounded to bfloat16); 2^(-inf) = 0
+__device__ __forceinline__ float power_of_two(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 16-byte piece `piece` (0..7) of row `row` of a part, swizzled
+__device__ __forceinline__ uint32_t piece_offset(int row, int piece) { return static_cast<uint32_t>(row * 128 + ((piece ^ (row & 7)) << 4)); }
+// A part as an operand: 128-byte rows, 128-byte swizzle, groups of eight rows 1024 bytes apart.  The same words serve
+// both readings (the contraction along the rows' bytes, or down the rows): within one part of 64 columns the leading
+// offset plays no role.
+__device__ __forceinline__ uint64_t descriptor(uint32_t saddr) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+         (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
+}
+
+// One request's tokens that follow one another in the tile, and the keys any of them sees.
+struct Segment { int begin, end, entry, first_key, end_key, first_tile, tiles; };
+__device__ __forceinline__ Segment segment_from(const Shared& s, int begin, int tokens, int window) {
+  Segment g{begin, begin, s.entry[begin], 0, 0, 0, 0};
+  int low = 0x7fffffff, high = -1;
+  while (g.end < tokens && s.entry[g.end] == g.entry) {
+    low = min(low, s.position[g.end]);
+    high = max(high, s.position[g.end]);
+    ++g.end;
+  }
+  g.first_key = window > 0 ? max(0, low - window + 1) : 0;
+  g.end_key = high + 1;
+  g.first_tile = g.first_key / kKeys;
+  g.tiles = (g.end_key + kKeys - 1) / kKeys - g.first_tile;
+  return g;
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+latent_fold_tc_kernel(const Params p) {
+  extern __shared__ uint8_t latent_tc_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(latent_tc_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* queries = base;                                   // parts of [128 rows][64 columns]
+  uint8_t* slots = base + kMostParts * kQueryBytes;          // parts of [64 keys][64 columns]
+  Shared& s = *reinterpret_cast<Shared*>(slots + kSlots * kPartBytes);
+  volatile int* abort_flag = &s.abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int latent_parts = p.rank / kPart, slices = (latent_parts + 3) / 4;
+  const int tile = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) / slices;   // the longest histories of a prompt first
+  const int slice = static_cast<int>(blockIdx.x) % slices;
+  // parts in the order they are read: those only the scores need (the other slices', the rotated one), then this slice's
+  const int value_parts = min(4, latent_parts - 4 * slice), score_parts = latent_parts + 1 - value_parts;
+  auto part_of = [&](int i) {   // the latent's part (latent_parts: the rotated one) that comes i-th
+    if (i >= score_parts) return 4 * slice + i - score_parts;
+    if (i == score_parts - 1) return latent_parts;
+    return i < 4 * slice ? i : i + value_parts;
+  };
+  const int parts = latent_parts + 1;
+  const int total_rows = p.num_tokens * p.heads, row0 = tile * kRows, rows = min(kRows, total_rows - row0);
+  const int token0 = row0 / p.heads, tokens = (row0 + rows - 1) / p.heads - token0 + 1;
+
+  pdl_launch_dependents();
+  if (tid == 0) {
+    for (int i = 0; i < kSlots; ++i) {
+      bar_init(&s.full[i], 32);
+      bar_init(&s.empty[i], 1);
+    }
+    for (int i = 0; i < kMostParts; ++i) bar_init(&s.query[i], 32);
+    for (int i = 0; i < 2; ++i) {
+      bar_init(&s.score[i], 1);
+      bar_init(&s.weight[i], kSoftmaxWarps * 32);
+    }
+    bar_init(&s.done, 1);
+    s.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kIssuer) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(addr(&s.tmem_base)), "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  // (the step's tokens are the host's, written before the step)
+  for (int i = tid; i < tokens; i += kThreads) {
+    s.entry[i] = p.token_entry[token0 + i];
+    s.position[i] = p.positions[token0 + i];
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = s.tmem_base;
+
+  if (warp < kSoftmaxWarps) {
+    // ---------------- softmax, ending: thread = row ----------------
+    pdl_wait();   // the output belongs to earlier kernels until now
+    const int row = tid, own_token = (row0 + min(row, rows - 1)) / p.heads - token0;
+    const int head = (row0 + min(row, rows - 1)) % p.heads;
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    int count = 0, passes = 0;   // tiles, and requests, so far
+    for (int begin = 0; begin < tokens; ++passes) {
+      const Segment g = segment_from(s, begin, tokens, p.window);
+      begin = g.end;
+      const bool mine = row < rows && own_token >= g.begin && own_token < g.end;
+      const int last = mine ? s.position[own_token] : -1;
+      const int first = mine && p.window > 0 ? last - p.window + 1 : 0;
+      float row_max = -INFINITY, row_sum = 0.0f;   // the max in powers of two
+      for (int t = 0; t < g.tiles; ++t, ++count) {
+        const uint32_t buffer = count & 1, parity = (count >> 1) & 1;
+        bar_wait(&s.score[buffer], parity, abort_flag, p.status);
+        fence_after();
+        uint32_t v[64];
+        tmem_load(lanes + kColsS + buffer * kKeys, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        tmem_load(lanes + kColsS + buffer * kKeys + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+        tmem_load_wait();
+        const int key0 = (g.first_tile + t) * kKeys;
+        if (key0 < first || key0 + kKeys - 1 > last) {
+#pragma unroll
+          for (int k = 0; k < kKeys; ++k)
+            if (key0 + k < first || key0 + k > last) v[k] = __float_as_uint(-INFINITY);
+        }
+        float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < kKeys; k += 4) {
+          m0 = fmaxf(m0, __uint_as_float(v[k]));
+          m1 = fmaxf(m1, __uint_as_float(v[k + 1]));
+          m2 = fmaxf(m2, __uint_as_float(v[k + 2]));
+          m3 = fmaxf(m3, __uint_as_float(v[k + 3]));
+        }
+        const float tile_max = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * kLog2e;
+        // the running max follows once it is behind by more than the slack: most tiles leave the output as it is
+        float new_max = row_max;
+        if (tile_max > row_max + kMaxSlack || row_max == -INFINITY) new_max = fmaxf(row_max, tile_max);
+        const float alpha = new_max == row_max ? 1.0f : power_of_two(row_max - new_max);
+        row_max = new_max;
+        row_sum *= alpha;
+        // (these scores are complete, so the output product of the tile before is)
+        if (t > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+#pragma unroll 1
+          for (int c = 0; c < value_parts * kPart; c += 32) {
+            uint32_t o[32];
+            tmem_load(lanes + kColsO + c, o);
+            tmem_load_wait();
+#pragma unroll
+            for (int k = 0; k < 32; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+            tmem_store(lanes + kColsO + c, o);
+          }
+        }
+        const float shift = row_max == -INFINITY ? 0.0f : row_max;
+        float sum0 = 0.0f, sum1 = 0.0f;
+        uint32_t packed[32];
+#pragma unroll
+        for (int k = 0; k < kKeys; k += 2) {
+          const __nv_bfloat162 w = __floats2bfloat162_rn(power_of_two(fmaf(__uint_as_float(v[k]), kLog2e, -shift)),
+                                                         power_of_two(fmaf(__uint_as_float(v[k + 1]), kLog2e, -shift)));
+          const float2 rounded = __bfloat1622float2(w);
+          sum0 += rounded.x;
+          sum1 += rounded.y;
+          packed[k >> 1] = *reinterpret_cast<const uint32_t*>(&w);
+        }
+        row_sum += sum0 + sum1;
+        tmem_store(lanes + kColsP + buffer * (kKeys / 2), packed);
+        tmem_store_wait();
+        fence_before();
+        bar_arrive(&s.weight[buffer]);
+      }
+      // the ending: the request's rows
+      bar_wait(&s.done, static_cast<uint32_t>(passes) & 1u, abort_flag, p.status);
+      fence_after();
+      float total = row_sum;
+      if (p.sink) total += exp2f(p.sink[head] * kLog2e - row_max);
+      const float inverse = 1.0f / total;
+      __nv_bfloat16* out = p.l_heads + (static_cast<size_t>(head) * p.padded_tokens + token0 + own_token) * p.rank + slice * 4 * kPart;
+#pragma unroll 1
+      for (int c = 0; c < value_parts * kPart; c += 32) {
+        uint32_t o[32];
+        tmem_load(lanes + kColsO + c, o);
+        tmem_load_wait();
+        if (mine && !*abort_flag) {
+#pragma unroll
+          for (int k = 0; k < 32; k += 8) {
+            uint4 packed;
+            __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              pairs[e] = __floats2bfloat162_rn(__uint_as_float(o[k + 2 * e]) * inverse, __uint_as_float(o[k + 2 * e + 1]) * inverse);
+            *reinterpret_cast<uint4*>(out + c + k) = packed;
+          }
+        }
+      }
+      fence_before();
+      asm volatile("bar.sync 1, 160;" ::: "memory");   // with the issuer: the next request's products overwrite O
+    }
+  } else if (warp == kIssuer) {
+    // ---------------- the products, one thread ----------------
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kRows >> 4) << 24) | (static_cast<uint32_t>(kKeys >> 3) << 17);
+    constexpr uint32_t kIdescValues = kIdesc | (1u << 16);   // B read down its rows
+    int score_number = 0, value_number = 0, count = 0;       // parts taken from the two rings, tiles issued
+    const int rot_steps = (p.rot + 15) / 16;
+    const int early = min(score_parts, 4);
+    auto issue_part = [&](int i, int buffer) {   // the i-th part of a tile's scores
+      int slot;
+      uint32_t parity;
+      if (i < score_parts) {
+        slot = score_number % kScoreSlots;
+        parity = (score_number / kScoreSlots) & 1;
+        ++score_number;
+      } else {
+        slot = kScoreSlots + value_number % kValueSlots;
+        parity = (value_number / kValueSlots) & 1;
+        ++value_number;
+      }
+      bar_wait(&s.full[slot], parity, abort_flag, p.status);
+      fence_after();
+      const uint32_t a = addr(queries + i * kQueryBytes), b = addr(slots + slot * kPartBytes);
+      const int steps = part_of(i) == latent_parts ? rot_steps : 4;
+      for (int ks = 0; ks < steps; ++ks)
+        mma_shared(tmem + kColsS + buffer * kKeys, descriptor(a + ks * 32), descriptor(b + ks * 32), kIdesc, i > 0 || ks > 0 ? 1u : 0u);
+      if (i < score_parts) commit(&s.empty[slot]);
+    };
+    for (int begin = 0; begin < tokens;) {
+      const Segment g = segment_from(s, begin, tokens, p.window);
+      begin = g.end;
+      if (lane == 0) {
+        int values_of_last = 0;   // the number of the first value part of the tile before
+        for (int t = 0; t <= g.tiles; ++t) {
+          // scores of tile t, and in their midst the output product of tile t - 1
+          const int number = count + t;
+          const bool very_first = number == 0;   // the queries may still be on their way
+          if (t < g.tiles)
+            for (int i = 0; i < early; ++i) {
+              if (very_first) bar_wait(&s.query[i], 0, abort_flag, p.status);
+              issue_part(i, number & 1);
+            }
+          if (t > 0) {
+            const int before = number - 1;
+            bar_wait(&s.weight[before & 1], (before >> 1) & 1, abort_flag, p.status);
+            fence_after();
+            for (int v = 0; v < value_parts; ++v) {
+              const int slot = kScoreSlots + (values_of_last + v) % kValueSlots;
+              const uint32_t b = addr(slots + slot * kPartBytes);
+#pragma unroll
+              for (int ks = 0; ks < kKeys / 16; ++ks)
+                mma_tensor(tmem + kColsO + v * kPart, tmem + kColsP + (before & 1) * (kKeys / 2) + ks * 8, descriptor(b + ks * 2048),
+                           kIdescValues, t > 1 || ks > 0 ? 1u : 0u);
+              commit(&s.empty[slot]);
+            }
+            if (t == g.tiles) commit(&s.done);
+          }
+          if (t < g.tiles) {
+            values_of_last = value_number;
+            for (int i = early; i < parts; ++i) {
+              if (very_first) bar_wait(&s.query[i], 0, abort_flag, p.status);
+              issue_part(i, number & 1);
+            }
+            commit(&s.score[number & 1]);
+          }
+        }
+      }
+      count += g.tiles;
+      __syncwarp();
+      fence_before();
+      asm volatile("bar.sync 1, 160;" ::: "memory");
+      fence_after();
+    }
+  } else {
+    // ---------------- a warp per slot: the parts that come to it, one after another ----------------
+    const int slot = warp - kFirstLoader;
+    const bool of_values = slot >= kScoreSlots;
+    const int ring = of_values ? kValueSlots : kScoreSlots, each = of_values ? value_parts : score_parts;   // slots, parts a tile
+    const int piece = lane & 7, sub = lane >> 3;
+    const uint32_t dst = addr(slots + slot * kPartBytes);
+    int number = of_values ? slot - kScoreSlots : slot, round = 0, count = 0;   // of the part, of the slot's use; tiles before this request
+    // where keys lane and lane + 32 of a tile lie in the pools, -1: nowhere (zeros)
+    int place_lo = -1, place_hi = -1;
+    auto look_up = [&](const Segment& g, int tile_index) {
+      const int* table = p.block_table + static_cast<size_t>(g.entry) * p.table_width;
+      const int lo = (g.first_tile + tile_index) * kKeys + lane, hi = lo + 32;
+      place_lo = place_hi = -1;
+      if (lo >= g.first_key && lo < g.end_key) {
+        const int page = table[lo / p.page_size];
+        if (page >= 0) place_lo = page * p.page_size + lo % p.page_size;
+      }
+      if (hi >= g.first_key && hi < g.end_key) {
+        const int page = table[hi / p.page_size];
+        if (page >= 0) place_hi = page * p.page_size + hi % p.page_size;
+      }
+    };
+    auto copy = [&](int i) {   // the i-th part of a tile
+      const int part = part_of(i);
+      const bool latent = part < latent_parts;
+      const __nv_bfloat16* pool = latent ? p.k_pool + part * kPart + piece * 8 : p.v_pool + piece * 8;
+      const int stride = latent ? p.rank : p.rot;
+      const bool column = latent || piece * 8 < p.rot;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int r = sub + 4 * j;   // (rows 32 and on from j = 8 on)
+        const int place = __shfl_sync(0xffffffffu, j < 8 ? place_lo : place_hi, r & 31);
+        const bool valid = place >= 0 && column;
+        copy_piece(dst + piece_offset(r, piece), valid ? pool + static_cast<size_t>(place) * stride : p.k_pool, valid);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    bool queries_due = slot < parts;
+    auto bring_queries = [&]() {   // part `slot` of the queries, sixteen rows of it at a time
+      queries_due = false;
+      const int part = part_of(slot);
+      const float f = part < latent_parts ? p.scale : 1.0f;
+      const int c = piece * 8;
+#pragma unroll 1
+      for (int r0 = 0; r0 < kRows; r0 += 32) {
+        float4 lo[8], hi[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int r = r0 + sub + 4 * j, global = row0 + r;
+          lo[j] = hi[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (r < rows && (part < latent_parts || c < p.rot)) {
+            const float* src = part < latent_parts
+                ? p.qa_heads + (static_cast<size_t>(global % p.heads) * p.padded_tokens + global / p.heads) * p.rank + part * kPart + c
+                : p.q_rot + static_cast<size_t>(global) * p.rot + c;
+            lo[j] = *reinterpret_cast<const float4*>(src);
+            hi[j] = *reinterpret_cast<const float4*>(src + 4);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          uint4 packed;
+          __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&packed);
+          pairs[0] = __floats2bfloat162_rn(lo[j].x * f, lo[j].y * f);
+          pairs[1] = __floats2bfloat162_rn(lo[j].z * f, lo[j].w * f);
+          pairs[2] = __floats2bfloat162_rn(hi[j].x * f, hi[j].y * f);
+          pairs[3] = __floats2bfloat162_rn(hi[j].z * f, hi[j].w * f);
+          *reinterpret_cast<uint4*>(queries + slot * kQueryBytes + piece_offset(r0 + sub + 4 * j, piece)) = packed;
+        }
+      }
+      fence_async();
+      bar_arrive(&s.query[slot]);
+    };
+    bool waited = false;
+    for (int begin = 0; begin < tokens;) {
+      const Segment g = segment_from(s, begin, tokens, p.window);
+      begin = g.end;
+      if (number < (count + g.tiles) * each) look_up(g, number / each - count);
+      if (!waited) {
+        pdl_wait();   // (the block table is the host's)
+        waited = true;
+      }
+      for (; number < (count + g.tiles) * each; number += ring, ++round) {
+        if (round > 0) bar_wait(&s.empty[slot], (round - 1) & 1, abort_flag, p.status);
+        copy((of_values ? score_parts : 0) + number % each);
+        if (number + ring < (count + g.tiles) * each) look_up(g, (number + ring) / each - count);
+        if (queries_due) bring_queries();
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        fence_async();
+        bar_arrive(&s.full[slot]);
+      }
+      count += g.tiles;
+    }
+    if (queries_due) bring_queries();   // (a slot that no part comes to)
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == kIssuer) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+  }
+}
+
+}  // namespace latent_tc

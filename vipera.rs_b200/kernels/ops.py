@@ -1737,7 +1737,7 @@ class _LatentParams(ctypes.Structure):
         ("stage", _c_int), ("padded_tokens", _c_int), ("a_heads", _c_void), ("qa_heads", _c_void), ("q_rot", _c_void),
         ("l_heads", _c_void), ("o_heads", _c_void), ("tile_group", _c_void),
         ("window", _c_int), ("pairing", _c_int), ("sink", _c_void), ("q", _c_void), ("q_width", ctypes.c_longlong),
-        ("cq_off", _c_int), ("q_rank", _c_int), ("cq_norm_weight", _c_void), ("cq", _c_void), ("single", _c_int),
+        ("cq_off", _c_int), ("q_rank", _c_int), ("cq_norm_weight", _c_void), ("cq", _c_void), ("single", _c_int), ("status", _c_void),
     ]
 
 
@@ -1835,6 +1835,7 @@ def latent_attention(proj: torch.Tensor, *, q_off: int, g_off: int, kv_off: int,
         raise InvalidArgumentError("latent_attention: the rotated part turns as interleaved pairs or as halves")
     p.window, p.pairing = int(window or 0), 1 if pairing == ROPE_NEOX else 0
     p.part, p.split_keys, p.num_splits, p.single = None, 0, 1, int(bool(single))
+    p.status = _tc_buffers(proj.device, 0)["status"].data_ptr() if head_major is not None else None
     if part is not None and max_keys > 0:
         _, _, split_keys, splits = latent_plan(tokens, heads, rank, rot_dim, int(max_keys), sm_count(proj.device), p.window, single)
         if splits > 1:
@@ -1859,7 +1860,8 @@ def latent_attention(proj: torch.Tensor, *, q_off: int, g_off: int, kv_off: int,
         _check(fn(ctypes.byref(p), code, _stream()), "attention", kernels=2 if kv_off >= 0 else 1)
         gemm_tc_grouped(m["a_heads"], m["up_k_t"], m["tile_group"], epilogue=EPI_STORE, out=m["qa_heads"], what="attention")
         p.stage = 2
-        _check(fn(ctypes.byref(p), code, _stream()), "attention", kernels=2 if p.num_splits > 1 else 1)
+        tensor = _function("latent", "vipera_latent_fold_tensor", [ctypes.POINTER(_LatentParams)])(ctypes.byref(p))
+        _check(fn(ctypes.byref(p), code, _stream()), "attention", kernels=2 if p.num_splits > 1 and not tensor else 1)
         gemm_tc_grouped(m["l_heads"], m["up_v_rows"], m["tile_group"], epilogue=EPI_STORE, out=m["o_heads"], what="attention")
         p.stage = 3
         _check(fn(ctypes.byref(p), code, _stream()), "attention")
