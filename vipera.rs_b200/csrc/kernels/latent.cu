@@ -994,7 +994,7 @@ static bool fold_takes_tensor(const LatentParams& p) {
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool) | reinterpret_cast<uintptr_t>(p.l_heads) |
                           reinterpret_cast<uintptr_t>(p.qa_heads) | reinterpret_cast<uintptr_t>(p.q_rot);
   return p.stage == 2 && !p.single && p.status != nullptr && static_cast<long>(p.num_tokens) * p.heads >= kTensorRows &&
-         p.rank % latent_tc::kPart == 0 && p.rot <= latent_tc::kPart && (bases & 15) == 0;
+         p.rank % latent_tc::kHalf == 0 && p.rot <= latent_tc::kHalf && (bases & 15) == 0;
 }
 
 static int launch_fold_tensor(const LatentParams& p, cudaStream_t s) {

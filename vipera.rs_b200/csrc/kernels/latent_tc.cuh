@@ -10,16 +10,20 @@
 //   O += P C             tcgen05.mma 128 x 64 columns x 64 keys per part of 64 columns, in tensor memory
 //
 // Two score and two weight buffers let the scores of one tile run while the softmax of the one before is
-// computed.  Keys and values are the same rows: a tile comes as parts of [64 keys][64 columns] (8 KB, 128-byte
-// swizzle), read along the columns for the scores and along the keys for the output.  The queries fill 144 KB of
-// shared memory, which leaves ten slots for parts: a ring for those that only the scores read, and one for
-// those the output product reads too (a tile's four and some of the next).  The scores are computed in the block of
-// each slice: with 512 columns of output beside them, tensor memory would not do (512 columns an SM).
+// computed.  Keys and values are the same rows: a tile comes as parts of [64 keys][128 columns] (two halves of 64
+// columns, 8 KB, 128-byte swizzle), read along the columns for the scores and along the keys for the output.  The
+// queries fill 144 KB of shared memory, which leaves five slots for parts: a ring of two for those that only the
+// scores read, and one of three for those the output product reads too (a tile's two and the next one's first).  The
+// scores are computed in the block of each slice: with 512 columns of output beside them, tensor memory would not do
+// (512 columns an SM).
 //
-// Roles: warps 0-3 softmax and ending, warp 4 issues the products, then a warp per slot, which brings one part after
-// another through the block table (cp.async; first of all each brings a part of the queries).  A thread that handed
-// over several parts in their order waited for the newest before the oldest could be used: 500 us where a warp per
-// slot takes MEASURED.  Tokens of several requests in a tile are folded one request after another.
+// Roles: warps 0-3 softmax and ending, warp 4 issues the products, then a warp per half of a slot, which brings one
+// half part after another through the block table (cp.async; first of all each brings a half part of the queries).
+// What bounds it is the issuing warp: a product of 16 values' depth keeps the tensor cores for 48 to 64 clocks and its
+// issue takes 35 (77 from a single lane in a diverged branch, whose operands travel one by one), a wait or a commit
+// about 100; hence the elected lane, the parts of 128 columns and the output products of 128.
+// MEASURED
+// Tokens of several requests in a tile are folded one request after another.
 // Every wait is bounded; one that runs out leaves a code in the status word and the rows unwritten.
 #pragma once
 
@@ -27,18 +31,18 @@
 
 namespace latent_tc {
 
-constexpr int kRows = 128, kKeys = 64, kPart = 64;   // rows, keys of a tile, columns of a part
-constexpr int kPartBytes = kKeys * kPart * 2, kQueryBytes = kRows * kPart * 2;
-constexpr int kScoreSlots = 4, kValueSlots = 6, kSlots = kScoreSlots + kValueSlots;
-constexpr int kMostParts = 9;                        // 512 / 64 and the rotated part
-constexpr int kSoftmaxWarps = 4, kIssuer = 4, kFirstLoader = 5;
-constexpr int kThreads = (kFirstLoader + kSlots) * 32;
+constexpr int kRows = 128, kKeys = 64, kHalf = 64, kPart = 128;   // rows, keys of a tile, columns of a half part and of a part
+constexpr int kHalfBytes = kKeys * kHalf * 2, kQueryBytes = kRows * kHalf * 2;
+constexpr int kScoreSlots = 2, kValueSlots = 3, kSlots = kScoreSlots + kValueSlots;
+constexpr int kMostHalves = 9;                       // 512 / 64 and the rotated part
+constexpr int kSoftmaxWarps = 4, kIssuer = 4, kFirstLoader = 5, kLoaders = 2 * kSlots;
+constexpr int kThreads = (kFirstLoader + kLoaders) * 32;
 constexpr uint32_t kColsO = 0, kColsS = 256, kColsP = 384, kTmemCols = 512;   // O 256, S 2 x 64, P 2 x 32
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMaxSlack = 8.0f;                    // in powers of two
 enum { WAIT_EXPIRED = 5 };
-static_assert(kSlots >= kMostParts, "a loading warp brings at most one part of the queries");
+static_assert(kLoaders >= kMostHalves, "a loading warp brings at most one half part of the queries");
 
 struct Params {
   const float* qa_heads;           // [heads, padded_tokens, rank], unscaled
@@ -56,13 +60,13 @@ struct Params {
 };
 
 struct Shared {
-  uint64_t full[kSlots], empty[kSlots], query[kMostParts], score[2], weight[2], done;
+  uint64_t full[kSlots], empty[kSlots], query[kMostHalves], score[2], weight[2], done;
   uint32_t tmem_base;
   int abort_flag;
   int entry[kRows], position[kRows];   // of the tile's tokens
 };
 
-constexpr int kSharedBytes = kMostParts * kQueryBytes + kSlots * kPartBytes + static_cast<int>(sizeof(Shared)) + 1024;
+constexpr int kSharedBytes = kMostHalves * kQueryBytes + 2 * kSlots * kHalfBytes + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(kSharedBytes <= 227 * 1024, "a block's shared memory");
 
 __device__ __forceinline__ uint32_t addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -93,16 +97,21 @@ __device__ __forceinline__ void copy_piece(uint32_t dst, const void* src, bool v
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Issued by a whole warp that walks the loop together, every lane with the same operands; one elected lane issues.
 __device__ __forceinline__ void commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(addr(bar)) : "memory");
+  asm volatile(
+      "{\n .reg .pred leader;\n elect.sync _|leader, 0xffffffff;\n"
+      " @leader tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(addr(bar)) : "memory");
 }
 __device__ __forceinline__ void mma_shared(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+  asm volatile(
+      "{\n .reg .pred p, leader;\n elect.sync _|leader, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+      " @leader tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void mma_tensor(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+  asm volatile(
+      "{\n .reg .pred p, leader;\n elect.sync _|leader, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+      " @leader tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
 #define LATENT_TC_8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
 __device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&r)[32]) {
@@ -132,13 +141,13 @@ __device__ __forceinline__ float power_of_two(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// 16-byte piece `piece` (0..7) of row `row` of a part, swizzled
+// 16-byte piece `piece` (0..7) of row `row` of a half part, swizzled
 __device__ __forceinline__ uint32_t piece_offset(int row, int piece) { return static_cast<uint32_t>(row * 128 + ((piece ^ (row & 7)) << 4)); }
-// A part as an operand: 128-byte rows, 128-byte swizzle, groups of eight rows 1024 bytes apart.  The same words serve
-// both readings (the contraction along the rows' bytes, or down the rows): within one part of 64 columns the leading
-// offset plays no role.
+// A half part as an operand: 128-byte rows, 128-byte swizzle, groups of eight rows 1024 bytes apart.  The same words
+// serve both readings, the contraction along the rows' bytes or down the rows; in the latter the second 64 of an
+// operand's columns are one half part further (along the rows that word is not used).
 __device__ __forceinline__ uint64_t descriptor(uint32_t saddr) {
-  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(kHalfBytes >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
          (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
 }
 
@@ -163,32 +172,29 @@ __global__ void __launch_bounds__(kThreads, 1)
 latent_fold_tc_kernel(const Params p) {
   extern __shared__ uint8_t latent_tc_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(latent_tc_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* queries = base;                                   // parts of [128 rows][64 columns]
-  uint8_t* slots = base + kMostParts * kQueryBytes;          // parts of [64 keys][64 columns]
-  Shared& s = *reinterpret_cast<Shared*>(slots + kSlots * kPartBytes);
+  uint8_t* queries = base;                                   // half parts of [128 rows][64 columns]
+  uint8_t* slots = base + kMostHalves * kQueryBytes;         // half parts of [64 keys][64 columns], two a slot
+  Shared& s = *reinterpret_cast<Shared*>(slots + 2 * kSlots * kHalfBytes);
   volatile int* abort_flag = &s.abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int latent_parts = p.rank / kPart, slices = (latent_parts + 3) / 4;
+  const int slices = (p.rank + 255) / 256;
   const int tile = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) / slices;   // the longest histories of a prompt first
   const int slice = static_cast<int>(blockIdx.x) % slices;
-  // parts in the order they are read: those only the scores need (the other slices', the rotated one), then this slice's
-  const int value_parts = min(4, latent_parts - 4 * slice), score_parts = latent_parts + 1 - value_parts;
-  auto part_of = [&](int i) {   // the latent's part (latent_parts: the rotated one) that comes i-th
-    if (i >= score_parts) return 4 * slice + i - score_parts;
-    if (i == score_parts - 1) return latent_parts;
-    return i < 4 * slice ? i : i + value_parts;
-  };
-  const int parts = latent_parts + 1;
+  // The columns in the order they are read: those only the scores need (the other slice's), the rotated part, this
+  // slice's.  Counted in half parts: others, then one, then own; in parts: others_parts, one, own_parts.
+  const int own = min(256, p.rank - 256 * slice) / kHalf, others = p.rank / kHalf - own, halves = others + 1 + own;
+  const int others_parts = (others + 1) / 2, own_parts = (own + 1) / 2, score_parts = others_parts + 1;
+  auto column_of = [&](int half) { return half > others ? 256 * slice + (half - others - 1) * kHalf : (slice ? 0 : 256) + half * kHalf; };
   const int total_rows = p.num_tokens * p.heads, row0 = tile * kRows, rows = min(kRows, total_rows - row0);
   const int token0 = row0 / p.heads, tokens = (row0 + rows - 1) / p.heads - token0 + 1;
 
   pdl_launch_dependents();
   if (tid == 0) {
     for (int i = 0; i < kSlots; ++i) {
-      bar_init(&s.full[i], 32);
+      bar_init(&s.full[i], 64);
       bar_init(&s.empty[i], 1);
     }
-    for (int i = 0; i < kMostParts; ++i) bar_init(&s.query[i], 32);
+    for (int i = 0; i < kMostHalves; ++i) bar_init(&s.query[i], 32);
     for (int i = 0; i < 2; ++i) {
       bar_init(&s.score[i], 1);
       bar_init(&s.weight[i], kSoftmaxWarps * 32);
@@ -257,7 +263,7 @@ latent_fold_tc_kernel(const Params p) {
         // (these scores are complete, so the output product of the tile before is)
         if (t > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll 1
-          for (int c = 0; c < value_parts * kPart; c += 32) {
+          for (int c = 0; c < own * kHalf; c += 32) {
             uint32_t o[32];
             tmem_load(lanes + kColsO + c, o);
             tmem_load_wait();
@@ -290,9 +296,9 @@ latent_fold_tc_kernel(const Params p) {
       float total = row_sum;
       if (p.sink) total += exp2f(p.sink[head] * kLog2e - row_max);
       const float inverse = 1.0f / total;
-      __nv_bfloat16* out = p.l_heads + (static_cast<size_t>(head) * p.padded_tokens + token0 + own_token) * p.rank + slice * 4 * kPart;
+      __nv_bfloat16* out = p.l_heads + (static_cast<size_t>(head) * p.padded_tokens + token0 + own_token) * p.rank + slice * 256;
 #pragma unroll 1
-      for (int c = 0; c < value_parts * kPart; c += 32) {
+      for (int c = 0; c < own * kHalf; c += 32) {
         uint32_t o[32];
         tmem_load(lanes + kColsO + c, o);
         tmem_load_wait();
@@ -312,84 +318,104 @@ latent_fold_tc_kernel(const Params p) {
       asm volatile("bar.sync 1, 160;" ::: "memory");   // with the issuer: the next request's products overwrite O
     }
   } else if (warp == kIssuer) {
-    // ---------------- the products, one thread ----------------
-    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kRows >> 4) << 24) | (static_cast<uint32_t>(kKeys >> 3) << 17);
-    constexpr uint32_t kIdescValues = kIdesc | (1u << 16);   // B read down its rows
-    int score_number = 0, value_number = 0, count = 0;       // parts taken from the two rings, tiles issued
+    // ---------------- the products: a warp that walks together, one elected lane issues ----------------
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kRows >> 4) << 24);
+    constexpr uint32_t kIdescScores = kIdesc | (static_cast<uint32_t>(kKeys >> 3) << 17);
+    constexpr uint32_t kIdescValues = kIdesc | (1u << 16) | (static_cast<uint32_t>(kPart >> 3) << 17);       // B read down its rows
+    constexpr uint32_t kIdescHalf = kIdesc | (1u << 16) | (static_cast<uint32_t>(kHalf >> 3) << 17);
+    const uint32_t query_addr = addr(queries), slot_addr = addr(slots);
+    uint32_t score_slot = 0, score_parity = 0, value_slot = 0, value_parity = 0;   // of the next part of either ring
+    int count = 0;                                                                // tiles issued
     const int rot_steps = (p.rot + 15) / 16;
-    const int early = min(score_parts, 4);
-    auto issue_part = [&](int i, int buffer) {   // the i-th part of a tile's scores
-      int slot;
-      uint32_t parity;
-      if (i < score_parts) {
-        slot = score_number % kScoreSlots;
-        parity = (score_number / kScoreSlots) & 1;
-        ++score_number;
-      } else {
-        slot = kScoreSlots + value_number % kValueSlots;
-        parity = (value_number / kValueSlots) & 1;
-        ++value_number;
-      }
-      bar_wait(&s.full[slot], parity, abort_flag, p.status);
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (lane == 0) bar_wait(bar, parity, abort_flag, p.status);
+      __syncwarp();
       fence_after();
-      const uint32_t a = addr(queries + i * kQueryBytes), b = addr(slots + slot * kPartBytes);
-      const int steps = part_of(i) == latent_parts ? rot_steps : 4;
-      for (int ks = 0; ks < steps; ++ks)
-        mma_shared(tmem + kColsS + buffer * kKeys, descriptor(a + ks * 32), descriptor(b + ks * 32), kIdesc, i > 0 || ks > 0 ? 1u : 0u);
-      if (i < score_parts) commit(&s.empty[slot]);
+    };
+    // `steps` products of 16 columns of a half part
+    auto scores_of = [&](int half, uint32_t keys, uint32_t buffer, int steps) {
+      const uint64_t a = descriptor(query_addr + half * kQueryBytes), b = descriptor(keys);
+      const uint32_t d = tmem + kColsS + buffer * kKeys;
+      if (steps == 4) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) mma_shared(d, a + 2 * ks, b + 2 * ks, kIdescScores, half > 0 || ks > 0 ? 1u : 0u);
+      } else {
+        for (int ks = 0; ks < steps; ++ks) mma_shared(d, a + 2 * ks, b + 2 * ks, kIdescScores, half > 0 || ks > 0 ? 1u : 0u);
+      }
+    };
+    auto score_part = [&](int i, uint32_t buffer, bool very_first) {   // a part that only the scores read (the last: the rotated one)
+      const int half = i == score_parts - 1 ? others : 2 * i, more = i < score_parts - 1 && half + 1 < others;
+      if (very_first) {
+        wait(&s.query[half], 0);
+        if (more) wait(&s.query[half + 1], 0);
+      }
+      wait(&s.full[score_slot], score_parity);
+      const uint32_t keys = slot_addr + score_slot * 2 * kHalfBytes;
+      scores_of(half, keys, buffer, i == score_parts - 1 ? rot_steps : 4);
+      if (more) scores_of(half + 1, keys + kHalfBytes, buffer, 4);
+      commit(&s.empty[score_slot]);
+      if (++score_slot == kScoreSlots) score_slot = 0, score_parity ^= 1;
     };
     for (int begin = 0; begin < tokens;) {
       const Segment g = segment_from(s, begin, tokens, p.window);
       begin = g.end;
-      if (lane == 0) {
-        int values_of_last = 0;   // the number of the first value part of the tile before
-        for (int t = 0; t <= g.tiles; ++t) {
-          // scores of tile t, and in their midst the output product of tile t - 1
-          const int number = count + t;
-          const bool very_first = number == 0;   // the queries may still be on their way
-          if (t < g.tiles)
-            for (int i = 0; i < early; ++i) {
-              if (very_first) bar_wait(&s.query[i], 0, abort_flag, p.status);
-              issue_part(i, number & 1);
-            }
-          if (t > 0) {
-            const int before = number - 1;
-            bar_wait(&s.weight[before & 1], (before >> 1) & 1, abort_flag, p.status);
-            fence_after();
-            for (int v = 0; v < value_parts; ++v) {
-              const int slot = kScoreSlots + (values_of_last + v) % kValueSlots;
-              const uint32_t b = addr(slots + slot * kPartBytes);
+      uint32_t values_slot = 0;   // of the first value part of the tile before
+      for (int t = 0; t <= g.tiles; ++t) {
+        // scores of tile t, and in their midst the output product of tile t - 1
+        const int number = count + t;
+        const uint32_t buffer = number & 1;
+        const bool very_first = number == 0;   // the queries may still be on their way
+        if (t < g.tiles) {
+          score_part(0, buffer, very_first);
+          if (score_parts > 2) score_part(1, buffer, very_first);
+        }
+        if (t > 0) {
+          const int before = number - 1;
+          wait(&s.weight[before & 1], (before >> 1) & 1);
+          const uint32_t weights = tmem + kColsP + (before & 1) * (kKeys / 2);
+          uint32_t slot = values_slot;
+          for (int v = 0; v < own_parts; ++v) {
+            const uint64_t b = descriptor(slot_addr + (kScoreSlots + slot) * 2 * kHalfBytes);
+            const uint32_t idesc = 2 * v + 1 < own ? kIdescValues : kIdescHalf;
 #pragma unroll
-              for (int ks = 0; ks < kKeys / 16; ++ks)
-                mma_tensor(tmem + kColsO + v * kPart, tmem + kColsP + (before & 1) * (kKeys / 2) + ks * 8, descriptor(b + ks * 2048),
-                           kIdescValues, t > 1 || ks > 0 ? 1u : 0u);
-              commit(&s.empty[slot]);
-            }
-            if (t == g.tiles) commit(&s.done);
+            for (int ks = 0; ks < kKeys / 16; ++ks)
+              mma_tensor(tmem + kColsO + v * kPart, weights + ks * 8, b + ks * (2048 >> 4), idesc, t > 1 || ks > 0 ? 1u : 0u);
+            commit(&s.empty[kScoreSlots + slot]);
+            if (++slot == kValueSlots) slot = 0;
           }
-          if (t < g.tiles) {
-            values_of_last = value_number;
-            for (int i = early; i < parts; ++i) {
-              if (very_first) bar_wait(&s.query[i], 0, abort_flag, p.status);
-              issue_part(i, number & 1);
+          if (t == g.tiles) commit(&s.done);
+        }
+        if (t < g.tiles) {
+          for (int i = score_parts > 2 ? 2 : 1; i < score_parts; ++i) score_part(i, buffer, very_first);
+          values_slot = value_slot;
+          for (int v = 0; v < own_parts; ++v) {
+            const int half = others + 1 + 2 * v;
+            const bool more = 2 * v + 1 < own;
+            if (very_first) {
+              wait(&s.query[half], 0);
+              if (more) wait(&s.query[half + 1], 0);
             }
-            commit(&s.score[number & 1]);
+            wait(&s.full[kScoreSlots + value_slot], value_parity);
+            const uint32_t keys = slot_addr + (kScoreSlots + value_slot) * 2 * kHalfBytes;
+            scores_of(half, keys, buffer, 4);
+            if (more) scores_of(half + 1, keys + kHalfBytes, buffer, 4);
+            if (++value_slot == kValueSlots) value_slot = 0, value_parity ^= 1;
           }
+          commit(&s.score[buffer]);
         }
       }
       count += g.tiles;
-      __syncwarp();
       fence_before();
       asm volatile("bar.sync 1, 160;" ::: "memory");
       fence_after();
     }
   } else {
-    // ---------------- a warp per slot: the parts that come to it, one after another ----------------
-    const int slot = warp - kFirstLoader;
+    // ---------------- a warp per half of a slot: the half parts that come to it, one after another ----------------
+    const int loader = warp - kFirstLoader, slot = loader >> 1, second = loader & 1;
     const bool of_values = slot >= kScoreSlots;
-    const int ring = of_values ? kValueSlots : kScoreSlots, each = of_values ? value_parts : score_parts;   // slots, parts a tile
+    const int ring = of_values ? kValueSlots : kScoreSlots, each = of_values ? own_parts : score_parts;   // slots, parts a tile
     const int piece = lane & 7, sub = lane >> 3;
-    const uint32_t dst = addr(slots + slot * kPartBytes);
+    const uint32_t dst = addr(slots + loader * kHalfBytes);
     int number = of_values ? slot - kScoreSlots : slot, round = 0, count = 0;   // of the part, of the slot's use; tiles before this request
     // where keys lane and lane + 32 of a tile lie in the pools, -1: nowhere (zeros)
     int place_lo = -1, place_hi = -1;
@@ -406,12 +432,15 @@ latent_fold_tc_kernel(const Params p) {
         if (page >= 0) place_hi = page * p.page_size + hi % p.page_size;
       }
     };
-    auto copy = [&](int i) {   // the i-th part of a tile
-      const int part = part_of(i);
-      const bool latent = part < latent_parts;
-      const __nv_bfloat16* pool = latent ? p.k_pool + part * kPart + piece * 8 : p.v_pool + piece * 8;
-      const int stride = latent ? p.rank : p.rot;
-      const bool column = latent || piece * 8 < p.rot;
+    auto copy = [&](int i) {   // this warp's half of the i-th part of its ring's in a tile
+      const bool rotated = !of_values && i == score_parts - 1;
+      const int half = rotated ? others : (of_values ? others + 1 : 0) + 2 * i + second;
+      // (a part may have one half only; the rotated one does)
+      const bool there = rotated ? second == 0 : 2 * i + second < (of_values ? own : others);
+      if (!there) return;
+      const __nv_bfloat16* pool = (rotated ? p.v_pool : p.k_pool + column_of(half)) + piece * 8;
+      const int stride = rotated ? p.rot : p.rank;
+      const bool column = !rotated || piece * 8 < p.rot;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int r = sub + 4 * j;   // (rows 32 and on from j = 8 on)
@@ -421,11 +450,12 @@ latent_fold_tc_kernel(const Params p) {
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    bool queries_due = slot < parts;
-    auto bring_queries = [&]() {   // part `slot` of the queries, sixteen rows of it at a time
+    bool queries_due = loader < halves;
+    auto bring_queries = [&]() {   // half part `loader` of the queries, 32 rows of it at a time
       queries_due = false;
-      const int part = part_of(slot);
-      const float f = part < latent_parts ? p.scale : 1.0f;
+      const bool rotated = loader == others;
+      const float f = rotated ? 1.0f : p.scale;
+      const int column = rotated ? 0 : column_of(loader);
       const int c = piece * 8;
 #pragma unroll 1
       for (int r0 = 0; r0 < kRows; r0 += 32) {
@@ -434,10 +464,9 @@ latent_fold_tc_kernel(const Params p) {
         for (int j = 0; j < 8; ++j) {
           const int r = r0 + sub + 4 * j, global = row0 + r;
           lo[j] = hi[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (r < rows && (part < latent_parts || c < p.rot)) {
-            const float* src = part < latent_parts
-                ? p.qa_heads + (static_cast<size_t>(global % p.heads) * p.padded_tokens + global / p.heads) * p.rank + part * kPart + c
-                : p.q_rot + static_cast<size_t>(global) * p.rot + c;
+          if (r < rows && (!rotated || c < p.rot)) {
+            const float* src = rotated ? p.q_rot + static_cast<size_t>(global) * p.rot + c
+                : p.qa_heads + (static_cast<size_t>(global % p.heads) * p.padded_tokens + global / p.heads) * p.rank + column + c;
             lo[j] = *reinterpret_cast<const float4*>(src);
             hi[j] = *reinterpret_cast<const float4*>(src + 4);
           }
@@ -450,11 +479,11 @@ latent_fold_tc_kernel(const Params p) {
           pairs[1] = __floats2bfloat162_rn(lo[j].z * f, lo[j].w * f);
           pairs[2] = __floats2bfloat162_rn(hi[j].x * f, hi[j].y * f);
           pairs[3] = __floats2bfloat162_rn(hi[j].z * f, hi[j].w * f);
-          *reinterpret_cast<uint4*>(queries + slot * kQueryBytes + piece_offset(r0 + sub + 4 * j, piece)) = packed;
+          *reinterpret_cast<uint4*>(queries + loader * kQueryBytes + piece_offset(r0 + sub + 4 * j, piece)) = packed;
         }
       }
       fence_async();
-      bar_arrive(&s.query[slot]);
+      bar_arrive(&s.query[loader]);
     };
     bool waited = false;
     for (int begin = 0; begin < tokens;) {
@@ -467,7 +496,7 @@ latent_fold_tc_kernel(const Params p) {
       }
       for (; number < (count + g.tiles) * each; number += ring, ++round) {
         if (round > 0) bar_wait(&s.empty[slot], (round - 1) & 1, abort_flag, p.status);
-        copy((of_values ? score_parts : 0) + number % each);
+        copy(number % each);
         if (number + ring < (count + g.tiles) * each) look_up(g, (number + ring) / each - count);
         if (queries_due) bring_queries();
         asm volatile("cp.async.wait_group 0;" ::: "memory");
