@@ -143,12 +143,12 @@ __device__ __forceinline__ float power_of_two(float x) {
 }
 // 16-byte piece `piece` (0..7) of row `row` of a half part, swizzled
 __device__ __forceinline__ uint32_t piece_offset(int row, int piece) { return static_cast<uint32_t>(row * 128 + ((piece ^ (row & 7)) << 4)); }
-// A half part as an operand: 128-byte rows, 128-byte swizzle, groups of eight rows 1024 bytes apart.  The same words
-// serve both readings, the contraction along the rows' bytes or down the rows; in the latter the second 64 of an
-// operand's columns are one half part further (along the rows that word is not used).
-__device__ __forceinline__ uint64_t descriptor(uint32_t saddr) {
-  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(kHalfBytes >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
-         (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
+// A half part as an operand: 128-byte rows, 128-byte swizzle, groups of eight rows 1024 bytes apart, read with the
+// contraction along the rows' bytes or (`down`) down the rows; in the latter the second 64 of an operand's columns are
+// one half part further.
+__device__ __forceinline__ uint64_t descriptor(uint32_t saddr, bool down) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(down ? kHalfBytes >> 4 : 1) << 16) |
+         (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
 }
 
 // One request's tokens that follow one another in the tile, and the keys any of them sees.
@@ -334,7 +334,7 @@ latent_fold_tc_kernel(const Params p) {
     };
     // `steps` products of 16 columns of a half part
     auto scores_of = [&](int half, uint32_t keys, uint32_t buffer, int steps) {
-      const uint64_t a = descriptor(query_addr + half * kQueryBytes), b = descriptor(keys);
+      const uint64_t a = descriptor(query_addr + half * kQueryBytes, false), b = descriptor(keys, false);
       const uint32_t d = tmem + kColsS + buffer * kKeys;
       if (steps == 4) {
 #pragma unroll
@@ -375,7 +375,7 @@ latent_fold_tc_kernel(const Params p) {
           const uint32_t weights = tmem + kColsP + (before & 1) * (kKeys / 2);
           uint32_t slot = values_slot;
           for (int v = 0; v < own_parts; ++v) {
-            const uint64_t b = descriptor(slot_addr + (kScoreSlots + slot) * 2 * kHalfBytes);
+            const uint64_t b = descriptor(slot_addr + (kScoreSlots + slot) * 2 * kHalfBytes, true);
             const uint32_t idesc = 2 * v + 1 < own ? kIdescValues : kIdescHalf;
 #pragma unroll
             for (int ks = 0; ks < kKeys / 16; ++ks)
