@@ -34,11 +34,53 @@ def test_product_tiles_and_slabs(m, n, k, types):
     ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, bias=bias, out=out)
     # the error of a chain of k roundings of random sign, 2^-24 each, is some sqrt(k) 2^-24 of the sum at most
     assert _rel(out, a.double() @ w.double().T + bias.double()) < 2.0 ** -24 * (k ** 0.5 + 4)
-    # a row's result does not depend on the rows beside it, within its class (up to eight rows, or more)
+    # a row's result does not depend on the rows beside it, within its class (up to eight rows, up to 64; with more the
+    # blocks that share an inner size depend on the count of tiles)
+    if m > 64:
+        return
     beside = 1 if m <= 8 else 9
     last = torch.empty(beside, n, device=DEV)
     ops.gemm_simt(a[-beside:].contiguous(), w, epilogue=ops.EPI_STORE, bias=bias, out=last)
     assert torch.equal(last[-1], out[-1])
+
+
+# the tensor-core form of many rows: tiles that end inside, one block and clusters of two and four that share K (one
+# share may be empty), all endings, numbers of very different sizes, and numbers that have no parts
+@pytest.mark.parametrize("m,n,k", [(65, 32, 4), (128, 128, 64), (129, 160, 68), (200, 96, 700), (300, 1152, 896), (1024, 896, 4864), (70, 5024, 300)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_product_in_parts(m, n, k, epilogue):
+    ops = _ops()
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device=DEV) * torch.exp(4 * torch.randn(m, 1, device=DEV))
+    w, bias = torch.randn(n, k, device=DEV), torch.randn(n, device=DEV)
+    y = a.double() @ w.double().T + bias.double()
+    if epilogue == 2:
+        a = a / a.norm(dim=1, keepdim=True)
+        y = a.double() @ w.double().T + bias.double()
+        gate, up = y.view(m, n // 32, 2, 16)[:, :, 0], y.view(m, n // 32, 2, 16)[:, :, 1]
+        y = (up * gate * torch.sigmoid(gate)).reshape(m, n // 2)
+    out = torch.randn(m, y.shape[1], device=DEV)
+    want = y + out.double() if epilogue == 1 else y
+    ops.gemm_simt(a, w, epilogue=epilogue, bias=bias, **({"resid": out} if epilogue == 1 else {"out": out}))
+    torch.cuda.synchronize()
+    ops.check_kernel_status(a.device)
+    # no worse than a chain of k roundings of 2^-24, row by row
+    error = (out.double() - want).norm(dim=1) / want.norm(dim=1)
+    assert float(error.max()) < 2.0 ** -24 * (k ** 0.5 + 6)
+
+
+def test_product_in_parts_without_parts():
+    ops = _ops()
+    a, w = torch.randn(140, 256, device=DEV), torch.randn(130, 256, device=DEV)
+    a[3, 7], a[5, 9], a[137, 200], w[129, 255] = float("inf"), float("nan"), float("-inf"), float("inf")
+    w[4, 7] = 0.0
+    out = torch.empty(140, 130, device=DEV)
+    ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, out=out)
+    want = a.double() @ w.double().T
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+    fine = torch.isfinite(want)
+    assert torch.equal(out[~fine & ~torch.isnan(want)].sign(), want[~fine & ~torch.isnan(want)].float().sign())
+    assert float((out.double() - want)[fine].norm() / want[fine].norm()) < 2.0 ** -20
 
 
 def _attention_want(q, keys, values, entry, position, heads, kv_heads, scale, mask, sink, chunk, window, keep_first, gate):

@@ -31,7 +31,7 @@
 //             out[m, f] = (up + bias) * act(gate + bias), act = silu, silu(z) = z/(1+exp(-z))
 //             (model.rs:4368-4374), or the tanh form of gelu,
 //             0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))
-#include "simt.cuh"
+#include "gemm_split.cuh"
 
 enum GemmEpilogue { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU = 2 };
 
@@ -62,6 +62,7 @@ struct GemmArgs {
   float* resid;
   int activation, epilogue, out_bf16;
   int wide;            // rows of whole pieces of eight values on 16-byte boundaries
+  int* status;         // for the bounded waits of the tensor-core form, or null: it is not used
 };
 
 __device__ __forceinline__ void load_eight(const float* src, float (&v)[8]) {
@@ -437,6 +438,9 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
       if (p.M <= kFewRows) return launch_few(p, s);
       if (p.M <= TileSome::BM) return launch_tile<TA, TW, TileSome, true>(p, s);
       if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileMid, true>(p, s);
+      if (p.status)   // more rows than a half tile: three parts of every number on the tensor cores
+        return gemm_split::launch({static_cast<const float*>(p.A), static_cast<const float*>(p.W), p.M, p.N, p.K, 1, 0, p.bias, p.out,
+                                   p.resid, p.activation, p.epilogue, p.out_bf16, p.status}, s);
       return launch_tile<TA, TW, TileMany, true>(p, s);
     }
   }
@@ -447,30 +451,30 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
 
 template <typename TA, typename TW>
 static int launch_typed(const TA* A, const TW* W, int M, int N, int K, int epilogue, const float* bias,
-                        void* out, int out_dtype, float* resid, int activation, cudaStream_t s) {
+                        void* out, int out_dtype, float* resid, int activation, int* status, cudaStream_t s) {
   const int slab = ((K + kSlabs - 1) / kSlabs + kChunk - 1) / kChunk * kChunk;
   if (epilogue != EPI_STORE && epilogue != EPI_RESIDUAL && epilogue != EPI_SWIGLU) return VIPERA_BAD_ARGUMENT;
   if (epilogue == EPI_RESIDUAL ? !resid : !out) return VIPERA_BAD_ARGUMENT;
   if (epilogue == EPI_SWIGLU && N % 32 != 0) return VIPERA_BAD_SHAPE;  // gate/up groups of 16 must pair up
   if (epilogue != EPI_RESIDUAL && out_dtype != VIPERA_F32 && out_dtype != VIPERA_BF16) return VIPERA_BAD_DTYPE;
   const int wide = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
-  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16, wide};
+  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16, wide, status};
   return launch_sizes<TA, TW>(p, s);
 }
 
 // A is [M, K] and W is [N, K], both row-major and contiguous.  For SWIGLU, N counts the
 // interleaved gate and up rows (twice the intermediate size) and out is [M, N/2].
 static int run_simt(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K, int epilogue,
-                    const float* bias, void* out, int out_dtype, float* resid, int activation, void* stream) {
+                    const float* bias, void* out, int out_dtype, float* resid, int activation, int* status, void* stream) {
   if (M <= 0) return VIPERA_OK;
   if (N <= 0 || K <= 0) return VIPERA_BAD_SHAPE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a_dtype == VIPERA_F32 && w_dtype == VIPERA_F32)
-    return launch_typed(static_cast<const float*>(A), static_cast<const float*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, s);
+    return launch_typed(static_cast<const float*>(A), static_cast<const float*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, s);
   if (a_dtype == VIPERA_BF16 && w_dtype == VIPERA_BF16)
-    return launch_typed(static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, s);
+    return launch_typed(static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, s);
   if (a_dtype == VIPERA_F32 && w_dtype == VIPERA_BF16)
-    return launch_typed(static_cast<const float*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, s);
+    return launch_typed(static_cast<const float*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, s);
   return VIPERA_BAD_DTYPE;
 }
 
@@ -479,7 +483,7 @@ VIPERA_API int vipera_gemm_simt(const void* A, int a_dtype, const void* W, int w
                                 void* stream) {
   // the form the earlier callers know: bias with STORE only, silu in the gated unit
   return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, epilogue == EPI_STORE ? bias : nullptr, out, out_dtype,
-                  resid, ACT_SILU, stream);
+                  resid, ACT_SILU, nullptr, stream);
 }
 
 // The same with a bias in every ending and the gated unit's activation chosen (ACT_SILU, ACT_GELU_TANH).
@@ -487,7 +491,16 @@ VIPERA_API int vipera_gemm_simt_act(const void* A, int a_dtype, const void* W, i
                                     int epilogue, const float* bias, void* out, int out_dtype, float* resid,
                                     int activation, void* stream) {
   if (activation != ACT_SILU && activation != ACT_GELU_TANH) return VIPERA_BAD_ARGUMENT;
-  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, stream);
+  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, nullptr, stream);
+}
+
+// The same with a device word that must be 0 before the launch and is not afterwards where a bounded wait ran out: 32-bit
+// products of many rows may then run on the tensor cores, three parts of every number.
+VIPERA_API int vipera_gemm_simt_status(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
+                                       int epilogue, const float* bias, void* out, int out_dtype, float* resid,
+                                       int activation, int* status, void* stream) {
+  if (activation != ACT_SILU && activation != ACT_GELU_TANH) return VIPERA_BAD_ARGUMENT;
+  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, stream);
 }
 
 VIPERA_API const char* vipera_gemm_simt_status_text(int status) { return vipera_status_text(status); }

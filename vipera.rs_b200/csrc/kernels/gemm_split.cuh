@@ -1,0 +1,314 @@
+// 32-bit matrix products of many rows on the fifth-generation tensor cores: out[M, N] = A[M, K] . W[N, K]^T with A, W
+// and the sums in 32 bits.
+//
+// A 32-bit number is the exact sum of three bfloat16 numbers (its leading 8 bits, the next 8, the last 8, by
+// truncation), and a product of two bfloat16 numbers is exact in 32 bits.  So a . w is a1 w1 + (a1 w2 + a2 w1 + a2 w2
+// + a1 w3 + a3 w1) up to terms of 2^-24 of |a w| and below, six products in place of one.  The tensor cores round
+// every step of their sums towards zero, which over a long K would cost more than 32-bit multiply-adds do: so the
+// leading product and the five small ones have accumulators of their own, both are read after every 64 values of K
+// and added to the tile's sums in registers, rounded to nearest.  Against 64 bits the result is closer than a chain of
+// fused multiply-adds over K (MEASUREDERR).  An infinity or a NaN has no such parts (its products with their zeros
+// would be NaN): a block that meets one computes its tile with multiply-adds instead.
+//
+// A block computes a tile of 128 x 128: eight warps read 64 values of K of both operands, split them and leave the
+// parts in shared memory (three images of 128 rows each, 128-byte swizzle, two stages of 96 KB); eight warps add up, the
+// first of which issues 24 products of 16 values a stage (a warp of its own for that would leave too few registers).  Two pairs of accumulators fill tensor memory.  Where the tiles
+// are too few to fill the chip, the blocks of a cluster share K and add their parts through distributed shared memory.
+// What bounds it: 24 products of 64 clocks a stage, whose operands' reads alone keep shared memory busy as long; the
+// split writes 96 KB more.  MEASURED
+#pragma once
+
+#include "simt.cuh"
+
+namespace gemm_split {
+
+constexpr int kTile = 128, kDepth = 64, kStages = 2, kParts = 3;
+constexpr int kImageBytes = kTile * kDepth * 2, kStageBytes = 2 * kParts * kImageBytes;
+constexpr int kSumWarps = 8, kIssuer = 0, kFirstSplitter = 8, kSplitters = 256;   // (the first of the adding warps issues)
+constexpr int kThreads = (kFirstSplitter + 8) * 32;
+constexpr int kSumPitch = kTile + 4;
+constexpr uint32_t kWaitLimit = 1u << 22;
+enum { WAIT_EXPIRED = 6 };
+
+struct Args {
+  const float* A;
+  const float* W;
+  int M, N, K, cluster, share;   // share: stages of K a block of the cluster takes
+  const float* bias;
+  void* out;
+  float* resid;
+  int activation, epilogue, out_bf16;
+  int* status;
+};
+
+struct Shared {
+  uint64_t full[kStages], empty[kStages], sums_full[2], sums_empty[2];
+  uint32_t tmem_base;
+  int abort_flag, not_finite;
+};
+constexpr int kSharedBytes = kStages * kStageBytes + static_cast<int>(sizeof(Shared)) + 1024;
+static_assert(kTile * kSumPitch * 4 <= kStages * kStageBytes, "the tile's sums take the stages' place");
+
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_address(bar)), "r"(count));
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(shared_address(bar)) : "memory");
+}
+__device__ __forceinline__ void bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(shared_address(bar)), "r"(parity) : "memory");
+    if (done) return;
+    if (spin > 8) __nanosleep(32);
+    if ((spin & 1023u) == 1023u && *abort_flag) return;
+  }
+  *abort_flag = 1;
+  atomicExch(status, WAIT_EXPIRED);
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Issued by a whole warp that walks together, one elected lane issues.
+__device__ __forceinline__ void commit(uint64_t* bar) {
+  asm volatile(
+      "{\n .reg .pred leader;\n elect.sync _|leader, 0xffffffff;\n"
+      " @leader tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(shared_address(bar)) : "memory");
+}
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p, leader;\n elect.sync _|leader, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+      " @leader tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+#define GEMM_SPLIT_8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
+__device__ __forceinline__ void tmem_load_16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : GEMM_SPLIT_8(r, 0), GEMM_SPLIT_8(r, 8) : "r"(taddr));
+}
+#undef GEMM_SPLIT_8
+// An image as an operand: rows of 64 values (128 bytes, 128-byte swizzle), groups of eight rows 1024 bytes apart, the
+// contraction along the rows.
+__device__ __forceinline__ uint64_t descriptor(uint32_t saddr) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+         (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
+}
+__device__ __forceinline__ float leading(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+// the upper halves of two 32-bit words, `lo`'s in the lower one
+__device__ __forceinline__ uint32_t uppers(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_split_kernel(const Args p) {
+  extern __shared__ uint8_t split_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(split_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  Shared& s = *reinterpret_cast<Shared*>(stages + kStages * kStageBytes);
+  float* sums = reinterpret_cast<float*>(stages);   // [128][kSumPitch], once the stages are read out
+  volatile int* abort_flag = &s.abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = blockIdx.x % p.cluster, n0 = blockIdx.x / p.cluster * kTile, m0 = blockIdx.y * kTile;
+  const int k_begin = min(rank * p.share * kDepth, p.K), k_end = min(k_begin + p.share * kDepth, p.K);
+  const int count = (k_end - k_begin + kDepth - 1) / kDepth;
+  pdl_launch_dependents();
+  if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      bar_init(&s.full[i], kSplitters);
+      bar_init(&s.empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      bar_init(&s.sums_full[i], 1);
+      bar_init(&s.sums_empty[i], kSumWarps * 32);
+    }
+    s.abort_flag = s.not_finite = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kIssuer) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(shared_address(&s.tmem_base)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = s.tmem_base;
+
+  if (warp < kSumWarps) {
+    // ---------------- sums: a row and 64 columns a thread; the first warp issues the products ----------------
+    const int row = (warp & 3) * 32 + lane, column0 = (warp >> 2) * 64;
+    const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + column0;
+    float total[64];
+#pragma unroll
+    for (int j = 0; j < 64; ++j) total[j] = 0.0f;
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTile >> 4) << 24) | (static_cast<uint32_t>(kTile >> 3) << 17);
+    const uint32_t base = shared_address(stages);
+    auto products = [&](int c) {
+      const uint32_t stage = c & 1, parity = (c >> 1) & 1;
+      if (lane == 0) {
+        if (c >= 2) bar_wait(&s.sums_empty[stage], parity ^ 1u, abort_flag, p.status);
+        bar_wait(&s.full[stage], parity, abort_flag, p.status);
+      }
+      __syncwarp();
+      fence_after();
+      const uint64_t a = descriptor(base + stage * kStageBytes), w = descriptor(base + stage * kStageBytes + kParts * kImageBytes);
+      constexpr uint64_t kNext = kImageBytes >> 4;   // the next part's image
+      const uint32_t large = tmem + stage * 256, small = large + 128;
+#pragma unroll
+      for (int ks = 0; ks < kDepth / 16; ++ks) {
+        const uint64_t x = a + 2 * ks, y = w + 2 * ks;
+        mma(small, x + 2 * kNext, y, kIdesc, ks > 0 ? 1u : 0u);
+        mma(small, x, y + 2 * kNext, kIdesc, 1u);
+        mma(small, x + kNext, y + kNext, kIdesc, 1u);
+        mma(small, x + kNext, y, kIdesc, 1u);
+        mma(small, x, y + kNext, kIdesc, 1u);
+        mma(large, x, y, kIdesc, ks > 0 ? 1u : 0u);
+      }
+      commit(&s.empty[stage]);
+      commit(&s.sums_full[stage]);
+    };
+    if (warp == kIssuer && count > 0) products(0);
+    for (int c = 0; c < count; ++c) {
+      if (warp == kIssuer && c + 1 < count) products(c + 1);   // (on their way while this warp adds)
+      const uint32_t pair = taddr + (c & 1) * 256;
+      bar_wait(&s.sums_full[c & 1], (c >> 1) & 1, abort_flag, p.status);
+      fence_after();
+#pragma unroll
+      for (int j = 0; j < 64; j += 16) {
+        uint32_t large[16], small[16];
+        tmem_load_16(pair + j, large);
+        tmem_load_16(pair + 128 + j, small);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 16; ++e) total[j + e] = (total[j + e] + __uint_as_float(small[e])) + __uint_as_float(large[e]);
+      }
+      fence_before();
+      bar_arrive(&s.sums_empty[c & 1]);
+    }
+    // (the last sums are complete, so every product that read the stages is)
+#pragma unroll
+    for (int j = 0; j < 64; j += 4)
+      *reinterpret_cast<float4*>(sums + row * kSumPitch + column0 + j) = make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]);
+  } else {
+    // ---------------- operands: eight runs of eight values a thread and stage, four of either operand ----------------
+    const int t = tid - kFirstSplitter * 32, piece = t & 7, sub = t >> 3;   // rows sub + 32 i
+    float4 lo[8], hi[8];
+    auto ask = [&](int i, int c) {
+      const bool of_a = i < 4;
+      const int r = sub + 32 * (i & 3), k = k_begin + c * kDepth + piece * 8;
+      const int row = (of_a ? m0 : n0) + r, extent = of_a ? p.M : p.N;
+      const float* src = (of_a ? p.A : p.W) + (row < extent ? static_cast<size_t>(row) * p.K + k : 0);
+      // (K is a multiple of four: each half of the run lies within it or not)
+      lo[i] = c < count && row < extent && k < k_end ? *reinterpret_cast<const float4*>(src) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      hi[i] = c < count && row < extent && k + 4 < k_end ? *reinterpret_cast<const float4*>(src + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    // the weights of the first stage are asked for before the kernel ahead has ended
+#pragma unroll
+    for (int i = 4; i < 8; ++i) ask(i, 0);
+    pdl_wait();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ask(i, 0);
+    bool odd = false;   // something that is not finite
+    for (int c = 0; c < count; ++c) {
+      const int stage = c & 1;
+      if (c >= 2) bar_wait(&s.empty[stage], ((c >> 1) & 1) ^ 1, abort_flag, p.status);
+      uint8_t* dst = stages + stage * kStageBytes;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float v[8] = {lo[i].x, lo[i].y, lo[i].z, lo[i].w, hi[i].x, hi[i].y, hi[i].z, hi[i].w};
+        uint32_t first[4], second[4], third[4];
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          const float r0 = v[e] - leading(v[e]), r1 = v[e + 1] - leading(v[e + 1]);
+          first[e >> 1] = uppers(v[e], v[e + 1]);
+          second[e >> 1] = uppers(r0, r1);
+          third[e >> 1] = uppers(r0 - leading(r0), r1 - leading(r1));
+          odd |= !(fabsf(v[e]) <= 3.402823466e38f) || !(fabsf(v[e + 1]) <= 3.402823466e38f);
+        }
+        if (c + 1 < count) ask(i, c + 1);   // the next stage's run takes this one's registers
+        const int r = sub + 32 * (i & 3);
+        uint8_t* at = dst + (i < 4 ? 0 : kParts * kImageBytes) + r * 128 + ((piece ^ (r & 7)) << 4);
+        *reinterpret_cast<uint4*>(at) = make_uint4(first[0], first[1], first[2], first[3]);
+        *reinterpret_cast<uint4*>(at + kImageBytes) = make_uint4(second[0], second[1], second[2], second[3]);
+        *reinterpret_cast<uint4*>(at + 2 * kImageBytes) = make_uint4(third[0], third[1], third[2], third[3]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      bar_arrive(&s.full[stage]);
+    }
+    if (odd) s.not_finite = 1;
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == kIssuer) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+  pdl_wait();   // (every thread may read A or the residual stream from here on)
+  if (s.not_finite) {
+    for (int i = tid; i < kTile * kTile; i += kThreads) {
+      const int m = i / kTile, n = i % kTile;
+      float sum = 0.0f;
+      if (m0 + m < p.M && n0 + n < p.N)
+        for (int k = k_begin; k < k_end; ++k) sum = fmaf(p.A[static_cast<size_t>(m0 + m) * p.K + k], p.W[static_cast<size_t>(n0 + n) * p.K + k], sum);
+      sums[m * kSumPitch + n] = sum;
+    }
+    __syncthreads();
+  }
+  if (p.cluster > 1) cluster_sync();
+
+  // The ending.  In a cluster each block finishes every cluster-th row of the tile.  A thread keeps one column.
+  auto total = [&](int m, int n) {
+    float* own = sums + m * kSumPitch + n;
+    if (p.cluster == 1) return *own;
+    const uint32_t at = shared_address(own);
+    float sum = remote_float(at, 0);
+    for (int r = 1; r < p.cluster; ++r) sum += remote_float(at, r);
+    return sum;
+  };
+  const bool gated = p.epilogue == 2;
+  const int columns = gated ? kTile / 2 : kTile, column_bits = gated ? 6 : 7, row_step = 512 >> column_bits;
+  const int c = tid & (columns - 1), n = gated ? (c / 16) * 32 + c % 16 : c;   // gated: the gate's column; the up value is 16 further
+  if (tid < 512 && n0 + n + (gated ? 16 : 0) < p.N && !*abort_flag) {
+    const float bias = p.bias ? p.bias[n0 + n] : 0.0f, up_bias = p.bias && gated ? p.bias[n0 + n + 16] : 0.0f;
+    const int pitch = gated ? p.N / 2 : p.N, column = gated ? n0 / 2 + c : n0 + c;
+    for (int row = tid >> column_bits; row < kTile / p.cluster; row += 4 * row_step) {
+      float value[4], before[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = (row + i * row_step) * p.cluster + rank;
+        if (m >= kTile || m0 + m >= p.M) continue;
+        if (p.epilogue == 1) before[i] = p.resid[static_cast<size_t>(m0 + m) * pitch + column];
+        value[i] = total(m, n) + bias;
+        if (gated) value[i] = (total(m, n + 16) + up_bias) * gate_activation(value[i], p.activation);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = (row + i * row_step) * p.cluster + rank;
+        if (m >= kTile || m0 + m >= p.M) continue;
+        const size_t at = static_cast<size_t>(m0 + m) * pitch + column;
+        if (p.epilogue == 1) p.resid[at] = before[i] + value[i];
+        else if (p.out_bf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value[i]);
+        else static_cast<float*>(p.out)[at] = value[i];
+      }
+    }
+  }
+  if (p.cluster > 1) cluster_sync();   // no block leaves while another reads its part
+}
+
+// Blocks of a cluster share K where that leaves fewer stages in a row: (waves of blocks) x (stages of a block + what it
+// costs besides).
+static int launch(const Args& args, cudaStream_t s) {
+  static SharedMemoryOptIn opt_in;
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(gemm_split_kernel), kSharedBytes);
+  if (opted) return opted;
+  constexpr long long kSms = 148;
+  Args p = args;
+  const long long tiles_n = (p.N + kTile - 1) / kTile, tiles_m = (p.M + kTile - 1) / kTile, depth = (p.K + kDepth - 1) / kDepth;
+  if (tiles_m > 65535) return VIPERA_BAD_SHAPE;
+  long long best = 0;
+  for (int cluster = 1; cluster <= 4; cluster *= 2) {
+    const long long share = (depth + cluster - 1) / cluster;
+    const long long cost = (tiles_n * tiles_m * cluster + kSms - 1) / kSms * (share + 4);
+    if (cluster == 1 || cost < best) best = cost, p.cluster = cluster, p.share = static_cast<int>(share);
+  }
+  return launch_in_clusters(gemm_split_kernel, p.cluster, dim3(static_cast<unsigned>(tiles_n * p.cluster), static_cast<unsigned>(tiles_m)),
+                            dim3(kThreads), kSharedBytes, s, p);
+}
+
+}  // namespace gemm_split

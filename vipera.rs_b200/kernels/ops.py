@@ -468,18 +468,19 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE,
     """a[M, K] times w[N, K] transposed, on the CUDA cores with float32 accumulation.  ``bias``
     counts in every ending (for the gated unit it is interleaved like the rows);
     ``activation`` is the gated unit's."""
-    fn = _function("gemm_simt", "vipera_gemm_simt_act",
+    fn = _function("gemm_simt", "vipera_gemm_simt_status",
                    [_c_void, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_int,
-                    _c_void, _c_int, _c_void])
+                    _c_void, _c_int, _c_void, _c_void])
     m, k = a.shape
     n = w.shape[0]
     if w.shape[1] != k:
         raise InvalidArgumentError(f"gemm: inner sizes differ ({k} and {w.shape[1]})")
     _check_gemm_outputs(m, n, epilogue, bias, out, resid)
-    _check(fn(_gpu(a, "a"), dtype_code(a.dtype), _gpu(w, "w"), dtype_code(w.dtype), m, n, k, epilogue,
+    pointer = _gpu(a, "a")
+    _check(fn(pointer, dtype_code(a.dtype), _gpu(w, "w"), dtype_code(w.dtype), m, n, k, epilogue,
               _opt(bias, "bias", torch.float32), _opt(out, "out"),
               dtype_code(out.dtype) if out is not None else F32, _opt(resid, "resid", torch.float32),
-              int(activation), _stream()), "gemm_simt")
+              int(activation), _tc_buffers(a.device, 0)["status"].data_ptr(), _stream()), "gemm_simt")
 
 
 def _check_gemm_outputs(m, n, epilogue, bias, out, resid) -> None:
