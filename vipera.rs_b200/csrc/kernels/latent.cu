@@ -919,6 +919,7 @@ struct LatentParams {
   void* cq;                      // [tokens, q_rank], the run's type
   int single;              // 1: every request of the step brings one token
   int* status;             // receives a code where a bounded wait ran out, or null: the fold stays with mma.sync
+  int max_keys;            // at least the longest history of the step (0: not known)
 };
 
 // How the tensor-core fold cuts a step.  Rows are tokens x heads.  Many rows: two groups of sixteen to a
@@ -987,13 +988,18 @@ static int launch_fold(const LatentFoldParams& f, dim3 grid, size_t shared, cuda
   return vipera_launch(latent_fold_kernel<NR, MT>, grid, kFoldThreads, shared, s, f);
 }
 
-// Rows from which the tcgen05 fold runs a step in the head-major form.  RULE
+// The tcgen05 fold runs a step in the head-major form from 1,536 rows on whose longest row sees more than 256 keys.  A
+// block's start (queries, tensor memory) weighs as much as a few tiles of 64 keys: mixers of 12 heads over prompts of
+// 128, 256 and 512 tokens take 75, 82 and 103 us with it and 62, 78 and 136 us without; 128 tokens behind 2,000: 181
+// and 194 us (32 heads: 202 and 364).
 constexpr long kTensorRows = 1536;
+constexpr int kTensorKeys = 256;
 
 static bool fold_takes_tensor(const LatentParams& p) {
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool) | reinterpret_cast<uintptr_t>(p.l_heads) |
                           reinterpret_cast<uintptr_t>(p.qa_heads) | reinterpret_cast<uintptr_t>(p.q_rot);
-  return p.stage == 2 && !p.single && p.status != nullptr && static_cast<long>(p.num_tokens) * p.heads >= kTensorRows &&
+  const long keys = p.window > 0 ? std::min<long>(p.max_keys, static_cast<long>(p.window) + p.num_tokens) : p.max_keys;
+  return p.stage == 2 && keys > kTensorKeys && !p.single && p.status != nullptr && static_cast<long>(p.num_tokens) * p.heads >= kTensorRows &&
          p.rank % latent_tc::kHalf == 0 && p.rot <= latent_tc::kHalf && (bases & 15) == 0;
 }
 
