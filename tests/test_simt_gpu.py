@@ -101,7 +101,8 @@ def _attention_want(q, keys, values, entry, position, heads, kv_heads, scale, ma
 
 # counts of tokens at the borders of the two forms (64) and of a tile (64 rows, several requests in one), head sizes of
 # every instance, rows that are not whole 16-byte pieces, every mask; a value nobody may see yet is infinite
-@pytest.mark.parametrize("counts,firsts", [([1], [0]), ([1, 1, 1], [5, 130, 700]), ([64], [3]), ([65], [0]), ([1, 70, 130, 1], [90, 0, 65, 200])])
+@pytest.mark.parametrize("counts,firsts", [([1], [0]), ([1, 1, 1], [5, 130, 700]), ([64], [3]), ([65], [0]), ([1, 70, 130, 1], [90, 0, 65, 200]),
+                                          ([1, 1, 70, 1, 1, 1], [0, 3, 40, 200, 7, 64])])
 @pytest.mark.parametrize("d,dv,heads,kv_heads", [(64, 64, 7, 1), (128, 96, 4, 2), (80, 256, 12, 1), (30, 18, 2, 2)])
 @pytest.mark.parametrize("mask", ["all", "window", "chunk"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -46,6 +46,7 @@ struct AttentionParams {
   const float* gate;
   long long gate_stride;
   int gate_per_head;
+  int singles;   // tokens that stand alone among their neighbours have a launch of their own
 };
 
 // What a query at `position` sees: keys 0 .. kept - 1 and first .. position.
@@ -110,6 +111,31 @@ __device__ __forceinline__ float ending_factor(const AttentionParams& p, int h, 
 // ---------------------------------------------------------------------------------------
 constexpr int kSplits = 8, kRows = 8, kScorePitch = 12;
 
+// The `index`-th token that stands alone (another request's before it and behind it), for the whole block; -1: none.
+__device__ __forceinline__ int single_token(const int* __restrict__ seq, int tokens, int index) {
+  __shared__ int counts[kAttentionThreads / 32], found;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) found = -1;
+  int before = 0;
+  for (int base = 0; base < tokens; base += kAttentionThreads) {
+    const int t = base + threadIdx.x;
+    const bool alone = t < tokens && (t == 0 || seq[t - 1] != seq[t]) && (t + 1 == tokens || seq[t + 1] != seq[t]);
+    const unsigned votes = __ballot_sync(0xffffffffu, alone);
+    __syncthreads();   // the counts before are read
+    if (lane == 0) counts[warp] = __popc(votes);
+    __syncthreads();
+    int own = before + __popc(votes & ((1u << lane) - 1u));
+    for (int w = 0; w < kAttentionThreads / 32; ++w) {
+      if (w < warp) own += counts[w];
+      before += counts[w];
+    }
+    if (alone && own == index) found = t;
+    if (before > index) break;
+  }
+  __syncthreads();
+  return found;
+}
+
 template <int DP>
 struct SplitShared {
   float q[kRows][DP];
@@ -128,7 +154,7 @@ attention_split_kernel(const AttentionParams p) {
   SplitShared<DP>& s = *reinterpret_cast<SplitShared<DP>*>(split_raw);
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int split = blockIdx.x, t = blockIdx.z;
+  const int split = blockIdx.x;
   const int group = p.num_heads / p.num_kv_heads, parts = (group + kRows - 1) / kRows;
   const int kv_head = blockIdx.y / parts, h0 = kv_head * group + (blockIdx.y % parts) * kRows;
   const int heads = min(kRows, (kv_head + 1) * group - h0);
@@ -136,6 +162,10 @@ attention_split_kernel(const AttentionParams p) {
   // columns that no row of a pool fills are read with the others: zeros
   for (int i = tid; i < kTileKeys * (DP + 4 - d); i += kAttentionThreads) s.k[i / (DP + 4 - d)][d + i % (DP + 4 - d)] = 0.0f;
   pdl_wait();
+  // a token a cluster; or the tokens that stand alone, as many clusters as there are requests (nearly always one round)
+  for (int turn = blockIdx.z;; turn += gridDim.z) {
+  const int t = p.singles ? single_token(p.token_seq, p.num_tokens, turn) : turn;
+  if (t < 0 || t >= p.num_tokens) return;   // (the same for every block of the cluster)
   const int position = p.positions[t];
   const int* table = p.block_table + static_cast<size_t>(p.token_seq[t]) * p.table_width;
   int kept, first;
@@ -272,7 +302,8 @@ attention_split_kernel(const AttentionParams p) {
       static_cast<T*>(p.out)[(static_cast<size_t>(t) * p.num_heads + h) * dv + c] = from_float<T>(value * factor * gate_factor(p, t, h, c));
     }
   }
-  cluster_sync();   // no block leaves while another reads its part
+  cluster_sync();   // no block goes on while another reads its part
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -282,7 +313,7 @@ attention_split_kernel(const AttentionParams p) {
 // within its warp.  Tokens of several requests in one tile are folded one request after another, the
 // others' rows masked.  Bound by the multiply-adds and the reads of shared memory that feed them: 64 x 64 tiles
 // read a key 64 times less often than a warp per row.  1,024 tokens of three requests (700, 1 and 323, histories
-// 0, 900, 40), 14 heads of 64 on 2, 32-bit: 269 us (a warp per (token, head): 1,146 us).
+// 0, 900, 40), 14 heads of 64 on 2, 32-bit: 133 us beside 21 us for the one alone (a warp per (token, head): 1,146 us).
 // ---------------------------------------------------------------------------------------
 constexpr int kTileRows = 64;
 
@@ -356,6 +387,13 @@ attention_tile_kernel(const AttentionParams p) {
       high = max(high, s.last[seg_end]);
       most_kept = max(most_kept, s.kept[seg_end]);
       ++seg_end;
+    }
+    if (p.singles && seg_end - seg == 1 && (t0 + seg == 0 || p.token_seq[t0 + seg - 1] != seq) &&
+        (t0 + seg_end == p.num_tokens || p.token_seq[t0 + seg_end] != seq)) {
+      if (tid == 0) s.last[seg] = -2;   // no row of this launch's
+      __syncthreads();
+      seg = seg_end;
+      continue;
     }
     const int* table = p.block_table + static_cast<size_t>(seq) * p.table_width;
     for (int run = 0; run < 2; ++run) {
@@ -494,7 +532,7 @@ attention_tile_kernel(const AttentionParams p) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int row = row0 + 2 * i;
-    if (row >= rows) continue;
+    if (row >= rows || s.last[row] == -2) continue;
     const int t = t0 + row;
     const float factor = ending_factor(p, h, row_max[i], row_sum[i]);
     T* out_row = static_cast<T*>(p.out) + (static_cast<size_t>(t) * p.num_heads + h) * dv;
@@ -513,16 +551,27 @@ attention_tile_kernel(const AttentionParams p) {
 constexpr int kSplitTokens = 64;
 
 template <typename T, int DP, bool VEC>
-static int launch_attention(const AttentionParams& p, cudaStream_t s) {
-  if (p.num_tokens <= kSplitTokens) {
-    static SharedMemoryOptIn opt_in;
-    constexpr int kBytes = static_cast<int>(sizeof(SplitShared<DP>));
-    const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_split_kernel<T, DP, VEC>), kBytes);
-    if (opted) return opted;
-    const int group = p.num_heads / p.num_kv_heads;
-    return launch_in_clusters(attention_split_kernel<T, DP, VEC>, kSplits,
-                              dim3(kSplits, p.num_kv_heads * ((group + kRows - 1) / kRows), p.num_tokens), dim3(kAttentionThreads),
-                              kBytes, s, p);
+static int launch_split(const AttentionParams& p, int clusters, cudaStream_t s) {
+  static SharedMemoryOptIn opt_in;
+  constexpr int kBytes = static_cast<int>(sizeof(SplitShared<DP>));
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_split_kernel<T, DP, VEC>), kBytes);
+  if (opted) return opted;
+  const int group = p.num_heads / p.num_kv_heads;
+  return launch_in_clusters(attention_split_kernel<T, DP, VEC>, kSplits, dim3(kSplits, p.num_kv_heads * ((group + kRows - 1) / kRows), clusters),
+                            dim3(kAttentionThreads), kBytes, s, p);
+}
+
+// In a step of portions beside tokens that stand alone (other requests' decode tokens) those would walk their whole
+// histories in a tile's rows that they do not fill, behind the tile's other requests: they go to the split form, a launch
+// of their own (1,024 tokens, one of them alone behind 900 keys: 270 us in the tiles alone, 133 + 21 us).
+template <typename T, int DP, bool VEC>
+static int launch_attention(const AttentionParams& asked, int requests, cudaStream_t s) {
+  AttentionParams p = asked;
+  if (p.num_tokens <= kSplitTokens) return launch_split<T, DP, VEC>(p, p.num_tokens, s);
+  if (requests > 1) {
+    p.singles = 1;
+    const int status = launch_split<T, DP, VEC>(p, requests < 65535 ? requests : 65535, s);
+    if (status) return status;
   }
   static SharedMemoryOptIn opt_in;
   constexpr int kBytes = static_cast<int>(sizeof(TileShared<DP>));
@@ -533,14 +582,14 @@ static int launch_attention(const AttentionParams& p, cudaStream_t s) {
 }
 
 template <typename T>
-static int launch_sizes(const AttentionParams& p, cudaStream_t s) {
+static int launch_sizes(const AttentionParams& p, int requests, cudaStream_t s) {
   constexpr int kPiece = 16 / static_cast<int>(sizeof(T));
   const bool vec = p.head_dim % kPiece == 0 && p.value_dim % kPiece == 0 &&
                    ((reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool)) & 15) == 0;
   const int largest = p.head_dim > p.value_dim ? p.head_dim : p.value_dim;
-  if (largest <= 64) return vec ? launch_attention<T, 64, true>(p, s) : launch_attention<T, 64, false>(p, s);
-  if (largest <= 128) return vec ? launch_attention<T, 128, true>(p, s) : launch_attention<T, 128, false>(p, s);
-  return vec ? launch_attention<T, 256, true>(p, s) : launch_attention<T, 256, false>(p, s);
+  if (largest <= 64) return vec ? launch_attention<T, 64, true>(p, requests, s) : launch_attention<T, 64, false>(p, requests, s);
+  if (largest <= 128) return vec ? launch_attention<T, 128, true>(p, requests, s) : launch_attention<T, 128, false>(p, requests, s);
+  return vec ? launch_attention<T, 256, true>(p, requests, s) : launch_attention<T, 256, false>(p, requests, s);
 }
 
 // q is [tokens, heads, d] and out [tokens, heads, value_dim]; the key pool is
@@ -552,12 +601,13 @@ static int launch_sizes(const AttentionParams& p, cudaStream_t s) {
 // sink_values (null: none) holds a learned sink score per query head; gate (null: none) the output
 // gate's 32-bit pre-activations, row t at gate + t * gate_stride, [heads * value_dim] values ([heads] with
 // gate_per_head).
-VIPERA_API int vipera_attention_gated(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,
+// `requests`: the rows of block_table (1: not known; every token then takes the tiles).
+VIPERA_API int vipera_attention_step(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,
                                       const int* token_seq, const int* positions, const int* block_table,
                                       int table_width, int page_size, int num_tokens, int num_heads,
                                       int num_kv_heads, int head_dim, int value_dim, float scale, int window,
                                       int keep_first, int sink, int chunk, float out_scale, const float* sink_values,
-                                      const float* gate, long long gate_stride, int gate_per_head, void* stream) {
+                                      const float* gate, long long gate_stride, int gate_per_head, int requests, void* stream) {
   if (num_tokens <= 0) return VIPERA_OK;
   if (chunk < 0 || (chunk > 0 && window > 0)) return VIPERA_BAD_ARGUMENT;
   if (head_dim <= 0 || head_dim > kMaxHeadDim) return VIPERA_BAD_SHAPE;
@@ -567,11 +617,22 @@ VIPERA_API int vipera_attention_gated(const void* q, void* out, int dtype, const
   if (num_heads > 65535) return VIPERA_BAD_SHAPE;
   const AttentionParams p{q, out, k_pool, v_pool, token_seq, positions, block_table, table_width, page_size, num_tokens, num_heads,
                           num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink, chunk, out_scale, sink_values, gate,
-                          gate_stride, gate_per_head};
+                          gate_stride, gate_per_head, 0};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == VIPERA_F32) return launch_sizes<float>(p, s);
-  if (dtype == VIPERA_BF16) return launch_sizes<__nv_bfloat16>(p, s);
+  if (dtype == VIPERA_F32) return launch_sizes<float>(p, requests, s);
+  if (dtype == VIPERA_BF16) return launch_sizes<__nv_bfloat16>(p, requests, s);
   return VIPERA_BAD_DTYPE;
+}
+
+VIPERA_API int vipera_attention_gated(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,
+                                      const int* token_seq, const int* positions, const int* block_table,
+                                      int table_width, int page_size, int num_tokens, int num_heads,
+                                      int num_kv_heads, int head_dim, int value_dim, float scale, int window,
+                                      int keep_first, int sink, int chunk, float out_scale, const float* sink_values,
+                                      const float* gate, long long gate_stride, int gate_per_head, void* stream) {
+  return vipera_attention_step(q, out, dtype, k_pool, v_pool, token_seq, positions, block_table, table_width, page_size, num_tokens,
+                               num_heads, num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink, chunk, out_scale,
+                               sink_values, gate, gate_stride, gate_per_head, 1, stream);
 }
 
 VIPERA_API int vipera_attention(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,

@@ -515,10 +515,10 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: 
     float32 [heads]: exp(sink_h) joins head h's denominator instead of one.  ``gate`` float32
     [tokens, width]: the output is multiplied by the sigmoid of the heads * value_dim values that
     start at column ``gate_offset`` of the token's row (``gate_per_head``: of heads values, one for a whole head)."""
-    fn = _function("attention", "vipera_attention_gated",
+    fn = _function("attention", "vipera_attention_step",
                    [_c_void, _c_void, _c_int, _c_void, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_int,
                     _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void,
-                    _c_void, ctypes.c_longlong, _c_int, _c_void])
+                    _c_void, ctypes.c_longlong, _c_int, _c_int, _c_void])
     if chunk and window:
         raise InvalidArgumentError("attention: a mask is a window or chunks, not both")
     count = q.shape[0]
@@ -544,7 +544,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: 
               num_heads, num_kv_heads, head_dim, value_dim, float(scale), int(window or 0),
               int(keep_first or 0) if window else 0, 1 if sink else 0, int(chunk or 0), float(out_scale),
               _opt(sink_values, "sink_values", torch.float32), gate_pointer, gate_stride, int(bool(gate_per_head)),
-              _stream()), "attention")
+              block_table.shape[0], _stream()), "attention", kernels=2 if count > 64 and block_table.shape[0] > 1 else 1)
 
 
 # ----------------------------------------------------------------------------------------
