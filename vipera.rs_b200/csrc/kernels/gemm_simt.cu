@@ -1,16 +1,19 @@
-// Matrix products on the CUDA cores with 32-bit accumulation: out[M, N] = A[M, K] . W[N, K]^T.
+// Matrix products with 32-bit accumulation: out[M, N] = A[M, K] . W[N, K]^T.
 //
-// This is the product kernel of the true 32-bit path (no tensor cores, no reduced-precision
-// mode) and the fallback of the bfloat16 path for sizes the tensor-core kernel refuses.
+// This is the product kernel of the true 32-bit path (no reduced-precision mode) and the fallback of the bfloat16 path for sizes the tensor-core kernel refuses.
 // The reference multiplies one weight matrix by all B activation rows in one pass over the
 // weights (crates/vipera-backend-cpu/src/model.rs:1005-1025) and promises that a row's
 // result does not depend on its neighbours in the batch (model.rs:881-882); here every output
-// element sums over K in an order that is fixed for its class of row counts: up to eight rows, or more.
+// element sums over K in an order that is fixed for its class of row counts: up to eight rows, up to 64 (and values that are
+// widened), or more, where the order also depends on how many blocks share K (gemm_split.cuh).
 //
 // Up to eight rows the stream of W bounds the product (gemv_rows_kernel): a warp reads eight rows of W
 // through a ring of its own, 512 neighbouring bytes of a row at a time, a lane's four values against all
 // rows of A, and adds its lanes' sums at the end.
-// More rows (gemm_simt_kernel): the multiply-add units and the reads of shared memory that feed them.  K is
+// 32-bit products of more than 64 rows (whole rows of 16-byte pieces) run on the tensor cores, three bfloat16 parts of every
+// number: gemm_split.cuh.  Multiply-adds / tensor cores: 65 rows, W 896 x 896: 17.4 / 17.3 us; W 9,728 x 896: 106 / 38; 128
+// rows, W 896 x 4,864: 70 / 47.
+// The others of more rows (gemm_simt_kernel): the multiply-add units and the reads of shared memory that feed them.  K is
 // cut into eight slabs (of whole chunks of 32), a slab's even and odd places are two chains of fused
 // multiply-adds (the two halves of a packed 32-bit pair) whose ends are added, and the slabs are added in
 // their order.  A block takes a tile of rows and columns through a ring of cp.async
@@ -20,8 +23,8 @@
 // scratch either way.
 //
 // Measured (B200; a 64 x 64 tile staged value by value before): 8 rows, W 17,920 x 1,536: 166 -> 30 us (3.7 TB/s);
-// 8 rows, W 1,536 x 1,536 and 1,536 x 8,960: 461 -> 16 us on average; 1,024 rows, W 9,728 x 896: 758 -> 535 us
-// (33 TFLOP/s).  Sums in parts are also closer to 64-bit ones: 8e-7 instead of 3e-6 on a decode step's logits.
+// 8 rows, W 1,536 x 1,536 and 1,536 x 8,960: 461 -> 16 us on average; 1,024 rows, W 9,728 x 896: 758 -> 503 us
+// here, 183 us on the tensor cores.  Sums in parts are also closer to 64-bit ones: 8e-7 instead of 3e-6 on a decode step's logits.
 //
 // Epilogues:
 //   STORE     out[m, n] = acc (+ bias[n]), stored as float or bfloat16
@@ -63,6 +66,8 @@ struct GemmArgs {
   int activation, epilogue, out_bf16;
   int wide;            // rows of whole pieces of eight values on 16-byte boundaries
   int* status;         // for the bounded waits of the tensor-core form, or null: it is not used
+  void* parts;         // room for its left operand's parts, or null
+  long long parts_bytes;
 };
 
 __device__ __forceinline__ void load_eight(const float* src, float (&v)[8]) {
@@ -440,7 +445,8 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
       if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileMid, true>(p, s);
       if (p.status)   // more rows than a half tile: three parts of every number on the tensor cores
         return gemm_split::launch({static_cast<const float*>(p.A), static_cast<const float*>(p.W), p.M, p.N, p.K, 1, 0, p.bias, p.out,
-                                   p.resid, p.activation, p.epilogue, p.out_bf16, p.status}, s);
+                                   p.resid, p.activation, p.epilogue, p.out_bf16, p.status,
+                                   static_cast<uint8_t*>(p.parts), nullptr, p.parts_bytes}, s);
       return launch_tile<TA, TW, TileMany, true>(p, s);
     }
   }
@@ -451,30 +457,34 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
 
 template <typename TA, typename TW>
 static int launch_typed(const TA* A, const TW* W, int M, int N, int K, int epilogue, const float* bias,
-                        void* out, int out_dtype, float* resid, int activation, int* status, cudaStream_t s) {
+                        void* out, int out_dtype, float* resid, int activation, int* status, void* parts, long long parts_bytes, cudaStream_t s) {
   const int slab = ((K + kSlabs - 1) / kSlabs + kChunk - 1) / kChunk * kChunk;
   if (epilogue != EPI_STORE && epilogue != EPI_RESIDUAL && epilogue != EPI_SWIGLU) return VIPERA_BAD_ARGUMENT;
   if (epilogue == EPI_RESIDUAL ? !resid : !out) return VIPERA_BAD_ARGUMENT;
   if (epilogue == EPI_SWIGLU && N % 32 != 0) return VIPERA_BAD_SHAPE;  // gate/up groups of 16 must pair up
   if (epilogue != EPI_RESIDUAL && out_dtype != VIPERA_F32 && out_dtype != VIPERA_BF16) return VIPERA_BAD_DTYPE;
   const int wide = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
-  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16, wide, status};
+  const GemmArgs p{A, W, M, N, K, slab, bias, out, resid, activation, epilogue, out_dtype == VIPERA_BF16, wide, status, parts, parts_bytes};
   return launch_sizes<TA, TW>(p, s);
 }
 
 // A is [M, K] and W is [N, K], both row-major and contiguous.  For SWIGLU, N counts the
 // interleaved gate and up rows (twice the intermediate size) and out is [M, N/2].
 static int run_simt(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K, int epilogue,
-                    const float* bias, void* out, int out_dtype, float* resid, int activation, int* status, void* stream) {
+                    const float* bias, void* out, int out_dtype, float* resid, int activation, int* status, void* parts,
+                    long long parts_bytes, void* stream) {
   if (M <= 0) return VIPERA_OK;
   if (N <= 0 || K <= 0) return VIPERA_BAD_SHAPE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a_dtype == VIPERA_F32 && w_dtype == VIPERA_F32)
-    return launch_typed(static_cast<const float*>(A), static_cast<const float*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, s);
+    return launch_typed(static_cast<const float*>(A), static_cast<const float*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status,
+                        parts, parts_bytes, s);
   if (a_dtype == VIPERA_BF16 && w_dtype == VIPERA_BF16)
-    return launch_typed(static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, s);
+    return launch_typed(static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status,
+                        parts, parts_bytes, s);
   if (a_dtype == VIPERA_F32 && w_dtype == VIPERA_BF16)
-    return launch_typed(static_cast<const float*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, s);
+    return launch_typed(static_cast<const float*>(A), static_cast<const __nv_bfloat16*>(W), M, N, K, epilogue, bias, out, out_dtype, resid, activation, status,
+                        parts, parts_bytes, s);
   return VIPERA_BAD_DTYPE;
 }
 
@@ -483,7 +493,7 @@ VIPERA_API int vipera_gemm_simt(const void* A, int a_dtype, const void* W, int w
                                 void* stream) {
   // the form the earlier callers know: bias with STORE only, silu in the gated unit
   return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, epilogue == EPI_STORE ? bias : nullptr, out, out_dtype,
-                  resid, ACT_SILU, nullptr, stream);
+                  resid, ACT_SILU, nullptr, nullptr, 0, stream);
 }
 
 // The same with a bias in every ending and the gated unit's activation chosen (ACT_SILU, ACT_GELU_TANH).
@@ -491,16 +501,21 @@ VIPERA_API int vipera_gemm_simt_act(const void* A, int a_dtype, const void* W, i
                                     int epilogue, const float* bias, void* out, int out_dtype, float* resid,
                                     int activation, void* stream) {
   if (activation != ACT_SILU && activation != ACT_GELU_TANH) return VIPERA_BAD_ARGUMENT;
-  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, nullptr, stream);
+  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, nullptr, nullptr, 0, stream);
 }
 
 // The same with a device word that must be 0 before the launch and is not afterwards where a bounded wait ran out: 32-bit
-// products of many rows may then run on the tensor cores, three parts of every number.
+// products of many rows may then run on the tensor cores, three parts of every number.  `parts`: room of
+// vipera_gemm_simt_parts bytes (16-byte aligned), or null.
 VIPERA_API int vipera_gemm_simt_status(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
                                        int epilogue, const float* bias, void* out, int out_dtype, float* resid,
-                                       int activation, int* status, void* stream) {
+                                       int activation, int* status, void* parts, long long parts_bytes, void* stream) {
   if (activation != ACT_SILU && activation != ACT_GELU_TANH) return VIPERA_BAD_ARGUMENT;
-  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, stream);
+  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, status, parts,
+                  parts_bytes, stream);
 }
+
+// The bytes that 32-bit products of such sizes want for the parts of their left operand (0: none).
+VIPERA_API int vipera_gemm_simt_parts(int M, int N, int K) { return gemm_split::parts_bytes(M, N, K); }
 
 VIPERA_API const char* vipera_gemm_simt_status_text(int status) { return vipera_status_text(status); }

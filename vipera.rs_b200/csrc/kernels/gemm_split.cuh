@@ -7,15 +7,19 @@
 // every step of their sums towards zero, which over a long K would cost more than 32-bit multiply-adds do: so the
 // leading product and the five small ones have accumulators of their own, both are read after every 64 values of K
 // and added to the tile's sums in registers, rounded to nearest.  Against 64 bits the result is closer than a chain of
-// fused multiply-adds over K (MEASUREDERR).  An infinity or a NaN has no such parts (its products with their zeros
+// fused multiply-adds over K (1,024 rows through a model of two layers and K up to 4,864: 4.8e-7 against 2.2e-6).  An infinity or a NaN has no such parts (its products with their zeros
 // would be NaN): a block that meets one computes its tile with multiply-adds instead.
 //
-// A block computes a tile of 128 x 128: eight warps read 64 values of K of both operands, split them and leave the
-// parts in shared memory (three images of 128 rows each, 128-byte swizzle, two stages of 96 KB); eight warps add up, the
-// first of which issues 24 products of 16 values a stage (a warp of its own for that would leave too few registers).  Two pairs of accumulators fill tensor memory.  Where the tiles
-// are too few to fill the chip, the blocks of a cluster share K and add their parts through distributed shared memory.
-// What bounds it: 24 products of 64 clocks a stage, whose operands' reads alone keep shared memory busy as long; the
-// split writes 96 KB more.  MEASURED
+// A block computes a tile of 128 x 128: eight warps read 64 values of K, split them and leave the parts in shared
+// memory (three images of 128 rows each, 128-byte swizzle, two stages of 96 KB); eight warps add up, the first of which
+// issues 24 products of 16 values a stage (a warp of its own for that would leave too few registers).  The left
+// operand's images are written once by a kernel ahead and copied in bulk where that pays (parts_bytes), else the same
+// warps split both.  Two pairs of accumulators fill tensor memory.  Where the tiles are too few to fill the chip, the
+// blocks of a cluster share K and add their parts through distributed shared memory.
+// What bounds it: a stage's 24 products of 64 clocks read shared memory for all of these 1,536 clocks, and the
+// images' 96 KB are written there beside them; 3,400 clocks a stage are left of that in long K, and what a block costs
+// before its first and after its last stage (about six stages).  1,024 x 9,728 of 896: 183 us (multiply-adds: 503), the
+// left operand split in every block: 262; 2,048 x 4,096 of 14,336: 1,624 us, 148 TFLOP/s (the CUDA cores' own peak is 74).
 #pragma once
 
 #include "simt.cuh"
@@ -39,6 +43,9 @@ struct Args {
   float* resid;
   int activation, epilogue, out_bf16;
   int* status;
+  uint8_t* parts;            // the left operand's images, written ahead: [tile of rows][64 of K][part], or null
+  int* odd;                  // of each of those threes of images: something in it is not finite
+  long long parts_bytes;     // what `parts` has room for (the flags lie behind the images)
 };
 
 struct Shared {
@@ -97,6 +104,54 @@ __device__ __forceinline__ float leading(float v) { return __uint_as_float(__flo
 // the upper halves of two 32-bit words, `lo`'s in the lower one
 __device__ __forceinline__ uint32_t uppers(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
 
+// Eight values' pieces of the three images; `odd` becomes NaN where a value is not finite (its remainder is NaN).
+struct Pieces {
+  uint32_t first[4], second[4], third[4];
+  __device__ __forceinline__ Pieces(const float4& lo, const float4& hi, float& odd) {
+    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const float r0 = v[e] - leading(v[e]), r1 = v[e + 1] - leading(v[e + 1]);
+      first[e >> 1] = uppers(v[e], v[e + 1]);
+      second[e >> 1] = uppers(r0, r1);
+      third[e >> 1] = uppers(r0 - leading(r0), r1 - leading(r1));
+      odd = fmaf(r0, 0.0f, fmaf(r1, 0.0f, odd));
+    }
+  }
+  __device__ __forceinline__ void store(uint8_t* at) const {
+    *reinterpret_cast<uint4*>(at) = make_uint4(first[0], first[1], first[2], first[3]);
+    *reinterpret_cast<uint4*>(at + kImageBytes) = make_uint4(second[0], second[1], second[2], second[3]);
+    *reinterpret_cast<uint4*>(at + 2 * kImageBytes) = make_uint4(third[0], third[1], third[2], third[3]);
+  }
+};
+
+// The left operand's parts, a block 128 rows and 64 values of K: the images as the products' blocks want them in shared
+// memory.  Every block along N would split the same rows again.
+__global__ void __launch_bounds__(kSplitters)
+gemm_split_left_kernel(const Args p) {
+  const int t = threadIdx.x, piece = t & 7, sub = t >> 3, k = blockIdx.x * kDepth + piece * 8, m0 = blockIdx.y * kTile;
+  const int three = blockIdx.y * gridDim.x + blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  float4 lo[4], hi[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + sub + 32 * i;
+    const float* src = p.A + static_cast<size_t>(m) * p.K + k;
+    lo[i] = hi[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (m < p.M && k < p.K) lo[i] = *reinterpret_cast<const float4*>(src);
+    if (m < p.M && k + 4 < p.K) hi[i] = *reinterpret_cast<const float4*>(src + 4);
+  }
+  uint8_t* dst = p.parts + static_cast<size_t>(three) * (kParts * kImageBytes) + sub * 128 + ((piece ^ (sub & 7)) << 4);
+  float odd = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) Pieces(lo[i], hi[i], odd).store(dst + i * 32 * 128);
+  const int any = __syncthreads_or(odd != odd);
+  if (t == 0) p.odd[three] = any;
+}
+
+// AHEAD: the left operand's images lie in p.parts and are copied; else this block splits both operands.
+template <bool AHEAD>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_split_kernel(const Args p) {
   extern __shared__ uint8_t split_raw[];
@@ -111,7 +166,7 @@ gemm_split_kernel(const Args p) {
   pdl_launch_dependents();
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
-      bar_init(&s.full[i], kSplitters);
+      bar_init(&s.full[i], kSplitters + (AHEAD ? 1 : 0));
       bar_init(&s.empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -186,52 +241,67 @@ gemm_split_kernel(const Args p) {
     for (int j = 0; j < 64; j += 4)
       *reinterpret_cast<float4*>(sums + row * kSumPitch + column0 + j) = make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]);
   } else {
-    // ---------------- operands: eight runs of eight values a thread and stage, four of either operand ----------------
+    // ---------------- operands: runs of eight values, four a thread and stage of either operand ----------------
+    constexpr int kRuns = AHEAD ? 4 : 8, kFirstW = kRuns - 4;
     const int t = tid - kFirstSplitter * 32, piece = t & 7, sub = t >> 3;   // rows sub + 32 i
-    float4 lo[8], hi[8];
+    float4 lo[kRuns], hi[kRuns];
+    // where this thread's runs start, and which of its rows exist
+    const float* a_rows = p.A + static_cast<size_t>(m0 + sub) * p.K + k_begin + piece * 8;
+    const float* w_rows = p.W + static_cast<size_t>(n0 + sub) * p.K + k_begin + piece * 8;
+    const size_t step = static_cast<size_t>(32) * p.K;
+    unsigned live = 0;
+#pragma unroll
+    for (int i = 0; i < kRuns; ++i)
+      live |= (i < kFirstW ? m0 + sub + 32 * i < p.M : n0 + sub + 32 * (i - kFirstW) < p.N) ? 1u << i : 0u;
+    const int whole = (k_end - k_begin) / kDepth;   // stages that lie within K
     auto ask = [&](int i, int c) {
-      const bool of_a = i < 4;
-      const int r = sub + 32 * (i & 3), k = k_begin + c * kDepth + piece * 8;
-      const int row = (of_a ? m0 : n0) + r, extent = of_a ? p.M : p.N;
-      const float* src = (of_a ? p.A : p.W) + (row < extent ? static_cast<size_t>(row) * p.K + k : 0);
-      // (K is a multiple of four: each half of the run lies within it or not)
-      lo[i] = c < count && row < extent && k < k_end ? *reinterpret_cast<const float4*>(src) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      hi[i] = c < count && row < extent && k + 4 < k_end ? *reinterpret_cast<const float4*>(src + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float* src = (i < kFirstW ? a_rows + i * step : w_rows + (i - kFirstW) * step) + c * kDepth;
+      lo[i] = hi[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (live >> i & 1u) {
+        // (K is a multiple of four: each half of the run lies within it or not)
+        if (c < whole || k_begin + c * kDepth + piece * 8 < k_end) lo[i] = *reinterpret_cast<const float4*>(src);
+        if (c < whole || k_begin + c * kDepth + piece * 8 + 4 < k_end) hi[i] = *reinterpret_cast<const float4*>(src + 4);
+      }
     };
     // the weights of the first stage are asked for before the kernel ahead has ended
 #pragma unroll
-    for (int i = 4; i < 8; ++i) ask(i, 0);
+    for (int i = kFirstW; i < kRuns; ++i)
+      if (count > 0) ask(i, 0);
     pdl_wait();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) ask(i, 0);
-    bool odd = false;   // something that is not finite
+    for (int i = 0; i < kFirstW; ++i)
+      if (count > 0) ask(i, 0);
+    const int three = blockIdx.y * ((p.K + kDepth - 1) / kDepth) + k_begin / kDepth;   // the first images of this block
+    float odd = 0.0f;   // NaN once something is not finite
+    if (AHEAD)
+      for (int c = t; c < count; c += kSplitters)
+        if (p.odd[three + c]) odd = NAN;
     for (int c = 0; c < count; ++c) {
       const int stage = c & 1;
       if (c >= 2) bar_wait(&s.empty[stage], ((c >> 1) & 1) ^ 1, abort_flag, p.status);
-      uint8_t* dst = stages + stage * kStageBytes;
+      if (AHEAD && t == 0) {
+        const uint32_t bytes = *abort_flag ? 0 : kParts * kImageBytes, bar = shared_address(&s.full[stage]);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        if (bytes)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           shared_address(stages + stage * kStageBytes)),
+                       "l"(p.parts + static_cast<size_t>(three + c) * (kParts * kImageBytes)), "r"(bytes), "r"(bar)
+                       : "memory");
+      }
+      uint8_t* dst = stages + stage * kStageBytes + sub * 128 + ((piece ^ (sub & 7)) << 4);   // (rows 32 apart are swizzled alike)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float v[8] = {lo[i].x, lo[i].y, lo[i].z, lo[i].w, hi[i].x, hi[i].y, hi[i].z, hi[i].w};
-        uint32_t first[4], second[4], third[4];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const float r0 = v[e] - leading(v[e]), r1 = v[e + 1] - leading(v[e + 1]);
-          first[e >> 1] = uppers(v[e], v[e + 1]);
-          second[e >> 1] = uppers(r0, r1);
-          third[e >> 1] = uppers(r0 - leading(r0), r1 - leading(r1));
-          odd |= !(fabsf(v[e]) <= 3.402823466e38f) || !(fabsf(v[e + 1]) <= 3.402823466e38f);
-        }
+      for (int i = 0; i < kRuns; ++i) {
+        const Pieces pieces(lo[i], hi[i], odd);
         if (c + 1 < count) ask(i, c + 1);   // the next stage's run takes this one's registers
-        const int r = sub + 32 * (i & 3);
-        uint8_t* at = dst + (i < 4 ? 0 : kParts * kImageBytes) + r * 128 + ((piece ^ (r & 7)) << 4);
-        *reinterpret_cast<uint4*>(at) = make_uint4(first[0], first[1], first[2], first[3]);
-        *reinterpret_cast<uint4*>(at + kImageBytes) = make_uint4(second[0], second[1], second[2], second[3]);
-        *reinterpret_cast<uint4*>(at + 2 * kImageBytes) = make_uint4(third[0], third[1], third[2], third[3]);
+        pieces.store(dst + (i < kFirstW ? 0 : kParts * kImageBytes) + ((i - kFirstW) & 3) * 32 * 128);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       bar_arrive(&s.full[stage]);
     }
-    if (odd) s.not_finite = 1;
+    if (odd != odd) s.not_finite = 1;
+    if (AHEAD && t == 0 && *abort_flag) {   // a copy may be on its way still: it ends long before this does
+      for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
   }
   fence_before();
   __syncthreads();
@@ -292,23 +362,70 @@ gemm_split_kernel(const Args p) {
 }
 
 // Blocks of a cluster share K where that leaves fewer stages in a row: (waves of blocks) x (stages of a block + what it
-// costs besides).
-static int launch(const Args& args, cudaStream_t s) {
-  static SharedMemoryOptIn opt_in;
-  const int opted = opt_in.ask(reinterpret_cast<const void*>(gemm_split_kernel), kSharedBytes);
-  if (opted) return opted;
+// costs besides).  Returns the stages in a row.
+static long long share_out(long long tiles, long long depth, int* cluster, int* share_of_block) {
   constexpr long long kSms = 148;
+  long long best = 0, in_a_row = 0;
+  for (int blocks = 1; blocks <= 4; blocks *= 2) {
+    const long long share = (depth + blocks - 1) / blocks, waves = (tiles * blocks + kSms - 1) / kSms;
+    if (blocks > 1 && waves * (share + 4) >= best) continue;
+    best = waves * (share + 4), in_a_row = waves * share;
+    *cluster = blocks, *share_of_block = static_cast<int>(share);
+  }
+  return in_a_row;
+}
+
+static int launch_rows(const Args& args, cudaStream_t s) {
   Args p = args;
   const long long tiles_n = (p.N + kTile - 1) / kTile, tiles_m = (p.M + kTile - 1) / kTile, depth = (p.K + kDepth - 1) / kDepth;
   if (tiles_m > 65535) return VIPERA_BAD_SHAPE;
-  long long best = 0;
-  for (int cluster = 1; cluster <= 4; cluster *= 2) {
-    const long long share = (depth + cluster - 1) / cluster;
-    const long long cost = (tiles_n * tiles_m * cluster + kSms - 1) / kSms * (share + 4);
-    if (cluster == 1 || cost < best) best = cost, p.cluster = cluster, p.share = static_cast<int>(share);
+  share_out(tiles_n * tiles_m, depth, &p.cluster, &p.share);
+  const dim3 grid(static_cast<unsigned>(tiles_n * p.cluster), static_cast<unsigned>(tiles_m));
+  if (!p.parts) return launch_in_clusters(gemm_split_kernel<false>, p.cluster, grid, dim3(kThreads), kSharedBytes, s, p);
+  const int status = vipera_launch(gemm_split_left_kernel, dim3(static_cast<unsigned>(depth), static_cast<unsigned>(tiles_m)),
+                                   dim3(kSplitters), 0, s, p);
+  if (status) return status;
+  return launch_in_clusters(gemm_split_kernel<true>, p.cluster, grid, dim3(kThreads), kSharedBytes, s, p);
+}
+
+// Room for the left operand's parts, or 0 where splitting them ahead does not pay: a launch more, and each stage shorter
+// (5,500 clocks to 3,400).  Not more room than the L2 holds well: more rows are taken in turns.  Both operands split in the
+// block / the left one ahead: 80 x 896 of 896, seven stages in a row: 17.5 / 18.5 us; 1,024 x 1,152 of 896, seven: 30.6 / 31.2;
+// 256 x 256 of 2,048, eight: 33.9 / 27.0; 128 x 9,728 of 896, fourteen: 53.7 / 39.3; 8,192 x 4,096 of 4,096: 2,852 / 1,797.
+constexpr long long kMostParts = 96ll << 20, kTileExtra = 4;   // (bytes beside each three of images: its flag)
+static int parts_bytes(int M, int N, int K) {
+  if (M <= 64 || N <= kTile || K % 4 != 0) return 0;   // (one tile along N: nobody else would split the same rows)
+  const long long tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile;
+  int cluster, share;
+  if (share_out(tiles_m * tiles_n, (K + kDepth - 1) / kDepth, &cluster, &share) < 8) return 0;
+  const long long of_tile = (K + kDepth - 1) / kDepth * (kParts * kImageBytes + kTileExtra);
+  const long long tiles = kMostParts / of_tile;
+  return static_cast<int>((tiles < tiles_m ? tiles : tiles_m) * of_tile);
+}
+
+static int launch(const Args& args, cudaStream_t s) {
+  static SharedMemoryOptIn opt_in, opt_in_ahead;
+  int status = opt_in.ask(reinterpret_cast<const void*>(gemm_split_kernel<false>), kSharedBytes);
+  if (!status) status = opt_in_ahead.ask(reinterpret_cast<const void*>(gemm_split_kernel<true>), kSharedBytes);
+  if (status) return status;
+  const long long of_tile = static_cast<long long>((args.K + kDepth - 1) / kDepth) * (kParts * kImageBytes + kTileExtra);
+  const long long tiles = args.parts ? args.parts_bytes / of_tile : 0;
+  if (tiles < 1) {
+    Args p = args;
+    p.parts = nullptr;
+    return launch_rows(p, s);
   }
-  return launch_in_clusters(gemm_split_kernel, p.cluster, dim3(static_cast<unsigned>(tiles_n * p.cluster), static_cast<unsigned>(tiles_m)),
-                            dim3(kThreads), kSharedBytes, s, p);
+  const size_t out_pitch = static_cast<size_t>(args.epilogue == 2 ? args.N / 2 : args.N);
+  for (long long m = 0; m < args.M && !status; m += tiles * kTile) {
+    Args p = args;
+    p.M = static_cast<int>(args.M - m < tiles * kTile ? args.M - m : tiles * kTile);
+    p.odd = reinterpret_cast<int*>(p.parts + tiles * ((p.K + kDepth - 1) / kDepth) * (kParts * kImageBytes));
+    p.A += static_cast<size_t>(m) * p.K;
+    if (p.epilogue == 1) p.resid += m * out_pitch;
+    else p.out = static_cast<char*>(p.out) + m * out_pitch * (p.out_bf16 ? 2 : 4);
+    status = launch_rows(p, s);
+  }
+  return status;
 }
 
 }  // namespace gemm_split

@@ -470,17 +470,26 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE,
     ``activation`` is the gated unit's."""
     fn = _function("gemm_simt", "vipera_gemm_simt_status",
                    [_c_void, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_int,
-                    _c_void, _c_int, _c_void, _c_void])
+                    _c_void, _c_int, _c_void, _c_void, ctypes.c_longlong, _c_void])
     m, k = a.shape
     n = w.shape[0]
     if w.shape[1] != k:
         raise InvalidArgumentError(f"gemm: inner sizes differ ({k} and {w.shape[1]})")
     _check_gemm_outputs(m, n, epilogue, bias, out, resid)
     pointer = _gpu(a, "a")
+    room, bytes_wanted = None, 0
+    if m > 64 and a.dtype == w.dtype == torch.float32:
+        bytes_wanted = _function("gemm_simt", "vipera_gemm_simt_parts", [_c_int, _c_int, _c_int])(m, n, k)
+        if bytes_wanted:
+            try:  # of the stream's own pool (a captured graph's, under capture): given back when the call returns
+                room = torch.empty(bytes_wanted, dtype=torch.uint8, device=a.device)
+            except torch.cuda.OutOfMemoryError:
+                bytes_wanted = 0  # the products then split both operands themselves
     _check(fn(pointer, dtype_code(a.dtype), _gpu(w, "w"), dtype_code(w.dtype), m, n, k, epilogue,
               _opt(bias, "bias", torch.float32), _opt(out, "out"),
               dtype_code(out.dtype) if out is not None else F32, _opt(resid, "resid", torch.float32),
-              int(activation), _tc_buffers(a.device, 0)["status"].data_ptr(), _stream()), "gemm_simt")
+              int(activation), _tc_buffers(a.device, 0)["status"].data_ptr(),
+              room.data_ptr() if room is not None else None, bytes_wanted, _stream()), "gemm_simt", kernels=2 if room is not None else 1)
 
 
 def _check_gemm_outputs(m, n, epilogue, bias, out, resid) -> None:
