@@ -102,6 +102,18 @@ __device__ __forceinline__ size_t gate_row(int feature, int group) {
   return static_cast<size_t>(feature / group) * 2 * group + feature % group;
 }
 
+template <typename T>
+__device__ __forceinline__ float4 four_values(const T* src);
+template <>
+__device__ __forceinline__ float4 four_values<float>(const float* src) { return *reinterpret_cast<const float4*>(src); }
+template <>
+__device__ __forceinline__ float4 four_values<__nv_bfloat16>(const __nv_bfloat16* src) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(src);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
 // The lane holding the largest value wins; equal values go to the lower index.
 __device__ __forceinline__ void warp_argmax(float& best, int& index) {
 #pragma unroll
@@ -115,68 +127,92 @@ __device__ __forceinline__ void warp_argmax(float& best, int& index) {
   }
 }
 
-// A block per token: its warps share the experts' logits between them (a lane sums every 32nd
-// product, the warp adds the lanes), then the first warp chooses.
-template <typename T>
+// A block per TOKENS tokens: its warps share the experts' logits between them (a lane sums every 32nd
+// product, the warp adds the lanes), then a warp per token chooses.  Bound by the reads of the router's
+// rows from L2: with four tokens a row read once serves them all (2,048 tokens of 1,536 values, 16 rows:
+// 37.1 us a block per token, 20.5 us four).  A token's sums are the same in both.
+template <typename T, int TOKENS>
 __global__ void __launch_bounds__(kRouteThreads)
 moe_route_kernel(MoeParams p) {
   extern __shared__ __align__(16) float route_shared[];
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x;
-  float* h_s = route_shared;                // [hidden] (first: read as vectors)
+  const int first_token = blockIdx.x * TOKENS, here = min(TOKENS, p.num_tokens - first_token);
+  float* h_all = route_shared;              // [TOKENS][hidden] (first: read as vectors)
   const int rows_total = p.experts + p.always_gate;
-  float* score = h_s + p.hidden;
-  float* open = score + rows_total;         // the score while the expert may still be chosen, else -inf
-  float* group_score = open + p.experts;
-  const T* h = static_cast<const T*>(p.h) + static_cast<size_t>(t) * p.hidden;
-  for (int i = threadIdx.x; i < p.hidden; i += kRouteThreads) h_s[i] = to_float<T>(h[i]);
+  float* score_all = h_all + TOKENS * p.hidden;   // [TOKENS][rows_total]
+  if (TOKENS == 1) {
+    const T* h = static_cast<const T*>(p.h) + static_cast<size_t>(first_token) * p.hidden;
+    for (int i = threadIdx.x; i < p.hidden; i += kRouteThreads) h_all[i] = to_float<T>(h[i]);
+  } else {
+    const T* h = static_cast<const T*>(p.h) + static_cast<size_t>(first_token) * p.hidden;
+#pragma unroll 4
+    for (int i = threadIdx.x * 4; i < TOKENS * p.hidden; i += kRouteThreads * 4) {   // (hidden is a multiple of four)
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (i < here * p.hidden) v = four_values<T>(h + i);
+      *reinterpret_cast<float4*>(h_all + i) = v;
+    }
+  }
   __syncthreads();
   constexpr int kWarpsHere = kRouteThreads / 32;
-  if ((p.hidden & 3) == 0 && (reinterpret_cast<uintptr_t>(p.router) & 15) == 0) {
+  if (TOKENS > 1 || ((p.hidden & 3) == 0 && (reinterpret_cast<uintptr_t>(p.router) & 15) == 0)) {
     // Four values at a time: a lane sums the products of values 4 (lane + 32 j) .. + 3, in that order.  A warp
-    // walks four of its rows side by side, so that their loads are in flight together (a step of one token is
+    // walks some of its rows side by side, so that their loads are in flight together (a step of one token is
     // one block, which waits for every row it asks for).
-    const float4* h4 = reinterpret_cast<const float4*>(h_s);
-    for (int e0 = warp; e0 < rows_total; e0 += 4 * kWarpsHere) {
-      const float4* rows[4];
-      float sums[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    constexpr int kRowsHere = TOKENS > 1 ? 2 : 4;
+    const float4* h4 = reinterpret_cast<const float4*>(h_all);
+    const int quarter = p.hidden / 4;
+    for (int e0 = warp; e0 < rows_total; e0 += kRowsHere * kWarpsHere) {
+      const float4* rows[kRowsHere];
+      float sums[kRowsHere][TOKENS];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < kRowsHere; ++j) {
         rows[j] = reinterpret_cast<const float4*>(p.router + static_cast<size_t>(min(e0 + j * kWarpsHere, rows_total - 1)) * p.hidden);
+#pragma unroll
+        for (int n = 0; n < TOKENS; ++n) sums[j][n] = 0.0f;
+      }
 #pragma unroll 4
-      for (int i = lane; i < p.hidden / 4; i += 32) {
-        const float4 a = h4[i];
-        float4 b[4];
+      for (int i = lane; i < quarter; i += 32) {
+        float4 b[kRowsHere];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = rows[j][i];
+        for (int j = 0; j < kRowsHere; ++j) b[j] = rows[j][i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          sums[j] = fmaf(a.x, b[j].x, sums[j]);
-          sums[j] = fmaf(a.y, b[j].y, sums[j]);
-          sums[j] = fmaf(a.z, b[j].z, sums[j]);
-          sums[j] = fmaf(a.w, b[j].w, sums[j]);
+        for (int n = 0; n < TOKENS; ++n) {
+          const float4 a = h4[n * quarter + i];
+#pragma unroll
+          for (int j = 0; j < kRowsHere; ++j) {
+            sums[j][n] = fmaf(a.x, b[j].x, sums[j][n]);
+            sums[j][n] = fmaf(a.y, b[j].y, sums[j][n]);
+            sums[j][n] = fmaf(a.z, b[j].z, sums[j][n]);
+            sums[j][n] = fmaf(a.w, b[j].w, sums[j][n]);
+          }
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float sum = warp_sum(sums[j]);
-        if (lane == 0 && e0 + j * kWarpsHere < rows_total) score[e0 + j * kWarpsHere] = sum;
-      }
+      for (int j = 0; j < kRowsHere; ++j)
+#pragma unroll
+        for (int n = 0; n < TOKENS; ++n) {
+          const float sum = warp_sum(sums[j][n]);
+          if (lane == 0 && e0 + j * kWarpsHere < rows_total) score_all[n * rows_total + e0 + j * kWarpsHere] = sum;
+        }
     }
   } else {
     for (int e = warp; e < rows_total; e += kWarpsHere) {
       const float* r = p.router + static_cast<size_t>(e) * p.hidden;
       float sum = 0.0f;
 #pragma unroll 4
-      for (int i = lane; i < p.hidden; i += 32) sum = fmaf(h_s[i], r[i], sum);
+      for (int i = lane; i < p.hidden; i += 32) sum = fmaf(h_all[i], r[i], sum);
       sum = warp_sum(sum);
-      if (lane == 0) score[e] = sum;
+      if (lane == 0) score_all[e] = sum;
     }
   }
   __syncthreads();
-  if (warp == 0) {
+  if (warp < here) {
+  const int t = first_token + warp;
+  float* score = score_all + warp * rows_total;
+  float* open = score_all + TOKENS * rows_total + warp * (p.experts + p.groups);   // the score while the expert may still be chosen, else -inf
+  float* group_score = open + p.experts;
   if (p.scores == 1) {
     float top_z = -INFINITY;
     for (int e = lane; e < p.experts; e += 32) top_z = fmaxf(top_z, score[e]);
@@ -270,84 +306,119 @@ moe_route_kernel(MoeParams p) {
   }
   if (p.identity == 0) return;
   __syncthreads();   // the choice is written
-  for (int place = 0; place < p.top; ++place) {
-    const size_t a = static_cast<size_t>(t) * p.slots + place;
+  for (int place = 0; place < here * p.top; ++place) {
+    const int n = place / p.top;
+    const size_t a = static_cast<size_t>(first_token + n) * p.slots + place % p.top;
     if (p.chosen[a] >= 0) continue;
     const float w = p.weight[a];
-    for (int i = threadIdx.x; i < p.hidden; i += kRouteThreads) p.rows[a * p.hidden + i] = w * h_s[i];
+    for (int i = threadIdx.x; i < p.hidden; i += kRouteThreads) p.rows[a * p.hidden + i] = w * h_all[n * p.hidden + i];
   }
 }
 
-// One block: assignments counted per expert, the experts' runs cut into tiles, the sorted order.
+// One block: assignments counted per expert, the experts' runs cut into tiles, the sorted order.  A chain of
+// dependent reads, atomics and barriers bounds it: a thread has eight assignments' reads in flight, and the runs'
+// places are a scan over the experts (10,240 assignments to
+// 17 units: 15.4 us one by one, GROUPED).
 __global__ void __launch_bounds__(1024)
 moe_group_kernel(MoeParams p) {
   __shared__ int count[kMaxExperts];
   __shared__ int start[kMaxExperts];
+  __shared__ int warp_tiles[32], warp_places[32];
   pdl_launch_dependents();
   pdl_wait();
-  const int assignments = p.num_tokens * p.slots;
+  constexpr int kBatch = 8;
+  const int assignments = p.num_tokens * p.slots, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int matrices = moe_matrices(p);
-  for (int e = threadIdx.x; e < matrices; e += blockDim.x) count[e] = 0;
-  for (int tile = threadIdx.x; tile < p.max_tiles; tile += blockDim.x) p.tile_expert[tile] = 0;
+  static_assert(kMaxExperts <= 1024, "a thread per unit");
+  if (tid < kMaxExperts) count[tid] = 0;
+  for (int tile = tid; tile < p.max_tiles; tile += blockDim.x) p.tile_expert[tile] = 0;
   if (p.padded)
-    for (int place = threadIdx.x; place < p.max_tiles * p.tile_rows; place += blockDim.x) p.order[place] = -1;
+    for (int place = tid; place < p.max_tiles * p.tile_rows; place += blockDim.x) p.order[place] = -1;
   __syncthreads();
-  for (int a = threadIdx.x; a < assignments; a += blockDim.x)
-    p.rank[a] = p.chosen[a] >= 0 ? atomicAdd(&count[p.chosen[a]], 1) : -1;   // (-1: no matrices, no place)
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int place = 0, tile = 0;
-    for (int e = 0; e < matrices; ++e) {
-      start[e] = place;
-      int first = 0;
-      for (; first < count[e] && tile < p.max_tiles; first += p.tile_rows, ++tile) {
-        p.tiles[1 + 3 * tile] = e;
-        p.tiles[2 + 3 * tile] = place + first;
-        p.tiles[3 + 3 * tile] = min(p.tile_rows, count[e] - first);
-        p.tile_expert[tile] = e;
-      }
-      place += p.padded ? first : count[e];
+  for (int base = 0; base < assignments; base += 1024 * kBatch) {
+    int unit[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int a = base + j * 1024 + tid;
+      unit[j] = a < assignments ? p.chosen[a] : -1;
     }
-    p.tiles[0] = tile;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int a = base + j * 1024 + tid;
+      if (base + j * 1024 >= assignments) break;
+      // (-1: no matrices, no place)
+      if (a < assignments) p.rank[a] = unit[j] >= 0 ? atomicAdd(&count[unit[j]], 1) : -1;
+    }
   }
   __syncthreads();
-  for (int a = threadIdx.x; a < assignments; a += blockDim.x) {
-    if (p.chosen[a] < 0) continue;
-    const int place = start[p.chosen[a]] + p.rank[a];
-    p.rank[a] = place;
-    p.order[place] = a;
+  // each unit's first tile and first place: a scan of both over the units
+  const int mine = tid < matrices ? count[tid] : 0, tiles = (mine + p.tile_rows - 1) / p.tile_rows;
+  const int places = p.padded ? tiles * p.tile_rows : mine;
+  int tiles_to = tiles, places_to = places;
+#pragma unroll
+  for (int offset = 1; offset < 32; offset <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, tiles_to, offset), q = __shfl_up_sync(0xffffffffu, places_to, offset);
+    if (lane >= offset) tiles_to += t, places_to += q;
+  }
+  if (lane == 31) warp_tiles[warp] = tiles_to, warp_places[warp] = places_to;
+  __syncthreads();
+  int tile = tiles_to - tiles, place = places_to - places;
+  for (int w = 0; w < warp; ++w) tile += warp_tiles[w], place += warp_places[w];
+  if (tid < matrices) {
+    start[tid] = place;
+    for (int first = 0; first < mine && tile < p.max_tiles; first += p.tile_rows, ++tile) {
+      p.tiles[1 + 3 * tile] = tid;
+      p.tiles[2 + 3 * tile] = place + first;
+      p.tiles[3 + 3 * tile] = min(p.tile_rows, mine - first);
+      p.tile_expert[tile] = tid;
+    }
+    if (tid == matrices - 1) p.tiles[0] = tile;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int a = tid; a < assignments; a += 1024) {
+    const int unit = p.chosen[a], rank = p.rank[a];
+    if (unit < 0) continue;
+    const int at = start[unit] + rank;
+    p.rank[a] = at;
+    p.order[at] = a;
   }
 }
 
-// Padded form: the tokens' rows in sorted order (zero where a place pads a run); a block per place.
+// Padded form: the tokens' rows in sorted order (zero where a place pads a run); a warp per place, eight vectors of a
+// lane in flight (12,416 places of 1,536 bfloat16 values: 15.3 us a block of 128 per place, 9.2 us).
+constexpr int kGatherRows = 8;   // places of a block
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * kGatherRows)
 moe_gather_kernel(MoeParams p) {
   pdl_launch_dependents();
   pdl_wait();
-  const int place = blockIdx.x;
+  const int place = blockIdx.x * kGatherRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;   // (a tile is whole blocks)
   if (place / p.tile_rows >= p.tiles[0]) return;
   const int a = p.order[place];
   const int vectors = p.hidden * static_cast<int>(sizeof(T)) / 16;   // the caller sees to whole vectors
   uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.xs) + static_cast<size_t>(place) * p.hidden);
-  if (a < 0) {
-    for (int i = threadIdx.x; i < vectors; i += blockDim.x) dst[i] = make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(p.h) + static_cast<size_t>(a / p.slots) * p.hidden);
-  if (p.input_weight && a % p.slots < p.top) {
-    constexpr int kPer = 16 / static_cast<int>(sizeof(T));
-    const float w = p.weight[a];
-    for (int i = threadIdx.x; i < vectors; i += blockDim.x) {
-      uint4 raw = src[i];
-      T* values = reinterpret_cast<T*>(&raw);
+  const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(p.h) + static_cast<size_t>(a < 0 ? 0 : a / p.slots) * p.hidden);
+  const bool weighted = a >= 0 && p.input_weight && a % p.slots < p.top;
+  const float w = weighted ? p.weight[a] : 1.0f;
+  constexpr int kPer = 16 / static_cast<int>(sizeof(T)), kBatch = 8;
+  for (int base = lane; base < vectors; base += 32 * kBatch) {
+    uint4 v[kBatch];
 #pragma unroll
-      for (int e = 0; e < kPer; ++e) values[e] = from_float<T>(w * to_float<T>(values[e]));
-      dst[i] = raw;
+    for (int j = 0; j < kBatch; ++j) {
+      v[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (a >= 0 && base + 32 * j < vectors) v[j] = src[base + 32 * j];
     }
-    return;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      if (weighted) {
+        T* values = reinterpret_cast<T*>(&v[j]);
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) values[e] = from_float<T>(w * to_float<T>(values[e]));
+      }
+      if (base + 32 * j < vectors) dst[base + 32 * j] = v[j];
+    }
   }
-  for (int i = threadIdx.x; i < vectors; i += blockDim.x) dst[i] = src[i];
 }
 
 // Padded form: rows[a, :] = w_a * ys[sorted place of a, :].
@@ -364,6 +435,43 @@ moe_scatter_kernel(MoeParams p) {
   float4 v = reinterpret_cast<const float4*>(p.ys + static_cast<size_t>(p.rank[a]) * p.hidden)[c];
   v.x *= w, v.y *= w, v.z *= w, v.w *= w;
   reinterpret_cast<float4*>(p.rows + static_cast<size_t>(a) * p.hidden)[c] = v;
+}
+
+// Padded form: target[t, :] += the sum over t's places of w_a * ys[sorted place of a, :], in the order of the places and
+// rounded as moe_scatter_kernel and moe_add_rows_kernel do: without their pass through `rows` (2,048 tokens of 5 places and
+// 1,536 values: 45 us the two, 18.5 us).
+__global__ void __launch_bounds__(256)
+moe_sum_kernel(MoeParams p, float* __restrict__ target) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int quarter = p.hidden / 4;
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= static_cast<long long>(p.num_tokens) * quarter) return;
+  const int t = static_cast<int>(i / quarter), c = static_cast<int>(i % quarter);
+  float4* at = reinterpret_cast<float4*>(target) + i;
+  const float4 before = *at;
+  float4 sum;
+  constexpr int kBatch = 4;
+  for (int first = 0; first < p.slots; first += kBatch) {
+    float4 v[kBatch];
+    float w[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      if (first + j >= p.slots) break;
+      const int a = t * p.slots + first + j, rank = p.rank[a];
+      // (without matrices: the router's block wrote the weighted row)
+      w[j] = rank < 0 ? 1.0f : moe_output_weight(p, a);
+      v[j] = reinterpret_cast<const float4*>(rank < 0 ? p.rows + static_cast<size_t>(a) * p.hidden : p.ys + static_cast<size_t>(rank) * p.hidden)[c];
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      if (first + j >= p.slots) break;
+      const float4 x = make_float4(__fmul_rn(v[j].x, w[j]), __fmul_rn(v[j].y, w[j]), __fmul_rn(v[j].z, w[j]), __fmul_rn(v[j].w, w[j]));
+      if (first + j == 0) sum = x;
+      else sum.x += x.x, sum.y += x.y, sum.z += x.z, sum.w += x.w;
+    }
+  }
+  *at = make_float4(before.x + sum.x, before.y + sum.y, before.z + sum.z, before.w + sum.w);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -605,21 +713,33 @@ static int launch_skinny(const MoeParams& p, cudaStream_t s) {
   return vipera_launch(moe_skinny_kernel<T, MODE, 1>, grid, 256, shared, s, p);
 }
 
-// The router, the grouping and (padded form) the gathered rows.
-template <typename T>
-static int launch_route(const MoeParams& p, cudaStream_t s) {
-  const size_t route_shared = static_cast<size_t>(2 * p.experts + p.always_gate + p.groups + p.hidden) * sizeof(float);
+template <typename T, int TOKENS>
+static int launch_router(const MoeParams& p, cudaStream_t s) {
+  const size_t shared = TOKENS * static_cast<size_t>(2 * p.experts + p.always_gate + p.groups + p.hidden) * sizeof(float);
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(moe_route_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(moe_route_kernel<T, TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
       return VIPERA_BAD_ARGUMENT;
     configured = true;
   }
-  int status = vipera_launch(moe_route_kernel<T>, p.num_tokens, kRouteThreads, route_shared, s, p);
+  return vipera_launch(moe_route_kernel<T, TOKENS>, (p.num_tokens + TOKENS - 1) / TOKENS, kRouteThreads, shared, s, p);
+}
+
+// The router, the grouping and (padded form) the gathered rows.
+template <typename T>
+static int launch_route(const MoeParams& p, cudaStream_t s) {
+  // four tokens a block where that still leaves every SM a block, their rows and the router's are whole vectors, and
+  // several blocks' rows fit an SM
+  constexpr int kTokens = 4;
+  const bool several = p.num_tokens >= kTokens * 148 && p.hidden % 4 == 0 && (reinterpret_cast<uintptr_t>(p.router) & 15) == 0 &&
+                       reinterpret_cast<uintptr_t>(p.h) % (4 * sizeof(T)) == 0 &&
+                       kTokens * static_cast<size_t>(2 * p.experts + p.always_gate + p.groups + p.hidden) * sizeof(float) <= 64 * 1024;
+  int status = several ? launch_router<T, kTokens>(p, s) : launch_router<T, 1>(p, s);
   if (status) return status;
   status = vipera_launch(moe_group_kernel, 1, 1024, 0, s, p);
   if (status || !p.padded) return status;
-  return vipera_launch(moe_gather_kernel<T>, p.max_tiles * p.tile_rows, 128, 0, s, p);
+  static_assert(128 % kGatherRows == 0, "a tile is whole blocks");
+  return vipera_launch(moe_gather_kernel<T>, p.max_tiles * p.tile_rows / kGatherRows, 32 * kGatherRows, 0, s, p);
 }
 
 template <typename T>
@@ -683,6 +803,15 @@ VIPERA_API int vipera_moe_scatter(const MoeParams* params, void* stream) {
   if (!p.padded || p.hidden % 4) return VIPERA_BAD_ARGUMENT;
   const long long count = static_cast<long long>(p.num_tokens) * p.slots * (p.hidden / 4);
   return vipera_launch(moe_scatter_kernel, static_cast<unsigned>((count + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), p);
+}
+
+// Instead of vipera_moe_scatter and the sum of its rows: target [tokens, hidden] (16-byte aligned) += the mixture's output.
+VIPERA_API int vipera_moe_sum(const MoeParams* params, float* target, void* stream) {
+  const MoeParams& p = *params;
+  if (p.num_tokens <= 0) return VIPERA_OK;
+  if (!p.padded || p.hidden % 4 || !target || (reinterpret_cast<uintptr_t>(target) & 15)) return VIPERA_BAD_ARGUMENT;
+  const long long count = static_cast<long long>(p.num_tokens) * (p.hidden / 4);
+  return vipera_launch(moe_sum_kernel, static_cast<unsigned>((count + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), p, target);
 }
 
 VIPERA_API int vipera_moe_params_size() { return static_cast<int>(sizeof(MoeParams)); }

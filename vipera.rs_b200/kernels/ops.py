@@ -2052,7 +2052,8 @@ def moe(h: torch.Tensor, *, router: torch.Tensor, gate_up: torch.Tensor, down: t
         xs: Optional[torch.Tensor] = None, ys: Optional[torch.Tensor] = None, gated: bool = True,
         correction: Optional[torch.Tensor] = None, identity: int = 0, always: int = 0, route_scale: float = 1.0,
         renorm_eps: float = 0.0, logit_scores: bool = False, always_gate: bool = False,
-        unit_limit: Optional[torch.Tensor] = None, unit_slope: float = 0.0, input_weight: bool = False) -> None:
+        unit_limit: Optional[torch.Tensor] = None, unit_slope: float = 0.0, input_weight: bool = False,
+        target: Optional[torch.Tensor] = None) -> None:
     """A mixture of gated units over a step.  ``h`` [tokens, hidden]; ``router`` float32 [experts,
     hidden]; ``gate_up`` [experts, 2 ff, hidden] (``gate_group`` gate rows, then the up rows of the
     same features, and so on) and ``down`` [experts, hidden, ff] in h's type.  ``chosen`` int32 and
@@ -2073,7 +2074,8 @@ def moe(h: torch.Tensor, *, router: torch.Tensor, gate_up: torch.Tensor, down: t
     weights the softmax over the chosen ones.  ``always_gate``: ``router`` has one row more, and the
     always-used units' weight is the sigmoid of its product with h.  Activation ACT_CLAMPED: gated units
     with the bounds ``unit_limit`` (float32, one per unit with matrices) and ``unit_slope``.
-    ``input_weight``: a chosen expert's weight multiplies what it reads and not its output."""
+    ``input_weight``: a chosen expert's weight multiplies what it reads and not its output.
+    ``target`` float32 [tokens, hidden]: the mixture's output is added to it, and what ``rows`` holds is not said."""
     fn = _function("moe", "vipera_moe", [ctypes.POINTER(_MoeParams), _c_int, _c_void])
     _check_struct("moe", "vipera_moe_params_size", _MoeParams)
     tokens, hidden = h.shape
@@ -2101,6 +2103,8 @@ def moe(h: torch.Tensor, *, router: torch.Tensor, gate_up: torch.Tensor, down: t
     if chosen.numel() < assignments or weight.numel() < assignments or scratch.numel() < moe_scratch_words(tokens, top, experts) or \
             act.numel() < capacity * ff or act.dtype != h.dtype or rows.numel() < assignments * hidden:
         raise InvalidArgumentError("moe: a scratch buffer is too small")
+    if target is not None and tuple(target.shape) != (tokens, hidden):
+        raise InvalidArgumentError("moe: target must be [tokens, hidden]")
     p = _MoeParams()
     p.h, p.router = _gpu(h, "h"), _gpu(router, "router", torch.float32)
     p.gate_up, p.down = _gpu(gate_up, "gate_up"), _gpu(down, "down")
@@ -2123,6 +2127,8 @@ def moe(h: torch.Tensor, *, router: torch.Tensor, gate_up: torch.Tensor, down: t
     p.gate_group, p.tile_rows, p.padded = int(gate_group), int(tile_rows), int(padded)
     if not padded:
         _check(fn(ctypes.byref(p), dtype_code(h.dtype), _stream()), "moe", kernels=4)
+        if target is not None:
+            add_rows(rows.view(-1)[:assignments * hidden], top, target)
         return
     if xs.numel() < capacity * hidden or ys.numel() < capacity * hidden or xs.dtype != h.dtype:
         raise InvalidArgumentError("moe: a scratch buffer is too small")
@@ -2136,8 +2142,14 @@ def moe(h: torch.Tensor, *, router: torch.Tensor, gate_up: torch.Tensor, down: t
                     activation=activation, unit_limit=unit_limit if activation == ACT_CLAMPED else None,
                     unit_slope=unit_slope, what="moe")
     gemm_tc_grouped(act_rows, down, tile_expert, epilogue=EPI_STORE, out=ys_rows, what="moe")
+    if target is not None and target.data_ptr() % 16 == 0:
+        total = _function("moe", "vipera_moe_sum", [ctypes.POINTER(_MoeParams), _c_void, _c_void])
+        _check(total(ctypes.byref(p), _gpu(target, "target", torch.float32), _stream()), "moe")
+        return
     scatter = _function("moe", "vipera_moe_scatter", [ctypes.POINTER(_MoeParams), _c_void])
     _check(scatter(ctypes.byref(p), _stream()), "moe")
+    if target is not None:
+        add_rows(rows.view(-1)[:assignments * hidden], top, target)
 
 
 def add_rows(rows: torch.Tensor, parts: int, target: torch.Tensor) -> None:

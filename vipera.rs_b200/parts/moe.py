@@ -201,11 +201,8 @@ class MixtureOfExperts(FeedForward):
                 act=act, rows=rows, xs=xs, ys=ys, gated=self.gated, correction=self.correction, identity=self.identity,
                 always=self.always, route_scale=self.route_scale, renorm_eps=self.renorm_eps, logit_scores=self.logit_scores,
                 always_gate=self.shared_gate, unit_limit=self.unit_limit, unit_slope=self.unit_slope,
-                input_weight=self.input_weight)
-        if residual is None:
-            return rows, self.slots
-        ops.add_rows(rows, self.slots, residual)
-        return None
+                input_weight=self.input_weight, target=residual)
+        return (rows, self.slots) if residual is None else None
 
 
 FEED_FORWARDS.register("moe_mlp", MixtureOfExperts)
