@@ -318,7 +318,7 @@ moe_route_kernel(MoeParams p) {
 // One block: assignments counted per expert, the experts' runs cut into tiles, the sorted order.  A chain of
 // dependent reads, atomics and barriers bounds it: a thread has eight assignments' reads in flight, and the runs'
 // places are a scan over the experts (10,240 assignments to
-// 17 units: 15.4 us one by one, GROUPED).
+// 17 units: 15.4 us one by one, 10.7 so).
 __global__ void __launch_bounds__(1024)
 moe_group_kernel(MoeParams p) {
   __shared__ int count[kMaxExperts];
