@@ -593,6 +593,38 @@ mlstm_chunk_tc_kernel(const MlstmParams p) {
 //      outputs of the chunk from the state, n and m at its start, exactly as in the kernel above.
 // The sums are associated differently from the walking kernel's (U is summed before it meets
 // S), which is 32-bit rounding only.
+// q, k, v and S lie in shared memory as they lie in memory, and the products' fragments that want them the other way
+// come through ldmatrix's transposition: values stored one by one into transposed rows met one bank sixteen
+// at a time, which bounded both kernels.  2,048 tokens, 8 heads of 256 x 512: parts 160 us, now 60; outputs 233 us, now 151;
+// the scan, with eight chunks' reads in flight instead of four and the gates' among them, 70 us, now 64.  What bounds them now:
+// the chunks' states of 32 bits (134 MB written, read, written and read) and the projections' rows read again for
+// every tile of value columns.
+__device__ __forceinline__ void load_four(uint32_t (&r)[4], const __nv_bfloat16* at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(at))) : "memory");
+}
+__device__ __forceinline__ void load_four_turned(uint32_t (&r)[4], const __nv_bfloat16* at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(at))) : "memory");
+}
+// Fragments of arrays of `stride` elements a row.  Left operand [row][inner] at (row0, k0), and the same from [inner][row];
+// right operand for sixteen columns, registers 0, 1 the first eight's and 2, 3 the others', from [column][inner] and [inner][column].
+__device__ __forceinline__ void left(uint32_t (&r)[4], const __nv_bfloat16* base, int stride, int row0, int k0, int lane) {
+  load_four(r, base + (row0 + (lane & 15)) * stride + k0 + (lane >> 4) * 8);
+}
+__device__ __forceinline__ void left_turned(uint32_t (&r)[4], const __nv_bfloat16* base, int stride, int row0, int k0, int lane) {
+  load_four_turned(r, base + (k0 + (lane & 7) + (lane >> 4) * 8) * stride + row0 + (lane >> 3 & 1) * 8);
+}
+__device__ __forceinline__ void right(uint32_t (&r)[4], const __nv_bfloat16* base, int stride, int column0, int k0, int lane) {
+  load_four(r, base + (column0 + (lane & 7) + (lane >> 4) * 8) * stride + k0 + (lane >> 3 & 1) * 8);
+}
+__device__ __forceinline__ void right_turned(uint32_t (&r)[4], const __nv_bfloat16* base, int stride, int column0, int k0, int lane) {
+  load_four_turned(r, base + (k0 + (lane & 15)) * stride + column0 + (lane >> 4) * 8);
+}
+__device__ __forceinline__ void store_four(__nv_bfloat16* at, const float4& v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(at) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
 __device__ __forceinline__ bool find_job(const MlstmParams& p, int job, int* entry, int* chunk) {
   int remaining = job;
   for (int e = 0; e < p.num_entries; ++e) {
@@ -610,8 +642,8 @@ __device__ __forceinline__ bool find_job(const MlstmParams& p, int job, int* ent
 
 template <int D>
 struct PartsLayout {
-  static constexpr int kLS = kTcChunk + 8;
-  static constexpr size_t kBytes = (static_cast<size_t>(D) * kLS + kTcTile * kLS) * 2 + (3 * kTcChunk + 8) * 4;
+  static constexpr int kQS = D + 8, kVS = kTcTile + 8;
+  static constexpr size_t kBytes = (static_cast<size_t>(kTcChunk) * kQS + kTcChunk * kVS) * 2 + (3 * kTcChunk + 8) * 4;
 };
 
 template <int D>
@@ -619,14 +651,14 @@ __global__ void __launch_bounds__(kTcThreads)
 mlstm_parts_kernel(const MlstmParams p) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int L = kTcChunk, TW = kTcTile, LS = PartsLayout<D>::kLS;
+  constexpr int L = kTcChunk, TW = kTcTile, QS = PartsLayout<D>::kQS, VS = PartsLayout<D>::kVS;
   constexpr int WM = D >= 128 ? 8 : 4, WN = 8 / WM, MT = D / 16 / WM, NT = 8 / WN;
   int e, chunk;
   if (!find_job(p, blockIdx.z, &e, &chunk)) return;
   extern __shared__ __align__(16) unsigned char raw[];
-  __nv_bfloat16* Kt = reinterpret_cast<__nv_bfloat16*>(raw);   // [D][LS]
-  __nv_bfloat16* Vt = Kt + D * LS;                             // [TW][LS]
-  float* lis = reinterpret_cast<float*>(Vt + TW * LS);         // [L]
+  __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(raw);   // [L][QS]
+  __nv_bfloat16* Vs = Ks + L * QS;                             // [L][VS]
+  float* lis = reinterpret_cast<float*>(Vs + L * VS);          // [L]
   float* lfs = lis + L;                                        // [L]
   float* we = lfs + L;                                         // [L] exp(a_s - A)
   float* scal = we + L;                                        // [0] A, [1] B
@@ -672,19 +704,21 @@ mlstm_parts_kernel(const MlstmParams p) {
     }
   }
   __syncthreads();
+  const bool wide_v = wide && p.v_off % 4 == 0;   // (the value size is a multiple of four)
+#pragma unroll 8
   for (int item = tid; item < L * (D / 4); item += kTcThreads) {
     const int t = item / (D / 4), dd = (item % (D / 4)) * 4;
     float4 k = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (t < len) k = load4(rows + static_cast<size_t>(t) * p.proj_width + p.k_off + h * d + dd, wide);
-    Kt[dd * LS + t] = __float2bfloat16_rn(k.x);
-    Kt[(dd + 1) * LS + t] = __float2bfloat16_rn(k.y);
-    Kt[(dd + 2) * LS + t] = __float2bfloat16_rn(k.z);
-    Kt[(dd + 3) * LS + t] = __float2bfloat16_rn(k.w);
+    store_four(Ks + t * QS + dd, k);
   }
-  for (int item = tid; item < L * TW; item += kTcThreads) {
-    const int t = item / TW, c = item % TW;
-    const float v = (t < len && c < cols) ? rows[static_cast<size_t>(t) * p.proj_width + p.v_off + h * dv + c0 + c] : 0.0f;
-    Vt[c * LS + t] = __float2bfloat16_rn(v * we[t]);
+#pragma unroll
+  for (int item = tid; item < L * (TW / 4); item += kTcThreads) {
+    const int t = item / (TW / 4), c = (item % (TW / 4)) * 4;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (t < len && c < cols) v = load4(rows + static_cast<size_t>(t) * p.proj_width + p.v_off + h * dv + c0 + c, wide_v);
+    const float w = we[t];
+    store_four(Vs + t * VS + c, make_float4(v.x * w, v.y * w, v.z * w, v.w * w));
   }
   __syncthreads();
   float S[MT][NT][4];
@@ -697,13 +731,15 @@ mlstm_parts_kernel(const MlstmParams p) {
 #pragma unroll
   for (int kk = 0; kk < L / 16; ++kk) {
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      uint32_t a[4];
-      load_a(a, Kt, LS, (sm * MT + mt) * 16, kk * 16, g, tq);
+    for (int nt = 0; nt < NT; nt += 2) {
+      uint32_t b[4];
+      right_turned(b, Vs, VS, (sn * NT + nt) * 8, kk * 16, lane);
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const __nv_bfloat16* at = Vt + ((sn * NT + nt) * 8 + g) * LS + kk * 16 + 2 * tq;
-        mma_bf16(S[mt][nt], a, ld32(at), ld32(at + 8));
+      for (int mt = 0; mt < MT; ++mt) {
+        uint32_t a[4];
+        left_turned(a, Ks, QS, (sm * MT + mt) * 16, kk * 16, lane);
+        mma_bf16(S[mt][nt], a, b[0], b[1]);
+        mma_bf16(S[mt][nt + 1], a, b[2], b[3]);
       }
     }
   }
@@ -722,7 +758,7 @@ mlstm_parts_kernel(const MlstmParams p) {
     float* u = p.chunk_n + (static_cast<size_t>(job) * p.heads + h) * d;
     for (int dd = tid; dd < d; dd += kTcThreads) {
       float acc = 0.0f;
-      for (int t = 0; t < len; ++t) acc = fmaf(we[t], __bfloat162float(Kt[dd * LS + t]), acc);
+      for (int t = 0; t < len; ++t) acc = fmaf(we[t], __bfloat162float(Ks[t * QS + dd]), acc);
       u[dd] = acc;
     }
     if (tid == 0) {
@@ -765,17 +801,23 @@ mlstm_scan_kernel(const MlstmParams p) {
     for (int i = 0; i < 2; ++i)
       if (threadIdx.x + 256 * i < d) n[i] = n_state[threadIdx.x + 256 * i];
   float* U = p.chunk_state + (static_cast<size_t>(job0) * p.heads + h) * total + index;
-  for (int c0 = 0; c0 < chunks; c0 += 4) {
-    float4 own[4];
+  constexpr int kAhead = 8;   // chunks whose reads are in flight
+  for (int c0 = 0; c0 < chunks; c0 += kAhead) {
+    float4 own[kAhead];
+    float tops[kAhead], sums[kAhead];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (live && c0 + j < chunks) own[j] = *reinterpret_cast<const float4*>(U + (c0 + j) * job_stride);
+    for (int j = 0; j < kAhead; ++j) {
+      if (c0 + j >= chunks) break;
+      if (live) own[j] = *reinterpret_cast<const float4*>(U + (c0 + j) * job_stride);
+      const float* aux = p.chunk_aux + (static_cast<size_t>(job0 + c0 + j) * p.heads + h) * 4;
+      tops[j] = aux[0], sums[j] = aux[1];
+    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < kAhead; ++j) {
       if (c0 + j >= chunks) break;
       const int job = job0 + c0 + j;
       float* aux = p.chunk_aux + (static_cast<size_t>(job) * p.heads + h) * 4;
-      const float A = aux[0], B = aux[1];
+      const float A = tops[j], B = sums[j];
       const float M = fmaxf(m, A);
       const float keep = expf(m - M), take = expf(A - M);
       if (live) {
@@ -809,9 +851,11 @@ mlstm_scan_kernel(const MlstmParams p) {
 
 template <int D>
 struct OutputsLayout {
-  static constexpr int kQS = D + 8, kLS = kTcChunk + 8;
-  // (S^T takes K's place once the scores are done: two blocks fit an SM at the largest size)
-  static constexpr size_t kBytes = (2 * static_cast<size_t>(kTcChunk) * kQS + kTcTile * kLS + kTcChunk * kLS) * 2 +
+  static constexpr int kQS = D + 8, kLS = kTcChunk + 8, kVS = kTcTile + 8;
+  // (S takes K's place once the scores are done: two blocks fit an SM at the largest size)
+  static constexpr size_t kKeys = static_cast<size_t>(kTcChunk) * kQS > static_cast<size_t>(D) * kVS ? static_cast<size_t>(kTcChunk) * kQS
+                                                                                                    : static_cast<size_t>(D) * kVS;
+  static constexpr size_t kBytes = (static_cast<size_t>(kTcChunk) * kQS + kKeys + kTcChunk * kVS + kTcChunk * kLS) * 2 +
                                    (D + 8 * kTcChunk + 8) * 4;
 };
 
@@ -820,16 +864,15 @@ __global__ void __launch_bounds__(kTcThreads)
 mlstm_outputs_kernel(const MlstmParams p) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int L = kTcChunk, TW = kTcTile, QS = OutputsLayout<D>::kQS, LS = OutputsLayout<D>::kLS;
+  constexpr int L = kTcChunk, TW = kTcTile, QS = OutputsLayout<D>::kQS, LS = OutputsLayout<D>::kLS, VS = OutputsLayout<D>::kVS;
   int e, chunk;
   if (!find_job(p, blockIdx.z, &e, &chunk)) return;
   extern __shared__ __align__(16) unsigned char raw[];
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(raw);   // [L][QS]
   __nv_bfloat16* Ks = Qs + L * QS;                             // [L][QS]
-  __nv_bfloat16* Vt = Ks + L * QS;                             // [TW][LS]
-  __nv_bfloat16* Ws = Vt + TW * LS;                            // [L][LS]
-  __nv_bfloat16* St = Ks;                                      // [TW][QS] in K's place, after the scores
-  static_assert(kTcTile <= kTcChunk, "S^T must fit where K lay");
+  __nv_bfloat16* Vs = Ks + OutputsLayout<D>::kKeys;            // [L][VS]
+  __nv_bfloat16* Ws = Vs + L * VS;                             // [L][LS]
+  __nv_bfloat16* Ss = Ks;                                      // [D][VS] in K's place, after the scores
   float* ns = reinterpret_cast<float*>(Ws + L * LS);           // [D] n at the chunk's start
   float* av = ns + D;
   float* Mv = av + L;
@@ -851,6 +894,9 @@ mlstm_outputs_kernel(const MlstmParams p) {
   const float* S_start = p.chunk_state + (static_cast<size_t>(job) * p.heads + h) * d * dv;
   const float* n_start = p.chunk_n + (static_cast<size_t>(job) * p.heads + h) * d;
   for (int dd = tid; dd < d; dd += kTcThreads) ns[dd] = n_start[dd];
+  const bool wide_v = wide && p.v_off % 4 == 0;   // (the value size is a multiple of four)
+  const bool pairs = (reinterpret_cast<uintptr_t>(p.o_raw) & 7) == 0;
+#pragma unroll 4
   for (int item = tid; item < L * (D / 4); item += kTcThreads) {
     const int t = item / (D / 4), dd = (item % (D / 4)) * 4;
     float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f), k = q;
@@ -859,15 +905,15 @@ mlstm_outputs_kernel(const MlstmParams p) {
       q = load4(row + p.q_off + h * d + dd, wide);
       k = load4(row + p.k_off + h * d + dd, wide);
     }
-    *reinterpret_cast<__nv_bfloat162*>(Qs + t * QS + dd) = __floats2bfloat162_rn(q.x * p.q_scale, q.y * p.q_scale);
-    *reinterpret_cast<__nv_bfloat162*>(Qs + t * QS + dd + 2) = __floats2bfloat162_rn(q.z * p.q_scale, q.w * p.q_scale);
-    *reinterpret_cast<__nv_bfloat162*>(Ks + t * QS + dd) = __floats2bfloat162_rn(k.x, k.y);
-    *reinterpret_cast<__nv_bfloat162*>(Ks + t * QS + dd + 2) = __floats2bfloat162_rn(k.z, k.w);
+    store_four(Qs + t * QS + dd, make_float4(q.x * p.q_scale, q.y * p.q_scale, q.z * p.q_scale, q.w * p.q_scale));
+    store_four(Ks + t * QS + dd, k);
   }
-  for (int item = tid; item < L * TW; item += kTcThreads) {
-    const int t = item / TW, c = item % TW;
-    const float v = (t < len && c < cols) ? rows[static_cast<size_t>(t) * p.proj_width + p.v_off + h * dv + c0 + c] : 0.0f;
-    Vt[c * LS + t] = __float2bfloat16_rn(v);
+#pragma unroll
+  for (int item = tid; item < L * (TW / 4); item += kTcThreads) {
+    const int t = item / (TW / 4), c = (item % (TW / 4)) * 4;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (t < len && c < cols) v = load4(rows + static_cast<size_t>(t) * p.proj_width + p.v_off + h * dv + c0 + c, wide_v);
+    store_four(Vs + t * VS + c, v);
   }
   if (tid < L) {
     float li = 0.0f, lf = 0.0f;
@@ -908,6 +954,15 @@ mlstm_outputs_kernel(const MlstmParams p) {
     Mv[2 * lane + 1] = fmaxf(m0, scan);
   }
   __syncthreads();
+  // the state at the chunk's start: asked for here, laid where K is once the scores are done (whole fours: the value size is)
+  constexpr int kStateFours = D * (TW / 4) / kTcThreads;
+  float4 state_fours[kStateFours];
+#pragma unroll
+  for (int i = 0; i < kStateFours; ++i) {
+    const int item = tid + i * kTcThreads, dd = item / (TW / 4), c = (item % (TW / 4)) * 4;
+    state_fours[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (c < cols) state_fours[i] = *reinterpret_cast<const float4*>(S_start + static_cast<size_t>(dd) * dv + c0 + c);
+  }
   {
     float G[4][4];
 #pragma unroll
@@ -916,12 +971,13 @@ mlstm_outputs_kernel(const MlstmParams p) {
       for (int i = 0; i < 4; ++i) G[j][i] = 0.0f;
 #pragma unroll 4
     for (int kk = 0; kk < D / 16; ++kk) {
-      uint32_t a[4];
-      load_a(a, Qs, QS, rm * 16, kk * 16, g, tq);
+      uint32_t a[4], b[4];
+      left(a, Qs, QS, rm * 16, kk * 16, lane);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const __nv_bfloat16* at = Ks + (cn * 32 + j * 8 + g) * QS + kk * 16 + 2 * tq;
-        mma_bf16(G[j], a, ld32(at), ld32(at + 8));
+      for (int j = 0; j < 4; j += 2) {
+        right(b, Ks, QS, cn * 32 + j * 8, kk * 16, lane);
+        mma_bf16(G[j], a, b[0], b[1]);
+        mma_bf16(G[j + 1], a, b[2], b[3]);
       }
     }
     float sums[2] = {0.0f, 0.0f};
@@ -956,20 +1012,10 @@ mlstm_outputs_kernel(const MlstmParams p) {
     if (part == 0) qn[t] = sum;
   }
   __syncthreads();
-  // the state at the chunk's start, transposed, where K lay
-  for (int item = tid; item < D * (TW / 4); item += kTcThreads) {
-    const int dd = item / (TW / 4), c = (item % (TW / 4)) * 4;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (c + 3 < cols) v = *reinterpret_cast<const float4*>(S_start + static_cast<size_t>(dd) * dv + c0 + c);
-    else {
-      float* lanes = reinterpret_cast<float*>(&v);
-      for (int i = 0; i < 4; ++i)
-        if (c + i < cols) lanes[i] = S_start[static_cast<size_t>(dd) * dv + c0 + c + i];
-    }
-    St[c * QS + dd] = __float2bfloat16_rn(v.x);
-    St[(c + 1) * QS + dd] = __float2bfloat16_rn(v.y);
-    St[(c + 2) * QS + dd] = __float2bfloat16_rn(v.z);
-    St[(c + 3) * QS + dd] = __float2bfloat16_rn(v.w);
+#pragma unroll
+  for (int i = 0; i < kStateFours; ++i) {
+    const int item = tid + i * kTcThreads, dd = item / (TW / 4), c = (item % (TW / 4)) * 4;
+    store_four(Ss + dd * VS + c, state_fours[i]);
   }
   __syncthreads();
   float O[4][4];
@@ -979,12 +1025,13 @@ mlstm_outputs_kernel(const MlstmParams p) {
     for (int i = 0; i < 4; ++i) O[j][i] = 0.0f;
 #pragma unroll 4
   for (int kk = 0; kk < D / 16; ++kk) {
-    uint32_t a[4];
-    load_a(a, Qs, QS, rm * 16, kk * 16, g, tq);
+    uint32_t a[4], b[4];
+    left(a, Qs, QS, rm * 16, kk * 16, lane);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat16* at = St + (cn * 32 + j * 8 + g) * QS + kk * 16 + 2 * tq;
-      mma_bf16(O[j], a, ld32(at), ld32(at + 8));
+    for (int j = 0; j < 4; j += 2) {
+      right_turned(b, Ss, VS, cn * 32 + j * 8, kk * 16, lane);
+      mma_bf16(O[j], a, b[0], b[1]);
+      mma_bf16(O[j + 1], a, b[2], b[3]);
     }
   }
   float inter[2], denominator[2];
@@ -1001,21 +1048,30 @@ mlstm_outputs_kernel(const MlstmParams p) {
     for (int i = 0; i < 4; ++i) O[j][i] *= inter[i >> 1];
 #pragma unroll
   for (int kk = 0; kk < L / 16; ++kk) {
-    uint32_t a[4];
-    load_a(a, Ws, LS, rm * 16, kk * 16, g, tq);
+    uint32_t a[4], b[4];
+    left(a, Ws, LS, rm * 16, kk * 16, lane);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat16* at = Vt + (cn * 32 + j * 8 + g) * LS + kk * 16 + 2 * tq;
-      mma_bf16(O[j], a, ld32(at), ld32(at + 8));
+    for (int j = 0; j < 4; j += 2) {
+      right_turned(b, Vs, VS, cn * 32 + j * 8, kk * 16, lane);
+      mma_bf16(O[j], a, b[0], b[1]);
+      mma_bf16(O[j + 1], a, b[2], b[3]);
     }
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = rm * 16 + g + 8 * (i >> 1), c = cn * 32 + j * 8 + 2 * tq + (i & 1);
-      if (t < len && c < cols)
-        p.o_raw[(static_cast<size_t>(t0 + start + t) * p.heads + h) * dv + c0 + c] = O[j][i] / denominator[i >> 1];
+    for (int i = 0; i < 4; i += 2) {
+      const int t = rm * 16 + g + 8 * (i >> 1), c = cn * 32 + j * 8 + 2 * tq;
+      if (t < len && c < cols) {
+        float* at = p.o_raw + (static_cast<size_t>(t0 + start + t) * p.heads + h) * dv + c0 + c;
+        const float2 value = make_float2(O[j][i] / denominator[i >> 1], O[j][i + 1] / denominator[i >> 1]);
+        if (pairs) {
+          *reinterpret_cast<float2*>(at) = value;
+        } else {
+          at[0] = value.x;
+          at[1] = value.y;
+        }
+      }
     }
 }
 
