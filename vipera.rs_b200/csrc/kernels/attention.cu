@@ -58,13 +58,13 @@ __device__ __forceinline__ void visible_keys(const AttentionParams& p, int posit
 
 // Rows of a pool (row r's place in place[r], -1: zeros) into shared memory as floats, `pitch` apart.  VEC: rows of
 // whole 16-byte pieces on 16-byte boundaries (32-bit ones are copied asynchronously: the caller waits).
-template <typename T, bool VEC>
+template <typename T, bool VEC, int THREADS = kAttentionThreads>
 __device__ __forceinline__ void stage_keys(float* dst, int pitch, const T* __restrict__ pool, size_t row_stride, int size,
                                            const int* place, int rows) {
   constexpr int kPiece = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;
   const int pieces = size / kPiece;
 #pragma unroll 4
-  for (int i = threadIdx.x; i < rows * pieces; i += kAttentionThreads) {
+  for (int i = threadIdx.x; i < rows * pieces; i += THREADS) {
     const int r = i / pieces, c = (i - r * pieces) * kPiece;
     const int at = place[r];
     const T* src = pool + (at >= 0 ? static_cast<size_t>(at) * row_stride + c : 0);
@@ -315,7 +315,7 @@ attention_split_kernel(const AttentionParams p) {
 // read a key 64 times less often than a warp per row.  1,024 tokens of three requests (700, 1 and 323, histories
 // 0, 900, 40), 14 heads of 64 on 2, 32-bit: 133 us beside 21 us for the one alone (a warp per (token, head): 1,146 us).
 // ---------------------------------------------------------------------------------------
-constexpr int kTileRows = 64;
+constexpr int kTileRows = 64, kTileThreads = 256, kOwn = kTileRows * 16 / kTileThreads;   // (sixteen lanes a row; kOwn rows a thread)
 
 template <int DP>
 struct TileShared {
@@ -327,7 +327,7 @@ struct TileShared {
 };
 
 template <typename T, int DP, bool VEC>
-__global__ void __launch_bounds__(kAttentionThreads)
+__global__ void __launch_bounds__(kTileThreads)
 attention_tile_kernel(const AttentionParams p) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
   TileShared<DP>& s = *reinterpret_cast<TileShared<DP>*>(tile_raw);
@@ -350,26 +350,26 @@ attention_tile_kernel(const AttentionParams p) {
     if (valid) visible_keys(p, s.last[tid], &s.kept[tid], &s.first[tid]);
   }
 #pragma unroll 4
-  for (int i = tid; i < kTileRows * d; i += kAttentionThreads) {
+  for (int i = tid; i < kTileRows * d; i += kTileThreads) {
     const int r = i / d, c = i - r * d;
     s.q[r][c] = r < rows ? to_float<T>(static_cast<const T*>(p.q)[(static_cast<size_t>(t0 + r) * p.num_heads + h) * d + c]) : 0.0f;
   }
   if (d < DP) {
     const int spare = DP - d;
-    for (int i = tid; i < kTileRows * spare; i += kAttentionThreads) s.q[i / spare][d + i % spare] = 0.0f;
+    for (int i = tid; i < kTileRows * spare; i += kTileThreads) s.q[i / spare][d + i % spare] = 0.0f;
   }
   if (dv < DP) {
     const int spare = DP - dv;
-    for (int i = tid; i < kTileKeys * spare; i += kAttentionThreads) s.v[i / spare][dv + i % spare] = 0.0f;
+    for (int i = tid; i < kTileKeys * spare; i += kTileThreads) s.v[i / spare][dv + i % spare] = 0.0f;
   }
   __syncthreads();
 
-  const int row0 = warp * 16 + (lane >> 4), column0 = lane & 15;   // rows row0 + 2 i; keys column0 + 16 j; values 4 column0 + 64 j
+  const int row0 = warp * 2 * kOwn + (lane >> 4), column0 = lane & 15;   // rows row0 + 2 i; keys column0 + 16 j; values 4 column0 + 64 j
   constexpr int kGroups = DP / 64;
-  float out[8][kGroups][4];
-  float row_max[8], row_sum[8];
+  float out[kOwn][kGroups][4];
+  float row_max[kOwn], row_sum[kOwn];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < kOwn; ++i) {
     row_max[i] = -INFINITY;
     row_sum[i] = 0.0f;
 #pragma unroll
@@ -411,21 +411,21 @@ attention_tile_kernel(const AttentionParams p) {
         if (tid < kTileKeys) s.place[tid] = ahead;
         if (d < DP) {   // the weights were here
           const int spare = DP - d;
-          for (int i = tid; i < kTileKeys * spare; i += kAttentionThreads) s.k[i / spare][d + i % spare] = 0.0f;
+          for (int i = tid; i < kTileKeys * spare; i += kTileThreads) s.k[i / spare][d + i % spare] = 0.0f;
         }
         __syncthreads();
-        stage_keys<T, VEC>(&s.k[0][0], DP + 4, static_cast<const T*>(p.k_pool) + static_cast<size_t>(kv_head) * d,
+        stage_keys<T, VEC, kTileThreads>(&s.k[0][0], DP + 4, static_cast<const T*>(p.k_pool) + static_cast<size_t>(kv_head) * d,
                            static_cast<size_t>(p.num_kv_heads) * d, d, s.place, kTileKeys);
         copy_commit();
-        stage_keys<T, VEC>(&s.v[0][0], DP, static_cast<const T*>(p.v_pool) + static_cast<size_t>(kv_head) * dv,
+        stage_keys<T, VEC, kTileThreads>(&s.v[0][0], DP, static_cast<const T*>(p.v_pool) + static_cast<size_t>(kv_head) * dv,
                            static_cast<size_t>(p.num_kv_heads) * dv, dv, s.place, kTileKeys);
         copy_commit();
         if (base + kTileKeys < run_end) ahead = look_up(base + kTileKeys);
         copy_wait<1>();
         __syncthreads();
-        unsigned long long dot[8][4];
+        unsigned long long dot[kOwn][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < kOwn; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) dot[i][j] = 0ull;
 #pragma unroll 2
@@ -434,7 +434,7 @@ attention_tile_kernel(const AttentionParams p) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const ulonglong2*>(&s.k[column0 + 16 * j][c]);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < kOwn; ++i) {
             const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&s.q[row0 + 2 * i][c]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -447,7 +447,7 @@ attention_tile_kernel(const AttentionParams p) {
         __syncthreads();   // the keys are read out (the weights take their place), and the values are there
         bool some_hidden = false;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < kOwn; ++i) {
           const int row = row0 + 2 * i;
           const int from = run == 0 ? 0 : s.first[row], to = run == 0 ? s.kept[row] : s.last[row] + 1;
           const bool mine = row >= seg && row < seg_end;
@@ -487,15 +487,15 @@ attention_tile_kernel(const AttentionParams p) {
         if (!edge) {
 #pragma unroll 2
           for (int key = 0; key < kTileKeys; key += 2) {
-            float2 w[8];
+            float2 w[kOwn];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = *reinterpret_cast<const float2*>(weights + (row0 + 2 * i) * kWeightPitch + key);
+            for (int i = 0; i < kOwn; ++i) w[i] = *reinterpret_cast<const float2*>(weights + (row0 + 2 * i) * kWeightPitch + key);
 #pragma unroll
             for (int j = 0; j < kGroups; ++j) {
               const float4 a = *reinterpret_cast<const float4*>(&s.v[key][4 * column0 + 64 * j]);
               const float4 b = *reinterpret_cast<const float4*>(&s.v[key + 1][4 * column0 + 64 * j]);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
+              for (int i = 0; i < kOwn; ++i) {
                 out[i][j][0] = fmaf(w[i].y, b.x, fmaf(w[i].x, a.x, out[i][j][0]));
                 out[i][j][1] = fmaf(w[i].y, b.y, fmaf(w[i].x, a.y, out[i][j][1]));
                 out[i][j][2] = fmaf(w[i].y, b.z, fmaf(w[i].x, a.z, out[i][j][2]));
@@ -507,14 +507,14 @@ attention_tile_kernel(const AttentionParams p) {
           // a value a row does not see is left out, whatever it holds (0 times infinity is not 0)
 #pragma unroll 2
           for (int key = 0; key < count; ++key) {
-            float w[8];
+            float w[kOwn];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = weights[(row0 + 2 * i) * kWeightPitch + key];
+            for (int i = 0; i < kOwn; ++i) w[i] = weights[(row0 + 2 * i) * kWeightPitch + key];
 #pragma unroll
             for (int j = 0; j < kGroups; ++j) {
               const float4 a = *reinterpret_cast<const float4*>(&s.v[key][4 * column0 + 64 * j]);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
+              for (int i = 0; i < kOwn; ++i) {
                 if (!(w[i] < 0.0f)) {
                   out[i][j][0] = fmaf(w[i], a.x, out[i][j][0]);
                   out[i][j][1] = fmaf(w[i], a.y, out[i][j][1]);
@@ -530,7 +530,7 @@ attention_tile_kernel(const AttentionParams p) {
     seg = seg_end;
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < kOwn; ++i) {
     const int row = row0 + 2 * i;
     if (row >= rows || s.last[row] == -2) continue;
     const int t = t0 + row;
@@ -578,7 +578,7 @@ static int launch_attention(const AttentionParams& asked, int requests, cudaStre
   const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_tile_kernel<T, DP, VEC>), kBytes);
   if (opted) return opted;
   return vipera_launch(attention_tile_kernel<T, DP, VEC>, dim3(p.num_heads, (p.num_tokens + kTileRows - 1) / kTileRows),
-                       dim3(kAttentionThreads), kBytes, s, p);
+                       dim3(kTileThreads), kBytes, s, p);
 }
 
 template <typename T>
