@@ -39,7 +39,7 @@ def _plain(w, h, kept, counts, firsts, heads, dim, rot, rank, vdim, window, sink
     return out.reshape(len(h), -1) @ w["p.o.weight"].T
 
 
-@pytest.mark.parametrize("counts,firsts", [([520], [0]), ([300, 1, 129, 130], [70, 200, 0, 63]), ([64, 65, 63, 400], [0, 1, 300, 0])])
+@pytest.mark.parametrize("counts,firsts", [([520], [0]), ([300, 1, 129, 130], [70, 200, 0, 63]), ([64, 65, 63, 400], [0, 1, 300, 0]), ([700, 1, 900], [0, 60, 10])])
 @pytest.mark.parametrize("heads,rank,rot,window,page", [(3, 512, 64, 0, 16), (12, 512, 64, 100, 16), (5, 256, 32, 0, 7), (7, 64, 8, 50, 64),
                                                         (32, 384, 24, 0, 1), (128, 320, 64, 333, 16)])
 def test_fold(counts, firsts, heads, rank, rot, window, page):

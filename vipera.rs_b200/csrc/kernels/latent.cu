@@ -920,6 +920,7 @@ struct LatentParams {
   int single;              // 1: every request of the step brings one token
   int* status;             // receives a code where a bounded wait ran out, or null: the fold stays with mma.sync
   int max_keys;            // at least the longest history of the step (0: not known)
+  int requests;            // of the step
 };
 
 // How the tensor-core fold cuts a step.  Rows are tokens x heads.  Many rows: two groups of sixteen to a
@@ -999,6 +1000,12 @@ static bool fold_takes_tensor(const LatentParams& p) {
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool) | reinterpret_cast<uintptr_t>(p.l_heads) |
                           reinterpret_cast<uintptr_t>(p.qa_heads) | reinterpret_cast<uintptr_t>(p.q_rot);
   const long keys = p.window > 0 ? std::min<long>(p.max_keys, static_cast<long>(p.window) + p.num_tokens) : p.max_keys;
+  // Its tiles hold 128 rows and their keys are not cut: a token behind a long history makes one block walk it alone (five
+  // microseconds per 64 keys).  With several requests that has to fit into what the step's own tokens surely cost without it
+  // (42,000 keys of a row per microsecond): 8 heads, 600 + 1 + 100 tokens, the one behind 2,000: 242 us with it, 134 without;
+  // 32 heads, 1,748 tokens of four requests behind up to 3,000: the mixer 666 and 1,158.
+  const double own = static_cast<double>(p.num_tokens) * p.heads * std::min<double>(keys, static_cast<double>(p.num_tokens) / std::max(p.requests, 1));
+  if (p.requests > 1 && own < 42000.0 * 2 * 5 / 64 * keys) return false;
   return p.stage == 2 && keys > kTensorKeys && !p.single && p.status != nullptr && static_cast<long>(p.num_tokens) * p.heads >= kTensorRows &&
          p.rank % latent_tc::kHalf == 0 && p.rot <= latent_tc::kHalf && (bases & 15) == 0;
 }

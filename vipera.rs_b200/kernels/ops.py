@@ -1747,7 +1747,7 @@ class _LatentParams(ctypes.Structure):
         ("stage", _c_int), ("padded_tokens", _c_int), ("a_heads", _c_void), ("qa_heads", _c_void), ("q_rot", _c_void),
         ("l_heads", _c_void), ("o_heads", _c_void), ("tile_group", _c_void),
         ("window", _c_int), ("pairing", _c_int), ("sink", _c_void), ("q", _c_void), ("q_width", ctypes.c_longlong),
-        ("cq_off", _c_int), ("q_rank", _c_int), ("cq_norm_weight", _c_void), ("cq", _c_void), ("single", _c_int), ("status", _c_void), ("max_keys", _c_int),
+        ("cq_off", _c_int), ("q_rank", _c_int), ("cq_norm_weight", _c_void), ("cq", _c_void), ("single", _c_int), ("status", _c_void), ("max_keys", _c_int), ("requests", _c_int),
     ]
 
 
@@ -1846,7 +1846,7 @@ def latent_attention(proj: torch.Tensor, *, q_off: int, g_off: int, kv_off: int,
     p.window, p.pairing = int(window or 0), 1 if pairing == ROPE_NEOX else 0
     p.part, p.split_keys, p.num_splits, p.single = None, 0, 1, int(bool(single))
     p.status = _tc_buffers(proj.device, 0)["status"].data_ptr() if head_major is not None else None
-    p.max_keys = int(max_keys)
+    p.max_keys, p.requests = int(max_keys), int(block_table.shape[0])
     if part is not None and max_keys > 0:
         _, _, split_keys, splits = latent_plan(tokens, heads, rank, rot_dim, int(max_keys), sm_count(proj.device), p.window, single)
         if splits > 1:
