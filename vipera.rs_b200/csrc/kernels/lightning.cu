@@ -267,11 +267,13 @@ static int launch_scans(const LightningParams& params, bool chunked, cudaStream_
   const int tiles = (p.dv + kColumns - 1) / kColumns;
   if (!chunked)
     return vipera_launch(lightning_scan_kernel<RPT, MODE_WALK>, dim3(tiles, p.heads, p.num_entries), kRowWarps * 32, shared, s, p);
-  // rows that are not whole 16-byte pieces walk their chunks
+  // Rows that are not whole 16-byte pieces walk their chunks, and so do small heads (up to 64 key channels): a walk's
+  // block holds their state in few registers, and the products' tiles are not filled.  Walks / products, the mixer: 4 heads of
+  // 64 x 128, 400 and 800 tokens: 75 / 86 and 81 / 95 us; 8 heads: 82 / 81 and 95 / 100; 4 heads of 128 x 256: 134 / 95 and 146 / 121.
   const LinearArgs chunks{p.proj, p.proj_width, p.q_off, p.k_off, p.v_off, nullptr, nullptr, p.decay, p.entry_starts, p.chunk_state,
                           nullptr, p.raw, p.num_entries, p.heads, p.d, p.dv, 1.0f};
   const size_t state_floats = static_cast<size_t>(p.heads) * p.d * p.dv;
-  if (linear_chunks_take(chunks)) {
+  if (p.d > 64 && linear_chunks_take(chunks)) {
     int status = launch_linear_ends<false>(chunks, p.num_jobs, s);
     if (status) return status;
     status = vipera_launch(lightning_carry_kernel, dim3(static_cast<unsigned>((state_floats + 255) / 256), p.num_entries), 256, 0, s, p);
