@@ -308,12 +308,12 @@ attention_split_kernel(const AttentionParams p) {
 
 // ---------------------------------------------------------------------------------------
 // Steps of more tokens: a block takes 64 neighbouring tokens and one head and walks the keys 64 at a time.  A
-// thread owns 8 rows x 4 keys of the scores (packed multiply-adds) and 8 rows x DP / 16 values of the output;
-// sixteen lanes share a row, a warp sixteen rows, so that a row's weights pass through shared memory
+// thread owns 4 rows x 4 keys of the scores (packed multiply-adds) and 4 rows x DP / 16 values of the output;
+// sixteen lanes share a row, a warp eight rows, so that a row's weights pass through shared memory
 // within its warp.  Tokens of several requests in one tile are folded one request after another, the
 // others' rows masked.  Bound by the multiply-adds and the reads of shared memory that feed them: 64 x 64 tiles
 // read a key 64 times less often than a warp per row.  1,024 tokens of three requests (700, 1 and 323, histories
-// 0, 900, 40), 14 heads of 64 on 2, 32-bit: 133 us beside 21 us for the one alone (a warp per (token, head): 1,146 us).
+// 0, 900, 40), 14 heads of 64 on 2, 32-bit: 101 us beside 21 us for the one alone (four warps of twice the rows: 133; a warp per (token, head): 1,146 us).
 // ---------------------------------------------------------------------------------------
 constexpr int kTileRows = 64, kTileThreads = 256, kOwn = kTileRows * 16 / kTileThreads;   // (sixteen lanes a row; kOwn rows a thread)
 
