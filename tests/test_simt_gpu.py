@@ -20,7 +20,7 @@ def _rel(got, want):
 # rows at the borders of the tiles (8, 32, 64, 128), columns that end inside one, inner sizes of a part of a chunk,
 # of fewer than eight slabs, of slabs that end early, of rows that do not start on 16 bytes
 @pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 33, 64, 65, 129])
-@pytest.mark.parametrize("n,k", [(64, 32), (70, 5), (96, 100), (130, 770), (200, 771), (1536, 808), (9600, 520)])
+@pytest.mark.parametrize("n,k", [(64, 32), (257, 16), (33, 4), (70, 5), (96, 100), (130, 770), (200, 771), (1536, 808), (9600, 520)])
 @pytest.mark.parametrize("types", ["f32", "bf16", "mixed"])
 def test_product_tiles_and_slabs(m, n, k, types):
     ops = _ops()
