@@ -7,8 +7,10 @@
 // every step of their sums towards zero, which over a long K would cost more than 32-bit multiply-adds do: so the
 // leading product and the five small ones have accumulators of their own, both are read after every 64 values of K
 // and added to the tile's sums in registers, rounded to nearest.  Against 64 bits the result is closer than a chain of
-// fused multiply-adds over K (1,024 rows through a model of two layers and K up to 4,864: 4.8e-7 against 2.2e-6).  An infinity or a NaN has no such parts (its products with their zeros
-// would be NaN): a block that meets one computes its tile with multiply-adds instead.
+// fused multiply-adds over K (1,024 rows through a model of two layers and K up to 4,864: 4.8e-7 against 2.2e-6).
+// An infinity or a NaN has no such parts (its products with their zeros would be NaN).  Nothing such a row of A or W
+// gives is finite, and no other row reads it: a block notes which of its rows hold one, writes NaN where a row holds a
+// NaN, and computes the outputs of rows with infinities alone with multiply-adds, a warp an output.
 //
 // A block computes a tile of 128 x 128: eight warps read 64 values of K, split them and leave the parts in shared
 // memory (three images of 128 rows each, 128-byte swizzle, two stages of 96 KB); eight warps add up, the first of which
@@ -31,6 +33,7 @@ constexpr int kImageBytes = kTile * kDepth * 2, kStageBytes = 2 * kParts * kImag
 constexpr int kSumWarps = 8, kIssuer = 0, kFirstSplitter = 8, kSplitters = 256;   // (the first of the adding warps issues)
 constexpr int kThreads = (kFirstSplitter + 8) * 32;
 constexpr int kSumPitch = kTile + 4;
+constexpr int kRowWords = kTile / 32;   // words of a bit per row
 constexpr uint32_t kWaitLimit = 1u << 22;
 enum { WAIT_EXPIRED = 6 };
 
@@ -44,14 +47,16 @@ struct Args {
   int activation, epilogue, out_bf16;
   int* status;
   uint8_t* parts;            // the left operand's images, written ahead: [tile of rows][64 of K][part], or null
-  int* odd;                  // of each of those threes of images: something in it is not finite
+  uint32_t* odd;             // of each of those threes of images: a bit for each row with something that is not finite
   long long parts_bytes;     // what `parts` has room for (the flags lie behind the images)
 };
 
 struct Shared {
   uint64_t full[kStages], empty[kStages], sums_full[2], sums_empty[2];
   uint32_t tmem_base;
-  int abort_flag, not_finite;
+  int abort_flag;
+  uint32_t odd[2 * kRowWords];   // rows of A, then of W, that hold something that is not finite
+  uint32_t nan[2 * kRowWords];   // of those, the ones that hold a NaN
 };
 constexpr int kSharedBytes = kStages * kStageBytes + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(kTile * kSumPitch * 4 <= kStages * kStageBytes, "the tile's sums take the stages' place");
@@ -104,10 +109,12 @@ __device__ __forceinline__ float leading(float v) { return __uint_as_float(__flo
 // the upper halves of two 32-bit words, `lo`'s in the lower one
 __device__ __forceinline__ uint32_t uppers(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
 
-// Eight values' pieces of the three images; `odd` becomes NaN where a value is not finite (its remainder is NaN).
+// Eight values' pieces of the three images; odd(): one of them is not finite (its remainder is NaN).
 struct Pieces {
   uint32_t first[4], second[4], third[4];
-  __device__ __forceinline__ Pieces(const float4& lo, const float4& hi, float& odd) {
+  float sum;
+  __device__ __forceinline__ bool odd() const { return sum != sum; }
+  __device__ __forceinline__ Pieces(const float4& lo, const float4& hi) : sum(0.0f) {
     const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
     for (int e = 0; e < 8; e += 2) {
@@ -115,7 +122,7 @@ struct Pieces {
       first[e >> 1] = uppers(v[e], v[e + 1]);
       second[e >> 1] = uppers(r0, r1);
       third[e >> 1] = uppers(r0 - leading(r0), r1 - leading(r1));
-      odd = fmaf(r0, 0.0f, fmaf(r1, 0.0f, odd));
+      sum = fmaf(r0, 0.0f, fmaf(r1, 0.0f, sum));
     }
   }
   __device__ __forceinline__ void store(uint8_t* at) const {
@@ -143,11 +150,17 @@ gemm_split_left_kernel(const Args p) {
     if (m < p.M && k + 4 < p.K) hi[i] = *reinterpret_cast<const float4*>(src + 4);
   }
   uint8_t* dst = p.parts + static_cast<size_t>(three) * (kParts * kImageBytes) + sub * 128 + ((piece ^ (sub & 7)) << 4);
-  float odd = 0.0f;
+  __shared__ uint32_t rows[kRowWords];
+  if (t < kRowWords) rows[t] = 0u;
+  __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 4; ++i) Pieces(lo[i], hi[i], odd).store(dst + i * 32 * 128);
-  const int any = __syncthreads_or(odd != odd);
-  if (t == 0) p.odd[three] = any;
+  for (int i = 0; i < 4; ++i) {
+    const Pieces pieces(lo[i], hi[i]);
+    pieces.store(dst + i * 32 * 128);
+    if (pieces.odd()) atomicOr(&rows[i], 1u << sub);
+  }
+  __syncthreads();
+  if (t < kRowWords) p.odd[three * kRowWords + t] = rows[t];
 }
 
 // AHEAD: the left operand's images lie in p.parts and are copied; else this block splits both operands.
@@ -173,7 +186,8 @@ gemm_split_kernel(const Args p) {
       bar_init(&s.sums_full[i], 1);
       bar_init(&s.sums_empty[i], kSumWarps * 32);
     }
-    s.abort_flag = s.not_finite = 0;
+    s.abort_flag = 0;
+    for (int i = 0; i < 2 * kRowWords; ++i) s.odd[i] = s.nan[i] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kIssuer) {
@@ -272,10 +286,9 @@ gemm_split_kernel(const Args p) {
     for (int i = 0; i < kFirstW; ++i)
       if (count > 0) ask(i, 0);
     const int three = blockIdx.y * ((p.K + kDepth - 1) / kDepth) + k_begin / kDepth;   // the first images of this block
-    float odd = 0.0f;   // NaN once something is not finite
     if (AHEAD)
-      for (int c = t; c < count; c += kSplitters)
-        if (p.odd[three + c]) odd = NAN;
+      for (int i = t; i < count * kRowWords; i += kSplitters)
+        if (const uint32_t rows = p.odd[three * kRowWords + i]) atomicOr(&s.odd[i % kRowWords], rows);
     for (int c = 0; c < count; ++c) {
       const int stage = c & 1;
       if (c >= 2) bar_wait(&s.empty[stage], ((c >> 1) & 1) ^ 1, abort_flag, p.status);
@@ -291,14 +304,14 @@ gemm_split_kernel(const Args p) {
       uint8_t* dst = stages + stage * kStageBytes + sub * 128 + ((piece ^ (sub & 7)) << 4);   // (rows 32 apart are swizzled alike)
 #pragma unroll
       for (int i = 0; i < kRuns; ++i) {
-        const Pieces pieces(lo[i], hi[i], odd);
+        const Pieces pieces(lo[i], hi[i]);
         if (c + 1 < count) ask(i, c + 1);   // the next stage's run takes this one's registers
+        if (pieces.odd()) atomicOr(&s.odd[i < kFirstW ? i : kRowWords + i - kFirstW], 1u << sub);
         pieces.store(dst + (i < kFirstW ? 0 : kParts * kImageBytes) + ((i - kFirstW) & 3) * 32 * 128);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       bar_arrive(&s.full[stage]);
     }
-    if (odd != odd) s.not_finite = 1;
     if (AHEAD && t == 0 && *abort_flag) {   // a copy may be on its way still: it ends long before this does
       for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
@@ -310,13 +323,38 @@ gemm_split_kernel(const Args p) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
   }
   pdl_wait();   // (every thread may read A or the residual stream from here on)
-  if (s.not_finite) {
-    for (int i = tid; i < kTile * kTile; i += kThreads) {
-      const int m = i / kTile, n = i % kTile;
-      float sum = 0.0f;
-      if (m0 + m < p.M && n0 + n < p.N)
-        for (int k = k_begin; k < k_end; ++k) sum = fmaf(p.A[static_cast<size_t>(m0 + m) * p.K + k], p.W[static_cast<size_t>(n0 + n) * p.K + k], sum);
-      sums[m * kSumPitch + n] = sum;
+  uint32_t any = 0u;
+#pragma unroll
+  for (int i = 0; i < 2 * kRowWords; ++i) any |= s.odd[i];
+  if (any) {
+    // which of these rows hold a NaN within this block's share of K: a warp a row (one that holds something exists)
+    for (int r = warp; r < 2 * kTile; r += kThreads / 32) {
+      if (!(s.odd[r >> 5] >> (r & 31) & 1u)) continue;
+      const float* row = r < kTile ? p.A + static_cast<size_t>(m0 + r) * p.K : p.W + static_cast<size_t>(n0 + r - kTile) * p.K;
+      bool nan = false;
+#pragma unroll 4
+      for (int k = k_begin + lane; k < k_end; k += 32) nan |= row[k] != row[k];
+      if (__any_sync(0xffffffffu, nan) && lane == 0) atomicOr(&s.nan[r >> 5], 1u << (r & 31));
+    }
+    __syncthreads();
+    // their outputs: row r of A against all of W's, then row r of W against all of A's
+    for (int word = 0; word < 2 * kRowWords; ++word) {
+      for (uint32_t left = s.odd[word]; left; left &= left - 1u) {
+        const int r = word % kRowWords * 32 + __ffs(static_cast<int>(left)) - 1;
+        const bool of_a = word < kRowWords, nan = s.nan[word] & left & -left;
+        const float* own = of_a ? p.A + static_cast<size_t>(m0 + r) * p.K : p.W + static_cast<size_t>(n0 + r) * p.K;
+        const float* others = of_a ? p.W + static_cast<size_t>(n0) * p.K : p.A + static_cast<size_t>(m0) * p.K;
+        const int count_others = min(kTile, of_a ? p.N - n0 : p.M - m0);
+        for (int i = warp; i < count_others; i += kThreads / 32) {
+          float sum = nan ? NAN : 0.0f;
+          if (!nan) {
+#pragma unroll 4
+            for (int k = k_begin + lane; k < k_end; k += 32) sum = fmaf(own[k], others[static_cast<size_t>(i) * p.K + k], sum);
+            sum = warp_sum(sum);
+          }
+          if (lane == 0) sums[(of_a ? r : i) * kSumPitch + (of_a ? i : r)] = sum;
+        }
+      }
     }
     __syncthreads();
   }
@@ -392,7 +430,7 @@ static int launch_rows(const Args& args, cudaStream_t s) {
 // (5,500 clocks to 3,400).  Not more room than the L2 holds well: more rows are taken in turns.  Both operands split in the
 // block / the left one ahead: 80 x 896 of 896, seven stages in a row: 17.5 / 18.5 us; 1,024 x 1,152 of 896, seven: 30.6 / 31.2;
 // 256 x 256 of 2,048, eight: 33.9 / 27.0; 128 x 9,728 of 896, fourteen: 53.7 / 39.3; 8,192 x 4,096 of 4,096: 2,852 / 1,797.
-constexpr long long kMostParts = 96ll << 20, kTileExtra = 4;   // (bytes beside each three of images: its flag)
+constexpr long long kMostParts = 96ll << 20, kTileExtra = kRowWords * 4;   // (bytes beside each three of images: its rows' bits)
 static int parts_bytes(int M, int N, int K) {
   if (M <= 64 || N <= kTile || K % 4 != 0) return 0;   // (one tile along N: nobody else would split the same rows)
   const long long tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile;
@@ -419,7 +457,7 @@ static int launch(const Args& args, cudaStream_t s) {
   for (long long m = 0; m < args.M && !status; m += tiles * kTile) {
     Args p = args;
     p.M = static_cast<int>(args.M - m < tiles * kTile ? args.M - m : tiles * kTile);
-    p.odd = reinterpret_cast<int*>(p.parts + tiles * ((p.K + kDepth - 1) / kDepth) * (kParts * kImageBytes));
+    p.odd = reinterpret_cast<uint32_t*>(p.parts + tiles * ((p.K + kDepth - 1) / kDepth) * (kParts * kImageBytes));
     p.A += static_cast<size_t>(m) * p.K;
     if (p.epilogue == 1) p.resid += m * out_pitch;
     else p.out = static_cast<char*>(p.out) + m * out_pitch * (p.out_bf16 ? 2 : 4);
