@@ -1,5 +1,5 @@
-"""The kernels that compute in 32 bits on the CUDA cores, at the sizes where their tiles, slabs and dispatch end,
-against 64-bit restatements."""
+"""The kernels that compute in 32 bits, on the CUDA cores or on the tensor cores in parts, at the sizes where their tiles,
+slabs and dispatch end, against 64-bit restatements."""
 import pytest
 import torch
 
@@ -42,6 +42,37 @@ def test_product_tiles_and_slabs(m, n, k, types):
     last = torch.empty(beside, n, device=DEV)
     ops.gemm_simt(a[-beside:].contiguous(), w, epilogue=ops.EPI_STORE, bias=bias, out=last)
     assert torch.equal(last[-1], out[-1])
+
+
+# inner sizes short enough to lie in shared memory whole (up to 320, and the next), rows that are and are not whole pieces,
+# all endings and types of the output
+@pytest.mark.parametrize("k", [1, 63, 128, 130, 256, 319, 320, 321])
+@pytest.mark.parametrize("m,n", [(1, 32), (9, 160), (31, 96), (33, 128), (100, 288)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+@pytest.mark.parametrize("types", ["f32", "bf16", "mixed"])
+def test_short_products(m, n, k, epilogue, types):
+    ops = _ops()
+    torch.manual_seed(m + n + k)
+    a = (torch.randn(m, k, device=DEV) * k ** -0.5).to(torch.bfloat16 if types == "bf16" else torch.float32)
+    w, bias = torch.randn(n, k, device=DEV).to(torch.float32 if types == "f32" else torch.bfloat16), torch.randn(n, device=DEV)
+    y = a.double() @ w.double().T + bias.double()
+    if epilogue == 2:
+        gate, up = y.view(m, n // 32, 2, 16)[:, :, 0], y.view(m, n // 32, 2, 16)[:, :, 1]
+        y = (up * gate * torch.sigmoid(gate)).reshape(m, n // 2)
+    out = torch.randn(m, y.shape[1], device=DEV)
+    want = y + out.double() if epilogue == 1 else y
+    ops.gemm_simt(a, w, epilogue=epilogue, bias=bias, **({"resid": out} if epilogue == 1 else {"out": out}))
+    # k roundings of random sign, 2^-24 each, and those of the ending
+    assert _rel(out, want) < 2.0 ** -24 * (k ** 0.5 + 8)
+    if epilogue == 0:
+        narrow = torch.empty(m, n, device=DEV, dtype=torch.bfloat16)
+        ops.gemm_simt(a, w, epilogue=epilogue, bias=bias, out=narrow)
+        assert torch.equal(narrow, out.bfloat16())
+        # a row's result does not depend on the rows beside it (from nine rows on)
+        if m > 17:
+            last = torch.empty(9, n, device=DEV)
+            ops.gemm_simt(a[-9:].contiguous(), w, epilogue=epilogue, bias=bias, out=last)
+            assert torch.equal(last, out[-9:]) or (types == "f32" and k > 128 and m > 64)
 
 
 # the tensor-core form of many rows: tiles that end inside, one block and clusters of two and four that share K (one

@@ -10,9 +10,10 @@
 // Up to eight rows the stream of W bounds the product (gemv_rows_kernel): a warp reads eight rows of W
 // through a ring of its own, 512 neighbouring bytes of a row at a time, a lane's four values against all
 // rows of A, and adds its lanes' sums at the end.
+// A K of up to 320 lies in shared memory whole (gemm_short_kernel).
 // 32-bit products of more than 64 rows (whole rows of 16-byte pieces) run on the tensor cores, three bfloat16 parts of every
 // number: gemm_split.cuh.  Multiply-adds / tensor cores: 65 rows, W 896 x 896: 17.4 / 17.3 us; W 9,728 x 896: 106 / 38; 128
-// rows, W 896 x 4,864: 70 / 47.
+// rows, W 896 x 4,864: 70 / 47; W 512 x 128, in shared memory whole / tensor cores: 10.5 / 16.8.
 // The others of more rows (gemm_simt_kernel): the multiply-add units and the reads of shared memory that feed them.  K is
 // cut into eight slabs (of whole chunks of 32), a slab's even and odd places are two chains of fused
 // multiply-adds (the two halves of a packed 32-bit pair) whose ends are added, and the slabs are added in
@@ -54,6 +55,7 @@ struct Tile {
 };
 using TileSome = Tile<32, 128, 4, 1, 1, 32, 8, 4, 3>;
 using TileMid = Tile<64, 128, 2, 2, 4, 8, 8, 8, 3>;
+using TileLow = Tile<64, 64, 4, 2, 4, 8, 4, 4, 2>;   // little shared memory: four blocks an SM hide the staging through registers
 using TileMany = Tile<128, 128, 4, 2, 4, 8, 8, 8, 3>;
 
 struct GemmArgs {
@@ -422,24 +424,31 @@ static int launch_form(const GemmArgs& p, cudaStream_t s) {
 }
 
 // A tile's slabs go to a cluster where whole tiles would leave much of the chip idle: fewer small tiles
-// than multiprocessors, or a last wave that is mostly empty for the large ones (a block a multiprocessor).
+// than multiprocessors, or a last wave that is mostly empty for the large ones (a block a multiprocessor).  The tiles
+// of rows that are staged through registers go to clusters up to a count that grows with K: in bfloat16, whole / cluster, 140
+// tiles of K = 896: 51.5 / 55.6 us, 70: 51.5 / 33.5; 320 of 2,048: 217 / 202, 512: 305 / 316; 64 of 300: 26.9 / 20.7.
+// (Tiles of 64 x 128 took 78.7, 47.4, 283, 338 and 20.6 us there, tiles of 64 x 64 with one chain over K
+// 72, 72, 313, 419 and 24.9.)
 template <typename TA, typename TW, typename T, bool DIRECT>
 static int launch_tile(const GemmArgs& p, cudaStream_t s) {
   constexpr long long kSms = 148;
   const long long tiles = static_cast<long long>((p.N + T::BN - 1) / T::BN) * ((p.M + T::BM - 1) / T::BM);
   bool cluster;
   if (T::BM <= 32) cluster = tiles < kSms;
+  else if (!DIRECT) cluster = tiles <= (p.K / 6 > 80 ? p.K / 6 : 80);
   else cluster = tiles * 5 < (tiles + kSms - 1) / kSms * kSms * 4;
   // a slab of less than three chunks is all start and ending
-  if (cluster && p.slab >= 3 * kChunk) return launch_form<TA, TW, T, DIRECT, true>(p, s);
+  if (cluster && (p.slab >= 3 * kChunk || (T::BM > 32 && !DIRECT))) return launch_form<TA, TW, T, DIRECT, true>(p, s);
   return launch_form<TA, TW, T, DIRECT, false>(p, s);
 }
 
-// A short inner size (up to 32 values, more than eight rows): the output's stores bound the product, and what the
-// forms of long K keep for it (rings, slabs, tensor memory) only delays the start.  A block takes 32 rows and 128 columns,
-// a thread four rows and four columns a warp apart; the sum's order is the tiles' (even and odd places, then both).
-// 2,002 rows, W 1,024 x 16 in bfloat16: 11.2 us in tiles of 64 x 128, 10.3 so; 100 rows, W 512 x 16: a mixer of 102 us takes 73.
-constexpr int kShortInner = 32, kShortRows = 32, kShortColumns = 128, kShortThreads = 256;
+// A short inner size: the trip to memory and the output's stores bound the product, and what the forms of long K keep for
+// it (rings, slabs, tensor memory) only delays the start.  A block takes 32 rows and 128 columns with all of K in shared
+// memory, a thread four rows and four columns a warp apart; a sum has two chains, even and odd places.  VEC: rows of whole
+// pieces of four values.  Tiles through slabs or the tensor cores / this: bfloat16, 300 rows, W 256 x 100: 24.9 / 10.6 us, W 512
+// x 256: 31.0 / 18.7; 32-bit, 300 rows, W 128 x 128: 18.7 / 8.5.
+constexpr int kShortRows = 32, kShortColumns = 128, kShortThreads = 256;
+constexpr int kShortInner = 320, kShortInnerParts = 128;   // the longest K, and where the tensor cores could take over
 
 __device__ __forceinline__ float4 load_four(const float* src) { return *reinterpret_cast<const float4*>(src); }
 __device__ __forceinline__ float4 load_four(const __nv_bfloat16* src) {
@@ -448,42 +457,58 @@ __device__ __forceinline__ float4 load_four(const __nv_bfloat16* src) {
   const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
+// fours of a row in shared memory: odd, so that neighbouring rows' 16-byte reads meet no bank twice
+__host__ __device__ __forceinline__ int short_pitch(int K) { return ((K + 3) / 4) | 1; }
 
-template <typename TA, typename TW>
+// `rows` rows from row0 on; zeros outside.
+template <typename T, bool VEC>
+__device__ __forceinline__ void stage_short(float4* dst, int pitch, const T* __restrict__ src, int row0, int extent, int rows, int K) {
+  const int pieces = (K + 3) / 4;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < rows * pieces; i += kShortThreads) {
+    const int r = i / pieces, c = i - r * pieces;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (row0 + r < extent) {
+      const T* at = src + static_cast<size_t>(row0 + r) * K + 4 * c;
+      if (VEC) {
+        v = load_four(at);
+      } else {
+        v.x = to_float<T>(at[0]);
+        if (4 * c + 1 < K) v.y = to_float<T>(at[1]);
+        if (4 * c + 2 < K) v.z = to_float<T>(at[2]);
+        if (4 * c + 3 < K) v.w = to_float<T>(at[3]);
+      }
+    }
+    dst[r * pitch + c] = v;
+  }
+}
+
+template <typename TA, typename TW, bool VEC>
 __global__ void __launch_bounds__(kShortThreads)
 gemm_short_kernel(const GemmArgs p) {
-  __shared__ __align__(16) float a_s[kShortRows][kShortInner + 4], w_s[kShortColumns][kShortInner + 4];
+  extern __shared__ float4 short_shared[];
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, m0 = blockIdx.y * kShortRows, n0 = blockIdx.x * kShortColumns;
-  const int pieces = p.K / 4;
-  const TW* W = static_cast<const TW*>(p.W);
-  const TA* A = static_cast<const TA*>(p.A);
-  for (int i = tid; i < kShortColumns * pieces; i += kShortThreads) {
-    const int r = i / pieces, c = (i - r * pieces) * 4;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (n0 + r < p.N) v = load_four(W + static_cast<size_t>(n0 + r) * p.K + c);
-    *reinterpret_cast<float4*>(&w_s[r][c]) = v;
-  }
+  const int pitch = short_pitch(p.K), pieces = (p.K + 3) / 4;
+  float4* w_s = short_shared;                       // [kShortColumns][pitch]
+  float4* a_s = w_s + kShortColumns * pitch;        // [kShortRows][pitch]
+  stage_short<TW, VEC>(w_s, pitch, static_cast<const TW*>(p.W), n0, p.N, kShortColumns, p.K);
   pdl_wait();
-  for (int i = tid; i < kShortRows * pieces; i += kShortThreads) {
-    const int r = i / pieces, c = (i - r * pieces) * 4;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (m0 + r < p.M) v = load_four(A + static_cast<size_t>(m0 + r) * p.K + c);
-    *reinterpret_cast<float4*>(&a_s[r][c]) = v;
-  }
+  stage_short<TA, VEC>(a_s, pitch, static_cast<const TA*>(p.A), m0, p.M, min(kShortRows, p.M - m0), p.K);
   __syncthreads();
+  if (m0 + warp * 4 >= p.M) return;
   unsigned long long sums[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) sums[i][j] = 0ull;
-  for (int k = 0; k < p.K; k += 4) {
+  for (int c = 0; c < pieces; ++c) {   // (rows of A that do not exist: whatever lies there, never stored)
     ulonglong2 w[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(&w_s[lane + 32 * j][k]);
+    for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + (lane + 32 * j) * pitch + c);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&a_s[warp * 4 + i][k]);
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + (warp * 4 + i) * pitch + c);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         fma_pair(sums[i][j], a.x, w[j].x);
@@ -496,29 +521,48 @@ gemm_short_kernel(const GemmArgs p) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int m = m0 + warp * 4 + i, n = n0 + lane + 32 * j;
+      float value = sum_of_pair(sums[i][j]) + (p.bias && n < p.N ? p.bias[n] : 0.0f);
+      int column = n, columns = p.N;
+      if (p.epilogue == EPI_SWIGLU) {   // the feature's up value is 16 columns, and lanes, further
+        const float up = __shfl_down_sync(0xffffffffu, value, 16);
+        value = up * gate_activation(value, p.activation);
+        column = n / 32 * 16 + n % 32, columns = p.N / 2;
+        if (lane >= 16) continue;
+      }
       if (m >= p.M || n >= p.N) continue;
-      const size_t at = static_cast<size_t>(m) * p.N + n;
-      const float value = sum_of_pair(sums[i][j]) + (p.bias ? p.bias[n] : 0.0f);
+      const size_t at = static_cast<size_t>(m) * columns + column;
       if (p.epilogue == EPI_RESIDUAL) p.resid[at] += value;
       else if (p.out_bf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value);
       else static_cast<float*>(p.out)[at] = value;
     }
 }
 
+template <typename TA, typename TW, bool VEC>
+static int launch_short(const GemmArgs& p, cudaStream_t s) {
+  constexpr int kRowsHeld = kShortColumns + kShortRows;
+  static SharedMemoryOptIn opt_in;
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(gemm_short_kernel<TA, TW, VEC>), kRowsHeld * ((kShortInner / 4) | 1) * 16);
+  if (opted) return opted;
+  const dim3 grid(static_cast<unsigned>((p.N + kShortColumns - 1) / kShortColumns), static_cast<unsigned>((p.M + kShortRows - 1) / kShortRows));
+  return vipera_launch(gemm_short_kernel<TA, TW, VEC>, grid, dim3(kShortThreads), kRowsHeld * short_pitch(p.K) * 16, s, p);
+}
+
 template <typename TA, typename TW>
 static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
   constexpr bool kBothFloat = sizeof(TA) == 4 && sizeof(TW) == 4;
-  const unsigned short_rows = static_cast<unsigned>((p.M + kShortRows - 1) / kShortRows);
-  if (p.K <= kShortInner && p.K % 4 == 0 && p.M > kFewRows && p.epilogue != EPI_SWIGLU && short_rows <= 65535u &&
-      reinterpret_cast<uintptr_t>(p.A) % (4 * sizeof(TA)) == 0 && reinterpret_cast<uintptr_t>(p.W) % (4 * sizeof(TW)) == 0)
-    return vipera_launch(gemm_short_kernel<TA, TW>, dim3(static_cast<unsigned>((p.N + kShortColumns - 1) / kShortColumns), short_rows),
-                         dim3(kShortThreads), 0, s, p);
+  const bool direct = kBothFloat && p.K % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.W)) & 15) == 0;
+  const bool parts = direct && p.M > TileMid::BM && p.status;   // many rows: three parts of every number on the tensor cores
+  if (p.K <= (parts ? kShortInnerParts : kShortInner) && (p.M > kFewRows || !direct) && (p.M + kShortRows - 1) / kShortRows <= 65535) {
+    const bool vec = p.K % 4 == 0 && reinterpret_cast<uintptr_t>(p.A) % (4 * sizeof(TA)) == 0 &&
+                     reinterpret_cast<uintptr_t>(p.W) % (4 * sizeof(TW)) == 0;
+    return vec ? launch_short<TA, TW, true>(p, s) : launch_short<TA, TW, false>(p, s);
+  }
   if constexpr (kBothFloat) {
-    if (p.K % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.W)) & 15) == 0) {
+    if (direct) {
       if (p.M <= kFewRows) return launch_few(p, s);
       if (p.M <= TileSome::BM) return launch_tile<TA, TW, TileSome, true>(p, s);
       if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileMid, true>(p, s);
-      if (p.status)   // more rows than a half tile: three parts of every number on the tensor cores
+      if (parts)
         return gemm_split::launch({static_cast<const float*>(p.A), static_cast<const float*>(p.W), p.M, p.N, p.K, 1, 0, p.bias, p.out,
                                    p.resid, p.activation, p.epilogue, p.out_bf16, p.status,
                                    static_cast<uint8_t*>(p.parts), nullptr, p.parts_bytes}, s);
@@ -527,7 +571,7 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
   }
   // rows that do not start on 16 bytes, or values that are widened on the way
   if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileSome, false>(p, s);
-  return launch_tile<TA, TW, TileMid, false>(p, s);
+  return launch_tile<TA, TW, TileLow, false>(p, s);
 }
 
 template <typename TA, typename TW>
