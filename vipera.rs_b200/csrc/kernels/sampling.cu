@@ -65,7 +65,7 @@ VIPERA_API int vipera_apply_penalties(float* logits, int vocab, int entries, con
 }
 
 // ---------------------------------------------------------------------------------------
-// argmax with ties to the lowest id, over the block
+// argmax with ties to the lowest id
 // ---------------------------------------------------------------------------------------
 struct Best {
   float value;
@@ -78,35 +78,6 @@ __device__ __forceinline__ Best better_of(Best a, Best b) {
   if (b.value > a.value) return b;
   return a.id < b.id ? a : b;
 }
-__device__ Best block_argmax(const float* __restrict__ row, int vocab, Best* scratch /* 32 */) {
-  Best best{0.0f, -1};
-  for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
-    const float v = row[i];
-    if (finite(v)) best = better_of(best, Best{v, i});
-  }
-#pragma unroll
-  for (int offset = 16; offset > 0; offset >>= 1) {
-    Best other;
-    other.value = __shfl_xor_sync(0xffffffffu, best.value, offset);
-    other.id = __shfl_xor_sync(0xffffffffu, best.id, offset);
-    best = better_of(best, other);
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) scratch[warp] = best;
-  __syncthreads();
-  const int warps = (blockDim.x + 31) >> 5;
-  best = lane < warps ? scratch[lane] : Best{0.0f, -1};
-#pragma unroll
-  for (int offset = 16; offset > 0; offset >>= 1) {
-    Best other;
-    other.value = __shfl_xor_sync(0xffffffffu, best.value, offset);
-    other.id = __shfl_xor_sync(0xffffffffu, best.id, offset);
-    best = better_of(best, other);
-  }
-  return best;
-}
-
 // Greedy over a wide vocabulary in two stages, so that many blocks read each row at once:
 // every block finds the best of its slice of the row (eight independent loads in flight per
 // thread), then one warp per row picks the best of the slices.  Ties still go to the lowest id.
