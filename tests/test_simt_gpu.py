@@ -34,11 +34,8 @@ def test_product_tiles_and_slabs(m, n, k, types):
     ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, bias=bias, out=out)
     # the error of a chain of k roundings of random sign, 2^-24 each, is some sqrt(k) 2^-24 of the sum at most
     assert _rel(out, a.double() @ w.double().T + bias.double()) < 2.0 ** -24 * (k ** 0.5 + 4)
-    # a row's result does not depend on the rows beside it, within its class (up to eight rows, up to 64; with more the
-    # blocks that share an inner size depend on the count of tiles)
-    if m > 64:
-        return
-    beside = 1 if m <= 8 else 9
+    # a row's result does not depend on the rows beside it, within its class (up to eight rows, up to 64, more)
+    beside = 1 if m <= 8 else 9 if m <= 64 else 65
     last = torch.empty(beside, n, device=DEV)
     ops.gemm_simt(a[-beside:].contiguous(), w, epilogue=ops.EPI_STORE, bias=bias, out=last)
     assert torch.equal(last[-1], out[-1])
@@ -98,6 +95,22 @@ def test_product_in_parts(m, n, k, epilogue):
     # no worse than a chain of k roundings of 2^-24, row by row
     error = (out.double() - want).norm(dim=1) / want.norm(dim=1)
     assert float(error.max()) < 2.0 ** -24 * (k ** 0.5 + 6)
+
+
+# a row of more than 64 is summed in one order, whatever the count of rows, its place among them, how many blocks share its
+# K (one, two and four), and what splits its numbers (its own block or the kernel ahead)
+@pytest.mark.parametrize("n,k", [(9728, 896), (1152, 896), (896, 4864), (256, 2048), (160, 700), (2048, 1540), (6144, 2048)])
+def test_a_row_of_many_does_not_depend_on_the_others(n, k):
+    ops = _ops()
+    torch.manual_seed(n + k)
+    a, w = torch.randn(4200, k, device=DEV), torch.randn(n, k, device=DEV)
+    whole = torch.empty(4200, n, device=DEV)
+    ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, out=whole)
+    for m in (65, 130, 257, 500, 700, 1100, 2300):
+        out = torch.empty(m, n, device=DEV)
+        ops.gemm_simt(a[-m:].contiguous(), w, epilogue=ops.EPI_STORE, out=out)
+        assert torch.equal(out, whole[-m:]), m
+    ops.check_kernel_status(a.device)
 
 
 # rows with an infinity or a NaN in the forms that split both operands and that split the left one ahead, one block and

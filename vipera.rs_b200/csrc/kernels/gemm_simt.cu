@@ -4,8 +4,8 @@
 // The reference multiplies one weight matrix by all B activation rows in one pass over the
 // weights (crates/vipera-backend-cpu/src/model.rs:1005-1025) and promises that a row's
 // result does not depend on its neighbours in the batch (model.rs:881-882); here every output
-// element sums over K in an order that is fixed for its class of row counts: up to eight rows, up to 64 (and values that are
-// widened), or more, where the order also depends on how many blocks share K (gemm_split.cuh).
+// element sums over K in an order that is fixed by N, K and the class of row counts: up to eight rows, up to 64, or more (one
+// class for values that are widened and for rows off 16 bytes).
 //
 // Up to eight rows the stream of W bounds the product (gemv_rows_kernel): a warp reads eight rows of W
 // through a ring of its own, 512 neighbouring bytes of a row at a time, a lane's four values against all
@@ -563,7 +563,7 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
       if (p.M <= TileSome::BM) return launch_tile<TA, TW, TileSome, true>(p, s);
       if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileMid, true>(p, s);
       if (parts)
-        return gemm_split::launch({static_cast<const float*>(p.A), static_cast<const float*>(p.W), p.M, p.N, p.K, 1, 0, p.bias, p.out,
+        return gemm_split::launch({static_cast<const float*>(p.A), static_cast<const float*>(p.W), p.M, p.N, p.K, 1, 0, 1, p.bias, p.out,
                                    p.resid, p.activation, p.epilogue, p.out_bf16, p.status,
                                    static_cast<uint8_t*>(p.parts), nullptr, p.parts_bytes}, s);
       return launch_tile<TA, TW, TileMany, true>(p, s);

@@ -16,8 +16,9 @@
 // memory (three images of 128 rows each, 128-byte swizzle, two stages of 96 KB); eight warps add up, the first of which
 // issues 24 products of 16 values a stage (a warp of its own for that would leave too few registers).  The left
 // operand's images are written once by a kernel ahead and copied in bulk where that pays (parts_bytes), else the same
-// warps split both.  Two pairs of accumulators fill tensor memory.  Where the tiles are too few to fill the chip, the
-// blocks of a cluster share K and add their parts through distributed shared memory.
+// warps split both.  Two pairs of accumulators fill tensor memory.  K is cut into up to four groups, each
+// summed on its own; where the tiles are too few to fill the chip, the blocks of a cluster share the groups and add their sums
+// through distributed shared memory.
 // What bounds it: a stage's 24 products of 64 clocks read shared memory for all of these 1,536 clocks, and the
 // images' 96 KB are written there beside them; 3,400 clocks a stage are left of that in long K, and what a block costs
 // before its first and after its last stage (about six stages).  1,024 x 9,728 of 896: 183 us (multiply-adds: 503), the
@@ -40,7 +41,8 @@ enum { WAIT_EXPIRED = 6 };
 struct Args {
   const float* A;
   const float* W;
-  int M, N, K, cluster, share;   // share: stages of K a block of the cluster takes
+  int M, N, K;
+  int groups, share, cluster;    // groups of `share` stages of K that are summed on their own, and how many blocks share them
   const float* bias;
   void* out;
   float* resid;
@@ -59,7 +61,7 @@ struct Shared {
   uint32_t nan[2 * kRowWords];   // of those, the ones that hold a NaN
 };
 constexpr int kSharedBytes = kStages * kStageBytes + static_cast<int>(sizeof(Shared)) + 1024;
-static_assert(kTile * kSumPitch * 4 <= kStages * kStageBytes, "the tile's sums take the stages' place");
+static_assert(2 * kTile * kSumPitch * 4 <= kStages * kStageBytes, "the tile's sums, of two groups, take the stages' place");
 
 __device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_address(bar)), "r"(count));
@@ -174,8 +176,12 @@ gemm_split_kernel(const Args p) {
   volatile int* abort_flag = &s.abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x % p.cluster, n0 = blockIdx.x / p.cluster * kTile, m0 = blockIdx.y * kTile;
-  const int k_begin = min(rank * p.share * kDepth, p.K), k_end = min(k_begin + p.share * kDepth, p.K);
+  const int own_groups = p.groups / p.cluster, group_depth = p.share * kDepth;
+  const int k_begin = min(rank * own_groups * group_depth, p.K), k_end = min(k_begin + own_groups * group_depth, p.K);
   const int count = (k_end - k_begin + kDepth - 1) / kDepth;
+  // The groups' sums are added in their order: the first block of a cluster adds its own up as it goes; the others keep
+  // theirs apart, one tile each in shared memory (there are two at most: four groups in two blocks).
+  const bool apart = rank > 0 && own_groups > 1;
   pdl_launch_dependents();
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
@@ -206,6 +212,8 @@ gemm_split_kernel(const Args p) {
     float total[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) total[j] = 0.0f;
+    volatile float before[64];   // the groups before this one; in local memory, registers are short
+    bool some_before = false;
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTile >> 4) << 24) | (static_cast<uint32_t>(kTile >> 3) << 17);
     const uint32_t base = shared_address(stages);
     auto products = [&](int c) {
@@ -233,27 +241,56 @@ gemm_split_kernel(const Args p) {
       commit(&s.sums_full[stage]);
     };
     if (warp == kIssuer && count > 0) products(0);
-    for (int c = 0; c < count; ++c) {
-      if (warp == kIssuer && c + 1 < count) products(c + 1);   // (on their way while this warp adds)
-      const uint32_t pair = taddr + (c & 1) * 256;
-      bar_wait(&s.sums_full[c & 1], (c >> 1) & 1, abort_flag, p.status);
-      fence_after();
+    for (int c = 0; c < count;) {
+      const int group_end = min(c + p.share, count);
+#pragma unroll 1
+      for (; c < group_end; ++c) {
+        if (warp == kIssuer && c + 1 < count) products(c + 1);   // (on their way while this warp adds)
+        const uint32_t pair = taddr + (c & 1) * 256;
+        bar_wait(&s.sums_full[c & 1], (c >> 1) & 1, abort_flag, p.status);
+        fence_after();
 #pragma unroll
-      for (int j = 0; j < 64; j += 16) {
-        uint32_t large[16], small[16];
-        tmem_load_16(pair + j, large);
-        tmem_load_16(pair + 128 + j, small);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int j = 0; j < 64; j += 16) {
+          uint32_t large[16], small[16];
+          tmem_load_16(pair + j, large);
+          tmem_load_16(pair + 128 + j, small);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int e = 0; e < 16; ++e) total[j + e] = (total[j + e] + __uint_as_float(small[e])) + __uint_as_float(large[e]);
+          for (int e = 0; e < 16; ++e) total[j + e] = (total[j + e] + __uint_as_float(small[e])) + __uint_as_float(large[e]);
+        }
+        fence_before();
+        bar_arrive(&s.sums_empty[c & 1]);
       }
-      fence_before();
-      bar_arrive(&s.sums_empty[c & 1]);
+      if (own_groups == 1) break;
+      if (some_before && !apart) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) total[j] = before[j] + total[j];
+      }
+      if (c < count) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) {
+          before[j] = total[j];
+          total[j] = 0.0f;
+        }
+        some_before = true;
+      }
     }
     // (the last sums are complete, so every product that read the stages is)
+    float* own = sums + row * kSumPitch + column0;
+    if (apart) {   // the first group's tile, then the second's
+      if (!some_before) {
 #pragma unroll
-    for (int j = 0; j < 64; j += 4)
-      *reinterpret_cast<float4*>(sums + row * kSumPitch + column0 + j) = make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]);
+        for (int j = 0; j < 64; ++j) {
+          before[j] = total[j];
+          total[j] = 0.0f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(own + j) = make_float4(before[j], before[j + 1], before[j + 2], before[j + 3]);
+      own += kTile * kSumPitch;
+    }
+#pragma unroll
+    for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(own + j) = make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]);
   } else {
     // ---------------- operands: runs of eight values, four a thread and stage of either operand ----------------
     constexpr int kRuns = AHEAD ? 4 : 8, kFirstW = kRuns - 4;
@@ -346,13 +383,24 @@ gemm_split_kernel(const Args p) {
         const float* others = of_a ? p.W + static_cast<size_t>(n0) * p.K : p.A + static_cast<size_t>(m0) * p.K;
         const int count_others = min(kTile, of_a ? p.N - n0 : p.M - m0);
         for (int i = warp; i < count_others; i += kThreads / 32) {
-          float sum = nan ? NAN : 0.0f;
-          if (!nan) {
+          float* at = sums + (of_a ? r : i) * kSumPitch + (of_a ? i : r);
+          float all = nan ? NAN : 0.0f;
+          for (int group = 0; group < own_groups; ++group) {
+            const int begin = min(k_begin + group * group_depth, k_end), end = min(begin + group_depth, k_end);
+            float sum = 0.0f;
+            if (!nan) {
 #pragma unroll 4
-            for (int k = k_begin + lane; k < k_end; k += 32) sum = fmaf(own[k], others[static_cast<size_t>(i) * p.K + k], sum);
-            sum = warp_sum(sum);
+              for (int k = begin + lane; k < end; k += 32) sum = fmaf(own[k], others[static_cast<size_t>(i) * p.K + k], sum);
+              sum = warp_sum(sum);
+            }
+            if (apart && group == 0) {
+              if (lane == 0) at[0] = all + sum;
+              all = 0.0f;
+            } else {
+              all += sum;
+            }
           }
-          if (lane == 0) sums[(of_a ? r : i) * kSumPitch + (of_a ? i : r)] = sum;
+          if (lane == 0) at[apart ? kTile * kSumPitch : 0] = all;
         }
       }
     }
@@ -366,7 +414,10 @@ gemm_split_kernel(const Args p) {
     if (p.cluster == 1) return *own;
     const uint32_t at = shared_address(own);
     float sum = remote_float(at, 0);
-    for (int r = 1; r < p.cluster; ++r) sum += remote_float(at, r);
+    for (int r = 1; r < p.cluster; ++r) {
+      sum += remote_float(at, r);
+      if (own_groups > 1) sum += remote_float(at + kTile * kSumPitch * 4, r);
+    }
     return sum;
   };
   const bool gated = p.epilogue == 2;
@@ -399,25 +450,28 @@ gemm_split_kernel(const Args p) {
   if (p.cluster > 1) cluster_sync();   // no block leaves while another reads its part
 }
 
-// Blocks of a cluster share K where that leaves fewer stages in a row: (waves of blocks) x (stages of a block + what it
-// costs besides).  Returns the stages in a row.
-static long long share_out(long long tiles, long long depth, int* cluster, int* share_of_block) {
-  constexpr long long kSms = 148;
-  long long best = 0, in_a_row = 0;
-  for (int blocks = 1; blocks <= 4; blocks *= 2) {
-    const long long share = (depth + blocks - 1) / blocks, waves = (tiles * blocks + kSms - 1) / kSms;
-    if (blocks > 1 && waves * (share + 4) >= best) continue;
-    best = waves * (share + 4), in_a_row = waves * share;
-    *cluster = blocks, *share_of_block = static_cast<int>(share);
-  }
-  return in_a_row;
+// How K is cut.  A call costs about (waves of blocks) x (stages of a block + what it costs besides).  The groups that are
+// summed on their own are as many as blocks would share K with a single tile of rows: they follow from N and K alone, so that
+// a row's sums have one order whatever the step's other rows are.  The blocks of a cluster share the groups where that is
+// faster for the rows there are.
+constexpr long long kSms = 148;   // (not asked of the device: the groups follow from it)
+static double cost_of(long long tiles, int blocks, int stages) { return static_cast<double>((tiles * blocks + kSms - 1) / kSms) * (stages + 4); }
+static void share_out(int M, int N, int K, int* groups, int* share, int* cluster) {
+  const long long tiles_n = (N + kTile - 1) / kTile, tiles = tiles_n * ((M + kTile - 1) / kTile);
+  const int depth = (K + kDepth - 1) / kDepth;
+  *groups = *cluster = 1;
+  for (int n = 2; n <= 4; n *= 2)
+    if (cost_of(tiles_n, n, (depth + n - 1) / n) < cost_of(tiles_n, *groups, (depth + *groups - 1) / *groups)) *groups = n;
+  *share = (depth + *groups - 1) / *groups;
+  for (int n = 2; n <= *groups; n *= 2)
+    if (cost_of(tiles, n, *groups / n * *share) < cost_of(tiles, *cluster, *groups / *cluster * *share)) *cluster = n;
 }
 
 static int launch_rows(const Args& args, cudaStream_t s) {
   Args p = args;
   const long long tiles_n = (p.N + kTile - 1) / kTile, tiles_m = (p.M + kTile - 1) / kTile, depth = (p.K + kDepth - 1) / kDepth;
   if (tiles_m > 65535) return VIPERA_BAD_SHAPE;
-  share_out(tiles_n * tiles_m, depth, &p.cluster, &p.share);
+  share_out(p.M, p.N, p.K, &p.groups, &p.share, &p.cluster);
   const dim3 grid(static_cast<unsigned>(tiles_n * p.cluster), static_cast<unsigned>(tiles_m));
   if (!p.parts) return launch_in_clusters(gemm_split_kernel<false>, p.cluster, grid, dim3(kThreads), kSharedBytes, s, p);
   const int status = vipera_launch(gemm_split_left_kernel, dim3(static_cast<unsigned>(depth), static_cast<unsigned>(tiles_m)),
@@ -434,8 +488,9 @@ constexpr long long kMostParts = 96ll << 20, kTileExtra = kRowWords * 4;   // (b
 static int parts_bytes(int M, int N, int K) {
   if (M <= 64 || N <= kTile || K % 4 != 0) return 0;   // (one tile along N: nobody else would split the same rows)
   const long long tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile;
-  int cluster, share;
-  if (share_out(tiles_m * tiles_n, (K + kDepth - 1) / kDepth, &cluster, &share) < 8) return 0;
+  int groups, share, cluster;
+  share_out(M, N, K, &groups, &share, &cluster);
+  if ((tiles_m * tiles_n * cluster + kSms - 1) / kSms * (groups / cluster * share) < 8) return 0;   // stages in a row
   const long long of_tile = (K + kDepth - 1) / kDepth * (kParts * kImageBytes + kTileExtra);
   const long long tiles = kMostParts / of_tile;
   return static_cast<int>((tiles < tiles_m ? tiles : tiles_m) * of_tile);
