@@ -97,6 +97,49 @@ def test_product_in_parts(m, n, k, epilogue):
     assert float(error.max()) < 2.0 ** -24 * (k ** 0.5 + 6)
 
 
+# Numbers whose parts are as large as they get and of one sign: what the left-out products of parts come to does not
+# average out.  Cut-off parts of 1 + 2^-7 - 2^-23 would leave out 4.7e-7 of every product; rounded ones leave out 2^-24 at most.
+@pytest.mark.parametrize("value", [1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -8 - 2.0 ** -23, 1 + 2.0 ** -8 + 2.0 ** -16 - 2.0 ** -23, 1.99999988079071])
+@pytest.mark.parametrize("m,n,k", [(65, 64, 192), (256, 256, 2048)])
+def test_product_in_parts_of_one_sign(value, m, n, k):
+    ops = _ops()
+    a, w = torch.full((m, k), value, device=DEV), torch.full((n, k), value, device=DEV)
+    a[1::2] *= -0.5
+    out = torch.empty(m, n, device=DEV)
+    ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, out=out)
+    want = a.double() @ w.double().T
+    # 2^-24 of what is left out, 2^-24 a step of the tensor cores' four within 64 values (the leading product's: towards zero),
+    # half of 2^-24 a sum of K / 64 in a row
+    assert float((out.double() / want - 1).abs().max()) < 2.0 ** -24 * (1 + 4 + 0.5 * k / 64)
+
+
+# positive numbers: the tensor cores' rounding towards zero does not average out either, and is held against what one chain
+# of fused multiply-adds loses
+def test_product_in_parts_of_positive_numbers():
+    ops = _ops()
+    torch.manual_seed(3)
+    a, w = torch.rand(300, 4864, device=DEV), torch.rand(256, 4864, device=DEV)
+    out, chain = torch.empty(300, 256, device=DEV), torch.zeros(300, 256, device=DEV)
+    ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, out=out)
+    for k in range(4864):
+        torch.addcmul(chain, a[:, k:k + 1], w[:, k].view(1, -1), out=chain)
+    want = a.double() @ w.double().T
+    assert _rel(out, want) < _rel(chain, want) < 2.0 ** -24 * 4864
+
+
+# a number above bfloat16's largest, a finite one, has no leading part: its row is computed with multiply-adds
+def test_product_in_parts_of_large_numbers():
+    ops = _ops()
+    torch.manual_seed(4)
+    a, w = torch.randn(130, 512, device=DEV), torch.randn(96, 512, device=DEV)
+    a[77, 5], a[90, 500] = 3.4028e38, -3.4028e38
+    w[:, 5], w[:, 500] = w[:, 5] * 1e-3, w[:, 500] * 1e-3
+    out = torch.empty(130, 96, device=DEV)
+    ops.gemm_simt(a, w, epilogue=ops.EPI_STORE, out=out)
+    want = a.double() @ w.double().T
+    assert float(((out.double() - want).norm(dim=1) / want.norm(dim=1)).max()) < 2.0 ** -24 * (512 ** 0.5 + 6)
+
+
 # a row of more than 64 is summed in one order, whatever the count of rows, its place among them, how many blocks share its
 # K (one, two and four), and what splits its numbers (its own block or the kernel ahead)
 @pytest.mark.parametrize("n,k", [(9728, 896), (1152, 896), (896, 4864), (256, 2048), (160, 700), (2048, 1540), (6144, 2048)])

@@ -1,16 +1,18 @@
 // 32-bit matrix products of many rows on the fifth-generation tensor cores: out[M, N] = A[M, K] . W[N, K]^T with A, W
 // and the sums in 32 bits.
 //
-// A 32-bit number is the exact sum of three bfloat16 numbers (its leading 8 bits, the next 8, the last 8, by
-// truncation), and a product of two bfloat16 numbers is exact in 32 bits.  So a . w is a1 w1 + (a1 w2 + a2 w1 + a2 w2
-// + a1 w3 + a3 w1) up to terms of 2^-24 of |a w| and below, six products in place of one.  The tensor cores round
+// A 32-bit number is the exact sum of three bfloat16 numbers (its first 8 bits rounded to nearest, the remainder's, and
+// what is left, at most 7 bits), and a product of two bfloat16 numbers is exact in 32 bits.  So a . w is a1 w1 + (a1 w2 + a2 w1
+// + a2 w2 + a1 w3 + a3 w1), six products in place of one, and a2 w3 + a3 w2 + a3 w3, left out: some 2^-24 of |a w| at most, 2^-28
+// on average, of either sign (parts cut off instead of rounded leave out up to 2^-21, always towards zero).  Of a number below
+// 2^-110 the last part has no place in bfloat16 any more: it is held to 2^-134.  The tensor cores round
 // every step of their sums towards zero, which over a long K would cost more than 32-bit multiply-adds do: so the
 // leading product and the five small ones have accumulators of their own, both are read after every 64 values of K
 // and added to the tile's sums in registers, rounded to nearest.  Against 64 bits the result is closer than a chain of
-// fused multiply-adds over K (1,024 rows through a model of two layers and K up to 4,864: 4.8e-7 against 2.2e-6).
-// An infinity or a NaN has no such parts (its products with their zeros would be NaN).  Nothing such a row of A or W
-// gives is finite, and no other row reads it: a block notes which of its rows hold one, writes NaN where a row holds a
-// NaN, and computes the outputs of rows with infinities alone with multiply-adds, a warp an output.
+// fused multiply-adds over K (1,024 rows through a model of two layers and K up to 4,864: 4.3e-7 against 2.1e-6).
+// An infinity or a NaN has no such parts (its products with their zeros would be NaN), nor has a number above bfloat16's
+// largest.  No other row reads such a row of A or W: a block notes which of its rows hold one, writes NaN where a row holds a
+// NaN, and computes the outputs of the others with multiply-adds, a warp an output.
 //
 // A block computes a tile of 128 x 128: eight warps read 64 values of K, split them and leave the parts in shared
 // memory (three images of 128 rows each, 128-byte swizzle, two stages of 96 KB); eight warps add up, the first of which
@@ -107,11 +109,15 @@ __device__ __forceinline__ uint64_t descriptor(uint32_t saddr) {
   return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
          (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
 }
-__device__ __forceinline__ float leading(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+// a number's bits with its upper half rounded to nearest (ties away from zero; a NaN's may end as a zero's, and its remainder
+// is NaN all the same)
+__device__ __forceinline__ uint32_t rounded(float v) { return __float_as_uint(v) + 0x8000u; }
+__device__ __forceinline__ float leading(float v) { return __uint_as_float(rounded(v) & 0xffff0000u); }
 // the upper halves of two 32-bit words, `lo`'s in the lower one
-__device__ __forceinline__ uint32_t uppers(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+__device__ __forceinline__ uint32_t uppers(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
 
-// Eight values' pieces of the three images; odd(): one of them is not finite (its remainder is NaN).
+// Eight values' pieces of the three images; odd(): one of them is not finite (its remainder is NaN), or so large that its
+// leading part is not.
 struct Pieces {
   uint32_t first[4], second[4], third[4];
   float sum;
@@ -121,9 +127,9 @@ struct Pieces {
 #pragma unroll
     for (int e = 0; e < 8; e += 2) {
       const float r0 = v[e] - leading(v[e]), r1 = v[e + 1] - leading(v[e + 1]);
-      first[e >> 1] = uppers(v[e], v[e + 1]);
-      second[e >> 1] = uppers(r0, r1);
-      third[e >> 1] = uppers(r0 - leading(r0), r1 - leading(r1));
+      first[e >> 1] = uppers(rounded(v[e]), rounded(v[e + 1]));
+      second[e >> 1] = uppers(rounded(r0), rounded(r1));
+      third[e >> 1] = uppers(__float_as_uint(r0 - leading(r0)), __float_as_uint(r1 - leading(r1)));
       sum = fmaf(r0, 0.0f, fmaf(r1, 0.0f, sum));
     }
   }
