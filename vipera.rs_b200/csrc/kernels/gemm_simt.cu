@@ -635,6 +635,6 @@ VIPERA_API int vipera_gemm_simt_status(const void* A, int a_dtype, const void* W
 }
 
 // The bytes that 32-bit products of such sizes want for the parts of their left operand (0: none).
-VIPERA_API int vipera_gemm_simt_parts(int M, int N, int K) { return gemm_split::parts_bytes(M, N, K); }
+VIPERA_API int vipera_gemm_simt_parts(int M, int N, int K) { return K <= kShortInnerParts ? 0 : gemm_split::parts_bytes(M, N, K); }
 
 VIPERA_API const char* vipera_gemm_simt_status_text(int status) { return vipera_status_text(status); }

@@ -20,6 +20,7 @@ from ..weights.loader import FREE_EXTENT
 DEVICE_RESERVE_BYTES = 16 << 20  # kept free on the device (crates/vipera-core/src/planner.rs:23)
 PLANNED_STEP_TOKENS = 2048       # the step the workspace is sized for
 PRODUCT_SCRATCH_BYTES = 32 << 20  # partial sums of split products (the buffer starts at this size)
+PRODUCT_PARTS_BYTES = 96 << 20    # the parts of a 32-bit product's left operand, at most (gemm_split.cuh: kMostParts)
 
 
 def _element_bytes(dtype: str) -> int:
@@ -82,12 +83,12 @@ def kv_bytes_per_token(spec: ModelSpec, element_bytes: int) -> int:
 
 def workspace_bytes(spec: ModelSpec, batch: int, element_bytes: int, tokens: int = PLANNED_STEP_TOKENS) -> int:
     """The 32-bit residual stream (twice where the embedding's rows are kept beside it), the normalised input, the most any layer asks for (layers
-    share their buffers), the products' scratch for partial sums, and the 32-bit logits rows of
-    a batch."""
+    share their buffers), the products' scratch for partial sums (and, in 32-bit runs, for the parts of
+    their left operands), and the 32-bit logits rows of a batch."""
     layers = max(BLOCKS.find(layer.block).workspace_bytes(layer, tokens, element_bytes) for layer in spec.layers)
     stream = 8 if any(entry.adds_embedding for entry in spec.schedule) else 4
-    return (tokens * spec.hidden_size * (stream + element_bytes) + layers + PRODUCT_SCRATCH_BYTES
-            + batch * spec.vocab_size * 4)
+    products = PRODUCT_SCRATCH_BYTES + (PRODUCT_PARTS_BYTES if element_bytes == 4 else 0)
+    return tokens * spec.hidden_size * (stream + element_bytes) + layers + products + batch * spec.vocab_size * 4
 
 
 def plan_memory(spec: ModelSpec, ctx: int, batch: int, dtype: str, device_bytes: Optional[int] = None,

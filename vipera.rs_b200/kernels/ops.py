@@ -462,12 +462,20 @@ def head_rows(qkv: torch.Tensor, q_out: torch.Tensor, *, num_heads: int, num_kv_
     _check(fn(ctypes.byref(p), dtype_code(q_out.dtype), _stream()), "rope_cache")
 
 
+def gemm_simt_room(m: int, n: int, k: int) -> int:
+    """The bytes that a float32 product of these sizes wants beside it for the parts of its left operand (0: none)."""
+    return _function("gemm_simt", "vipera_gemm_simt_parts", [_c_int, _c_int, _c_int])(m, n, k) if m > 64 else 0
+
+
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE,
               bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-              resid: Optional[torch.Tensor] = None, activation: int = ACT_SILU) -> None:
-    """a[M, K] times w[N, K] transposed, on the CUDA cores with float32 accumulation.  ``bias``
-    counts in every ending (for the gated unit it is interleaved like the rows);
-    ``activation`` is the gated unit's."""
+              resid: Optional[torch.Tensor] = None, activation: int = ACT_SILU,
+              room: Optional[torch.Tensor] = None) -> None:
+    """a[M, K] times w[N, K] transposed with float32 accumulation: on the CUDA cores, or (float32, more than 64
+    rows) on the tensor cores in three bfloat16 parts of every number.  ``bias`` counts in every ending (for the
+    gated unit it is interleaved like the rows); ``activation`` is the gated unit's.  ``room``: gemm_simt_room bytes
+    that no other stream uses meanwhile.  Without it they come from the allocator for the call (and stay with a graph
+    that is being captured)."""
     fn = _function("gemm_simt", "vipera_gemm_simt_status",
                    [_c_void, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_int,
                     _c_void, _c_int, _c_void, _c_void, ctypes.c_longlong, _c_void])
@@ -477,14 +485,20 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE,
         raise InvalidArgumentError(f"gemm: inner sizes differ ({k} and {w.shape[1]})")
     _check_gemm_outputs(m, n, epilogue, bias, out, resid)
     pointer = _gpu(a, "a")
-    room, bytes_wanted = None, 0
-    if m > 64 and a.dtype == w.dtype == torch.float32:
-        bytes_wanted = _function("gemm_simt", "vipera_gemm_simt_parts", [_c_int, _c_int, _c_int])(m, n, k)
-        if bytes_wanted:
-            try:  # of the stream's own pool (a captured graph's, under capture): given back when the call returns
-                room = torch.empty(bytes_wanted, dtype=torch.uint8, device=a.device)
-            except torch.cuda.OutOfMemoryError:
-                bytes_wanted = 0  # the products then split both operands themselves
+    bytes_wanted = gemm_simt_room(m, n, k) if a.dtype == w.dtype == torch.float32 else 0
+    if not bytes_wanted:
+        room = None
+    elif room is not None:
+        if room.numel() * room.element_size() < bytes_wanted or room.data_ptr() % 16:
+            raise InvalidArgumentError(f"gemm: room must be {bytes_wanted} bytes on a 16-byte boundary")
+        _gpu(room, "room")
+    else:
+        try:  # of the stream's own pool: given back when the call returns
+            room = torch.empty(bytes_wanted, dtype=torch.uint8, device=a.device)
+        except torch.cuda.OutOfMemoryError:
+            pass  # the product then splits both operands itself
+    if room is None:
+        bytes_wanted = 0
     _check(fn(pointer, dtype_code(a.dtype), _gpu(w, "w"), dtype_code(w.dtype), m, n, k, epilogue,
               _opt(bias, "bias", torch.float32), _opt(out, "out"),
               dtype_code(out.dtype) if out is not None else F32, _opt(resid, "resid", torch.float32),

@@ -2,9 +2,9 @@
 
 The product is ``a[M, K] . w[N, K]^T`` with one of three endings: store (with an optional
 bias), add into the 32-bit residual stream, or SwiGLU over interleaved gate and up rows.
-Which kernel runs is decided here, by dtype and size: the 32-bit path always uses the
-CUDA-core kernel; the bfloat16 path uses the tensor-core kernel where it takes the sizes
-and the CUDA-core kernel elsewhere.
+Which kernel runs is decided here, by dtype and size: the 32-bit path always uses the 32-bit
+product (``ops.gemm_simt``); the bfloat16 path uses the tensor-core kernel where it takes the
+sizes and ``ops.gemm_simt`` elsewhere.
 """
 from __future__ import annotations
 
@@ -130,4 +130,12 @@ class Linear:
         if self.tensor_core and a.dtype == torch.bfloat16 and a.is_contiguous() and a.data_ptr() % 16 == 0:
             ops.gemm_tc(a, self.weight, epilogue=epilogue, bias=bias, out=out, resid=resid, activation=activation)
             return
-        ops.gemm_simt(a, self.weight, epilogue=epilogue, bias=bias, out=out, resid=resid, activation=activation)
+        room = None
+        if a.dtype == self.weight.dtype == torch.float32:
+            # one for all products of a step, which run one after another: a captured graph would keep its own otherwise
+            wanted = ops.gemm_simt_room(a.shape[0], self.out_features, self.in_features)
+            try:
+                room = ctx.workspace.get("linear.parts", (wanted,), torch.uint8) if wanted else None
+            except torch.cuda.OutOfMemoryError:
+                pass   # the product does without
+        ops.gemm_simt(a, self.weight, epilogue=epilogue, bias=bias, out=out, resid=resid, activation=activation, room=room)
