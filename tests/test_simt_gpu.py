@@ -156,6 +156,32 @@ def test_a_row_of_many_does_not_depend_on_the_others(n, k):
     ops.check_kernel_status(a.device)
 
 
+# more rows than the room for the left operand's parts holds are taken in turns: every ending's rows are those of products of
+# one turn
+@pytest.mark.parametrize("epilogue,dtype", [(0, torch.float32), (0, torch.bfloat16), (1, torch.float32), (2, torch.float32), (2, torch.bfloat16)])
+def test_rows_in_turns(epilogue, dtype):
+    ops = _ops()
+    m, n, k, one = 2400, 160, 14336, 700
+    of_tile, room = ops.gemm_simt_room(128, n, k), ops.gemm_simt_room(m, n, k)
+    assert room < -(-m // 128) * of_tile // 2 and ops.gemm_simt_room(one, n, k) == -(-one // 128) * of_tile   # three turns, and one
+    torch.manual_seed(epilogue)
+    a, w, bias = torch.randn(m, k, device=DEV) * k ** -0.5, torch.randn(n, k, device=DEV), torch.randn(n, device=DEV)
+    before = torch.randn(m, n // 2 if epilogue == 2 else n, device=DEV).to(dtype)
+
+    def product(rows):
+        out = before[rows].clone()
+        ops.gemm_simt(a[rows].contiguous(), w, epilogue=epilogue, bias=bias, **({"resid": out} if epilogue == 1 else {"out": out}))
+        return out
+
+    whole = product(slice(0, m))
+    for first in range(0, m, one):
+        rows = slice(min(first, m - one), min(first, m - one) + one)
+        assert torch.equal(whole[rows], product(rows)), first
+    if epilogue == 0 and dtype == torch.float32:
+        assert _rel(whole, a.double() @ w.double().T + bias.double()) < 2.0 ** -24 * (k ** 0.5 + 6)
+    ops.check_kernel_status(a.device)
+
+
 # rows with an infinity or a NaN in the forms that split both operands and that split the left one ahead, one block and
 # clusters: what such a row gives is as multiply-adds give it, and the rows beside it do not notice
 @pytest.mark.parametrize("m,n,k,ahead", [(140, 130, 256, False), (256, 256, 2048, True), (1024, 896, 1300, True)])
