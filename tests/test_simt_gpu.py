@@ -221,12 +221,13 @@ def _attention_want(q, keys, values, entry, position, heads, kv_heads, scale, ma
     return out * torch.sigmoid(gate.double()).view(len(q), heads, 1)
 
 
-# counts of tokens at the borders of the two forms (64) and of a tile (64 rows, several requests in one), head sizes of
-# every instance, rows that are not whole 16-byte pieces, every mask; a value nobody may see yet is infinite
-@pytest.mark.parametrize("counts,firsts", [([1], [0]), ([1, 1, 1], [5, 130, 700]), ([64], [3]), ([65], [0]), ([1, 70, 130, 1], [90, 0, 65, 200]),
+# counts of tokens at the borders of two forms (64) and of a tile (64 rows, several requests in one), head sizes of
+# every instance, rows that are not whole 16-byte pieces, every mask, narrow (a warp per token and head takes most of those) and
+# wide; a value nobody may see yet is infinite
+@pytest.mark.parametrize("counts,firsts", [([1], [0]), ([1, 1, 1], [5, 130, 700]), ([7, 40, 1, 30, 7], [100, 3, 64, 0, 33]), ([64], [3]), ([65], [0]), ([1, 70, 130, 1], [90, 0, 65, 200]),
                                           ([1, 1, 70, 1, 1, 1], [0, 3, 40, 200, 7, 64])])
 @pytest.mark.parametrize("d,dv,heads,kv_heads", [(64, 64, 7, 1), (128, 96, 4, 2), (80, 256, 12, 1), (30, 18, 2, 2)])
-@pytest.mark.parametrize("mask", ["all", "window", "chunk"])
+@pytest.mark.parametrize("mask", ["all", "window", "chunk", "wide window", "wide chunk"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_forms(counts, firsts, d, dv, heads, kv_heads, mask, dtype):
     ops = _ops()
@@ -252,8 +253,9 @@ def test_attention_forms(counts, firsts, d, dv, heads, kv_heads, mask, dtype):
     q = torch.randn(tokens, heads, d).to(dtype)
     sink, gate = torch.randn(heads), torch.randn(tokens, heads)
     options = {"all": dict(window=0, keep_first=0, chunk=0), "window": dict(window=50, keep_first=3, chunk=0),
-               "chunk": dict(window=0, keep_first=0, chunk=48)}[mask]
-    learned = sink if mask != "chunk" else None
+               "chunk": dict(window=0, keep_first=0, chunk=48), "wide window": dict(window=600, keep_first=7, chunk=0),
+               "wide chunk": dict(window=0, keep_first=0, chunk=520)}[mask]
+    learned = sink if "chunk" not in mask else None
     want = _attention_want(q, keys, values, entry, position, heads, kv_heads, scale, mask, learned, gate=gate, **options)
     out = torch.full((tokens, heads * dv), float("nan"), device=DEV, dtype=dtype)
     ops.attention(q.view(tokens, -1).to(DEV), out, k_pool.to(DEV), v_pool.to(DEV), token_seq=entry.to(DEV), positions=position.to(DEV),

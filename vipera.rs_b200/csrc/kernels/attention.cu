@@ -7,7 +7,7 @@
 // Traversal: a block folds the keys 64 at a time with a running (max, sum, output) per row, the online
 // form of the reference's chunk fold (model.rs:2752-2857) and of its device kernels' partials
 // (crates/vipera-backend-gpu/src/layer.cu:307-467); few tokens split their keys between the blocks of a
-// cluster, more share what they read in tiles (see the two kernels).
+// cluster, more share what they read in tiles, and where few keys are visible a warp folds those of a (token, head) (see the three kernels).
 // Keys are found through the block table: position j lives in page table[j / page], slot
 // j % page (model.rs:1507-1542).
 //
@@ -24,6 +24,8 @@
 // This is the attention of the 32-bit path and of bfloat16 head sizes without tensor-core kernels.  It takes
 // every head size up to 256 (keys and values each; rows that are not whole 16-byte pieces are read value by
 // value), any number of heads and groups, any page size.
+#include <algorithm>
+
 #include "simt.cuh"
 
 constexpr int kMaxHeadDim = 256;
@@ -546,6 +548,133 @@ attention_tile_kernel(const AttentionParams p) {
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Few visible keys: a warp per (token, head) folds them 32 at a time, a lane's score from its own key's row, the weights
+// handed round by shuffles.  Nothing is staged or shared, so many warps fit a multiprocessor; what bounds it is a warp's
+// chain of reads, some 16 us per 32 keys.
+// ---------------------------------------------------------------------------------------
+constexpr int kWarpsPerBlock = 4;
+
+// Dot product of `n` floats in shared memory with a row of T in memory.
+template <typename T, bool VEC>
+__device__ __forceinline__ float dot_row(const float* q, const T* __restrict__ row, int n) {
+  float sum = 0.0f;
+  if constexpr (!VEC) {
+    for (int i = 0; i < n; ++i) sum = fmaf(q[i], to_float<T>(row[i]), sum);
+  } else if constexpr (sizeof(T) == 4) {
+#pragma unroll 4
+    for (int i = 0; i < n; i += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(row + i);
+      sum = fmaf(q[i], f.x, sum);
+      sum = fmaf(q[i + 1], f.y, sum);
+      sum = fmaf(q[i + 2], f.z, sum);
+      sum = fmaf(q[i + 3], f.w, sum);
+    }
+  } else {
+#pragma unroll 4
+    for (int i = 0; i < n; i += 8) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(row + i);
+      const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(pairs[e]);
+        sum = fmaf(q[i + 2 * e], f.x, sum);
+        sum = fmaf(q[i + 2 * e + 1], f.y, sum);
+      }
+    }
+  }
+  return sum;
+}
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+attention_warp_kernel(const AttentionParams p) {
+  __shared__ float q_shared[kWarpsPerBlock][kMaxHeadDim];
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x, h = blockIdx.y * kWarpsPerBlock + warp;
+  if (h >= p.num_heads) return;
+  const int kv_head = h / (p.num_heads / p.num_kv_heads), d = p.head_dim, dv = p.value_dim;
+  pdl_wait();
+  const int position = p.positions[t];
+  const int* table = p.block_table + static_cast<size_t>(p.token_seq[t]) * p.table_width;
+  int kept, first;
+  visible_keys(p, position, &kept, &first);
+  const T* q_row = static_cast<const T*>(p.q) + (static_cast<size_t>(t) * p.num_heads + h) * d;
+  float* qs = q_shared[warp];
+  for (int i = lane; i < d; i += 32) qs[i] = to_float<T>(q_row[i]);
+  __syncwarp();
+  const T* k_head = static_cast<const T*>(p.k_pool) + static_cast<size_t>(kv_head) * d;
+  const T* v_head = static_cast<const T*>(p.v_pool) + static_cast<size_t>(kv_head) * dv;
+  const size_t k_stride = static_cast<size_t>(p.num_kv_heads) * d, v_stride = static_cast<size_t>(p.num_kv_heads) * dv;
+
+  constexpr int kColumns = kMaxHeadDim / 32;
+  float acc[kColumns];
+#pragma unroll
+  for (int i = 0; i < kColumns; ++i) acc[i] = 0.0f;
+  float row_max = -INFINITY, row_sum = 0.0f;
+  // two runs of keys: the kept first ones that the window has left behind, then the window
+  for (int run = 0; run < 2; ++run) {
+    const int begin = run == 0 ? 0 : first, end = run == 0 ? kept : position + 1;
+    for (int base = begin; base < end; base += 32) {
+      const int count = min(32, end - base);
+      int place = 0;
+      float score = -INFINITY;
+      if (lane < count) {
+        const int key = base + lane;
+        place = table[key / p.page_size] * p.page_size + key % p.page_size;
+        score = dot_row<T, VEC>(qs, k_head + static_cast<size_t>(place) * k_stride, d) * p.scale;
+      }
+      const float top = fmaxf(row_max, warp_max(score)), shift = top == -INFINITY ? 0.0f : top;
+      const float alpha = row_max == top ? 1.0f : expf(row_max - top);
+      const float weight = lane < count ? expf(score - shift) : 0.0f;
+      row_sum = row_sum * alpha + warp_sum(weight);
+      row_max = top;
+#pragma unroll
+      for (int i = 0; i < kColumns; ++i) acc[i] *= alpha;
+#pragma unroll 4
+      for (int k = 0; k < count; ++k) {
+        const float w = __shfl_sync(0xffffffffu, weight, k);
+        const T* v_row = v_head + static_cast<size_t>(__shfl_sync(0xffffffffu, place, k)) * v_stride;
+#pragma unroll
+        for (int i = 0; i < kColumns; ++i)
+          if (lane + 32 * i < dv) acc[i] = fmaf(w, to_float<T>(v_row[lane + 32 * i]), acc[i]);
+      }
+    }
+  }
+  const float factor = ending_factor(p, h, row_max, row_sum);
+  T* out_row = static_cast<T*>(p.out) + (static_cast<size_t>(t) * p.num_heads + h) * dv;
+#pragma unroll
+  for (int i = 0; i < kColumns; ++i)
+    if (lane + 32 * i < dv) out_row[lane + 32 * i] = from_float<T>(acc[i] * factor * gate_factor(p, t, h, lane + 32 * i));
+}
+
+// Whether a warp per (token, head) is the faster one: only where no token sees more than 128 keys (of the block table's
+// width, a window or a chunk), by what the forms take, in microseconds (largest errors a third).  A warp: 14 + d / 32 per 32 keys
+// and 3 besides, or 450 / d pairs of a query and a key per nanosecond, whichever is more.  Split: a start, and a cluster
+// after the other.  Tiles: the 64 x 64 tiles of keys that a tile's requests walk one after another.  Warps / before: 100 tokens
+// of one request each with a window of 32, 14 heads of 64 on 2 in 32 bits 23 / 48 us, 8 heads of 96 21 / 216, 4 of 256 on 1
+// 25 / 94; 30 portions of 7 behind 100: 72 / 133, 68 / 310, 82 / 363; 64 tokens of one prompt: 36 / 17, 35 / 109, 42 / 43.
+static bool warps_win(const AttentionParams& p, int dp, bool vec, bool narrow, int requests) {
+  long long most = static_cast<long long>(p.table_width) * p.page_size;
+  if (p.window > 0) most = std::min<long long>(most, static_cast<long long>(p.window) + p.keep_first);
+  if (p.chunk > 0) most = std::min<long long>(most, p.chunk);
+  const double run = static_cast<double>(p.num_tokens) / std::max(requests, 1);   // tokens of a request, on average
+  // (many requests of a token each in bfloat16: the split form's clusters are worth more keys; 100 behind 300, 8 heads of 96: 220 / 380 us)
+  if (most > (narrow && run < 2 ? 512 : 128) || (p.num_tokens > kTileRows && requests <= 1)) return false;
+  const int group = p.num_heads / p.num_kv_heads;
+  // the keys there probably are: widths are in whole pages, and an engine's in powers of two from eight pages on
+  const double keys = most >= 128 ? 0.7 * most : most - 0.5 * p.page_size, d = std::max(p.head_dim, p.value_dim);
+  const double warps = std::max(3.0 + (14.0 + d / 32) * keys / 32, static_cast<double>(p.num_tokens) * p.num_heads * keys * std::max(d, 90.0) / 450e3);
+  const double start = dp == 64 ? 7.0 : dp == 128 ? 8.0 : 10.0, cluster = dp == 64 ? 0.11 : dp == 128 ? 0.21 : 0.6;
+  const double split = start + static_cast<double>(p.num_tokens) * p.num_kv_heads * ((group + kRows - 1) / kRows) * cluster *
+                                   (1.0 + std::max(keys - 128.0, 0.0) / 600);
+  if (p.num_tokens <= kTileRows) return warps < split;
+  if (run < 2) return warps < 8.0 + split;
+  const double walked = std::min(kTileRows / run + 1, static_cast<double>(requests)) * ((most + kTileKeys - 1) / kTileKeys);
+  return warps < 8.0 + walked * (dp == 64 ? (vec ? 7.0 : 10.0) : dp == 128 ? 12.0 : 19.0);
+}
+
 // Up to this many tokens (a tile's rows) a step's keys are split between blocks: a single tile per head would leave
 // the chip idle.  With more, tiles of 64 tokens share what they read.
 constexpr int kSplitTokens = 64;
@@ -567,6 +696,9 @@ static int launch_split(const AttentionParams& p, int clusters, cudaStream_t s) 
 template <typename T, int DP, bool VEC>
 static int launch_attention(const AttentionParams& asked, int requests, cudaStream_t s) {
   AttentionParams p = asked;
+  if (warps_win(p, DP, VEC, sizeof(T) == 2, requests))
+    return vipera_launch(attention_warp_kernel<T, VEC>, dim3(p.num_tokens, (p.num_heads + kWarpsPerBlock - 1) / kWarpsPerBlock),
+                         dim3(kWarpsPerBlock * 32), 0, s, p);
   if (p.num_tokens <= kSplitTokens) return launch_split<T, DP, VEC>(p, p.num_tokens, s);
   if (requests > 1) {
     p.singles = 1;
