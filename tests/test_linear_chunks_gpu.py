@@ -35,7 +35,7 @@ def _step(counts):
 
 @pytest.mark.parametrize("counts", COUNTS)
 @pytest.mark.parametrize("dim,vdim", SIZES)
-@pytest.mark.parametrize("far", [False, True])
+@pytest.mark.parametrize("far", [False, True, "all", "deep"])
 def test_decays_per_channel(counts, dim, vdim, far):
     from vipera_rs_b200.kernels import ops
 
@@ -46,6 +46,10 @@ def test_decays_per_channel(counts, dim, vdim, far):
     if far:   # single tokens that forget everything, and channels that forget within a few
         z[::17] = -3000.0
         z[:, ::5] -= 40.0
+    if far in ("all", "deep"):   # every channel leaves the products' range within a chunk; within sixteen tokens, one in seven
+        z = torch.randn(tokens, heads * dim) - 16.0 * 1.25
+        if far == "deep":
+            z[:, 1::7] -= 70.0
     offsets = (0, heads * dim, 2 * heads * dim, 2 * heads * dim + heads * vdim)
     state = torch.randn(entries + 1, heads * dim * vdim)
     starts, slots, fresh = _step(counts)

@@ -10,8 +10,11 @@
 // and the caller walks the chunks in between (start' = e^(B_end) start + E).  CHANNEL: a decay per key
 // channel, its logarithms in `log_decay`; A is then a plain product of q e^(B_t - B_m) and k e^(B_m - B_s)
 // with B_m in the chunk's middle, as long as no channel decays by more than e^-60 over the chunk (the
-// factors stay in range); else the terms' decays are multiplied up token by token.  Otherwise a constant
-// decay per head: A = (q k) a^(t - s) from a table of powers, whatever the decay, and q, k and v are
+// factors stay in range).  Else the chunk is taken as four of 16 tokens: q against its sixteen's start, k against its
+// end, each at most 1, and what lies between (or, within a sixteen, is too much) as a factor of its own; where some
+// channel decays by more than e^-60 within a sixteen, that sixteen's decays are multiplied up token by token.  4 heads of
+// 128 x 256, 400 tokens, every channel far: 126 us the mixer (walks: 135, multiplied up through whole chunks: 378), 120 with
+// none.  Otherwise a constant decay per head: A = (q k) a^(t - s) from a table of powers, whatever the decay, and q, k and v are
 // the silu of what `proj` holds.
 //
 // What bounds it: multiply-adds, and the instructions around them.  A walk pays five
@@ -46,7 +49,8 @@ struct LinearArgs {
 
 // What the chunked form takes: rows of whole 16-byte pieces, heads of up to 256 key channels.
 static inline bool linear_chunks_take(const LinearArgs& p) {
-  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.chunk_state) | reinterpret_cast<uintptr_t>(p.out);
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.chunk_state) | reinterpret_cast<uintptr_t>(p.out) |
+                          reinterpret_cast<uintptr_t>(p.alpha);
   return p.d % 4 == 0 && p.dv % 4 == 0 && p.d <= 256 && p.proj_width % 4 == 0 && p.v_off % 4 == 0 && (bases & 15) == 0;
 }
 
@@ -186,11 +190,12 @@ linear_ends_kernel(const LinearArgs p) {
 // while these are used.
 // ---------------------------------------------------------------------------------------
 constexpr int kStageRows = 16;
+constexpr int kSixteen = 16, kSixteens = kLinearChunk / kSixteen;
 
 template <int COLUMNS>
 static inline int linear_outputs_bytes(int d) {
   const int keys = d * kLinearPitch, ring = 2 * kStageRows * COLUMNS;
-  return (d * kLinearPitch + (keys > ring ? keys : ring) + kLinearChunk * kLinearPitch + d + kLinearChunk + 1) * 4;
+  return (d * kLinearPitch + (keys > ring ? keys : ring) + kLinearChunk * kLinearPitch + 2 * kSixteens * d + kLinearChunk + 1) * 4;
 }
 
 template <bool CHANNEL, int COLUMNS>
@@ -201,8 +206,8 @@ linear_outputs_kernel(const LinearArgs p) {
   float* qt = outputs_shared;                               // [d][kLinearPitch]
   float* kt = qt + p.d * kLinearPitch;                      // [d][kLinearPitch], then two stages [kStageRows][COLUMNS]
   float* at = kt + keys_floats;                             // [s][kLinearPitch]
-  float* middle = at + kLinearChunk * kLinearPitch;         // CHANNEL: [d] B_m
-  float* power = middle + p.d;                              // otherwise: a^0 .. a^64
+  float* middle = at + kLinearChunk * kLinearPitch;         // CHANNEL: [d] B_m; or [sixteen][d] what each decays by, and 1 over it
+  float* power = middle + 2 * kSixteens * p.d;              // otherwise: a^0 .. a^64
   pdl_launch_dependents();
   const int tid = threadIdx.x, h = blockIdx.y, job = blockIdx.z;
   const int column0 = blockIdx.x * COLUMNS;
@@ -270,7 +275,7 @@ linear_outputs_kernel(const LinearArgs p) {
       middle[i] = to_middle;
     }
   }
-  far = __syncthreads_or(far);   // some channel decays too far for the factors: q and k stay as they are
+  far = __syncthreads_or(far);   // some channel decays too far for the factors: q and k stay as they are, for now
   for (int i = tid; i < p.d * parts; i += kThreads) {
     const int c = i % p.d, from = i / p.d * per;
     const float* q = p.proj + p.q_off + static_cast<size_t>(h) * p.d + c + static_cast<size_t>(first) * p.proj_width;
@@ -351,32 +356,102 @@ linear_outputs_kernel(const LinearArgs p) {
       }
     }
   } else {
-    // a thread a key token and a part of the channels: its keys decay token by token, sixteen outputs at a time
     constexpr int kShares = kThreads / kLinearChunk;
-    const int s = tid % kLinearChunk, share = tid / kLinearChunk;
+    bool deep = false;   // some channel decays too far over sixteen tokens
+    for (int i = tid; i < p.d * kSixteens; i += kThreads) {
+      const int c = i % p.d, t0 = i / p.d * kSixteen;
+      const float* b = p.log_decay + (static_cast<size_t>(first) * p.heads + h) * p.d + c;
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kSixteen; ++j) sum += t0 + j < count ? b[static_cast<size_t>(t0 + j) * p.heads * p.d] : 0.0f;
+      deep |= !(sum > -kLinearMostDecay);
+    }
+    deep = __syncthreads_or(deep);
+    if (deep) {
+      // within a sixteen: a thread a key token and a part of the channels, its keys decay token by token
+      const int s = tid % kLinearChunk, share = tid / kLinearChunk, t0 = s / kSixteen * kSixteen;
+      float a[kSixteen];
+#pragma unroll
+      for (int j = 0; j < kSixteen; ++j) a[j] = 0.0f;
+      const float* alpha = p.alpha + (static_cast<size_t>(first) * p.heads + h) * p.d;
+      // two channels at a time: sixteen reads in flight bound this
 #pragma unroll 1
-    for (int t0 = 0; t0 < kLinearChunk; t0 += 16) {
-      float a[16];
+      for (int c = 2 * share; c < p.d; c += 2 * kShares) {
+        float2 decay[kSixteen];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) a[j] = 0.0f;
-      for (int c = share; c < p.d; c += kShares) {
-        const float* alpha = p.alpha + (static_cast<size_t>(first) * p.heads + h) * p.d + c;
-        float w = kt[c * kLinearPitch + s];
-        for (int t = s + 1; t < t0; ++t) w *= alpha[static_cast<size_t>(min(t, count - 1)) * p.heads * p.d];
+        for (int j = 0; j < kSixteen; ++j)
+          decay[j] = *reinterpret_cast<const float2*>(alpha + static_cast<size_t>(min(t0 + j, count - 1)) * p.heads * p.d + c);
+        float lo = kt[c * kLinearPitch + s], hi = kt[(c + 1) * kLinearPitch + s];
+        const float* x = qt + c * kLinearPitch + t0;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float decay = alpha[static_cast<size_t>(min(t0 + j, count - 1)) * p.heads * p.d];
-          if (t0 + j > s) w *= decay;
-          if (t0 + j >= s) a[j] = fmaf(qt[c * kLinearPitch + t0 + j], w, a[j]);
+        for (int j = 0; j < kSixteen; ++j) {
+          if (t0 + j > s) lo *= decay[j].x, hi *= decay[j].y;
+          if (t0 + j >= s) a[j] = fmaf(x[kLinearPitch + j], hi, fmaf(x[j], lo, a[j]));
         }
       }
       for (int turn = 0; turn < kShares; ++turn) {
         if (share == turn) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) at[s * kLinearPitch + t0 + j] = turn == 0 ? a[j] : at[s * kLinearPitch + t0 + j] + a[j];
+          for (int j = 0; j < kSixteen; ++j) at[s * kLinearPitch + t0 + j] = turn == 0 ? a[j] : at[s * kLinearPitch + t0 + j] + a[j];
         }
         __syncthreads();
       }
+    }
+    // q from its sixteen's start on, k to its sixteen's end, and what a sixteen decays by
+    for (int i = tid; i < p.d * kSixteens; i += kThreads) {
+      const int c = i % p.d, sixteen = i / p.d, t0 = sixteen * kSixteen;
+      const float* b = p.log_decay + (static_cast<size_t>(first) * p.heads + h) * p.d + c;
+      float z[kSixteen], sum = 0.0f, rest = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kSixteen; ++j) z[j] = t0 + j < count ? b[static_cast<size_t>(t0 + j) * p.heads * p.d] : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kSixteen; ++j) qt[c * kLinearPitch + t0 + j] *= expf(sum += z[j]);
+#pragma unroll
+      for (int j = kSixteen - 1; j >= 0; --j) {
+        kt[c * kLinearPitch + t0 + j] *= expf(rest);
+        rest += z[j];
+      }
+      middle[sixteen * p.d + c] = expf(sum);
+      middle[(kSixteens + sixteen) * p.d + c] = expf(-sum);   // (used where it stays in range)
+    }
+    __syncthreads();
+    // between sixteens, and within one where its own decay is a factor: tokens x 4 keys a thread
+    constexpr int kRowsA = kLinearChunk * kLinearChunk / 4 / kThreads;   // 4 or 8
+    const int row = tid / 16 * kRowsA, key = tid % 16 * 4, to = row / kSixteen, from = key / kSixteen;
+    if (from != to || !deep) {
+      float a[kRowsA][4];
+#pragma unroll
+      for (int i = 0; i < kRowsA; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[i][j] = 0.0f;
+      if (from <= to) {
+        // the factor between: of the second and third sixteen where they lie between, 1 over its own within one
+        const float* second = middle + (from == to ? kSixteens + to : 1) * p.d;
+        const bool by_second = from == to || (from < 1 && to > 1), by_third = from < 2 && to > 2;
+#pragma unroll 4
+        for (int c = 0; c < p.d; ++c) {
+          float4 k = *reinterpret_cast<const float4*>(kt + c * kLinearPitch + key);
+          const float m1 = second[c], m2 = middle[2 * p.d + c];
+          const float between = (by_second ? m1 : 1.0f) * (by_third ? m2 : 1.0f);
+          k = make_float4(k.x * between, k.y * between, k.z * between, k.w * between);
+#pragma unroll
+          for (int i4 = 0; i4 < kRowsA; i4 += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(qt + c * kLinearPitch + row + i4);
+            const float x[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              a[i4 + i][0] = fmaf(x[i], k.x, a[i4 + i][0]);
+              a[i4 + i][1] = fmaf(x[i], k.y, a[i4 + i][1]);
+              a[i4 + i][2] = fmaf(x[i], k.z, a[i4 + i][2]);
+              a[i4 + i][3] = fmaf(x[i], k.w, a[i4 + i][3]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < kRowsA; ++i) at[(key + j) * kLinearPitch + row + i] = key + j > row + i ? 0.0f : a[i][j];
     }
   }
   __syncthreads();   // the keys are read out; A is there
@@ -390,11 +465,13 @@ linear_outputs_kernel(const LinearArgs p) {
           *x = make_float4(x->x * factor, x->y * factor, x->z * factor, x->w * factor);
         }
       } else {
-        const float* b = p.log_decay + (static_cast<size_t>(first) * p.heads + h) * p.d + c;
-        float sum = 0.0f;
-        for (int t = 0; t < count; ++t) {
-          sum += b[static_cast<size_t>(t) * p.heads * p.d];
-          qt[c * kLinearPitch + t] *= expf(sum);
+        float before = 1.0f;   // what the sixteens before decay by
+        for (int t0 = 0; t0 < kLinearChunk; t0 += kSixteen) {
+          for (int t = t0; t < t0 + kSixteen; t += 4) {
+            float4* x = reinterpret_cast<float4*>(qt + c * kLinearPitch + t);
+            *x = make_float4(x->x * before, x->y * before, x->z * before, x->w * before);
+          }
+          before *= middle[t0 / kSixteen * p.d + c];
         }
       }
     }
