@@ -101,3 +101,34 @@ def test_decays_per_head(counts, dim, vdim):
     assert _rel(out, want) < 1e-5
     assert _rel(kept[:entries].view(entries, heads, dim, vdim), ends) < 1e-5
     assert torch.equal(kept[entries].cpu(), state[entries])
+
+
+# a value that is not finite shows in its own token's output and in later ones', not in the ones before it in its chunk
+@pytest.mark.parametrize("kind", ["channel", "head"])
+@pytest.mark.parametrize("dim,vdim", [(128, 256), (128, 96)])
+@pytest.mark.parametrize("token", [0, 7, 8, 45, 63, 77])
+def test_values_that_are_not_finite(kind, dim, vdim, token):
+    from vipera_rs_b200.kernels import ops
+
+    torch.manual_seed(dim + vdim)
+    heads, tokens = 2, 100
+    proj = torch.randn(tokens, heads * (2 * dim + 2 * vdim), device=DEV)
+    offsets = (0, heads * dim, 2 * heads * dim, 2 * heads * dim + heads * vdim)
+    starts, slots, fresh = _step([tokens])
+    jobs, outs = ops.scan_jobs(tokens, 1), []
+    for value in (1.0, float("inf"), float("nan")):
+        proj[token, offsets[2]:offsets[2] + heads * vdim] = value
+        state, out = torch.zeros(2, heads * dim * vdim, device=DEV), torch.full((tokens, heads * vdim), -7.0, device=DEV)
+        common = dict(offsets=offsets, heads=heads, dim=dim, vdim=vdim, norm_eps=1e-6, state=state, entry_starts=starts, state_slots=slots,
+                      fresh=fresh, num_entries=1, out=out)
+        scratch = torch.empty(jobs, heads * dim * vdim, device=DEV)
+        if kind == "channel":
+            ops.gla(proj, torch.ones(tokens, heads * dim, device=DEV), q_scale=dim ** -0.5, tau=16.0, norm_weight=torch.ones(vdim, device=DEV), out_scale=1.0,
+                    partial=torch.empty(ops.gla_shares(dim), tokens, heads * vdim, device=DEV), log_decay=torch.empty(tokens, heads * dim, device=DEV),
+                    chunk_scratch=(scratch, torch.empty(jobs, heads * dim, device=DEV)), **common)
+        else:
+            ops.lightning(proj, decay=torch.tensor([0.99, 0.5], device=DEV), norm_weight=torch.ones(heads * vdim, device=DEV),
+                          raw=torch.empty(tokens, heads * vdim, device=DEV), chunk_state=scratch, **common)
+        outs.append(out)
+    for out in outs[1:]:
+        assert torch.equal(out[:token], outs[0][:token]) and not torch.isfinite(out[token:]).any()

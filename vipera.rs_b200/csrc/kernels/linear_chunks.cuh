@@ -498,8 +498,11 @@ linear_outputs_kernel(const LinearArgs p) {
     const float* x_rows = (of_state ? qt : at) + row0 * kLinearPitch + group_t;
     const float* y_rows = kt + (stage & 1) * kStageRows * COLUMNS + group_n;
     const int rows = min(kStageRows, (of_state ? p.d : count) - row0);
+    // (of the chunk's values: those of the tokens before this thread's eight, whole, then its eight's own: a token takes no
+    // part of a value behind it, whatever that holds)
+    const int whole = of_state ? rows : min(max(group_t - row0, 0), rows);
 #pragma unroll 2
-    for (int r = 0; r < rows; ++r) {
+    for (int r = 0; r < whole; ++r) {
       const float4 lo = *reinterpret_cast<const float4*>(x_rows + r * kLinearPitch), hi = *reinterpret_cast<const float4*>(x_rows + r * kLinearPitch + 4);
       const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
@@ -511,6 +514,27 @@ linear_outputs_kernel(const LinearArgs p) {
           acc[i][4 * j + 1] = fmaf(x[i], y.y, acc[i][4 * j + 1]);
           acc[i][4 * j + 2] = fmaf(x[i], y.z, acc[i][4 * j + 2]);
           acc[i][4 * j + 3] = fmaf(x[i], y.w, acc[i][4 * j + 3]);
+        }
+      }
+    }
+    if (!of_state && group_t >= row0 && group_t < row0 + rows) {
+      const int own = min(8, row0 + rows - group_t);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        if (e >= own) break;
+        const float* at_x = x_rows + (group_t - row0 + e) * kLinearPitch;
+        const float4 lo = *reinterpret_cast<const float4*>(at_x), hi = *reinterpret_cast<const float4*>(at_x + 4);
+        const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int j = 0; j < kGroups; ++j) {
+          const float4 y = *reinterpret_cast<const float4*>(y_rows + (group_t - row0 + e) * COLUMNS + COLUMNS / 2 * j);
+#pragma unroll
+          for (int i = e; i < 8; ++i) {
+            acc[i][4 * j] = fmaf(x[i], y.x, acc[i][4 * j]);
+            acc[i][4 * j + 1] = fmaf(x[i], y.y, acc[i][4 * j + 1]);
+            acc[i][4 * j + 2] = fmaf(x[i], y.z, acc[i][4 * j + 2]);
+            acc[i][4 * j + 3] = fmaf(x[i], y.w, acc[i][4 * j + 3]);
+          }
         }
       }
     }
