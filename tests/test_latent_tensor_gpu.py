@@ -39,19 +39,33 @@ def _plain(w, h, kept, counts, firsts, heads, dim, rot, rank, vdim, window, sink
     return out.reshape(len(h), -1) @ w["p.o.weight"].T
 
 
-@pytest.mark.parametrize("counts,firsts", [([520], [0]), ([300, 1, 129, 130], [70, 200, 0, 63]), ([64, 65, 63, 400], [0, 1, 300, 0]), ([700, 1, 900], [0, 60, 10])])
-@pytest.mark.parametrize("heads,rank,rot,window,page", [(3, 512, 64, 0, 16), (12, 512, 64, 100, 16), (5, 256, 32, 0, 7), (7, 64, 8, 50, 64),
-                                                        (32, 384, 24, 0, 1), (128, 320, 64, 333, 16)])
-def test_fold(counts, firsts, heads, rank, rot, window, page):
+# few heads want many tokens: the rule sends shorter steps to the other form
+LONG = [([1100], [0]), ([2000, 1, 2100], [3, 60, 0]), ([1500, 1501], [0, 70]), ([700], [333])]
+SHORT = [([520], [0]), ([300, 1, 129, 130], [70, 200, 0, 63]), ([64, 65, 63, 400], [0, 1, 300, 0]), ([700, 1, 900], [0, 60, 10])]
+SOME = [([520], [0]), ([700, 1, 900], [0, 60, 10]), ([1000, 63, 1100], [5, 300, 0]), ([2000, 1, 2100], [3, 60, 0])]
+CASES = [(case, sizes) for cases, sizes in [(LONG, (3, 512, 64, 0, 16)), (SOME, (12, 512, 64, 100, 16)), (LONG[:3] + SOME[2:3], (5, 256, 32, 0, 7)),
+                                             (SOME, (7, 64, 8, 50, 64)), (SHORT, (32, 384, 24, 0, 1)), (SHORT, (128, 320, 64, 333, 16))] for case in cases]
+
+
+@pytest.mark.parametrize("case,sizes", CASES)
+def test_fold(case, sizes, monkeypatch):
+    (counts, firsts), (heads, rank, rot, window, page) = case, sizes
     from vipera_rs_b200.config.registry import MIXERS
     from vipera_rs_b200.config.spec import PartSpec
     from vipera_rs_b200.kernels import ops
     from vipera_rs_b200.parts.base import PagedKVView, StepContext, Workspace
 
+    real, took = ops._function, []
+
+    def asked(family, name, arguments):
+        function = real(family, name, arguments)
+        return (lambda params: took.append(function(params)) or took[-1]) if name == "vipera_latent_fold_tensor" else function
+
+    monkeypatch.setattr(ops, "_function", asked)
     torch.manual_seed(sum(counts) + heads + rank)
     hidden, dim, vdim, sink, tokens, entries = 256, 32, 64, bool(window), sum(counts), len(counts)
     position = PartSpec("rope_interleaved", {"head_dim": rot, "rotary_dims": rot, "theta": 10000.0, "scaling": None,
-                                             "exact_angles": True, "max_positions": 2048})
+                                             "exact_angles": True, "max_positions": 4096})
     params = {"hidden_size": hidden, "num_heads": heads, "head_dim": dim, "rot_dim": rot, "value_dim": vdim, "kv_rank": rank,
               "softmax_scale": (dim + rot) ** -0.5, "norm_eps": 1e-6, "position": position}
     if window:
@@ -63,7 +77,7 @@ def test_fold(counts, firsts, heads, rank, rot, window, page):
         tensor = torch.randn(*spec.shape, device=DEV) * std + (1.0 if "norm" in name else 0.0)
         w[name] = tensor if "norm" in name or "sink" in name else tensor.bfloat16()
     part = cls(params, "p", w, torch.bfloat16, DEV)
-    part.prepare(2048)
+    part.prepare(4096)
     h = torch.randn(tokens, hidden, device=DEV).bfloat16()
     kept = [(torch.randn(f, rank, device=DEV).bfloat16(), torch.randn(f, rot, device=DEV).bfloat16()) for f in firsts]
     longest = max(c + f for c, f in zip(counts, firsts))
@@ -92,6 +106,7 @@ def test_fold(counts, firsts, heads, rank, rot, window, page):
     part.forward(context, h, out, PagedKVView(0, k, v, page, window or None), True)
     torch.cuda.synchronize()
     ops.check_kernel_status(DEV)
+    assert took == [1]   # the tcgen05 form ran
     want = _plain({n: t.double() for n, t in w.items()}, h.double(), kept, counts, firsts, heads, dim, rot, rank, vdim, window, sink)
     # bfloat16 operands of five products in a row (queries, latents, weights, mixed latents, heads): 2^-9 each and a little
     assert float((out.double() - want).norm() / want.norm()) < 1e-2

@@ -989,25 +989,29 @@ static int launch_fold(const LatentFoldParams& f, dim3 grid, size_t shared, cuda
   return vipera_launch(latent_fold_kernel<NR, MT>, grid, kFoldThreads, shared, s, f);
 }
 
-// The tcgen05 fold runs a step in the head-major form from 1,536 rows on whose longest row sees more than 256 keys.  A
-// block's start (queries, tensor memory) weighs as much as a few tiles of 64 keys: mixers of 12 heads over prompts of
-// 128, 256 and 512 tokens take 75, 82 and 103 us with it and 62, 78 and 136 us without; 128 tokens behind 2,000: 181
-// and 194 us (32 heads: 202 and 364).
-constexpr long kTensorRows = 1536;
-constexpr int kTensorKeys = 256;
-
+// Where the tcgen05 fold is the faster one, in the head-major form: more than 2,048 rows whose longest sees more than 512 keys,
+// or 4,608 and 256.  A block's start (queries, tensor memory) weighs as much as a few tiles of 64 keys, and its 128 rows walk the
+// keys uncut, 3.6 us per 64 of them, so few rows leave most of the chip idle however long the history is.  One request, with
+// it / without, us of the mixer: 8 heads, 192 tokens behind 0 and 4,000: 84 / 73 and 283 / 238; 12 heads, 128 tokens behind 400,
+// 2,000 and 7,000: 98 / 91, 183 / 194, 447 / 485; 12 heads, 256 behind 8,000: 507 / 1,119; 12 heads, prompts of 300 and 512: 95 / 92 and
+// 103 / 136; 8 heads, a prompt of 512: 95 / 90; 32 heads, 128 behind 130 and 8,000: 104 / 100 and 523 / 1,033.  (266 such steps, 8 to 32
+// heads, 48 to 1,024 tokens behind up to 7,000, with and without a window of 512: the rule loses none and 1.2 % against the
+// better one of each.)
+// A token behind a long history makes one block walk it alone.  Histories are not known here one by one, so with several
+// requests the longest walk, taken at 5 us per 64 keys, has to fit into what the step's own tokens surely cost without it: half
+// of an even share of them seen by each on average, 42,000 keys of a row per microsecond.  8 heads, 600 + 1 + 100 tokens, the one
+// behind 2,000: 242 us with it, 134 without; 32 heads, 1,748 tokens of four requests behind up to 3,000: 666 and 1,158.  (It leaves
+// gains: two portions of 512 behind 3,000 each stay without.)
 static bool fold_takes_tensor(const LatentParams& p) {
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool) | reinterpret_cast<uintptr_t>(p.l_heads) |
                           reinterpret_cast<uintptr_t>(p.qa_heads) | reinterpret_cast<uintptr_t>(p.q_rot);
+  const long rows = static_cast<long>(p.num_tokens) * p.heads;
   const long keys = p.window > 0 ? std::min<long>(p.max_keys, static_cast<long>(p.window) + p.num_tokens) : p.max_keys;
-  // Its tiles hold 128 rows and their keys are not cut: a token behind a long history makes one block walk it alone (five
-  // microseconds per 64 keys).  With several requests that has to fit into what the step's own tokens surely cost without it
-  // (42,000 keys of a row per microsecond): 8 heads, 600 + 1 + 100 tokens, the one behind 2,000: 242 us with it, 134 without;
-  // 32 heads, 1,748 tokens of four requests behind up to 3,000: the mixer 666 and 1,158.
-  const double own = static_cast<double>(p.num_tokens) * p.heads * std::min<double>(keys, static_cast<double>(p.num_tokens) / std::max(p.requests, 1));
-  if (p.requests > 1 && own < 42000.0 * 2 * 5 / 64 * keys) return false;
-  return p.stage == 2 && keys > kTensorKeys && !p.single && p.status != nullptr && static_cast<long>(p.num_tokens) * p.heads >= kTensorRows &&
-         p.rank % latent_tc::kHalf == 0 && p.rot <= latent_tc::kHalf && (bases & 15) == 0;
+  if (p.stage != 2 || p.single || p.status == nullptr || p.rank % latent_tc::kHalf != 0 || p.rot > latent_tc::kHalf || (bases & 15) != 0) return false;
+  if (!(rows > 2048 && keys > 512) && !(rows > 4608 && keys > 256)) return false;
+  if (p.requests <= 1) return true;
+  const double own = 0.5 * rows * std::min<double>(keys, static_cast<double>(p.num_tokens) / p.requests);
+  return own / 42000.0 >= 5.0 / 64 * keys;
 }
 
 static int launch_fold_tensor(const LatentParams& p, cudaStream_t s) {
