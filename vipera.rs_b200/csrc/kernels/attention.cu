@@ -756,25 +756,4 @@ VIPERA_API int vipera_attention_step(const void* q, void* out, int dtype, const 
   return VIPERA_BAD_DTYPE;
 }
 
-VIPERA_API int vipera_attention_gated(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,
-                                      const int* token_seq, const int* positions, const int* block_table,
-                                      int table_width, int page_size, int num_tokens, int num_heads,
-                                      int num_kv_heads, int head_dim, int value_dim, float scale, int window,
-                                      int keep_first, int sink, int chunk, float out_scale, const float* sink_values,
-                                      const float* gate, long long gate_stride, int gate_per_head, void* stream) {
-  return vipera_attention_step(q, out, dtype, k_pool, v_pool, token_seq, positions, block_table, table_width, page_size, num_tokens,
-                               num_heads, num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink, chunk, out_scale,
-                               sink_values, gate, gate_stride, gate_per_head, 1, stream);
-}
-
-VIPERA_API int vipera_attention(const void* q, void* out, int dtype, const void* k_pool, const void* v_pool,
-                                const int* token_seq, const int* positions, const int* block_table,
-                                int table_width, int page_size, int num_tokens, int num_heads,
-                                int num_kv_heads, int head_dim, int value_dim, float scale, int window,
-                                int keep_first, int sink, int chunk, float out_scale, void* stream) {
-  return vipera_attention_gated(q, out, dtype, k_pool, v_pool, token_seq, positions, block_table, table_width, page_size,
-                                num_tokens, num_heads, num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink,
-                                chunk, out_scale, nullptr, nullptr, 0, 0, stream);
-}
-
 VIPERA_API const char* vipera_attention_status_text(int status) { return vipera_status_text(status); }

@@ -56,7 +56,6 @@ struct Tile {
 using TileSome = Tile<32, 128, 4, 1, 1, 32, 8, 4, 3>;
 using TileMid = Tile<64, 128, 2, 2, 4, 8, 8, 8, 3>;
 using TileLow = Tile<64, 64, 4, 2, 4, 8, 4, 4, 2>;   // little shared memory: four blocks an SM hide the staging through registers
-using TileMany = Tile<128, 128, 4, 2, 4, 8, 8, 8, 3>;
 
 struct GemmArgs {
   const void* A;
@@ -67,7 +66,7 @@ struct GemmArgs {
   float* resid;
   int activation, epilogue, out_bf16;
   int wide;            // rows of whole pieces of eight values on 16-byte boundaries
-  int* status;         // for the bounded waits of the tensor-core form, or null: it is not used
+  int* status;         // for the bounded waits of the tensor-core form
   void* parts;         // room for its left operand's parts, or null
   long long parts_bytes;
 };
@@ -551,7 +550,7 @@ template <typename TA, typename TW>
 static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
   constexpr bool kBothFloat = sizeof(TA) == 4 && sizeof(TW) == 4;
   const bool direct = kBothFloat && p.K % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.W)) & 15) == 0;
-  const bool parts = direct && p.M > TileMid::BM && p.status;   // many rows: three parts of every number on the tensor cores
+  const bool parts = direct && p.M > TileMid::BM;   // many rows: three parts of every number on the tensor cores
   if (p.K <= (parts ? kShortInnerParts : kShortInner) && (p.M > kFewRows || !direct) && (p.M + kShortRows - 1) / kShortRows <= 65535) {
     const bool vec = p.K % 4 == 0 && reinterpret_cast<uintptr_t>(p.A) % (4 * sizeof(TA)) == 0 &&
                      reinterpret_cast<uintptr_t>(p.W) % (4 * sizeof(TW)) == 0;
@@ -562,11 +561,11 @@ static int launch_sizes(const GemmArgs& p, cudaStream_t s) {
       if (p.M <= kFewRows) return launch_few(p, s);
       if (p.M <= TileSome::BM) return launch_tile<TA, TW, TileSome, true>(p, s);
       if (p.M <= TileMid::BM) return launch_tile<TA, TW, TileMid, true>(p, s);
-      if (parts)
+      if (p.status)
         return gemm_split::launch({static_cast<const float*>(p.A), static_cast<const float*>(p.W), p.M, p.N, p.K, 1, 0, 1, p.bias, p.out,
                                    p.resid, p.activation, p.epilogue, p.out_bf16, p.status,
                                    static_cast<uint8_t*>(p.parts), nullptr, p.parts_bytes}, s);
-      return launch_tile<TA, TW, TileMany, true>(p, s);
+      return VIPERA_BAD_ARGUMENT;
     }
   }
   // rows that do not start on 16 bytes, or values that are widened on the way
@@ -607,25 +606,9 @@ static int run_simt(const void* A, int a_dtype, const void* W, int w_dtype, int 
   return VIPERA_BAD_DTYPE;
 }
 
-VIPERA_API int vipera_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
-                                int epilogue, const float* bias, void* out, int out_dtype, float* resid,
-                                void* stream) {
-  // the form the earlier callers know: bias with STORE only, silu in the gated unit
-  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, epilogue == EPI_STORE ? bias : nullptr, out, out_dtype,
-                  resid, ACT_SILU, nullptr, nullptr, 0, stream);
-}
-
-// The same with a bias in every ending and the gated unit's activation chosen (ACT_SILU, ACT_GELU_TANH).
-VIPERA_API int vipera_gemm_simt_act(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
-                                    int epilogue, const float* bias, void* out, int out_dtype, float* resid,
-                                    int activation, void* stream) {
-  if (activation != ACT_SILU && activation != ACT_GELU_TANH) return VIPERA_BAD_ARGUMENT;
-  return run_simt(A, a_dtype, W, w_dtype, M, N, K, epilogue, bias, out, out_dtype, resid, activation, nullptr, nullptr, 0, stream);
-}
-
-// The same with a device word that must be 0 before the launch and is not afterwards where a bounded wait ran out: 32-bit
-// products of many rows may then run on the tensor cores, three parts of every number.  `parts`: room of
-// vipera_gemm_simt_parts bytes (16-byte aligned), or null.
+// A bias counts in every ending; `activation` is the gated unit's (ACT_SILU, ACT_GELU_TANH).  `status`: a device word that must
+// be 0 before the launch and is not afterwards where a bounded wait ran out; only 32-bit products of more than 64 rows need it.
+// `parts`: room of vipera_gemm_simt_parts bytes (16-byte aligned), or null.
 VIPERA_API int vipera_gemm_simt_status(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
                                        int epilogue, const float* bias, void* out, int out_dtype, float* resid,
                                        int activation, int* status, void* parts, long long parts_bytes, void* stream) {

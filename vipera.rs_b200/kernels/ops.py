@@ -502,7 +502,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE,
     _check(fn(pointer, dtype_code(a.dtype), _gpu(w, "w"), dtype_code(w.dtype), m, n, k, epilogue,
               _opt(bias, "bias", torch.float32), _opt(out, "out"),
               dtype_code(out.dtype) if out is not None else F32, _opt(resid, "resid", torch.float32),
-              int(activation), _tc_buffers(a.device, 0)["status"].data_ptr(),
+              int(activation), kernel_status_word(a.device).data_ptr() if m > 64 else None,
               room.data_ptr() if room is not None else None, bytes_wanted, _stream()), "gemm_simt", kernels=2 if room is not None else 1)
 
 
