@@ -27,9 +27,11 @@
 // left operand split in every block: 262; 2,048 x 4,096 of 14,336: 1,624 us, 148 TFLOP/s (the CUDA cores' own peak is 74).
 #pragma once
 
-#include "simt.cuh"
+#include "tcgen05.cuh"
 
 namespace gemm_split {
+
+using namespace tcgen05;
 
 constexpr int kTile = 128, kDepth = 64, kStages = 2, kParts = 3;
 constexpr int kImageBytes = kTile * kDepth * 2, kStageBytes = 2 * kParts * kImageBytes;
@@ -37,7 +39,6 @@ constexpr int kSumWarps = 8, kIssuer = 0, kFirstSplitter = 8, kSplitters = 256; 
 constexpr int kThreads = (kFirstSplitter + 8) * 32;
 constexpr int kSumPitch = kTile + 4;
 constexpr int kRowWords = kTile / 32;   // words of a bit per row
-constexpr uint32_t kWaitLimit = 1u << 22;
 enum { WAIT_EXPIRED = 6 };
 
 struct Args {
@@ -65,37 +66,6 @@ struct Shared {
 constexpr int kSharedBytes = kStages * kStageBytes + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(2 * kTile * kSumPitch * 4 <= kStages * kStageBytes, "the tile's sums, of two groups, take the stages' place");
 
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_address(bar)), "r"(count));
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(shared_address(bar)) : "memory");
-}
-__device__ __forceinline__ void bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done) : "r"(shared_address(bar)), "r"(parity) : "memory");
-    if (done) return;
-    if (spin > 8) __nanosleep(32);
-    if ((spin & 1023u) == 1023u && *abort_flag) return;
-  }
-  *abort_flag = 1;
-  atomicExch(status, WAIT_EXPIRED);
-}
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Issued by a whole warp that walks together, one elected lane issues.
-__device__ __forceinline__ void commit(uint64_t* bar) {
-  asm volatile(
-      "{\n .reg .pred leader;\n elect.sync _|leader, 0xffffffff;\n"
-      " @leader tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(shared_address(bar)) : "memory");
-}
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p, leader;\n elect.sync _|leader, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
-      " @leader tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
 #define GEMM_SPLIT_8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
 __device__ __forceinline__ void tmem_load_16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -225,8 +195,8 @@ gemm_split_kernel(const Args p) {
     auto products = [&](int c) {
       const uint32_t stage = c & 1, parity = (c >> 1) & 1;
       if (lane == 0) {
-        if (c >= 2) bar_wait(&s.sums_empty[stage], parity ^ 1u, abort_flag, p.status);
-        bar_wait(&s.full[stage], parity, abort_flag, p.status);
+        if (c >= 2) bar_wait<WAIT_EXPIRED>(&s.sums_empty[stage], parity ^ 1u, abort_flag, p.status);
+        bar_wait<WAIT_EXPIRED>(&s.full[stage], parity, abort_flag, p.status);
       }
       __syncwarp();
       fence_after();
@@ -236,12 +206,12 @@ gemm_split_kernel(const Args p) {
 #pragma unroll
       for (int ks = 0; ks < kDepth / 16; ++ks) {
         const uint64_t x = a + 2 * ks, y = w + 2 * ks;
-        mma(small, x + 2 * kNext, y, kIdesc, ks > 0 ? 1u : 0u);
-        mma(small, x, y + 2 * kNext, kIdesc, 1u);
-        mma(small, x + kNext, y + kNext, kIdesc, 1u);
-        mma(small, x + kNext, y, kIdesc, 1u);
-        mma(small, x, y + kNext, kIdesc, 1u);
-        mma(large, x, y, kIdesc, ks > 0 ? 1u : 0u);
+        mma_shared(small, x + 2 * kNext, y, kIdesc, ks > 0 ? 1u : 0u);
+        mma_shared(small, x, y + 2 * kNext, kIdesc, 1u);
+        mma_shared(small, x + kNext, y + kNext, kIdesc, 1u);
+        mma_shared(small, x + kNext, y, kIdesc, 1u);
+        mma_shared(small, x, y + kNext, kIdesc, 1u);
+        mma_shared(large, x, y, kIdesc, ks > 0 ? 1u : 0u);
       }
       commit(&s.empty[stage]);
       commit(&s.sums_full[stage]);
@@ -253,7 +223,7 @@ gemm_split_kernel(const Args p) {
       for (; c < group_end; ++c) {
         if (warp == kIssuer && c + 1 < count) products(c + 1);   // (on their way while this warp adds)
         const uint32_t pair = taddr + (c & 1) * 256;
-        bar_wait(&s.sums_full[c & 1], (c >> 1) & 1, abort_flag, p.status);
+        bar_wait<WAIT_EXPIRED>(&s.sums_full[c & 1], (c >> 1) & 1, abort_flag, p.status);
         fence_after();
 #pragma unroll
         for (int j = 0; j < 64; j += 16) {
@@ -334,7 +304,7 @@ gemm_split_kernel(const Args p) {
         if (const uint32_t rows = p.odd[three * kRowWords + i]) atomicOr(&s.odd[i % kRowWords], rows);
     for (int c = 0; c < count; ++c) {
       const int stage = c & 1;
-      if (c >= 2) bar_wait(&s.empty[stage], ((c >> 1) & 1) ^ 1, abort_flag, p.status);
+      if (c >= 2) bar_wait<WAIT_EXPIRED>(&s.empty[stage], ((c >> 1) & 1) ^ 1, abort_flag, p.status);
       if (AHEAD && t == 0) {
         const uint32_t bytes = *abort_flag ? 0 : kParts * kImageBytes, bar = shared_address(&s.full[stage]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -352,7 +322,7 @@ gemm_split_kernel(const Args p) {
         if (pieces.odd()) atomicOr(&s.odd[i < kFirstW ? i : kRowWords + i - kFirstW], 1u << sub);
         pieces.store(dst + (i < kFirstW ? 0 : kParts * kImageBytes) + ((i - kFirstW) & 3) * 32 * 128);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      fence_async();
       bar_arrive(&s.full[stage]);
     }
     if (AHEAD && t == 0 && *abort_flag) {   // a copy may be on its way still: it ends long before this does

@@ -28,9 +28,11 @@
 // Every wait is bounded; one that runs out leaves a code in the status word and the rows unwritten.
 #pragma once
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace latent_tc {
+
+using namespace tcgen05;
 
 constexpr int kRows = 128, kKeys = 64, kHalf = 64, kPart = 128;   // rows, keys of a tile, columns of a half part and of a part
 constexpr int kHalfBytes = kKeys * kHalf * 2, kQueryBytes = kRows * kHalf * 2;
@@ -39,7 +41,6 @@ constexpr int kMostHalves = 9;                       // 512 / 64 and the rotated
 constexpr int kSoftmaxWarps = 4, kIssuer = 4, kFirstLoader = 5, kLoaders = 2 * kSlots;
 constexpr int kThreads = (kFirstLoader + kLoaders) * 32;
 constexpr uint32_t kColsO = 0, kColsS = 256, kColsP = 384, kTmemCols = 512;   // O 256, S 2 x 64, P 2 x 32
-constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr float kLog2e = 1.4426950408889634f;
 enum { WAIT_EXPIRED = 5 };
 static_assert(kLoaders >= kMostHalves, "a loading warp brings at most one half part of the queries");
@@ -69,45 +70,6 @@ struct Shared {
 constexpr int kSharedBytes = kMostHalves * kQueryBytes + 2 * kSlots * kHalfBytes + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(kSharedBytes <= 227 * 1024, "a block's shared memory");
 
-__device__ __forceinline__ uint32_t addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(addr(bar)), "r"(count));
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(addr(bar)) : "memory");
-}
-__device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(done) : "r"(addr(bar)), "r"(parity) : "memory");
-  return done != 0;
-}
-__device__ __forceinline__ void bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
-    if (bar_try(bar, parity)) return;
-    if (spin > 8) __nanosleep(32);
-    if ((spin & 1023u) == 1023u && *abort_flag) return;
-  }
-  *abort_flag = 1;
-  atomicExch(status, WAIT_EXPIRED);
-}
-__device__ __forceinline__ void copy_piece(uint32_t dst, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Issued by a whole warp that walks the loop together, every lane with the same operands; one elected lane issues.
-__device__ __forceinline__ void commit(uint64_t* bar) {
-  asm volatile(
-      "{\n .reg .pred leader;\n elect.sync _|leader, 0xffffffff;\n"
-      " @leader tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mma_shared(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p, leader;\n elect.sync _|leader, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
-      " @leader tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void mma_tensor(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p, leader;\n elect.sync _|leader, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
@@ -204,7 +166,7 @@ latent_fold_tc_kernel(const Params p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kIssuer) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(addr(&s.tmem_base)), "r"(kTmemCols));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(shared_address(&s.tmem_base)), "r"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   // (the step's tokens are the host's, written before the step)
@@ -233,7 +195,7 @@ latent_fold_tc_kernel(const Params p) {
       float row_max = -INFINITY, row_sum = 0.0f;   // the max in powers of two
       for (int t = 0; t < g.tiles; ++t, ++count) {
         const uint32_t buffer = count & 1, parity = (count >> 1) & 1;
-        bar_wait(&s.score[buffer], parity, abort_flag, p.status);
+        bar_wait<WAIT_EXPIRED>(&s.score[buffer], parity, abort_flag, p.status);
         fence_after();
         uint32_t v[64];
         tmem_load(lanes + kColsS + buffer * kKeys, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
@@ -291,7 +253,7 @@ latent_fold_tc_kernel(const Params p) {
         bar_arrive(&s.weight[buffer]);
       }
       // the ending: the request's rows
-      bar_wait(&s.done, static_cast<uint32_t>(passes) & 1u, abort_flag, p.status);
+      bar_wait<WAIT_EXPIRED>(&s.done, static_cast<uint32_t>(passes) & 1u, abort_flag, p.status);
       fence_after();
       float total = row_sum;
       if (p.sink) total += exp2f(p.sink[head] * kLog2e - row_max);
@@ -323,12 +285,12 @@ latent_fold_tc_kernel(const Params p) {
     constexpr uint32_t kIdescScores = kIdesc | (static_cast<uint32_t>(kKeys >> 3) << 17);
     constexpr uint32_t kIdescValues = kIdesc | (1u << 16) | (static_cast<uint32_t>(kPart >> 3) << 17);       // B read down its rows
     constexpr uint32_t kIdescHalf = kIdesc | (1u << 16) | (static_cast<uint32_t>(kHalf >> 3) << 17);
-    const uint32_t query_addr = addr(queries), slot_addr = addr(slots);
+    const uint32_t query_addr = shared_address(queries), slot_addr = shared_address(slots);
     uint32_t score_slot = 0, score_parity = 0, value_slot = 0, value_parity = 0;   // of the next part of either ring
     int count = 0;                                                                // tiles issued
     const int rot_steps = (p.rot + 15) / 16;
     auto wait = [&](uint64_t* bar, uint32_t parity) {
-      if (lane == 0) bar_wait(bar, parity, abort_flag, p.status);
+      if (lane == 0) bar_wait<WAIT_EXPIRED>(bar, parity, abort_flag, p.status);
       __syncwarp();
       fence_after();
     };
@@ -415,7 +377,7 @@ latent_fold_tc_kernel(const Params p) {
     const bool of_values = slot >= kScoreSlots;
     const int ring = of_values ? kValueSlots : kScoreSlots, each = of_values ? own_parts : score_parts;   // slots, parts a tile
     const int piece = lane & 7, sub = lane >> 3;
-    const uint32_t dst = addr(slots + loader * kHalfBytes);
+    const uint32_t dst = shared_address(slots + loader * kHalfBytes);
     int number = of_values ? slot - kScoreSlots : slot, round = 0, count = 0;   // of the part, of the slot's use; tiles before this request
     // where keys lane and lane + 32 of a tile lie in the pools, -1: nowhere (zeros)
     int place_lo = -1, place_hi = -1;
@@ -446,9 +408,9 @@ latent_fold_tc_kernel(const Params p) {
         const int r = sub + 4 * j;   // (rows 32 and on from j = 8 on)
         const int place = __shfl_sync(0xffffffffu, j < 8 ? place_lo : place_hi, r & 31);
         const bool valid = place >= 0 && column;
-        copy_piece(dst + piece_offset(r, piece), valid ? pool + static_cast<size_t>(place) * stride : p.k_pool, valid);
+        copy_16(dst + piece_offset(r, piece), valid ? pool + static_cast<size_t>(place) * stride : p.k_pool, valid);
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
+      copy_commit();
     };
     bool queries_due = loader < halves;
     auto bring_queries = [&]() {   // half part `loader` of the queries, 32 rows of it at a time
@@ -495,11 +457,11 @@ latent_fold_tc_kernel(const Params p) {
         waited = true;
       }
       for (; number < (count + g.tiles) * each; number += ring, ++round) {
-        if (round > 0) bar_wait(&s.empty[slot], (round - 1) & 1, abort_flag, p.status);
+        if (round > 0) bar_wait<WAIT_EXPIRED>(&s.empty[slot], (round - 1) & 1, abort_flag, p.status);
         copy(number % each);
         if (number + ring < (count + g.tiles) * each) look_up(g, (number + ring) / each - count);
         if (queries_due) bring_queries();
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        copy_wait<0>();
         fence_async();
         bar_arrive(&s.full[slot]);
       }
