@@ -651,7 +651,7 @@ attention_warp_kernel(const AttentionParams p) {
 
 // Whether a warp per (token, head) is the faster one: only where no token sees more than 128 keys (of the block table's
 // width, a window or a chunk), by what the forms take, in microseconds (largest errors a third).  A warp: 14 + d / 32 per 32 keys
-// and 3 besides, or 450 / d pairs of a query and a key per nanosecond, whichever is more.  Split: a start, and a cluster
+// and 3 besides, 4 + d / 36 at least, or 450 / d pairs of a query and a key per nanosecond, whichever is more.  Split: a start, and a cluster
 // after the other.  Tiles: the 64 x 64 tiles of keys that a tile's requests walk one after another.  Warps / before: 100 tokens
 // of one request each with a window of 32, 14 heads of 64 on 2 in 32 bits 23 / 48 us, 8 heads of 96 21 / 216, 4 of 256 on 1
 // 25 / 94; 30 portions of 7 behind 100: 72 / 133, 68 / 310, 82 / 363; 64 tokens of one prompt: 36 / 17, 35 / 109, 42 / 43.
@@ -665,7 +665,8 @@ static bool warps_win(const AttentionParams& p, int dp, bool vec, bool narrow, i
   const int group = p.num_heads / p.num_kv_heads;
   // the keys there probably are: widths are in whole pages, and an engine's in powers of two from eight pages on
   const double keys = most >= 128 ? 0.7 * most : most - 0.5 * p.page_size, d = std::max(p.head_dim, p.value_dim);
-  const double warps = std::max(3.0 + (14.0 + d / 32) * keys / 32, static_cast<double>(p.num_tokens) * p.num_heads * keys * std::max(d, 90.0) / 450e3);
+  const double warps = std::max({3.0 + (14.0 + d / 32) * keys / 32, 4.0 + d / 36,
+                                 static_cast<double>(p.num_tokens) * p.num_heads * keys * std::max(d, 90.0) / 450e3});
   const double start = dp == 64 ? 7.0 : dp == 128 ? 8.0 : 10.0, cluster = dp == 64 ? 0.11 : dp == 128 ? 0.21 : 0.6;
   const double split = start + static_cast<double>(p.num_tokens) * p.num_kv_heads * ((group + kRows - 1) / kRows) * cluster *
                                    (1.0 + std::max(keys - 128.0, 0.0) / 600);

@@ -23,8 +23,9 @@
 // through distributed shared memory.
 // What bounds it: a stage's 24 products of 64 clocks read shared memory for all of these 1,536 clocks, and the
 // images' 96 KB are written there beside them; 3,400 clocks a stage are left of that in long K, and what a block costs
-// before its first and after its last stage (about six stages).  1,024 x 9,728 of 896: 183 us (multiply-adds: 503), the
-// left operand split in every block: 262; 2,048 x 4,096 of 14,336: 1,624 us, 148 TFLOP/s (the CUDA cores' own peak is 74).
+// before its first and after its last stage (about six stages).  1,024 x 9,728 of 896: 188 us (multiply-adds: 503; parts
+// cut off instead of rounded: 185), the left operand split in every block: 279; 8,192 x 4,096 of 4,096: 1,860 us, 148 TFLOP/s (the
+// CUDA cores' own peak is 74).
 #pragma once
 
 #include "tcgen05.cuh"
@@ -388,13 +389,14 @@ gemm_split_kernel(const Args p) {
   auto total = [&](int m, int n) {
     float* own = sums + m * kSumPitch + n;
     if (p.cluster == 1) return *own;
+    // (every part is asked for before the first is added)
     const uint32_t at = shared_address(own);
-    float sum = remote_float(at, 0);
-    for (int r = 1; r < p.cluster; ++r) {
-      sum += remote_float(at, r);
-      if (own_groups > 1) sum += remote_float(at + kTile * kSumPitch * 4, r);
-    }
-    return sum;
+    float part[4], second = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) part[r] = r < p.cluster ? remote_float(at, r) : 0.0f;
+    if (own_groups > 1) second = remote_float(at + kTile * kSumPitch * 4, 1);   // (four groups in two blocks)
+    if (p.cluster == 2) return own_groups > 1 ? (part[0] + part[1]) + second : part[0] + part[1];
+    return ((part[0] + part[1]) + part[2]) + part[3];
   };
   const bool gated = p.epilogue == 2;
   const int columns = gated ? kTile / 2 : kTile, column_bits = gated ? 6 : 7, row_step = 512 >> column_bits;
@@ -429,7 +431,8 @@ gemm_split_kernel(const Args p) {
 // How K is cut.  A call costs about (waves of blocks) x (stages of a block + what it costs besides).  The groups that are
 // summed on their own are as many as blocks would share K with a single tile of rows: they follow from N and K alone, so that
 // a row's sums have one order whatever the step's other rows are.  The blocks of a cluster share the groups where that is
-// faster for the rows there are.
+// faster for the rows there are.  (As many blocks for every count of rows, those that lose least on average: 256 x 896 of 896
+// 35 us, 2,048 x 896 of 4,864 192; so 26 and 166.)
 constexpr long long kSms = 148;   // (not asked of the device: the groups follow from it)
 static double cost_of(long long tiles, int blocks, int stages) { return static_cast<double>((tiles * blocks + kSms - 1) / kSms) * (stages + 4); }
 static void share_out(int M, int N, int K, int* groups, int* share, int* cluster) {
@@ -459,7 +462,8 @@ static int launch_rows(const Args& args, cudaStream_t s) {
 // Room for the left operand's parts, or 0 where splitting them ahead does not pay: a launch more, and each stage shorter
 // (5,500 clocks to 3,400).  Not more room than the L2 holds well: more rows are taken in turns.  Both operands split in the
 // block / the left one ahead: 80 x 896 of 896, seven stages in a row: 17.5 / 18.5 us; 1,024 x 1,152 of 896, seven: 30.6 / 31.2;
-// 256 x 256 of 2,048, eight: 33.9 / 27.0; 128 x 9,728 of 896, fourteen: 53.7 / 39.3; 8,192 x 4,096 of 4,096: 2,852 / 1,797.
+// 256 x 256 of 2,048, eight: 33.9 / 27.0 (these three with parts cut off); 128 x 9,728 of 896, fourteen: 57.9 / 41.2; 8,192 x 4,096
+// of 4,096: 3,057 / 1,860.
 constexpr long long kMostParts = 96ll << 20, kTileExtra = kRowWords * 4;   // (bytes beside each three of images: its rows' bits)
 static int parts_bytes(int M, int N, int K) {
   if (M <= 64 || N <= kTile || K % 4 != 0) return 0;   // (one tile along N: nobody else would split the same rows)
