@@ -80,28 +80,30 @@ __device__ __forceinline__ uint64_t descriptor(uint32_t saddr) {
   return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
          (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
 }
-// a number's bits with its upper half rounded to nearest (ties away from zero; a NaN's may end as a zero's, and its remainder
-// is NaN all the same)
-__device__ __forceinline__ uint32_t rounded(float v) { return __float_as_uint(v) + 0x8000u; }
-__device__ __forceinline__ float leading(float v) { return __uint_as_float(rounded(v) & 0xffff0000u); }
-// the upper halves of two 32-bit words, `lo`'s in the lower one
-__device__ __forceinline__ uint32_t uppers(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
+// Two numbers in one 64-bit register: what rounding both to bfloat16 gives, packed (ties away from zero; a NaN's may end as a
+// zero's, and its remainder is NaN all the same), and what it leaves of them.
+__device__ __forceinline__ uint32_t take_leading(unsigned long long& two) {
+  const uint32_t lo = static_cast<uint32_t>(two) + 0x8000u, hi = static_cast<uint32_t>(two >> 32) + 0x8000u;
+  const uint32_t minus_lo = (lo & 0xffff0000u) ^ 0x80000000u, minus_hi = (hi & 0xffff0000u) ^ 0x80000000u;
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(two) : "l"(static_cast<unsigned long long>(minus_hi) << 32 | minus_lo));
+  return __byte_perm(lo, hi, 0x7632);
+}
 
 // Eight values' pieces of the three images; odd(): one of them is not finite (its remainder is NaN), or so large that its
 // leading part is not.
 struct Pieces {
   uint32_t first[4], second[4], third[4];
-  float sum;
-  __device__ __forceinline__ bool odd() const { return sum != sum; }
-  __device__ __forceinline__ Pieces(const float4& lo, const float4& hi) : sum(0.0f) {
+  unsigned long long sums;
+  __device__ __forceinline__ bool odd() const { return sum_of_pair(sums) != 0.0f; }
+  __device__ __forceinline__ Pieces(const float4& lo, const float4& hi) : sums(0ull) {
     const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
     for (int e = 0; e < 8; e += 2) {
-      const float r0 = v[e] - leading(v[e]), r1 = v[e + 1] - leading(v[e + 1]);
-      first[e >> 1] = uppers(rounded(v[e]), rounded(v[e + 1]));
-      second[e >> 1] = uppers(rounded(r0), rounded(r1));
-      third[e >> 1] = uppers(__float_as_uint(r0 - leading(r0)), __float_as_uint(r1 - leading(r1)));
-      sum = fmaf(r0, 0.0f, fmaf(r1, 0.0f, sum));
+      unsigned long long two = static_cast<unsigned long long>(__float_as_uint(v[e + 1])) << 32 | __float_as_uint(v[e]);
+      first[e >> 1] = take_leading(two);
+      fma_pair(sums, two, 0ull);   // (0, or NaN)
+      second[e >> 1] = take_leading(two);
+      third[e >> 1] = __byte_perm(static_cast<uint32_t>(two), static_cast<uint32_t>(two >> 32), 0x7632);
     }
   }
   __device__ __forceinline__ void store(uint8_t* at) const {
