@@ -1,0 +1,119 @@
+"""Latent attention that expands every head's keys and values once a step (csrc/kernels/latent_heads.cuh), through the mixer,
+against a 64-bit restatement: tiles of 128 queries and keys that end inside one, several requests, windows that begin inside
+a tile, both rotations, pages of odd sizes, pages that hold no number; and the rule that chooses the form."""
+import numpy as np
+import pytest
+import torch
+
+from test_latent_tensor_gpu import _plain
+
+DEV = "cuda:0"
+DIM, ROT, VDIM, HIDDEN = 128, 64, 128, 256
+
+
+def _part(sizes, seed, device):
+    from vipera_rs_b200.config.registry import MIXERS
+    from vipera_rs_b200.config.spec import PartSpec
+
+    heads, rank, window, page, style, gated = sizes
+    position = PartSpec("rope_" + style, {"head_dim": ROT, "rotary_dims": ROT, "theta": 10000.0, "scaling": None,
+                                          "exact_angles": True, "max_positions": 4096})
+    params = {"hidden_size": HIDDEN, "num_heads": heads, "head_dim": DIM, "rot_dim": ROT, "value_dim": VDIM, "kv_rank": rank,
+              "softmax_scale": (DIM + ROT) ** -0.5, "norm_eps": 1e-6, "position": position, "output_gate": gated}
+    if window:
+        params.update(window=window, sink="learned")
+    cls, w = MIXERS.find("latent_attention"), {}
+    torch.manual_seed(seed)
+    for name, spec in cls.schema(params, "p").items():
+        std = {"p.q.weight": 0.06, "p.uk.weight": 0.06, "p.uv.weight": 0.06, "p.sink.weight": 1.5}.get(name, 0.06)
+        tensor = torch.randn(*spec.shape, device=device) * std + (1.0 if "norm" in name else 0.0)
+        w[name] = tensor if "norm" in name or "sink" in name else tensor.bfloat16()
+    part = cls(params, "p", w, torch.bfloat16, device)
+    return part, w
+
+
+STEPS = [([64], [0]), ([128], [128]), ([129, 1, 127], [0, 300, 5]), ([1, 257], [700, 1]), ([500, 3], [333, 0]), ([1030], [0])]
+SIZES = [(3, 512, 0, 16, "interleaved", False), (5, 256, 100, 7, "interleaved", True), (2, 64, 333, 1, "neox", True), (33, 320, 0, 64, "neox", False)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step", STEPS)
+@pytest.mark.parametrize("sizes", SIZES)
+def test_expanded(step, sizes, monkeypatch):
+    from vipera_rs_b200.kernels import ops
+    from vipera_rs_b200.parts import latent
+    from vipera_rs_b200.parts.base import PagedKVView, StepContext, Workspace
+
+    monkeypatch.setattr(latent, "EXPANDED_SHARE", 0)
+    (counts, firsts), (heads, rank, window, page, style, gated) = step, sizes
+    tokens, entries = sum(counts), len(counts)
+    part, w = _part(sizes, tokens + heads + rank, DEV)
+    part.prepare(4096)
+    h = torch.randn(tokens, HIDDEN, device=DEV).bfloat16()
+    kept = [(torch.randn(f, rank, device=DEV).bfloat16(), torch.randn(f, ROT, device=DEV).bfloat16()) for f in firsts]
+    longest = max(c + f for c, f in zip(counts, firsts))
+    width = -(-longest // page)
+    table = torch.randperm(entries * width).view(entries, width).to(torch.int32)
+    k = torch.full((entries * width, page, 1, rank), float("nan"), device=DEV, dtype=torch.bfloat16)
+    v = torch.full((entries * width, page, 1, ROT), float("nan"), device=DEV, dtype=torch.bfloat16)
+    for e, (c, r) in enumerate(kept):
+        at = torch.arange(firsts[e])
+        where = (table[e].long()[at // page].to(DEV), (at % page).to(DEV))
+        k[where[0], where[1], 0], v[where[0], where[1], 0] = c, r
+        gone = max(0, firsts[e] - window + 1) // page if window else 0   # pages no window reaches any more are given back
+        k[table[e, :gone].long().to(DEV)], v[table[e, :gone].long().to(DEV)] = float("nan"), float("nan")
+        table[e, :gone] = -1
+    device = lambda values: torch.from_numpy(np.ascontiguousarray(values, dtype=np.int32)).to(DEV)  # noqa: E731
+    context = StepContext(
+        num_tokens=tokens, num_entries=entries, tokens=device(np.zeros(tokens)),
+        positions=device(np.concatenate([np.arange(f, f + c) for c, f in zip(counts, firsts)])),
+        token_entry=device(np.repeat(np.arange(entries), counts)), entry_starts=device(np.cumsum([0] + counts)), entry_pos0=device(firsts),
+        state_slots=device(np.arange(entries)), fresh=device(np.zeros(entries)), block_tables=[table.to(DEV)], logit_rows=None,
+        num_logit_rows=0, host_counts=counts, host_pos0=firsts, max_count=max(counts), max_kv_len=longest, all_single=False,
+        any_single=1 in counts, dtype=torch.bfloat16, workspace=Workspace(DEV))
+    for known in (True, False):   # as a step whose requests the host knows, and as a captured one
+        context.host_counts = counts if known else []
+        assert part.expanded_rows(context) > 0
+        out = torch.zeros(tokens, HIDDEN, device=DEV)
+        part.forward(context, h, out, PagedKVView(0, k, v, page, window or None), True)
+        torch.cuda.synchronize()
+        ops.check_kernel_status(DEV)
+        wide = {n: t.double() for n, t in w.items()}
+        if style == "neox":   # the restatement turns neighbours: put the values that turn together side by side
+            order = torch.arange(ROT, device=DEV).view(2, ROT // 2).T.reshape(-1)
+            rows = torch.cat([torch.arange(DIM, device=DEV), DIM + order])
+            wide["p.q.weight"] = wide["p.q.weight"].view(heads, DIM + ROT, HIDDEN)[:, rows].reshape(heads * (DIM + ROT), HIDDEN)
+            wide["p.dkv.weight"] = torch.cat([wide["p.dkv.weight"][:rank], wide["p.dkv.weight"][rank:][order]])
+        past = [(c, r[:, order] if style == "neox" else r) for c, r in kept]
+        eye = dict(wide, **{"p.o.weight": torch.eye(heads * VDIM, dtype=torch.float64, device=DEV)})
+        mixed = _plain(eye, h.double(), past, counts, firsts, heads, DIM, ROT, rank, VDIM, window, bool(window))
+        if gated:
+            mixed = mixed * torch.sigmoid(h.double() @ wide["p.g.weight"].T)
+        want = mixed @ wide["p.o.weight"].T
+        # bfloat16 operands of five products in a row (queries, latents, keys or values, weights, heads): 2^-9 each and a little
+        assert float((out.double() - want).norm() / want.norm()) < 1e-2
+        assert float(((out.double() - want).norm(dim=1) / want.norm(dim=1)).max()) < 4e-2
+
+
+def test_rule():
+    """Rows are each request's visible keys rounded up to 128; lone tokens, few tokens, rows that outweigh their queries and
+    other shapes of head stay with the latents, and what a captured step counts on holds for every step of its class."""
+    from types import SimpleNamespace
+
+    part, _ = _part((3, 512, 1024, 16, "interleaved", True), 0, "cpu")
+
+    def step(counts, firsts, **changes):
+        fields = dict(host_counts=counts, host_pos0=firsts, num_tokens=sum(counts), num_entries=len(counts), dtype=torch.bfloat16,
+                      all_single=max(counts) == 1, max_kv_len=max(c + f for c, f in zip(counts, firsts)))
+        return SimpleNamespace(**dict(fields, **changes))
+
+    assert part.expanded_rows(step([2048], [0])) == 2048
+    assert part.expanded_rows(step([300, 1], [3000, 5000])) == 1408 + 1024     # no further back than the window
+    assert part.expanded_rows(step([1] * 64, [2000] * 64)) == 0
+    assert part.expanded_rows(step([63], [0])) == 0
+    assert part.expanded_rows(step([64] + [1] * 10, [0] + [2000] * 10)) == 0
+    assert part.expanded_rows(step([2048], [0], dtype=torch.float32)) == 0
+    for counts, firsts in (([900, 100, 24], [0, 70, 3000]), ([1024], [7000]), ([1023, 1], [0, 4000])):
+        known, captured = step(counts, firsts), step(counts, firsts, host_counts=[])
+        if part.expanded_rows(captured):
+            assert 0 < part.expanded_rows(known) <= part.expanded_rows(captured)

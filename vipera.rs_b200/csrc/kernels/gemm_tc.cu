@@ -893,7 +893,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
               }
               use ^= 1;
             }
-          } else if (EXT && p.epilogue == EPI_STORE && p.out_dtype == VIPERA_BF16) {
+          } else if (p.epilogue == EPI_STORE && p.out_dtype == VIPERA_BF16) {
             // A plain store into bfloat16, with the activation of a unit without a gate on the way:
             // 64 accumulator columns make 64 outputs = one 128-byte row of bfloat16
 #pragma unroll 1
@@ -913,7 +913,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                     v[i] += n < p.features ? p.bias[n] : 0.0f;
                   }
                 }
-                if (p.activation == ACT_RELU2) {
+                if (EXT && p.activation == ACT_RELU2) {
 #pragma unroll
                   for (int i = 0; i < 32; ++i) {
                     const float r = fmaxf(v[i], 0.0f);
@@ -1733,7 +1733,7 @@ static int run_gemm(const void* A, const void* W, int T, int N, int K, int epilo
                (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
       if ((r = make_out_map(&map_out, out, T, N, false)) != VIPERA_OK) return r;
       p.tma_ending = 1;
-    } else if (ext && epilogue == EPI_STORE && out_dtype == VIPERA_BF16 && N % 8 == 0 &&
+    } else if (epilogue == EPI_STORE && out_dtype == VIPERA_BF16 && N % 8 == 0 &&
                (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
       if ((r = make_out_map(&map_out, out, T, N, true)) != VIPERA_OK) return r;
       p.tma_ending = 1;

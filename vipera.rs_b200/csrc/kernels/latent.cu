@@ -10,7 +10,7 @@
 //                                                    (latent_attention_kernel, latent_fold_kernel)
 //   out_h = (V_h l_h) * sigmoid(gate_h)              (latent_expand_kernel)
 //
-// so the keys and values of earlier tokens are never expanded.  Scores, softmax, the sums over
+// so the keys and values of earlier tokens are not expanded (long steps do expand them: latent_heads.cuh).  Scores, softmax, the sums over
 // keys, the latent's norm and the rotation are 32-bit.  Rotation: values (2i, 2i + 1) of the
 // rotated part (`pairing` 0) or values (i, i + rot/2) (`pairing` 1) turn by the angle whose cosine
 // and sine the tables hold at [position, i].  With a window w > 0 the query at position p sees keys
@@ -18,6 +18,7 @@
 // sink per head the softmax's denominator also holds exp(sink_h): a term without a key or a value,
 // which the scale does not touch.
 #include "attention_mma.cuh"
+#include "latent_heads.cuh"
 #include "latent_tc.cuh"
 #include "simt.cuh"
 
@@ -1143,6 +1144,15 @@ VIPERA_API int vipera_latent_attention(const LatentParams* params, int dtype, vo
 
 // 1 where the fold of these parameters runs on tcgen05 (one launch, whatever the splits), else 0.
 VIPERA_API int vipera_latent_fold_tensor(const LatentParams* params) { return fold_takes_tensor(*params) ? 1 : 0; }
+
+// The form of latent_heads.cuh, stage 1 ahead of the product that leaves `expanded`, stage 2 behind it.
+VIPERA_API int vipera_latent_heads(const latent_heads::Params* params, const void* expanded, int num_tokens, int stage, void* stream) {
+  if (num_tokens <= 0) return VIPERA_OK;
+  if (params->heads <= 0 || params->rank <= 0 || params->page_size <= 0 || params->table_width <= 0 || params->row_capacity <= 0) return VIPERA_BAD_SHAPE;
+  if (stage < 1 || stage > 2 || params->window < 0 || params->pairing < 0 || params->pairing > 1 || !(params->scale > 0.0f)) return VIPERA_BAD_ARGUMENT;
+  return latent_heads::launch(*params, expanded, num_tokens, stage, static_cast<cudaStream_t>(stream));
+}
+VIPERA_API int vipera_latent_heads_size() { return static_cast<int>(sizeof(latent_heads::Params)); }
 
 VIPERA_API int vipera_latent_params_size() { return static_cast<int>(sizeof(LatentParams)); }
 VIPERA_API const char* vipera_latent_status_text(int status) { return vipera_status_text(status); }

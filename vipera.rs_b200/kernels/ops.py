@@ -1894,6 +1894,69 @@ def latent_attention(proj: torch.Tensor, *, q_off: int, g_off: int, kv_off: int,
     _check(fn(ctypes.byref(p), dtype_code(k_pool.dtype), _stream()), "attention", kernels=4 if kv_off >= 0 else 3)
 
 
+class _LatentHeadsParams(ctypes.Structure):
+    _fields_ = [
+        ("q", _c_void), ("q_width", ctypes.c_longlong), ("q_off", _c_int), ("gate", _c_void), ("gate_width", ctypes.c_longlong),
+        ("cos_table", _c_void), ("sin_table", _c_void), ("sink", _c_void), ("entry_starts", _c_void), ("entry_pos0", _c_void),
+        ("block_table", _c_void), ("k_pool", _c_void), ("v_pool", _c_void), ("rows", _c_void), ("rot_rows", _c_void), ("out", _c_void),
+        ("requests", _c_int), ("heads", _c_int), ("rank", _c_int), ("table_width", _c_int), ("page_size", _c_int), ("window", _c_int),
+        ("pairing", _c_int), ("row_capacity", _c_int), ("scale", _c_float), ("status", _c_void),
+    ]
+
+
+LATENT_HEADS_ROWS = 128   # a request's run of rows starts on a multiple of this
+
+
+def latent_heads(q: torch.Tensor, *, q_off: int, gate: Optional[torch.Tensor], gate_off: int, up_kv: torch.Tensor,
+                 entry_starts: torch.Tensor, entry_pos0: torch.Tensor, block_table: torch.Tensor, cos: torch.Tensor,
+                 sin: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, rows: torch.Tensor, rot_rows: torch.Tensor,
+                 expanded: torch.Tensor, out: torch.Tensor, heads: int, scale: float, window: int = 0,
+                 pairing: int = ROPE_INTERLEAVED, sink: Optional[torch.Tensor] = None) -> None:
+    """Attention over a cached latent by expanding every head's keys and values of the step's requests once, for steps whose
+    tokens share them (bfloat16; heads of 128 values and 64 rotated ones, values of 128).  ``q`` float32 [tokens, width] holds
+    the queries at column ``q_off``, head by head [128 | 64 not yet rotated]; ``gate`` (None: none) float32 [tokens, width]
+    the output gate's pre-activations at ``gate_off``.  The step's own latents are in the pools (latent_store).  ``up_kv``
+    [heads * 256, rank]: every head's key matrix, then every head's value matrix.  ``entry_starts`` [requests + 1] and
+    ``entry_pos0`` [requests] say which tokens are whose and where they begin.  Scratch in bfloat16, all of the same number of
+    rows, a multiple of 128 that holds every request's visible keys, each request's rounded up to one: ``rows`` [., rank],
+    ``rot_rows`` [., 64], ``expanded`` [., heads * 256]."""
+    fn = _function("latent", "vipera_latent_heads", [ctypes.POINTER(_LatentHeadsParams), _c_void, _c_int, _c_int, _c_void])
+    _check_struct("latent", "vipera_latent_heads_size", _LatentHeadsParams)
+    tokens, rank, page_size, requests = q.shape[0], k_pool.shape[3], k_pool.shape[1], block_table.shape[0]
+    capacity = rows.shape[0]
+    if tuple(k_pool.shape[1:]) != (page_size, 1, rank) or tuple(v_pool.shape[1:]) != (page_size, 1, 64) or v_pool.shape[0] != k_pool.shape[0]:
+        raise InvalidArgumentError("latent_heads: the pools must be [pages, page_size, 1, rank] and [pages, page_size, 1, 64]")
+    if tuple(up_kv.shape) != (heads * 256, rank) or tuple(out.shape) != (tokens, heads * 128) or q.shape[1] < q_off + heads * 192 or \
+            (gate is not None and (gate.shape[0] != tokens or gate.shape[1] < gate_off + heads * 128)):
+        raise InvalidArgumentError("latent_heads: the up matrices, the queries, the gate or the output have the wrong size")
+    if capacity % LATENT_HEADS_ROWS or tuple(rows.shape) != (capacity, rank) or tuple(rot_rows.shape) != (capacity, 64) or \
+            tuple(expanded.shape) != (capacity, heads * 256):
+        raise InvalidArgumentError("latent_heads: the scratch must have a multiple of 128 rows of rank, 64 and heads * 256 values")
+    if tuple(cos.shape[1:]) != (32,) or cos.shape != sin.shape or entry_starts.numel() != requests + 1 or entry_pos0.numel() != requests or \
+            (sink is not None and sink.numel() != heads):
+        raise InvalidArgumentError("latent_heads: the tables, the requests' starts or the sinks have the wrong size")
+    if pairing not in (ROPE_INTERLEAVED, ROPE_NEOX):
+        raise InvalidArgumentError("latent_heads: the rotated part turns as interleaved pairs or as halves")
+    p = _LatentHeadsParams()
+    p.q, p.q_width, p.q_off = _gpu(q, "q", torch.float32), q.shape[1], int(q_off)
+    if gate is not None:
+        p.gate, p.gate_width = _gpu(gate, "gate", torch.float32) + 4 * int(gate_off), gate.shape[1]
+    p.cos_table, p.sin_table = _gpu(cos, "cos", torch.float32), _gpu(sin, "sin", torch.float32)
+    p.sink = _opt(sink, "sink", torch.float32)
+    p.entry_starts, p.entry_pos0 = _gpu(entry_starts, "entry_starts", torch.int32), _gpu(entry_pos0, "entry_pos0", torch.int32)
+    p.block_table = _gpu(block_table, "block_table", torch.int32)
+    p.k_pool, p.v_pool = _gpu(k_pool, "k_pool", torch.bfloat16), _gpu(v_pool, "v_pool", torch.bfloat16)
+    p.rows, p.rot_rows = _gpu(rows, "rows", torch.bfloat16), _gpu(rot_rows, "rot_rows", torch.bfloat16)
+    p.out = _gpu(out, "out", torch.bfloat16)
+    p.requests, p.heads, p.rank, p.table_width, p.page_size = int(requests), int(heads), int(rank), int(block_table.shape[1]), int(page_size)
+    p.window, p.pairing, p.row_capacity, p.scale = int(window or 0), 1 if pairing == ROPE_NEOX else 0, int(capacity), float(scale)
+    p.status = _tc_buffers(q.device, 0)["status"].data_ptr()
+    to = _gpu(expanded, "expanded", torch.bfloat16)
+    _check(fn(ctypes.byref(p), to, tokens, 1, _stream()), "attention")
+    gemm_tc(rows, up_kv, epilogue=EPI_STORE, out=expanded)
+    _check(fn(ctypes.byref(p), to, tokens, 2, _stream()), "attention")
+
+
 def latent_store(proj: torch.Tensor, *, kv_off: int, norm_weight: Optional[torch.Tensor], eps: float,
                  positions: torch.Tensor, token_entry: torch.Tensor, block_table: torch.Tensor, cos: torch.Tensor,
                  sin: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, rot_dim: int,

@@ -10,9 +10,10 @@ learned number per head that stands for no token (``sink``).  The concatenated h
 (where the mixer has an output gate) and sent through the output matrix, which adds into the stream
 the mixer is handed.
 
-Since ``q . (U_h c) = (U_h^T q) . c`` and ``sum_j p_j V_h c_j = V_h sum_j p_j c_j``, the heads attend
-to the latents themselves (``csrc/kernels/latent.cu``): no earlier token's keys or values are ever
-expanded.  The pages hold the latents where other attention keeps keys (one "KV head" of ``rank``
+Since ``q . (U_h c) = (U_h^T q) . c`` and ``sum_j p_j V_h c_j = V_h sum_j p_j c_j``, the heads can attend
+to the latents themselves (``csrc/kernels/latent.cu``), without expanding any token's keys or values.
+A step of many tokens in bfloat16 does expand them, once for all of its queries, and attends plainly
+(``csrc/kernels/latent_heads.cuh``): a pair of a query and a key then costs a third.  The pages hold the latents where other attention keeps keys (one "KV head" of ``rank``
 values) and the rotated key part where it keeps values (``rot_dim`` values).  A layer built with
 ``own_cache = False`` has no down projection: it reads the pages another layer of the same latent
 geometry wrote in this step (the schedule hands it that layer's cache slot without write access).
@@ -32,6 +33,14 @@ from .base import Mixer, PagedKV
 from .linear import Linear
 
 
+# Where every head's keys and values are expanded for a step (csrc/kernels/latent_heads.cuh), us of the mixer over the latents
+# and expanded.  From 64 tokens on it is the faster one in all of 100 steps of 8 to 32 heads, ranks 256 and 512, behind up to
+# 7,000 tokens: 12 heads, a prompt of 2,048 under a window of 1,024: 287 / 109; 32 heads, 1,748 tokens of four requests behind
+# up to 3,000: 663 / 325; closest where few heads walk many keys, 8 heads, 64 behind 7,000: 182 / 161.  Below, few heads lose:
+# 8 heads, 32 and 48 behind 3,000: 71 / 89 and 85 / 90; 12 heads of rank 256, a prompt of 32: 37 / 41.
+EXPANDED_FROM = 64
+EXPANDED_SHARE = 1.4    # (query, key) pairs per row, at least: 32 heads, 64 + 1 + 1 behind 0, 2,000, 2,000 has 1.4 and 191 / 117
+EXPANDED_ROWS = 16384   # most rows of keys; memory is planned for them
 HEAD_MAJOR_FROM = 64   # tokens of a step from which the up products run head by head on the tensor cores
 
 
@@ -109,11 +118,16 @@ class LatentAttention(Mixer):
         # for long steps in bfloat16 both products run as grouped tensor-core products, a head a group:
         # U_h transposed [heads, rank, d] and V_h as stored [heads, value_dim, rank]
         self.head_major = (dtype == torch.bfloat16 and self.rank % 8 == 0 and self.rot % 8 == 0 and self.dim % 8 == 0)
-        self.up_k_t = self.up_v_rows = None
+        self.up_kv = self.up_k_t = self.up_v_rows = None
         if self.head_major:
+            # every head's key matrix, then every head's value matrix, as stored: what expands latents into keys and values
+            self.up_kv = torch.cat([self.up_k, tensors[f"{prefix}.uv.weight"].to(device=device, dtype=dtype)]).contiguous()
+            self.up_k = self.up_kv[:self.heads * self.dim]
             self.up_k_t = self.up_k.view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
-            self.up_v_rows = tensors[f"{prefix}.uv.weight"].to(device=device, dtype=dtype).view(
-                self.heads, self.vdim, self.rank).contiguous()
+            self.up_v_rows = self.up_kv[self.heads * self.dim:].view(self.heads, self.vdim, self.rank)
+        # what the form that expands keys and values takes (csrc/kernels/latent_heads.cuh)
+        self.expands = (self.head_major and self.dim == 128 and self.rot == 64 and self.vdim == 128 and self.scale > 0 and
+                        all(off < 0 or off % 4 == 0 for off in (self.q_off, self.g_off)) and self.proj.out_features % 4 == 0)
         self.latent_norm = None
         if self.own_cache:
             self.latent_norm = tensors[f"{prefix}.dkv.norm.weight"].to(device=device, dtype=torch.float32).contiguous()
@@ -129,6 +143,26 @@ class LatentAttention(Mixer):
         up_q = self.up_q.kernel_families() if self.up_q is not None else ()
         return tuple(dict.fromkeys(("latent",) + grouped + self.proj.kernel_families() + up_q + self.out.kernel_families()))
 
+    def expanded_rows(self, ctx) -> int:
+        """Rows the step's keys take where every head's keys and values are expanded for it, or 0 where the heads attend to the
+        latents instead.  Expanding costs a head 512 rank operations per key and 640 per (query, key) pair, the latents 4 rank +
+        128 per pair."""
+        if not self.expands or ctx.all_single or ctx.dtype != torch.bfloat16 or ctx.num_tokens < EXPANDED_FROM:
+            return 0
+        reach = self.window if self.window else 1 << 30
+        block = ops.LATENT_HEADS_ROWS
+        if ctx.host_counts:
+            rows, pairs = 0, 0.0
+            for count, first in zip(ctx.host_counts, ctx.host_pos0):
+                kept = min(first, reach - 1)
+                rows += -(-(kept + count) // block) * block
+                pairs += count * min(kept + 0.5 * count, reach)
+        else:   # a captured step: any request may have the longest history, and the tokens may all be one request's own
+            longest = min(max(int(ctx.max_kv_len), 1), reach - 1 + ctx.num_tokens)
+            rows = ctx.num_entries * (-(-longest // block) * block)
+            pairs = 0.5 * ctx.num_tokens * min(ctx.num_tokens / ctx.num_entries, reach)
+        return rows if rows <= EXPANDED_ROWS and pairs >= EXPANDED_SHARE * rows else 0
+
     def prepare(self, max_positions: int) -> None:
         self.position.prepare(max_positions)
 
@@ -143,6 +177,8 @@ class LatentAttention(Mixer):
         # (the splits of a step of few tokens: at most some 600 blocks of 16 rows more than the step's own)
         padded = tokens + 127
         head_major = heads * padded * (params["head_dim"] * 2 + rank * 6 + params["value_dim"] * 4) + tokens * heads * r * 4 + 4096
+        if params["head_dim"] == 128 and r == 64 and params["value_dim"] == 128:
+            head_major += EXPANDED_ROWS * (heads * 256 + rank + r) * 2
         return (tokens * (width * 4 + heads * (2 * rank + r) * 4 + heads * params["value_dim"] * element_bytes)
                 + 16 * (rank + 2) * 4 * 1300 + head_major)
 
@@ -152,10 +188,14 @@ class LatentAttention(Mixer):
         count, ws = ctx.num_tokens, ctx.workspace
         proj = ws.get("latent.proj", (count, self.proj.out_features), torch.float32)
         self.proj(ctx, h, epilogue=ops.EPI_STORE, out=proj)
-        qa = ws.get("latent.qa", (count, self.heads, self.rank + self.rot), torch.float32)
-        mixed_latent = ws.get("latent.mixed", (count, self.heads, self.rank), torch.float32)
         mixed = ws.get("latent.out", (count, self.heads * self.vdim), ctx.dtype)
         cos, sin = self.position.tables()
+        expanded = self.expanded_rows(ctx)
+        if expanded:
+            self._attend_expanded(ctx, cache, proj, mixed, expanded)
+            return self._leave(ctx, mixed, residual)
+        qa = ws.get("latent.qa", (count, self.heads, self.rank + self.rot), torch.float32)
+        mixed_latent = ws.get("latent.mixed", (count, self.heads, self.rank), torch.float32)
         max_keys = max(int(ctx.max_kv_len), 1)
         single = bool(ctx.all_single)
         floats = ops.latent_part_floats(count, self.heads, self.rank, self.rot, max_keys, ops.sm_count(h.device), self.window,
@@ -175,14 +215,7 @@ class LatentAttention(Mixer):
             }
         q, q_off, kv_off = None, self.q_off, self.kv_off
         if self.q_rank:
-            # the norm of the query latent shares a kernel with the cache write; its product follows
-            cq = ws.get("latent.cq", (count, self.q_rank), ctx.dtype)
-            ops.latent_store(proj, kv_off=kv_off, norm_weight=self.latent_norm, eps=self.norm_eps, positions=ctx.positions,
-                             token_entry=ctx.token_entry, block_table=ctx.block_tables[cache.group], cos=cos, sin=sin,
-                             k_pool=cache.k, v_pool=cache.v, rot_dim=self.rot, pairing=self.position.style,
-                             cq_off=self.q_off, cq_norm_weight=self.q_norm, cq=cq)
-            q = ws.get("latent.q", (count, self.up_q.out_features), torch.float32)
-            self.up_q(ctx, cq, epilogue=ops.EPI_STORE, out=q)
+            q = self._store(ctx, cache, proj)
             q_off, kv_off = 0, -1
         ops.latent_attention(proj, q_off=q_off, g_off=self.g_off, kv_off=kv_off, up_k=self.up_k, up_v=self.up_v,
                              norm_weight=self.latent_norm, eps=self.norm_eps, positions=ctx.positions,
@@ -191,6 +224,39 @@ class LatentAttention(Mixer):
                              head_dim=self.dim, rot_dim=self.rot, value_dim=self.vdim, scale=self.scale, max_keys=max_keys,
                              part=part, head_major=head_major, window=self.window, pairing=self.position.style,
                              sink=self.sink, q=q, single=single)
+        return self._leave(ctx, mixed, residual)
+
+    def _store(self, ctx, cache, proj):
+        """The step's latents into their pages and, with a query latent, the queries [tokens, heads * (head_dim + rot_dim)]."""
+        ws, cq = ctx.workspace, None
+        cos, sin = self.position.tables()
+        if self.q_rank:   # the norm of the query latent shares a kernel with the cache write; its product follows
+            cq = ws.get("latent.cq", (ctx.num_tokens, self.q_rank), ctx.dtype)
+        if self.own_cache or self.q_rank:
+            ops.latent_store(proj, kv_off=self.kv_off, norm_weight=self.latent_norm, eps=self.norm_eps, positions=ctx.positions,
+                             token_entry=ctx.token_entry, block_table=ctx.block_tables[cache.group], cos=cos, sin=sin,
+                             k_pool=cache.k, v_pool=cache.v, rot_dim=self.rot, pairing=self.position.style,
+                             cq_off=self.q_off if self.q_rank else -1, cq_norm_weight=self.q_norm, cq=cq)
+        if not self.q_rank:
+            return None
+        q = ws.get("latent.q", (ctx.num_tokens, self.up_q.out_features), torch.float32)
+        self.up_q(ctx, cq, epilogue=ops.EPI_STORE, out=q)
+        return q
+
+    def _attend_expanded(self, ctx, cache, proj, mixed, rows):
+        ws = ctx.workspace
+        cos, sin = self.position.tables()
+        q = self._store(ctx, cache, proj)
+        ops.latent_heads(proj if q is None else q, q_off=self.q_off if q is None else 0, gate=proj if self.gated else None,
+                         gate_off=self.g_off, up_kv=self.up_kv, entry_starts=ctx.entry_starts, entry_pos0=ctx.entry_pos0,
+                         block_table=ctx.block_tables[cache.group], cos=cos, sin=sin, k_pool=cache.k, v_pool=cache.v,
+                         rows=ws.get("latent.rows_kept", (rows, self.rank), torch.bfloat16),
+                         rot_rows=ws.get("latent.rows_rotated", (rows, self.rot), torch.bfloat16),
+                         expanded=ws.get("latent.expanded", (rows, 2 * self.heads * self.dim), torch.bfloat16),
+                         out=mixed, heads=self.heads, scale=self.scale, window=self.window, pairing=self.position.style, sink=self.sink)
+
+    def _leave(self, ctx, mixed, residual):
+        count, ws = ctx.num_tokens, ctx.workspace
         if residual is None:
             rows = ws.get("latent.rows", (count, self.hidden), torch.float32)
             self.out(ctx, mixed, epilogue=ops.EPI_STORE, out=rows)
