@@ -169,30 +169,39 @@ VIPERA_API int vipera_argmax(const float* logits, int rows, int vocab, int* toke
 //
 // A cluster of eight blocks takes a row.  Block b keeps the logits whose index modulo 1024 is in [128 b, 128 b + 128)
 // in shared memory (one trip to memory for the whole draw), so that each of 1024 chains of the softmax sum lies in one
-// block.  Then a histogram over 2,048 equal steps below the best value (few ids meet in a bin, unlike the leading
-// bits of the values) tells the first block how far down it has to go: to the bound-th largest, or to where the
-// weights' sum is past top-p with a margin.  If what lies above is at most 4,096 ids, it goes to the first block,
-// which sorts it and draws; the others leave.  Otherwise the bound-th largest (value, lowest id first) is found
-// digit by digit.  The weights' sum that top-p cuts and the mass are added in order, best first, by one thread from
-// weights in shared memory.
-// What bounds it: the chain of these steps, some 50 us a row, 33 rows at once.  64 rows of 151,936 (a quarter each
-// top-k 50, top-p alone, min-p, greedy): 104 us; with one block a row and a pass over memory per step 440 us.
+// block.  Four threads of a chain compute weights ahead and add them in turn.  Then a histogram over 2,048 equal steps
+// below the best value (few ids meet in a bin, unlike the leading bits of the values; the upper bins first, which most
+// draws do not look beyond) tells the first block how far down it has to go: to the bound-th largest, or to where the
+// weights' sum is past top-p with a margin.  If what lies above is at most 4,096 ids, it goes to the first block, which
+// puts it in order bin by bin, a bin's few by counting, and draws; the others leave.  Otherwise the bound-th largest
+// (value, lowest id first) is found digit by digit, and sorted.  The weights' sum that top-p cuts and the mass are added
+// in order, best first, by one thread from weights in shared memory, and what the floor leaves is read off on the way.
+// What bounds it: instructions, two blocks of 512 threads an SM (clocks of a row with top-p, of 57 K: load 3, best 6,
+// weights 8, bins 13, gathering and order 8, sum of 1,219 weights 10, draw 3), and 64 rows being two waves.  64 rows of
+// 151,936 (a quarter each top-k 50, top-p alone, min-p, greedy): 48 us, 8 of 128,256: 24 us (with one thread a chain, a
+// sort, two sums in order and every bin filled: 102 and 60; one block a row and a pass over memory per step: 440).
 // ---------------------------------------------------------------------------------------
 constexpr int kSampleBlocks = 8, kSampleThreads = 512;
 constexpr int kChains = 1024, kOwnChains = kChains / kSampleBlocks;
 constexpr int kBins = 2048;
+constexpr int kFirstBins = 576;         // the bins that are filled first: far more than most draws look down to
+constexpr int kAhead = 20;              // weights a thread has computed ahead of its turn in a chain
+constexpr int kMostInBin = 64;          // of the candidates; more are sorted without the bins
 constexpr int kMostKept = 200 * 1024;   // bytes of logits a block keeps; longer rows are read again for each step
 
 struct SampleShared {
   unsigned int histogram[kBins];
   int ids[kMaxCandidates];              // the first block's candidates, then its weights
-  Best best[kSampleThreads / 32];
   float least[kSampleThreads / 32];
-  Best row_best;
-  float row_min;
+  // what every block found of the row, and its chains' sums, told by each to all
+  Best block_best[kSampleBlocks];
+  float block_least[kSampleBlocks];
+  unsigned int block_finite[kSampleBlocks];
+  float chain_sums[kSampleBlocks * kOwnChains / 32];
+  int best_item;
   float scan_float[kSampleThreads / 32];
-  float chain_sums[kOwnChains / 32];
-  unsigned int finite_count, count, bin, seen;
+  float partial[kOwnChains];            // the chains' sums so far
+  unsigned int count, bin, seen, listed, place;
   unsigned int scan[kSampleThreads / 32];
   double scan_double[kSampleThreads / 32];
   int cut, chosen, last;
@@ -227,13 +236,15 @@ __device__ __forceinline__ unsigned long long ranked(float v, int id) {
 }
 
 template <bool KEPT>
-__global__ void __launch_bounds__(kSampleThreads)
+__global__ void __launch_bounds__(kSampleThreads, 2)
 sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
               const double* __restrict__ uniform, int* __restrict__ tokens, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char sample_raw[];
   SampleShared& s = *reinterpret_cast<SampleShared*>(sample_raw);
   float* kept = reinterpret_cast<float*>(sample_raw + (sizeof(SampleShared) + 15) / 16 * 16);   // [runs][kOwnChains]
+  // (nothing is stored into another block before that has begun: the wait is ahead of the first such store)
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int own = blockIdx.x, r = blockIdx.y;
   const float* row = logits + static_cast<size_t>(r) * vocab;
@@ -244,8 +255,22 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     const int id = id_of(item);
     return id < vocab ? row[id] : NAN;
   };
+  // every item of this thread: four neighbours at a time where the row is kept
+  auto each_value = [&](auto take) {
+    if (KEPT) {
+#pragma unroll 2
+      for (int i = tid * 4; i < items; i += kSampleThreads * 4) {
+        const float4 v = *reinterpret_cast<const float4*>(kept + i);
+        take(v.x, i), take(v.y, i + 1), take(v.z, i + 2), take(v.w, i + 3);
+      }
+    } else {
+#pragma unroll 4
+      for (int i = tid; i < items; i += kSampleThreads) take(value_of(i), i);
+    }
+  };
   for (int i = tid; i < kBins; i += kSampleThreads) s.histogram[i] = 0;
-  if (tid == 0) s.finite_count = s.count = 0;
+  if (tid < kOwnChains) s.partial[tid] = 0.0f;
+  if (tid == 0) s.count = s.listed = 0;
   pdl_wait();
   if (KEPT) {
     if ((vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
@@ -266,40 +291,61 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
 
   // the best finite logit of the row, ties to the lowest id, and how many are finite
   {
-    Best best{0.0f, -1};
+    float most = -INFINITY, least = INFINITY;
     unsigned int own_finite = 0;
-    float least = INFINITY;
-#pragma unroll 4
-    for (int i = tid; i < items; i += kSampleThreads) {
-      const float v = value_of(i);
-      if (finite(v)) {
-        best = better_of(best, Best{v, id_of(i)});
-        least = fminf(least, v);
-        ++own_finite;
+    auto one = [&](float v) {
+      if (!finite(v)) return;
+      most = fmaxf(most, v);
+      least = fminf(least, v);
+      ++own_finite;
+    };
+    if (KEPT) {
+      // (twice a number's bits are at least 0xff000000 where it is none)
+#pragma unroll 2
+      for (int i = tid * 4; i < items; i += kSampleThreads * 4) {
+        const float4 v = *reinterpret_cast<const float4*>(kept + i);
+        const unsigned int bits = max(max(__float_as_uint(v.x) << 1, __float_as_uint(v.y) << 1), max(__float_as_uint(v.z) << 1, __float_as_uint(v.w) << 1));
+        if (bits < 0xff000000u) {
+          most = fmaxf(most, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+          least = fminf(least, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
+          own_finite += 4;
+        } else {
+          one(v.x), one(v.y), one(v.z), one(v.w);
+        }
       }
+    } else {
+#pragma unroll 4
+      for (int i = tid; i < items; i += kSampleThreads) one(value_of(i));
     }
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-      Best other;
-      other.value = __shfl_xor_sync(0xffffffffu, best.value, offset);
-      other.id = __shfl_xor_sync(0xffffffffu, best.id, offset);
-      best = better_of(best, other);
-      own_finite += __shfl_xor_sync(0xffffffffu, own_finite, offset);
-      least = fminf(least, __shfl_xor_sync(0xffffffffu, least, offset));
-    }
+    const float warp_most = warp_max(most);
+    least = -warp_max(-least);
+    own_finite = __reduce_add_sync(0xffffffffu, own_finite);
     if (lane == 0) {
-      s.best[warp] = best;
+      s.scan_float[warp] = warp_most;
       s.least[warp] = least;
-      atomicAdd(&s.finite_count, own_finite);
+      s.scan[warp] = own_finite;
+    }
+    if (tid == 0) s.best_item = 0x7fffffff;
+    __syncthreads();
+    float block_most = -INFINITY;
+    for (int w = 0; w < kSampleThreads / 32; ++w) block_most = fmaxf(block_most, s.scan_float[w]);
+    if (most == block_most && block_most > -INFINITY) {   // who has it looks for where it is first
+      int where = 0x7fffffff;
+      each_value([&](float v, int i) {
+        if (v == block_most) where = min(where, i);
+      });
+      atomicMin(&s.best_item, where);
     }
     __syncthreads();
-    if (tid == 0) {
-      for (int w = 1; w < kSampleThreads / 32; ++w) {
-        best = better_of(best, s.best[w]);
-        least = fminf(least, s.least[w]);
-      }
-      s.row_best = best;
-      s.row_min = least;
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (tid < kSampleBlocks) {   // told to every block
+      least = INFINITY, own_finite = 0;
+      for (int w = 0; w < kSampleThreads / 32; ++w) least = fminf(least, s.least[w]), own_finite += s.scan[w];
+      const int id = block_most > -INFINITY ? id_of(s.best_item) : -1;
+      remote_store(&s.block_best[own].value, tid, __float_as_uint(block_most));
+      remote_store(&s.block_best[own].id, tid, static_cast<unsigned int>(id));
+      remote_store(&s.block_least[own], tid, __float_as_uint(least));
+      remote_store(&s.block_finite[own], tid, own_finite);
     }
   }
   cluster_sync();
@@ -308,9 +354,9 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   float least = INFINITY;
 #pragma unroll
   for (int b = 0; b < kSampleBlocks; ++b) {
-    least = fminf(least, __uint_as_float(remote_word(&s.row_min, b)));
-    best = better_of(best, Best{__uint_as_float(remote_word(&s.row_best.value, b)), static_cast<int>(remote_word(&s.row_best.id, b))});
-    finite_total += remote_word(&s.finite_count, b);
+    least = fminf(least, s.block_least[b]);
+    best = better_of(best, s.block_best[b]);
+    finite_total += s.block_finite[b];
   }
   const float temp = temperature[r];
   if (best.id < 0 || temp == 0.0f) {
@@ -318,26 +364,42 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
       tokens[r] = best.id < 0 ? 0 : best.id;
       status[r] = best.id < 0 ? SAMPLE_NO_FINITE : SAMPLE_OK;
     }
-    cluster_sync();   // the others have read this block's best
     return;
   }
   const float scale = 1.0f / temp;
   const float peak = best.value * scale;
 
-  // softmax mass over every finite logit: chain t adds the weights of ids t, t + 1024, ... in order
-  if (tid < kOwnChains) {
-    float partial = 0.0f;
-#pragma unroll 8
-    for (int run = 0; run < runs; ++run) {
-      const float v = value_of(run * kOwnChains + tid);
-      if (finite(v)) partial += expf(v * scale - peak);
+  // softmax mass over every finite logit: chain t adds the weights of ids t, t + 1024, ... in order.  Four threads a chain:
+  // all compute the weights of their next runs at once, then each in its turn adds them to what the ones before have.
+  {
+    constexpr int kTurns = kSampleThreads / kOwnChains;
+    const int chain = tid % kOwnChains, turn = tid / kOwnChains;
+    for (int first = 0; first < runs; first += kTurns * kAhead) {
+      float weight[kAhead];
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        const int run = first + turn * kAhead + j;
+        const float v = run < runs ? value_of(run * kOwnChains + chain) : NAN;
+        weight[j] = finite(v) ? expf(v * scale - peak) : 0.0f;
+      }
+      for (int now = 0; now < kTurns; ++now) {
+        if (turn == now) {
+          float partial = s.partial[chain];
+#pragma unroll
+          for (int j = 0; j < kAhead; ++j) partial += weight[j];
+          s.partial[chain] = partial;
+        }
+        __syncthreads();
+      }
     }
-    partial = warp_sum(partial);
-    if (lane == 0) s.chain_sums[warp] = partial;
+    if (tid < kOwnChains) {
+      const float partial = warp_sum(s.partial[tid]);
+      if (lane < kSampleBlocks) remote_store(&s.chain_sums[own * (kOwnChains / 32) + warp], lane, __float_as_uint(partial));
+    }
   }
   cluster_sync();
-  const int per_block = kOwnChains / 32;
-  const float total = warp_sum(__uint_as_float(remote_word(&s.chain_sums[lane % per_block], lane / per_block)));
+  static_assert(kSampleBlocks * kOwnChains / 32 == 32, "a lane has 32 chains' sum");
+  const float total = warp_sum(s.chain_sums[lane]);
   const int requested = top_k[r];
   const bool uncut = requested == 0;
   if (!(total > 0.0f) || !finite(total) || requested > kMaxCandidates) {
@@ -345,7 +407,6 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
       tokens[r] = 0;
       status[r] = !(total > 0.0f) || !finite(total) ? SAMPLE_NO_MASS : SAMPLE_NEEDS_HOST;
     }
-    cluster_sync();   // the others have read this block's sums
     return;
   }
   const unsigned int bound = min(min(uncut ? static_cast<unsigned int>(kMaxCandidates) : static_cast<unsigned int>(requested),
@@ -356,12 +417,22 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   const bool spread = step > 0.0f && finite(step) && finite(per_step);
   auto bin_of = [&](float v) { return min(static_cast<int>((best.value - v) * per_step), kBins - 1); };
   int last_bin = -1;   // ids up to this bin go to the first block; below 0: bins cannot tell
-  if (spread) {
-#pragma unroll 4
-    for (int i = tid; i < items; i += kSampleThreads) {
-      const float v = value_of(i);
-      if (finite(v)) atomicAdd(&s.histogram[bin_of(v)], 1u);
-    }
+  // The upper bins first; the others only where these do not reach far enough.
+  const float floor_value = best.value - (kFirstBins + 2) * step;   // (no value of the upper bins is below)
+  unsigned long long upper = 0;   // which of this thread's items, the first 64 of them, may lie in the upper bins
+  for (int pass = 0; spread && pass < 2; ++pass) {
+    const int from = pass ? kFirstBins : 0, to = pass ? kBins : kFirstBins;
+    int number_of = 0;
+    each_value([&](float v, int) {
+      if (pass || v >= floor_value) {
+        const int bin = finite(v) ? bin_of(v) : kBins;
+        if (bin >= from && bin < to) {
+          atomicAdd(&s.histogram[bin], 1u);
+          if (number_of < 64) upper |= 1ull << number_of;
+        }
+      }
+      ++number_of;
+    });
     if (tid == 0) s.bin = kBins;
     cluster_sync();
     if (own == 0) {
@@ -401,22 +472,36 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
       // 4,096 roundings of 2^-24 and the exponentials' own stay far within a thousandth
       const float enough = top_p[r] * total * 1.001f;
       int found = kBins;
-      unsigned int found_number = 0;
+      unsigned int found_number = 0, upto = number_before;
 #pragma unroll
       for (int j = 0; j < kPer; ++j) {
-        number_before += mine[j], weight_before += lower[j];
-        if (found == kBins && (number_before >= bound || weight_before >= enough)) found = tid * kPer + j, found_number = number_before;
+        upto += mine[j], weight_before += lower[j];
+        if (found == kBins && (upto >= bound || weight_before >= enough)) found = tid * kPer + j, found_number = upto;
       }
-      if (found < kBins) atomicMin(&s.bin, static_cast<unsigned int>(found));
+      if (found < to) atomicMin(&s.bin, static_cast<unsigned int>(found));
       __syncthreads();
       if (found < kBins && s.bin == static_cast<unsigned int>(found)) s.seen = found_number;
+      // where each bin's candidates begin
+      if (s.bin < kBins) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          s.histogram[tid * kPer + j] = number_before;
+          number_before += mine[j];
+        }
+      }
     }
     cluster_sync();
-    if (remote_word(&s.seen, 0) <= kMaxCandidates) last_bin = static_cast<int>(remote_word(&s.bin, 0));
+    const unsigned int reached = remote_word(&s.bin, 0);
+    if (reached >= kBins) {
+      cluster_sync();   // the answer is read before the next one is begun
+      continue;
+    }
+    if (remote_word(&s.seen, 0) <= kMaxCandidates) last_bin = static_cast<int>(reached);
     else {
       for (int i = tid; i < kBins; i += kSampleThreads) s.histogram[i] = 0;
       cluster_sync();   // the answer is read and every histogram is empty before anything is added to the first
     }
+    break;
   }
 
   // The bound-th largest of (value, id): digits of its number from the highest on.  After each digit, everything
@@ -480,26 +565,39 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   // what is good enough goes to the first block
   {
     auto taken = [&](float v, int i) { return finite(v) && (last_bin >= 0 ? bin_of(v) <= last_bin : (ranked(v, id_of(i)) >> shift) >= prefix); };
-    unsigned int mine = 0;
-#pragma unroll 4
-    for (int i = tid; i < items; i += kSampleThreads) mine += taken(value_of(i), i);
-    unsigned int upto = mine;
-#pragma unroll
-    for (int offset = 1; offset < 32; offset <<= 1) {
-      const unsigned int other = __shfl_up_sync(0xffffffffu, upto, offset);
-      if (lane >= offset) upto += other;
-    }
-    unsigned int place = 0;
-    if (lane == 31 && upto) place = remote_fetch_add(&s.count, 0, upto);
-    place = __shfl_sync(0xffffffffu, place, 31) + upto - mine;
-    if (mine) {
-      for (int i = tid; i < items; i += kSampleThreads) {
-        if (taken(value_of(i), i)) {
-          if (place < kMaxCandidates) remote_store(&s.ids[place], 0, static_cast<unsigned int>(id_of(i)));
-          ++place;
-        }
+    // The other blocks list theirs where their bins were (the first block has read them) and hand the list over at once.
+    auto give = [&](float v, int i) {
+      if (!taken(v, i)) return;
+      const unsigned int id = static_cast<unsigned int>(id_of(i));
+      if (own == 0) {
+        const unsigned int at = atomicAdd(&s.count, 1u);
+        if (at < kMaxCandidates) s.ids[at] = static_cast<int>(id);
+        return;
       }
+      const unsigned int place = atomicAdd(&s.listed, 1u);
+      if (place < kBins) {
+        s.histogram[place] = id;
+      } else {
+        const unsigned int at = remote_fetch_add(&s.count, 0, 1u);
+        if (at < kMaxCandidates) remote_store(&s.ids[at], 0, id);
+      }
+    };
+    if (KEPT && last_bin >= 0) {   // (what the bins hold was noted as it was counted)
+      for (; upper; upper &= upper - 1) {
+        const int number = __ffsll(static_cast<long long>(upper)) - 1, i = tid * 4 + number / 4 * (kSampleThreads * 4) + number % 4;
+        give(kept[i], i);
+      }
+      for (int i = tid * 4 + 16 * (kSampleThreads * 4); i < items; i += kSampleThreads * 4)
+        for (int j = 0; j < 4; ++j) give(kept[i + j], i + j);
+    } else {
+      each_value(give);
     }
+    __syncthreads();
+    const unsigned int listed = min(s.listed, static_cast<unsigned int>(kBins));
+    if (tid == 0 && listed) s.place = remote_fetch_add(&s.count, 0, listed);
+    __syncthreads();
+    for (unsigned int i = tid; i < listed; i += kSampleThreads)
+      if (s.place + i < kMaxCandidates) remote_store(&s.ids[s.place + i], 0, s.histogram[i]);
   }
   cluster_sync();
   if (own != 0) return;
@@ -507,20 +605,47 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   const unsigned int gathered = min(s.count, static_cast<unsigned int>(kMaxCandidates)), count = min(gathered, bound);
   // the candidates' numbers take the place of the logits (and, where those are not kept, room of their own)
   unsigned long long* candidates = reinterpret_cast<unsigned long long*>(kept);
-  unsigned int padded = 1;
-  while (padded < gathered) padded <<= 1;
-  for (unsigned int i = tid; i < padded; i += kSampleThreads) candidates[i] = i < gathered ? ranked(row[s.ids[i]], s.ids[i]) : 0ull;
-  __syncthreads();
-  // bitonic sort, descending
-  for (unsigned int size = 2; size <= padded; size <<= 1) {
-    for (unsigned int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (unsigned int pair = tid; pair < padded / 2; pair += kSampleThreads) {
-        const unsigned int i = 2 * pair - (pair & (stride - 1)), partner = i + stride;
-        const bool descending = (i & size) == 0;
-        const unsigned long long a = candidates[i], b = candidates[partner];
-        if (descending ? a < b : a > b) { candidates[i] = b; candidates[partner] = a; }
+  bool ordered = last_bin >= 0;
+  if (ordered) {
+    // Each goes among its bin's, and there behind those that are better.  (gathered is what the bins hold up to the last.)
+    unsigned long long* grouped = candidates + kMaxCandidates;
+    auto bin_at = [&](unsigned long long number) { return bin_of(key_value(static_cast<uint32_t>(number >> 32))); };
+    for (unsigned int i = tid; i < gathered; i += kSampleThreads) {
+      const unsigned long long number = ranked(row[s.ids[i]], s.ids[i]);
+      grouped[min(atomicAdd(&s.histogram[bin_at(number)], 1u), static_cast<unsigned int>(kMaxCandidates - 1))] = number;
+    }
+    __syncthreads();
+    bool crowded = false;
+    for (unsigned int i = tid; i < gathered; i += kSampleThreads) {
+      const unsigned long long number = grouped[i];
+      const int bin = bin_at(number);
+      const unsigned int begin = bin ? s.histogram[bin - 1] : 0, end = s.histogram[bin];
+      if (end - begin > kMostInBin) {
+        crowded = true;
+        continue;
       }
-      __syncthreads();
+      unsigned int place = begin;
+      for (unsigned int j = begin; j < end; ++j) place += grouped[j] > number;
+      candidates[place] = number;
+    }
+    ordered = !__syncthreads_or(crowded);
+  }
+  if (!ordered) {
+    unsigned int padded = 1;
+    while (padded < gathered) padded <<= 1;
+    for (unsigned int i = tid; i < padded; i += kSampleThreads) candidates[i] = i < gathered ? ranked(row[s.ids[i]], s.ids[i]) : 0ull;
+    __syncthreads();
+    // bitonic sort, descending
+    for (unsigned int size = 2; size <= padded; size <<= 1) {
+      for (unsigned int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (unsigned int pair = tid; pair < padded / 2; pair += kSampleThreads) {
+          const unsigned int i = 2 * pair - (pair & (stride - 1)), partner = i + stride;
+          const bool descending = (i & size) == 0;
+          const unsigned long long a = candidates[i], b = candidates[partner];
+          if (descending ? a < b : a > b) { candidates[i] = b; candidates[partner] = a; }
+        }
+        __syncthreads();
+      }
     }
   }
   auto id_at = [&](unsigned int i) { return static_cast<int>(0xffffffffu - static_cast<unsigned int>(candidates[i] & 0xffffffffull)); };
@@ -529,28 +654,50 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     weights[i] = i < count ? expf(key_value(static_cast<uint32_t>(candidates[i] >> 32)) * scale - peak) : 0.0f;
   __syncthreads();
   const float best_weight = weights[0], floor_weight = min_p[r] * best_weight;
+  // How many are not below the floor, and whether these are the first ones (weights fall, but for an exponential's last bit).
+  unsigned int above = 0, behind = 0;
+  for (unsigned int i0 = 0; i0 < count; i0 += kSampleThreads) {
+    const unsigned int i = i0 + tid;
+    const bool in = i < count && weights[i] >= floor_weight;
+    above += __syncthreads_count(in);
+    behind += __syncthreads_count(in && i > 0 && !(weights[i - 1] >= floor_weight));
+  }
   if (tid == 0) {
-    // the top-p cut: weights added in order, best first, eight reads at a time
+    // The top-p cut: weights added in order, best first, 32 at a time with nothing between the additions, then again within
+    // the 32 that the cut, or the floor, falls in.  What the floor leaves has the sum the weights had when it was met.
     const float target_mass = top_p[r] * total;
-    float cumulative = 0.0f;
+    float* upto = reinterpret_cast<float*>(s.histogram);   // before each 32
+    float cumulative = 0.0f, mass = 0.0f;
     int cut = -1;
-    for (unsigned int i = 0; i < count && cut < 0; i += 8) {
-      const float4 lo = *reinterpret_cast<const float4*>(weights + i), hi = *reinterpret_cast<const float4*>(weights + i + 4);
-      const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-      float upto[8];
+    unsigned int reached = 0;
+#pragma unroll 1
+    for (unsigned int i = 0; i < count; i += 32) {
+      float w[32];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) upto[j] = cumulative = cumulative + w[j];
+      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(w + j) = *reinterpret_cast<const float4*>(weights + i + j);
+      upto[i / 32] = cumulative;
 #pragma unroll
-      for (int j = 7; j >= 0; --j)
-        if (upto[j] >= target_mass && i + j < count) cut = static_cast<int>(i) + j + 1;
+      for (int j = 0; j < 32; ++j) cumulative += w[j];
+      reached = i;
+      if (cumulative >= target_mass) break;
     }
-    const unsigned int kept_end = cut >= 0 ? static_cast<unsigned int>(cut) : count;
-    float mass = 0.0f;
-    for (unsigned int i = 0; i < kept_end; i += 8) {
-      const float4 lo = *reinterpret_cast<const float4*>(weights + i), hi = *reinterpret_cast<const float4*>(weights + i + 4);
-      const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) mass += i + j < kept_end && w[j] >= floor_weight ? w[j] : 0.0f;
+    if (cumulative >= target_mass) {
+      float again = upto[reached / 32];
+      for (unsigned int i = reached; cut < 0; ++i) {
+        again += weights[i];
+        if (again >= target_mass) cut = static_cast<int>(i) + 1;
+      }
+    }
+    const unsigned int end = cut >= 0 ? min(above, static_cast<unsigned int>(cut)) : above;
+    if (end > 0) {
+      mass = upto[(end - 1) / 32];
+      for (unsigned int i = (end - 1) / 32 * 32; i < end; ++i) mass += weights[i];
+    }
+    if (behind) {
+      const unsigned int kept_end = cut >= 0 ? static_cast<unsigned int>(cut) : count;
+      mass = 0.0f;
+      for (unsigned int i = 0; i < kept_end; ++i)
+        if (weights[i] >= floor_weight) mass += weights[i];
     }
     s.cut = cut;
     s.mass = mass;
@@ -606,7 +753,7 @@ VIPERA_API int vipera_sample(const float* logits, int rows, int vocab, const flo
   if (rows <= 0) return VIPERA_OK;
   if (vocab <= 0) return VIPERA_BAD_SHAPE;
   if (!status || !tokens) return VIPERA_BAD_ARGUMENT;
-  constexpr int kHead = static_cast<int>((sizeof(SampleShared) + 15) / 16 * 16), kRanks = kMaxCandidates * 8;
+  constexpr int kHead = static_cast<int>((sizeof(SampleShared) + 15) / 16 * 16), kRanks = 2 * kMaxCandidates * 8;
   const long long logits_bytes = (static_cast<long long>(vocab) + kChains - 1) / kChains * kOwnChains * 4;
   const bool keep = logits_bytes <= kMostKept;
   const int bytes = kHead + static_cast<int>(keep && logits_bytes > kRanks ? logits_bytes : kRanks);
