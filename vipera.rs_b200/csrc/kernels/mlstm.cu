@@ -26,6 +26,7 @@
 // divides each head's output by its root mean square, scales it, and gates it with
 // sigmoid(g).
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 constexpr int kChunk = 32;      // tokens of a chunk
 constexpr int kThreads = 256;
@@ -50,6 +51,14 @@ struct MlstmParams {
   float* chunk_n;           // [jobs, heads, dim]       the same for n
   float* chunk_aux;         // [jobs, heads, 4]         the chunk's largest a_s, its sum of log forget gates, m at its start
   int max_jobs;
+  // the walk over chunks that are prepared ahead (see mlstm_walk.cuh); chunk_n and chunk_aux as above
+  void* walk_q;             // [jobs, heads, 64, dim + 8] bfloat16
+  void* walk_k;
+  void* walk_w;             // [jobs, heads, 64, 72] bfloat16
+  void* walk_v;             // [jobs, heads, vdim / 32, 2, 64, 40] bfloat16
+  float* walk_token;        // [jobs, heads, 4, 64]
+  float* walk_factors;      // [jobs, heads, 132]
+  int* status;              // receives a code where a bounded wait ran out
 };
 
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
@@ -1192,52 +1201,113 @@ mlstm_decode_kernel(const MlstmParams p) {
   }
 }
 
+#include "mlstm_walk.cuh"
+
+template <int D>
+static int launch_walk(const MlstmParams& p, cudaStream_t s) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t error = cudaFuncSetAttribute(mlstm_prepare_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(PrepareLayout<D>::kBytes));
+    if (error == cudaSuccess)
+      error = cudaFuncSetAttribute(mlstm_walk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, WalkLayout<D>::kBytes);
+    if (error != cudaSuccess) return static_cast<int>(error);
+    configured = true;
+  }
+  const WalkBuffers buffers{static_cast<__nv_bfloat16*>(p.walk_q), static_cast<__nv_bfloat16*>(p.walk_k), static_cast<__nv_bfloat16*>(p.walk_w),
+                            static_cast<__nv_bfloat16*>(p.walk_v), p.walk_token, p.walk_factors, p.status};
+  const dim3 jobs(p.heads, p.max_jobs);
+  int status = vipera_launch(mlstm_prepare_kernel<D>, jobs, kTcThreads, PrepareLayout<D>::kBytes, s, p, buffers);
+  if (status == 0) status = vipera_launch(mlstm_nm_kernel, dim3(p.heads, p.num_entries), 256, 0, s, p);
+  if (status == 0) status = vipera_launch(mlstm_factors_kernel<D>, dim3(p.heads, p.max_jobs, (p.vdim + kFactorCols - 1) / kFactorCols), 256, 0, s, p, buffers);
+  if (status == 0)
+    status = vipera_launch(mlstm_walk_kernel<D>, dim3(p.vdim / kWalkCols, p.heads, p.num_entries), kWalkThreads, WalkLayout<D>::kBytes, s, p, buffers);
+  return status;
+}
+
 // ---------------------------------------------------------------------------------------
 // the ending: head norm, scale, output gate; and the new n and m into the state
 // ---------------------------------------------------------------------------------------
-// One block per (token, head).  out[t, h*dv + c] = o / rms(o) * weight[h*dv + c] * sigmoid(g[t, h*dv + c]).
-template <typename T>
-__global__ void __launch_bounds__(128)
-mlstm_finish_kernel(const MlstmParams p, const float* __restrict__ weight, float eps, T* __restrict__ out,
+// A warp per (token, head).  out[t, h*dv + c] = o / rms(o) * weight[h*dv + c] * sigmoid(g[t, h*dv + c]).  Values come four
+// at a time where rows start on 16 bytes (FOURS), and up to 512 of them stay in registers between the two passes.
+// What bounds it: memory.  2,048 tokens, 8 heads of 512: 24 us (a block per (token, head), a value at a time: 27).
+constexpr int kFinishWarps = 8;
+
+template <typename T, bool FOURS>
+__global__ void __launch_bounds__(kFinishWarps * 32)
+mlstm_finish_kernel(const MlstmParams p, int num_tokens, const float* __restrict__ weight, float eps, T* __restrict__ out,
                     const int* __restrict__ token_entry) {
-  __shared__ float scratch_sum[32];
   pdl_launch_dependents();
   pdl_wait();
-  const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const long long item = static_cast<long long>(blockIdx.x) * kFinishWarps + (threadIdx.x >> 5);
+  if (item >= static_cast<long long>(num_tokens) * p.heads) return;
+  const int t = static_cast<int>(item / p.heads), h = static_cast<int>(item % p.heads);
   const int dv = p.vdim, d = p.dim;
-  const float* o = p.o_raw + (static_cast<size_t>(t) * p.heads + h) * dv;
+  const float* o = p.o_raw + static_cast<size_t>(item) * dv;
   const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off + h * dv;
-  // up to four values a thread stay in registers between the two passes (value sizes up to 512)
-  float mine[4], gates[4];
+  const float* w = weight + h * dv;
+  T* dst = out + static_cast<size_t>(item) * dv;
+  constexpr int kWidth = FOURS ? 4 : 1, kKept = 16 / kWidth;   // values a thread takes at a time, and how often
+  float mine[kKept][kWidth], gates[kKept][kWidth];
+  auto read = [&](const float* from, int c, float (&to)[kWidth]) {
+    if constexpr (FOURS) {
+      const float4 v = *reinterpret_cast<const float4*>(from + c);
+      to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w;
+    } else {
+      to[0] = from[c];
+    }
+  };
   float squares = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int c = tid + 128 * i;
-    mine[i] = c < dv ? o[c] : 0.0f;
-    gates[i] = c < dv ? gate[c] : 0.0f;
-    squares = fmaf(mine[i], mine[i], squares);
-  }
-  for (int c = tid + 512; c < dv; c += 128) squares = fmaf(o[c], o[c], squares);
-  squares = block_sum(squares, scratch_sum);
-  const float inverse = rsqrtf(squares / static_cast<float>(dv) + eps);
-  const float* w = weight + h * dv;
-  T* dst = out + static_cast<size_t>(t) * p.heads * dv + h * dv;
+  for (int i = 0; i < kKept; ++i) {
+    const int c = (i * 32 + lane) * kWidth;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int c = tid + 128 * i;
-    if (c < dv) dst[c] = from_float<T>(mine[i] * inverse * w[c] * (1.0f / (1.0f + expf(-gates[i]))));
+    for (int j = 0; j < kWidth; ++j) mine[i][j] = gates[i][j] = 0.0f;
+    if (c < dv) {
+      read(o, c, mine[i]);
+      read(gate, c, gates[i]);
+    }
   }
-  for (int c = tid + 512; c < dv; c += 128)
-    dst[c] = from_float<T>(o[c] * inverse * w[c] * (1.0f / (1.0f + expf(-gate[c]))));
+#pragma unroll
+  for (int i = 0; i < kKept; ++i)
+#pragma unroll
+    for (int j = 0; j < kWidth; ++j) squares = fmaf(mine[i][j], mine[i][j], squares);
+  for (int c = 512 + lane; c < dv; c += 32) squares = fmaf(o[c], o[c], squares);
+  const float inverse = rsqrtf(warp_sum(squares) / static_cast<float>(dv) + eps);
+#pragma unroll
+  for (int i = 0; i < kKept; ++i) {
+    const int c = (i * 32 + lane) * kWidth;
+    if (c >= dv) continue;
+    float scale[kWidth];
+    read(w, c, scale);
+    T y[kWidth];
+#pragma unroll
+    for (int j = 0; j < kWidth; ++j) y[j] = from_float<T>(mine[i][j] * inverse * scale[j] * (1.0f / (1.0f + expf(-gates[i][j]))));
+    if constexpr (!FOURS) dst[c] = y[0];
+    else if constexpr (sizeof(T) == 2) *reinterpret_cast<uint2*>(dst + c) = *reinterpret_cast<const uint2*>(y);
+    else *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(y);
+  }
+  for (int c = 512 + lane; c < dv; c += 32) dst[c] = from_float<T>(o[c] * inverse * w[c] * (1.0f / (1.0f + expf(-gate[c]))));
   const int e = token_entry[t];
   if (t == p.entry_starts[e + 1] - 1) {
     float* state = p.state + static_cast<long long>(p.state_slots[e]) * p.state_stride;
     float* n_state = state + static_cast<size_t>(p.heads) * d * dv + static_cast<size_t>(h) * d;
     float* m_state = state + static_cast<size_t>(p.heads) * d * (dv + 1) + h;
     const float* scratch = p.nm_scratch + (static_cast<size_t>(e) * p.heads + h) * (d + 1);
-    for (int dd = tid; dd < d; dd += 128) n_state[dd] = scratch[dd];
-    if (tid == 0) m_state[0] = scratch[d];
+    for (int dd = lane; dd < d; dd += 32) n_state[dd] = scratch[dd];
+    if (lane == 0) m_state[0] = scratch[d];
   }
+}
+
+template <typename T>
+static int launch_finish(const MlstmParams& p, int num_tokens, const float* weight, float eps, T* out, const int* token_entry, cudaStream_t s) {
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.o_raw) | reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(out);
+  const bool fours = (bases & 15) == 0 && p.vdim % 4 == 0 && p.proj_width % 4 == 0 && p.g_off % 4 == 0;
+  const long long warps = static_cast<long long>(num_tokens) * p.heads;
+  const dim3 grid(static_cast<unsigned>((warps + kFinishWarps - 1) / kFinishWarps));
+  return fours ? vipera_launch(mlstm_finish_kernel<T, true>, grid, kFinishWarps * 32, 0, s, p, num_tokens, weight, eps, out, token_entry)
+               : vipera_launch(mlstm_finish_kernel<T, false>, grid, kFinishWarps * 32, 0, s, p, num_tokens, weight, eps, out, token_entry);
 }
 
 static size_t chunk_shared_bytes(int d, int tile) {
@@ -1288,6 +1358,12 @@ VIPERA_API int vipera_mlstm(const MlstmParams* params, int num_tokens, int singl
     if (shared > 48 * 1024)
       cudaFuncSetAttribute(mlstm_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));
     status = vipera_launch(mlstm_decode_kernel, grid, kThreads, shared, s, p);
+  } else if (tensor_cores && vipera_mlstm_tc_takes(p.dim) && p.walk_q) {
+    // a walk over prepared chunks (the caller gave the room for it)
+    if (!p.walk_k || !p.walk_w || !p.walk_v || !p.walk_token || !p.walk_factors || !p.status || !p.chunk_n || !p.chunk_aux || p.max_jobs <= 0 || p.max_jobs > 65535 || p.vdim % kWalkCols != 0)
+      return VIPERA_BAD_ARGUMENT;
+    if ((reinterpret_cast<uintptr_t>(p.proj) & 15) || p.proj_width % 4 || p.q_off % 4 || p.k_off % 4 || p.v_off % 4) return VIPERA_BAD_ARGUMENT;
+    status = p.dim == 64 ? launch_walk<64>(p, s) : p.dim == 128 ? launch_walk<128>(p, s) : launch_walk<256>(p, s);
   } else if (tensor_cores && vipera_mlstm_tc_takes(p.dim) && p.chunk_state && p.chunk_n && p.chunk_aux && p.max_jobs > 0 &&
              p.vdim % 4 == 0) {
     // all chunks at once (the caller gave the scratch for it: a long step)
@@ -1312,13 +1388,9 @@ VIPERA_API int vipera_mlstm(const MlstmParams* params, int num_tokens, int singl
     status = vipera_launch(mlstm_chunk_kernel, grid, kThreads, shared, s, p);
   }
   if (status != 0) return status;
-  dim3 grid(num_tokens, p.heads);
-  if (out_dtype == VIPERA_F32)
-    return vipera_launch(mlstm_finish_kernel<float>, grid, 128, 0, s, p, norm_weight, norm_eps, static_cast<float*>(out),
-                         token_entry);
+  if (out_dtype == VIPERA_F32) return launch_finish<float>(p, num_tokens, norm_weight, norm_eps, static_cast<float*>(out), token_entry, s);
   if (out_dtype == VIPERA_BF16)
-    return vipera_launch(mlstm_finish_kernel<__nv_bfloat16>, grid, 128, 0, s, p, norm_weight, norm_eps,
-                         static_cast<__nv_bfloat16*>(out), token_entry);
+    return launch_finish<__nv_bfloat16>(p, num_tokens, norm_weight, norm_eps, static_cast<__nv_bfloat16*>(out), token_entry, s);
   return VIPERA_BAD_DTYPE;
 }
 

@@ -1147,6 +1147,8 @@ class _MlstmParams(ctypes.Structure):
         ("entry_starts", _c_void), ("state_slots", _c_void), ("fresh", _c_void), ("state", _c_void),
         ("state_stride", ctypes.c_longlong), ("o_raw", _c_void), ("nm_scratch", _c_void),
         ("chunk_state", _c_void), ("chunk_n", _c_void), ("chunk_aux", _c_void), ("max_jobs", _c_int),
+        ("walk_q", _c_void), ("walk_k", _c_void), ("walk_w", _c_void), ("walk_v", _c_void), ("walk_token", _c_void),
+        ("walk_factors", _c_void), ("status", _c_void),
     ]
 
 
@@ -1167,6 +1169,20 @@ def mlstm_tc_takes(dim: int, vdim: int) -> bool:
     return dim in (64, 128, 256)
 
 
+def mlstm_walk_scratch(heads: int, dim: int, vdim: int):
+    """What the walk over prepared chunks needs per chunk of the step: name -> (values, type)."""
+    half, full = torch.bfloat16, torch.float32
+    return {"q": (heads * 64 * (dim + 8), half), "k": (heads * 64 * (dim + 8), half), "w": (heads * 64 * 72, half),
+            "v": (heads * (vdim // 32) * 2 * 64 * 40, half), "token": (heads * 256, full), "factors": (heads * 132, full),
+            "n": (heads * dim, full), "aux": (heads * 4, full)}
+
+
+def mlstm_walk_takes(proj: torch.Tensor, offsets, dim: int, vdim: int) -> bool:
+    """Whether the walk over prepared chunks takes these sizes and this product's rows."""
+    return (mlstm_tc_takes(dim, vdim) and vdim % 32 == 0 and proj.shape[1] % 4 == 0 and all(int(o) % 4 == 0 for o in offsets[:3]) and
+            proj.data_ptr() % 16 == 0)
+
+
 def mlstm_takes(dim: int, vdim: int) -> bool:
     fn = getattr(load_kernel_library("mlstm"), "vipera_mlstm_tile")
     fn.argtypes, fn.restype = [_c_int, _c_int], _c_int
@@ -1177,14 +1193,16 @@ def mlstm(proj: torch.Tensor, *, offsets, heads: int, dim: int, vdim: int, q_sca
           denom_eps: float, entry_starts: torch.Tensor, state_slots: torch.Tensor, fresh: torch.Tensor,
           token_entry: torch.Tensor, num_entries: int, single: bool, state: torch.Tensor, o_raw: torch.Tensor,
           nm_scratch: torch.Tensor, norm_weight: torch.Tensor, norm_eps: float, out: torch.Tensor,
-          chunk_scratch=None) -> None:
+          chunk_scratch=None, walk_scratch=None) -> None:
     """The mLSTM cell over a step.  ``proj`` is the float32 product [tokens, width] that holds q, k,
     v, the output gate and the two gates' pre-activations at ``offsets`` (q, k, v, g, i, f);
     ``state`` is [slots, mlstm_state_floats]; ``out`` [tokens, heads * vdim] receives the cell's
     output after the head norm (times ``norm_weight``) and the output gate.  ``single`` promises
     that every entry brings one token.  ``chunk_scratch`` (float32 tensors: states [jobs, heads * d
     * dv], n [jobs, heads * d], aux [jobs, heads * 4], with jobs >= tokens // MLSTM_CHUNK + entries)
-    lets a bfloat16 run compute all chunks of the step at once instead of walking each entry's."""
+    lets a bfloat16 run compute all chunks of the step at once instead of walking each entry's.
+    ``walk_scratch`` (mlstm_walk_scratch's tensors) lets it walk them with their products prepared ahead; it
+    takes rows that start on 16 bytes and value sizes that are multiples of 32 (mlstm_walk_takes)."""
     global _mlstm_checked
     fn = _function("mlstm", "vipera_mlstm",
                    [ctypes.POINTER(_MlstmParams), _c_int, _c_int, _c_int, _c_void, _c_float, _c_void, _c_int, _c_void,
@@ -1223,13 +1241,21 @@ def mlstm(proj: torch.Tensor, *, offsets, heads: int, dim: int, vdim: int, q_sca
             raise InvalidArgumentError("mlstm: the chunk scratch has the wrong row sizes")
         p.chunk_state, p.chunk_n = _gpu(states, "chunk states", torch.float32), _gpu(ns, "chunk n", torch.float32)
         p.chunk_aux, p.max_jobs = _gpu(aux, "chunk aux", torch.float32), tokens // MLSTM_CHUNK + num_entries
+    if walk_scratch is not None:
+        jobs, wanted = tokens // MLSTM_CHUNK + num_entries, mlstm_walk_scratch(heads, dim, vdim)
+        if any(walk_scratch[name].shape[0] < jobs or walk_scratch[name].shape[1] != size for name, (size, _) in wanted.items()) or \
+                not mlstm_walk_takes(proj, offsets, dim, vdim):
+            raise InvalidArgumentError("mlstm: the walk's scratch does not match the step, or its sizes are not taken")
+        (p.walk_q, p.walk_k, p.walk_w, p.walk_v, p.walk_token, p.walk_factors, p.chunk_n, p.chunk_aux) = (
+            _gpu(walk_scratch[name], "walk " + name, dtype) for name, (_, dtype) in wanted.items())
+        p.max_jobs, p.status = jobs, _tc_buffers(proj.device, 0)["status"].data_ptr()
     # a bfloat16 run's portions go through the tensor-core form where it takes the sizes
     # (VIPERA_MLSTM_TC=0 keeps them on the CUDA cores)
     tensor_cores = out.dtype == torch.bfloat16 and os.environ.get("VIPERA_MLSTM_TC", "1") != "0"
     _check(fn(ctypes.byref(p), tokens, 1 if single else 0, 1 if tensor_cores else 0,
               _gpu(norm_weight, "norm_weight", torch.float32),
               float(norm_eps), _gpu(out, "out"), dtype_code(out.dtype), _gpu(token_entry, "token_entry", torch.int32),
-              _stream()), "mlstm", kernels=4 if (chunk_scratch is not None and tensor_cores and not single) else 2)
+              _stream()), "mlstm", kernels=5 if (walk_scratch is not None and tensor_cores and not single) else 4 if (chunk_scratch is not None and tensor_cores and not single) else 2)
 
 
 def kernel_status_word(device) -> torch.Tensor:

@@ -108,7 +108,28 @@ class MLSTM(Mixer):
     def workspace_bytes(cls, params, tokens, element_bytes):
         heads, d, dv = params["num_heads"], params["head_dim"], params["value_dim"]
         width = 2 * heads * (d + dv) + 2 * heads
-        return tokens * (width * 4 + heads * dv * (4 + element_bytes)) + tokens * heads * (d + 1) * 4
+        walk = 0
+        if element_bytes == 2 and ops.mlstm_tc_takes(d, dv) and dv % 32 == 0:
+            chunk = sum(size * dtype.itemsize for size, dtype in ops.mlstm_walk_scratch(heads, d, dv).values())
+            walk = (tokens // ops.MLSTM_CHUNK + 8) * chunk
+        return tokens * (width * 4 + heads * dv * (4 + element_bytes)) + tokens * heads * (d + 1) * 4 + walk
+
+    def walks(self, ctx, proj) -> bool:
+        """Whether a step's portions walk chunks that were prepared ahead (csrc/kernels/mlstm_walk.cuh).  Such a walk takes 30 us
+        and 2.0 us per chunk of the longest request, or of all blocks where they are more than the multiprocessors; all chunks
+        at once (long steps) take 2.1 us per megabyte of states at the chunks' starts.  us of the mixer at once / walking: 8 heads
+        of 256 x 512, 2,048 tokens 511 / 332, 512 tokens 154 / 129; 4 heads, 512 tokens 73 / 77; 8 heads of 128 x 256, 2,048
+        tokens 158 / 168, three requests of 1,024, 901 and 77 152 / 134.  Short steps, against the walk without preparation: 4
+        heads of 256 x 512, 128 tokens 67 / 49; of 128 x 256 51 / 42; of 64 x 128, 65 tokens 39 / 38, 17 + 1 + 1 23 / 28."""
+        tokens, entries = ctx.num_tokens, ctx.num_entries
+        if not ops.mlstm_walk_takes(proj, self.offsets, self.dim, self.vdim) or tokens < 6 * entries:
+            return False
+        if tokens < self.AT_ONCE_FROM:
+            return self.dim >= 128 or tokens >= 128
+        chunks = -(-max(ctx.host_counts or [ctx.max_count]) // ops.MLSTM_CHUNK)
+        blocks = (tokens / ops.MLSTM_CHUNK + 0.5 * entries) * self.heads * (self.vdim // 32)
+        states = (tokens // ops.MLSTM_CHUNK + entries) * self.heads * self.dim * self.vdim * 4e-6
+        return 30.0 + 2.0 * max(chunks, blocks / 148) < 4.0 + 2.1 * states
 
     def forward(self, ctx, h, residual, cache, writes_cache):
         count = ctx.num_tokens
@@ -118,9 +139,12 @@ class MLSTM(Mixer):
         o_raw = ws.get("mlstm.cell", (count, self.heads * self.vdim), torch.float32)
         scratch = ws.get("mlstm.nm", (ctx.num_entries, self.heads * (self.dim + 1)), torch.float32)
         mixed = ws.get("mlstm.out", (count, self.heads * self.vdim), ctx.dtype)
-        chunk_scratch = None
+        chunk_scratch = walk_scratch = None
         jobs = count // ops.MLSTM_CHUNK + ctx.num_entries
-        if (ctx.dtype == torch.bfloat16 and not ctx.all_single and count >= self.AT_ONCE_FROM
+        if (ctx.dtype == torch.bfloat16 and not ctx.all_single and self.walks(ctx, proj)):
+            walk_scratch = {name: ws.get("mlstm.walk_" + name, (jobs, size), dtype)
+                            for name, (size, dtype) in ops.mlstm_walk_scratch(self.heads, self.dim, self.vdim).items()}
+        elif (ctx.dtype == torch.bfloat16 and not ctx.all_single and count >= self.AT_ONCE_FROM
                 and ops.mlstm_tc_takes(self.dim, self.vdim) and self.vdim % 4 == 0
                 and jobs * self.heads * self.dim * self.vdim * 4 <= self.AT_ONCE_MOST_BYTES):
             # a long step: all its chunks at once (a block per chunk) instead of each entry's one after another
@@ -132,7 +156,7 @@ class MLSTM(Mixer):
                   entry_starts=ctx.entry_starts, state_slots=ctx.state_slots, fresh=ctx.fresh,
                   token_entry=ctx.token_entry, num_entries=ctx.num_entries, single=ctx.all_single,
                   state=cache.data, o_raw=o_raw, nm_scratch=scratch, norm_weight=self.norm_weight,
-                  norm_eps=self.norm_eps, out=mixed, chunk_scratch=chunk_scratch)
+                  norm_eps=self.norm_eps, out=mixed, chunk_scratch=chunk_scratch, walk_scratch=walk_scratch)
         self.out(ctx, mixed, epilogue=ops.EPI_RESIDUAL, resid=residual)
 
 
