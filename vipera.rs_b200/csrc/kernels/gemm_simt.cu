@@ -254,14 +254,51 @@ gemm_simt_kernel(const GemmArgs p) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Up to eight rows.  A group of `warps` warps (1, 2, 4 or 8, as many as it takes to give every
-// multiprocessor a dozen) shares eight rows of W, each warp every `warps`-th run of 128 values of K.  Two
-// runs are in flight while one is used, the first two before the kernel ahead has ended.  MR: rows of A
-// computed (1, 2, 4 or 8; the sums' order does not depend on it).
+// Up to eight rows.  `members` (1, 2, 4 or 8, as many as it takes to give every multiprocessor a dozen warps of eight rows of
+// W) share rows of W, each every `members`-th run of 128 values of K; a lane adds its places in one chain, the lanes' sums and
+// then the members' are added in their order.  Two runs are in flight while one is used, the first two of W before the kernel
+// ahead has ended.  MR: rows of A computed (1, 2, 4 or 8).  No sum's order depends on MR, nor on which of two forms runs:
+//   gemv_rows_kernel         the members are warps of a block, each with eight rows of W; a warp reads its runs of A itself.
+//   gemv_rows_shared_kernel  the members are blocks of a cluster, a block has eight rows of W for each of its eight warps, and
+//                            a run of A comes once for all of them.
+// Eight rows of A read by every warp are as many bytes from L2 as its rows of W, which bounds the first form at half of the
+// memory's rate; the cluster's two barriers cost the second 1.2 us.  8 rows, us in warps / shared: W 32,000 x 1,536 50.6 / 41.2
+// (4.8 TB/s), 17,920 x 1,536 27.1 / 22.2, 1,536 x 8,960 20.0 / 16.3, 896 x 4,864 11.2 / 9.5; 2,048 x 1,536 6.1 / 7.6.  4 rows:
+// 32,000 x 1,536 37.5 / 35.5, but 1,536 x 8,960 in eight parts 11.9 / 12.9.  (Pairs of chains with packed multiply-adds and four
+// rows a warp: 42.4 and 24.3 us where these take 41.2 and 22.2: what bounds it now is shared memory, which feeds W and A.)
 // ---------------------------------------------------------------------------------------
 constexpr int kFewRows = 8;     // rows of A, and rows of W a warp holds
 constexpr int kFewWarps = 8;    // of a block
 constexpr int kFewStages = 3;   // runs of a warp's ring
+constexpr int kFewRun = 128;    // values of K
+constexpr int kFewSplit = 8;    // most members
+constexpr long long kSharedFrom = 4000000;   // numbers of W
+
+// The lanes' sums of N values: at each step a lane keeps one half of the values it holds and hands over the other, until
+// it holds one or two; then every lane holds the same value's.  Returns the first value a lane ends with, and how many.
+template <int N>
+__device__ __forceinline__ int sum_lanes(float (&acc)[N], int lane, int& held) {
+  int first = 0;
+  held = N;
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1) {
+    const bool upper = (lane & offset) != 0;
+    if (held > 1) {
+      held >>= 1;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) {
+        if (i < held) {
+          const float keep = upper ? acc[i + held] : acc[i], give = upper ? acc[i] : acc[i + held];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, offset);
+        }
+      }
+      if (upper) first += held;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], offset);
+    }
+  }
+  return first;
+}
 
 template <int MR>
 __global__ void __launch_bounds__(kFewWarps * 32, 2)
@@ -329,26 +366,8 @@ gemv_rows_kernel(const GemmArgs p, int warps) {
     }
     stage = stage == kFewStages - 1 ? 0 : stage + 1;
   }
-  // The lanes' sums: at each step a lane keeps one half of the values it holds and hands over the other, until
-  // it holds one or two; then every lane holds the same value's.
-  int held = kFewRows * MR, first = 0;
-#pragma unroll
-  for (int offset = 16; offset > 0; offset >>= 1) {
-    const bool upper = (lane & offset) != 0;
-    if (held > 1) {
-      held >>= 1;
-#pragma unroll
-      for (int i = 0; i < kFewRows * MR / 2; ++i) {
-        if (i < held) {
-          const float keep = upper ? acc[i + held] : acc[i], give = upper ? acc[i] : acc[i + held];
-          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, offset);
-        }
-      }
-      if (upper) first += held;
-    } else {
-      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], offset);
-    }
-  }
+  int held;
+  const int first = sum_lanes<kFewRows * MR>(acc, lane, held);
 #pragma unroll
   for (int i = 0; i < kFewRows * MR / 2; ++i)
     if (i < held) parts[warp][first + i] = acc[i];
@@ -390,23 +409,166 @@ gemv_rows_kernel(const GemmArgs p, int warps) {
 }
 
 template <int MR>
-static int launch_few_rows(const GemmArgs& p, int warps, dim3 grid, dim3 block, cudaStream_t s) {
-  constexpr int kBytes = kFewWarps * kFewStages * kFewRows * 32 * 16;
+__global__ void __launch_bounds__(kFewWarps * 32, 2)
+gemv_rows_shared_kernel(const GemmArgs p, int split) {
+  constexpr int R = kFewRows;
+  __shared__ float parts[kFewWarps][R * MR];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = static_cast<int>(blockIdx.x) / split, member = static_cast<int>(blockIdx.x) % split;
+  const int group = tile * kFewWarps + warp;
+  const float* A = static_cast<const float*>(p.A);
+  const float* W = static_cast<const float*>(p.W);
+  const bool gated = p.epilogue == EPI_SWIGLU;
+  // the warp's rows: neighbours, or the gates and the ups of neighbouring features
+  auto row_of = [&](int r) {
+    if (!gated) return group * R + r;
+    const int feature = group * (R / 2) + r % (R / 2);
+    return feature / 16 * 32 + feature % 16 + (r >= R / 2 ? 16 : 0);
+  };
+  // A lane copies the 16 bytes of each row of W that it will use itself; the run of A is everyone's.
+  extern __shared__ __align__(16) float few_shared[];
+  float* ring = few_shared + (warp * kFewStages * R * 32 + lane) * 4;
+  float* shared_rows = few_shared + kFewWarps * kFewStages * R * kFewRun;   // [stage][MR][run]
+  const float* rows[R];
+  bool live[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int n = row_of(r);
+    live[r] = n < p.N;
+    rows[r] = W + (live[r] ? static_cast<size_t>(n) * p.K : 0);
+  }
+  const int step = split * kFewRun;
+  auto ask = [&](int stage, int k) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool valid = live[r] && k < p.K;
+      copy_16(shared_address(ring + (stage * R + r) * kFewRun), rows[r] + (valid ? k : 0), valid);
+    }
+  };
+  auto ask_a = [&](int stage, int k) {
+    if (warp < MR) {
+      const bool valid = warp < p.M && k < p.K;
+      copy_16(shared_address(shared_rows + (stage * MR + warp) * kFewRun + lane * 4), A + (valid ? static_cast<size_t>(warp) * p.K + k : 0), valid);
+    }
+  };
+  int k = member * kFewRun + lane * 4;
+  pdl_launch_dependents();
+#pragma unroll
+  for (int stage = 0; stage < kFewStages - 1; ++stage) ask(stage, k + stage * step);
+  pdl_wait();
+#pragma unroll
+  for (int stage = 0; stage < kFewStages - 1; ++stage) {
+    ask_a(stage, k + stage * step);
+    copy_commit();   // (with the first, all that was asked for before the wait)
+  }
+  float acc[R * MR];
+#pragma unroll
+  for (int i = 0; i < R * MR; ++i) acc[i] = 0.0f;
+  int stage = 0;
+  for (int k0 = member * kFewRun; k0 < p.K; k0 += step, k += step) {
+    copy_wait<kFewStages - 2>();
+    __syncthreads();   // this run of A is there, the one before is read out
+    const int last = stage == 0 ? kFewStages - 1 : stage - 1;
+    ask(last, k + (kFewStages - 1) * step);
+    ask_a(last, k + (kFewStages - 1) * step);
+    copy_commit();
+    float4 a[MR];
+#pragma unroll
+    for (int m = 0; m < MR; ++m) a[m] = *reinterpret_cast<const float4*>(shared_rows + (stage * MR + m) * kFewRun + lane * 4);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 w = *reinterpret_cast<const float4*>(ring + (stage * R + r) * kFewRun);
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        float& sum = acc[m * R + r];
+        sum = fmaf(a[m].x, w.x, sum);
+        sum = fmaf(a[m].y, w.y, sum);
+        sum = fmaf(a[m].z, w.z, sum);
+        sum = fmaf(a[m].w, w.w, sum);
+      }
+    }
+    stage = stage == kFewStages - 1 ? 0 : stage + 1;
+  }
+  int held;
+  const int first = sum_lanes<R * MR>(acc, lane, held);
+#pragma unroll
+  for (int i = 0; i < R * MR / 2; ++i)
+    if (i < held) parts[warp][first + i] = acc[i];
+  if (split > 1) cluster_sync();
+  else __syncthreads();
+  auto total = [&](int own, int i) {   // value i of warp `own`, the cluster's blocks in their order
+    if (split == 1) return parts[own][i];
+    const uint32_t at = shared_address(&parts[own][i]);
+    float each[kFewSplit];
+#pragma unroll
+    for (int o = 0; o < kFewSplit; ++o) each[o] = o < split ? remote_float(at, o) : 0.0f;
+    float sum = each[0];
+#pragma unroll
+    for (int o = 1; o < kFewSplit; ++o)
+      if (o < split) sum += each[o];
+    return sum;
+  };
+  auto store = [&](size_t at, float value) {
+    if (p.out_bf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value);
+    else static_cast<float*>(p.out)[at] = value;
+  };
+  // the tile's outputs, row of A by row of A, an even share a block
+  const int columns = kFewWarps * (gated ? R / 2 : R), items = columns * MR, share = (items + split - 1) / split;
+  for (int i = member * share + static_cast<int>(threadIdx.x); i < min(items, (member + 1) * share); i += kFewWarps * 32) {
+    const int m = i / columns, column = i % columns;
+    if (m >= p.M) break;
+    if (gated) {
+      const int own = column / (R / 2), r = column % (R / 2);
+      const int feature = tile * columns + column, n = feature / 16 * 32 + feature % 16;
+      if (n + 16 >= p.N) continue;
+      float gate = total(own, m * R + r), up = total(own, m * R + r + R / 2);
+      if (p.bias) {
+        gate += p.bias[n];
+        up += p.bias[n + 16];
+      }
+      store(static_cast<size_t>(m) * (p.N / 2) + feature, up * gate_activation(gate, p.activation));
+    } else {
+      const int n = tile * columns + column;
+      if (n >= p.N) continue;
+      float value = total(column / R, m * R + column % R);
+      if (p.bias) value += p.bias[n];
+      const size_t at = static_cast<size_t>(m) * p.N + n;
+      if (p.epilogue == EPI_STORE) store(at, value);
+      else p.resid[at] += value;
+    }
+  }
+  if (split > 1) cluster_sync();   // no block leaves while another reads its sums
+}
+
+template <int MR>
+static int launch_few_rows(const GemmArgs& p, int members, cudaStream_t s) {
+  constexpr int kBytes = kFewWarps * kFewStages * kFewRows * kFewRun * 4;
   static SharedMemoryOptIn opt_in;
   const int opted = opt_in.ask(reinterpret_cast<const void*>(gemv_rows_kernel<MR>), kBytes);
-  return opted ? opted : vipera_launch(gemv_rows_kernel<MR>, grid, block, kBytes, s, p, warps);
+  const long long groups = (p.N + kFewRows - 1) / kFewRows;
+  const dim3 grid(static_cast<unsigned>((groups * members + kFewWarps - 1) / kFewWarps));
+  return opted ? opted : vipera_launch(gemv_rows_kernel<MR>, grid, dim3(kFewWarps * 32), kBytes, s, p, members);
+}
+
+template <int MR>
+static int launch_few_shared(const GemmArgs& p, int members, cudaStream_t s) {
+  constexpr int kBytes = (kFewWarps * kFewRows + MR) * kFewStages * kFewRun * 4;
+  static SharedMemoryOptIn opt_in;
+  const int opted = opt_in.ask(reinterpret_cast<const void*>(gemv_rows_shared_kernel<MR>), kBytes);
+  const long long tiles = (static_cast<long long>(p.N) + kFewWarps * kFewRows - 1) / (kFewWarps * kFewRows);
+  return opted ? opted : launch_in_clusters(gemv_rows_shared_kernel<MR>, members, dim3(static_cast<unsigned>(tiles * members)), dim3(kFewWarps * 32), kBytes, s, p, members);
 }
 
 static int launch_few(const GemmArgs& p, cudaStream_t s) {
   constexpr int kWarpsWanted = 148 * 12;
   const long long groups = (p.N + kFewRows - 1) / kFewRows;
-  int warps = 1;
-  while (warps < kFewWarps && groups * warps < kWarpsWanted) warps *= 2;
-  const dim3 grid(static_cast<unsigned>((groups * warps + kFewWarps - 1) / kFewWarps)), block(kFewWarps * 32);
-  if (p.M == 1) return launch_few_rows<1>(p, warps, grid, block, s);
-  if (p.M == 2) return launch_few_rows<2>(p, warps, grid, block, s);
-  if (p.M <= 4) return launch_few_rows<4>(p, warps, grid, block, s);
-  return launch_few_rows<8>(p, warps, grid, block, s);
+  int members = 1;
+  while (members < kFewSplit && groups * members < kWarpsWanted) members *= 2;
+  if (p.M == 1) return launch_few_rows<1>(p, members, s);
+  if (p.M == 2) return launch_few_rows<2>(p, members, s);
+  const bool large = static_cast<long long>(p.N) * p.K >= kSharedFrom;
+  if (p.M <= 4) return members == 1 && large ? launch_few_shared<4>(p, members, s) : launch_few_rows<4>(p, members, s);
+  return large ? launch_few_shared<8>(p, members, s) : launch_few_rows<8>(p, members, s);
 }
 
 template <typename TA, typename TW, typename T, bool DIRECT, bool CLUSTER>
