@@ -314,8 +314,10 @@ attention_split_kernel(const AttentionParams p) {
 // sixteen lanes share a row, a warp eight rows, so that a row's weights pass through shared memory
 // within its warp.  Tokens of several requests in one tile are folded one request after another, the
 // others' rows masked.  Bound by the multiply-adds and the reads of shared memory that feed them: 64 x 64 tiles
-// read a key 64 times less often than a warp per row.  1,024 tokens of three requests (700, 1 and 323, histories
-// 0, 900, 40), 14 heads of 64 on 2, 32-bit: 101 us beside 21 us for the one alone (four warps of twice the rows: 133; a warp per (token, head): 1,146 us).
+// read a key 64 times less often than a warp per row.  The longest walk bounds a step of few tiles: blocks of a cluster then
+// share a tile's keys (tile_members).  1,024 tokens of three requests (700, 1 and 323, histories 0, 900, 40), 14 heads of 64 on 2,
+// 32-bit, with 21 us for the one alone: 95 us by two blocks, 128 by one (four warps of twice the rows: 154; a warp per (token,
+// head): 1,146 us).  (The next keys asked for ahead, with a place for the weights beside them: no faster.)
 // ---------------------------------------------------------------------------------------
 constexpr int kTileRows = 64, kTileThreads = 256, kOwn = kTileRows * 16 / kTileThreads;   // (sixteen lanes a row; kOwn rows a thread)
 
@@ -326,11 +328,14 @@ struct TileShared {
   float v[kTileKeys][DP];
   int place[kTileKeys];
   int seq[kTileRows], last[kTileRows], first[kTileRows], kept[kTileRows];
+  float top[kTileRows], sum[kTileRows];   // JOIN: a block's, for the others of its cluster (its outputs take the values' place)
 };
+constexpr int kMostMembers = 4;
 
-template <typename T, int DP, bool VEC>
+// JOIN: the `members` blocks of a cluster share a tile's keys, each every members-th 64 of them, and join their outputs.
+template <typename T, int DP, bool VEC, bool JOIN>
 __global__ void __launch_bounds__(kTileThreads)
-attention_tile_kernel(const AttentionParams p) {
+attention_tile_kernel(const AttentionParams p, int members) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
   TileShared<DP>& s = *reinterpret_cast<TileShared<DP>*>(tile_raw);
   constexpr int kWeightPitch = kTileKeys + 4;
@@ -338,7 +343,8 @@ attention_tile_kernel(const AttentionParams p) {
   float* weights = &s.k[0][0];
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.x, kv_head = h / (p.num_heads / p.num_kv_heads);
+  const int h = JOIN ? blockIdx.x / members : blockIdx.x, member = JOIN ? blockIdx.x % members : 0, stride = JOIN ? members * kTileKeys : kTileKeys;
+  const int kv_head = h / (p.num_heads / p.num_kv_heads);
   const int t0 = (gridDim.y - 1 - blockIdx.y) * kTileRows;   // the longest histories of a prompt first
   const int rows = min(kTileRows, p.num_tokens - t0);
   const int d = p.head_dim, dv = p.value_dim;
@@ -399,7 +405,7 @@ attention_tile_kernel(const AttentionParams p) {
     }
     const int* table = p.block_table + static_cast<size_t>(seq) * p.table_width;
     for (int run = 0; run < 2; ++run) {
-      const int run_first = run == 0 ? 0 : low, run_end = run == 0 ? most_kept : high + 1;
+      const int run_first = (run == 0 ? 0 : low) + member * kTileKeys, run_end = run == 0 ? most_kept : high + 1;
       auto look_up = [&](int base) {   // where the key of this thread lies in the tile from `base` on, -1: nowhere
         const int key = base + (tid & (kTileKeys - 1));
         if (key >= run_end) return -1;
@@ -407,7 +413,7 @@ attention_tile_kernel(const AttentionParams p) {
         return page >= 0 ? page * p.page_size + key % p.page_size : -1;
       };
       int ahead = run_first < run_end ? look_up(run_first) : -1;
-      for (int base = run_first; base < run_end; base += kTileKeys) {
+      for (int base = run_first; base < run_end; base += stride) {
         const int count = min(kTileKeys, run_end - base);
         __syncthreads();   // the tile before is read out
         if (tid < kTileKeys) s.place[tid] = ahead;
@@ -422,7 +428,7 @@ attention_tile_kernel(const AttentionParams p) {
         stage_keys<T, VEC, kTileThreads>(&s.v[0][0], DP, static_cast<const T*>(p.v_pool) + static_cast<size_t>(kv_head) * dv,
                            static_cast<size_t>(p.num_kv_heads) * dv, dv, s.place, kTileKeys);
         copy_commit();
-        if (base + kTileKeys < run_end) ahead = look_up(base + kTileKeys);
+        if (base + stride < run_end) ahead = look_up(base + stride);
         copy_wait<1>();
         __syncthreads();
         unsigned long long dot[kOwn][4];
@@ -531,20 +537,65 @@ attention_tile_kernel(const AttentionParams p) {
     }
     seg = seg_end;
   }
+  if constexpr (JOIN) {
+    __syncthreads();   // the values are read out
 #pragma unroll
-  for (int i = 0; i < kOwn; ++i) {
-    const int row = row0 + 2 * i;
-    if (row >= rows || s.last[row] == -2) continue;
-    const int t = t0 + row;
-    const float factor = ending_factor(p, h, row_max[i], row_sum[i]);
-    T* out_row = static_cast<T*>(p.out) + (static_cast<size_t>(t) * p.num_heads + h) * dv;
+    for (int i = 0; i < kOwn; ++i) {
+      const int row = row0 + 2 * i;
+      if (column0 == 0) s.top[row] = row_max[i], s.sum[row] = row_sum[i];
 #pragma unroll
-    for (int j = 0; j < kGroups; ++j)
+      for (int j = 0; j < kGroups; ++j) *reinterpret_cast<float4*>(&s.v[row][4 * column0 + 64 * j]) = make_float4(out[i][j][0], out[i][j][1], out[i][j][2], out[i][j][3]);
+    }
+    cluster_sync();
+    // an even share of the rows a block, sixteen lanes a row
+    const int share = kTileRows / members;
+    for (int row = member * share + (tid >> 4); row < min(rows, (member + 1) * share); row += kTileThreads / 16) {
+      if (s.last[row] == -2) continue;
+      const int t = t0 + row;
+      float weight[kMostMembers], sums[kMostMembers], most = -INFINITY, sum = 0.0f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int c = 4 * column0 + 64 * j + e;
-        if (c < dv) out_row[c] = from_float<T>(out[i][j][e] * factor * gate_factor(p, t, h, c));
+      for (int b = 0; b < kMostMembers; ++b) {
+        weight[b] = b < members ? remote_float(shared_address(&s.top[row]), b) : -INFINITY;
+        sums[b] = b < members ? remote_float(shared_address(&s.sum[row]), b) : 0.0f;
       }
+#pragma unroll
+      for (int b = 0; b < kMostMembers; ++b) most = fmaxf(most, weight[b]);
+#pragma unroll
+      for (int b = 0; b < kMostMembers; ++b) {
+        weight[b] = weight[b] == -INFINITY ? 0.0f : expf(weight[b] - most);
+        sum = fmaf(sums[b], weight[b], sum);
+      }
+      const float factor = ending_factor(p, h, most, sum);
+      T* out_row = static_cast<T*>(p.out) + (static_cast<size_t>(t) * p.num_heads + h) * dv;
+#pragma unroll
+      for (int e = 0; e < 4 * kGroups; ++e) {
+        const int c = column0 + 16 * e;
+        float part[kMostMembers], value = 0.0f;
+#pragma unroll
+        for (int b = 0; b < kMostMembers; ++b) part[b] = b < members ? remote_float(shared_address(&s.v[row][c]), b) : 0.0f;
+#pragma unroll
+        for (int b = 0; b < kMostMembers; ++b)
+          if (b < members) value = fmaf(part[b], weight[b], value);
+        if (c < dv) out_row[c] = from_float<T>(value * factor * gate_factor(p, t, h, c));
+      }
+    }
+    cluster_sync();   // no block leaves while another reads its part
+  } else {
+#pragma unroll
+    for (int i = 0; i < kOwn; ++i) {
+      const int row = row0 + 2 * i;
+      if (row >= rows || s.last[row] == -2) continue;
+      const int t = t0 + row;
+      const float factor = ending_factor(p, h, row_max[i], row_sum[i]);
+      T* out_row = static_cast<T*>(p.out) + (static_cast<size_t>(t) * p.num_heads + h) * dv;
+#pragma unroll
+      for (int j = 0; j < kGroups; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = 4 * column0 + 64 * j + e;
+          if (c < dv) out_row[c] = from_float<T>(out[i][j][e] * factor * gate_factor(p, t, h, c));
+        }
+    }
   }
 }
 
@@ -691,6 +742,35 @@ static int launch_split(const AttentionParams& p, int clusters, cudaStream_t s) 
                             dim3(kAttentionThreads), kBytes, s, p);
 }
 
+// Among how many blocks a tile's keys are cut: 1, 2 or 4, by the longest of what a block walks and what all of them cost a
+// multiprocessor, in microseconds: a tile of 64 keys `tile`, a block's start and ending `start`, joining 4.  The keys are those the
+// block table, a window or a chunk leaves room for; several requests see half of them on average (the longest history may be
+// a lone token's, whose launch is another), and below 128 tokens of several requests it may be a lone token's alone.  1 / 2 / 4
+// blocks: 14 heads of 64 on 2, 200 tokens 28 / 25 / 21 us, 800 106 / 75 / 85, 2,048 299 / 292 / 342, 800 under a window of 256 55 / 60 / 72,
+// 100 behind 1,000 119 / 68 / 52; 12 heads of 128 on 2, 1,024 tokens of three requests 206 / 138 / 146, 100 behind 3,000 556 / 285 /
+// 190; 4 heads of 256 on 1, 800 tokens 245 / 146 / 109; two tiles of keys: 65 tokens, 14 heads of 64 14.8 / 17.2.
+static int tile_members(const AttentionParams& p, int dp, int requests) {
+  long long most = static_cast<long long>(p.table_width) * p.page_size;
+  if (p.window > 0) most = std::min<long long>(most, static_cast<long long>(p.window) + kTileRows + p.keep_first);
+  if (p.chunk > 0) most = std::min<long long>(most, p.chunk);
+  const long long walked = (most + kTileKeys - 1) / kTileKeys;
+  if (walked < 3 || (requests > 1 && p.num_tokens < 2 * kTileRows)) return 1;
+  const double run = static_cast<double>(p.num_tokens) / std::max(requests, 1);
+  const double in_tile = requests > 1 ? std::min(kTileRows / run + 1.0, static_cast<double>(requests)) : 1.0;
+  const double seen = requests > 1 ? 0.5 * most : p.window > 0 || p.chunk > 0 ? most : most - 0.5 * std::min<double>(run, most);
+  const double tile = dp == 64 ? 6.2 : dp == 128 ? 11.8 : 18.5, start = dp == 64 ? 4.7 : dp == 128 ? 7.0 : 12.0;
+  const double blocks = static_cast<double>(p.num_heads) * ((p.num_tokens + kTileRows - 1) / kTileRows);
+  double best = 0.0;
+  int members = 1;
+  for (int m = 1; m <= kMostMembers; m *= 2) {
+    const double longest = start + tile * in_tile * ((walked + m - 1) / m);
+    const double all = blocks * (m * start + in_tile * seen / kTileKeys * tile) / 148;
+    const double cost = (m > 1 ? 4.0 : 0.0) + std::max(longest, all);
+    if (m == 1 || cost < best) best = cost, members = m;
+  }
+  return members;
+}
+
 // In a step of portions beside tokens that stand alone (other requests' decode tokens) those would walk their whole
 // histories in a tile's rows that they do not fill, behind the tile's other requests: they go to the split form, a launch
 // of their own (1,024 tokens, one of them alone behind 900 keys: 270 us in the tiles alone, 133 + 21 us).
@@ -706,12 +786,16 @@ static int launch_attention(const AttentionParams& asked, int requests, cudaStre
     const int status = launch_split<T, DP, VEC>(p, requests < 65535 ? requests : 65535, s);
     if (status) return status;
   }
-  static SharedMemoryOptIn opt_in;
+  static SharedMemoryOptIn opt_in, opt_in_join;
   constexpr int kBytes = static_cast<int>(sizeof(TileShared<DP>));
-  const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_tile_kernel<T, DP, VEC>), kBytes);
-  if (opted) return opted;
-  return vipera_launch(attention_tile_kernel<T, DP, VEC>, dim3(p.num_heads, (p.num_tokens + kTileRows - 1) / kTileRows),
-                       dim3(kTileThreads), kBytes, s, p);
+  const dim3 grid(p.num_heads, (p.num_tokens + kTileRows - 1) / kTileRows);
+  const int members = tile_members(p, DP, requests);
+  if (members == 1) {
+    const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_tile_kernel<T, DP, VEC, false>), kBytes);
+    return opted ? opted : vipera_launch(attention_tile_kernel<T, DP, VEC, false>, grid, dim3(kTileThreads), kBytes, s, p, 1);
+  }
+  const int opted = opt_in_join.ask(reinterpret_cast<const void*>(attention_tile_kernel<T, DP, VEC, true>), kBytes);
+  return opted ? opted : launch_in_clusters(attention_tile_kernel<T, DP, VEC, true>, members, dim3(grid.x * members, grid.y), dim3(kTileThreads), kBytes, s, p, members);
 }
 
 template <typename T>
