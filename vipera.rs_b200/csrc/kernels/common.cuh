@@ -56,6 +56,24 @@ __device__ __forceinline__ float gate_activation(float z, int activation) {
   return z / (1.0f + expf(-z));
 }
 
+// 1 / (1 + e^-z) for a result that is stored as T: where that is bfloat16 (2^-9) by the approximate exponential and quotient,
+// some 2^-21 off, in a third of the instructions.
+template <typename T>
+__device__ __forceinline__ float sigmoid_for(float z) {
+  if constexpr (sizeof(T) == 2) return __fdividef(1.0f, 1.0f + __expf(-z));
+  return 1.0f / (1.0f + expf(-z));
+}
+// Four neighbours of a row of T.
+template <typename T>
+__device__ __forceinline__ void store_four_as(T* to, float a, float b, float c, float d) {
+  if constexpr (sizeof(T) == 2) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+    *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  } else {
+    *reinterpret_cast<float4*>(to) = make_float4(a, b, c, d);
+  }
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int offset = 16; offset > 0; offset >>= 1) v += __shfl_xor_sync(0xffffffffu, v, offset);
