@@ -159,7 +159,7 @@ latent_gather_kernel(const Params p) {
 
 struct Shared {
   // per group and, but for the output's, per buffer
-  uint64_t query, key_full[2][2], key_empty[2][2], value_landed[2][2], value_zeroed[2][2], value_empty[2][2], score[2][2], weight[2][2], done[2];
+  uint64_t query, key_full[2][2], key_empty[2][2], value_landed[2][2], value_zeroed[2][2], value_empty[2][2], score[2][2], weight[2][2], done[2], finished[2];
   uint32_t tmem_base;
   int abort_flag;
   Run run;
@@ -255,6 +255,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         bar_init(&s.weight[g][b], kGroupThreads);
       }
       bar_init(&s.done[g], 1);
+      bar_init(&s.finished[g], 1);
     }
     s.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -405,7 +406,8 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         gate[j][0] = z[0], gate[j][1] = z[1];
       }
     }
-    if (group_tiles > 0) bar_wait<WAIT_EXPIRED>(&s.done[group], (group_tiles - 1) & 1, abort_flag, p.status);
+    // (`done` would not do: the last scores tell only that the third product from the end is done, whose parity is the last's)
+    if (group_tiles > 0) bar_wait<WAIT_EXPIRED>(&s.finished[group], 0, abort_flag, p.status);
     fence_after();
     s.told[group][row] = make_float2(row_max, row_sum);
     fence_before();
@@ -499,6 +501,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         for (int k = 0; k < kKeys / 16; ++k)
           mma_tensor(o_tmem, s_tmem + buffer * kKeys + 8 * k, descriptor(v_addr + buffer * kValueBytes + k * 2048, true), kOutputs, (i > 0 || k > 0) ? 1u : 0u);
         commit(&s.done[g]);
+        if (i + 1 == group_tiles) commit(&s.finished[g]);
         commit(&s.value_empty[g][buffer]);
         if (i + 2 < group_tiles) {
           bar_wait<WAIT_EXPIRED>(&s.done[g], i & 1, abort_flag, p.status);   // (it reads the weights from the scores' columns)
