@@ -15,10 +15,12 @@
 // accumulator, two buffers for keys and two for values, an issuing warp and two loading warps of its own: a group's next
 // scores are computed under its softmax, the two groups drift against one another, and the ending joins them.  208 KB of
 // shared memory: Q 48, keys 4 x 24, values 4 x 16 (weights that stay in tensor memory are what makes room for these).
-// What bounds it: a block's start (set-up, queries: some 10 K clocks) and its softmax, 2.4 K clocks per 64 keys and group, of
+// The queries and, for the ending, the rows of the gate come by TMA as they are, in 32 bits, into space that the keys do not need
+// yet or any more.  (The gate read from memory by the ending's threads held it up by some 9,000 clocks: 327 us below.)
+// What bounds it: a block's start (set-up, queries: some 8 K clocks) and its softmax, 2.4 K clocks per 64 keys and group, of
 // which the exponentials are 512 and scaling the output to a new maximum some 400; tensor cores are busy a third of the time.
-// Measured: 2,048 tokens, 12 heads, rank 512, window 1,024: the mixer 287 -> 109 us; 1,748 tokens of four requests behind up
-// to 3,000, 32 heads, a gate: 663 -> 325 us (over the latents, latent_tc.cuh, before).
+// Measured: 2,048 tokens, 12 heads, rank 512, window 1,024: the mixer 287 -> 108 us; 1,748 tokens of four requests behind up
+// to 3,000, 32 heads, a gate: 663 -> 306 us (over the latents, latent_tc.cuh, before).
 // Every wait is bounded; one that runs out leaves a code in the status word.
 #pragma once
 
@@ -43,6 +45,7 @@ constexpr int kRunRows = 128;                        // a request's run of rows 
 constexpr int kQueryHalf = kQ * 128, kHalf = kKeys * 128;   // bytes of [rows][64 values]
 constexpr int kQueryBytes = 3 * kQueryHalf, kKeyBytes = 3 * kHalf, kValueBytes = 2 * kHalf;
 constexpr int kStagedPitch = kValues + 4;            // floats between rows of the ending's tile
+constexpr int kRawPitch = kDim + kRot;               // and of the queries as they come
 constexpr int kGroupThreads = 128, kSoftmaxThreads = 2 * kGroupThreads;
 constexpr int kIssuer = 8, kLoader = 12, kThreads = 16 * 32;   // (two warps idle: register shares go by four warps)
 constexpr int kSoftmaxRegisters = 184, kOtherRegisters = 72;
@@ -159,16 +162,17 @@ latent_gather_kernel(const Params p) {
 
 struct Shared {
   // per group and, but for the output's, per buffer
-  uint64_t query, key_full[2][2], key_empty[2][2], value_landed[2][2], value_zeroed[2][2], value_empty[2][2], score[2][2], weight[2][2], done[2], finished[2];
+  uint64_t raw, query, scored, gate, key_full[2][2], key_empty[2][2], value_landed[2][2], value_zeroed[2][2], value_empty[2][2], score[2][2], weight[2][2], done[2], finished[2];
   uint32_t tmem_base;
   int abort_flag;
   Run run;
   int tile;
   float2 told[2][kQ];   // a group's maxima and sums, for the other
 };
+constexpr int kGateBytes = kQ * kValues * 4;
 constexpr int kSharedBytes = kQueryBytes + 4 * kKeyBytes + 4 * kValueBytes + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(kSharedBytes <= 227 * 1024, "a block's shared memory");
-static_assert(kQ * kStagedPitch * 4 <= 4 * kKeyBytes, "the ending's tile lies where the keys were");
+static_assert(kGateBytes + kQ * kStagedPitch * 4 <= kQueryBytes + 4 * kKeyBytes && kQ * kRawPitch * 4 <= 4 * kKeyBytes, "what lies where queries and keys did, or will");
 
 __device__ __forceinline__ void expect_bytes(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(bar)), "r"(bytes) : "memory");
@@ -214,7 +218,8 @@ __device__ __forceinline__ uint32_t weights_of(uint32_t a, uint32_t b, float sca
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __grid_constant__ CUtensorMap rot_map, const Params p) {
+latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __grid_constant__ CUtensorMap rot_map,
+                    const __grid_constant__ CUtensorMap query_map, const __grid_constant__ CUtensorMap gate_map, const Params p) {
   extern __shared__ uint8_t latent_heads_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(latent_heads_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* queries = base;                          // three halves
@@ -243,7 +248,10 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
   const int key_base = run.first_key + first_tile * kKeys;                    // position of the first tile's first key
 
   if (tid == 0) {
+    bar_init(&s.raw, 1);
     bar_init(&s.query, kSoftmaxThreads);
+    bar_init(&s.scored, 2);
+    bar_init(&s.gate, 1);
     for (int g = 0; g < 2; ++g) {
       for (int b = 0; b < 2; ++b) {
         bar_init(&s.key_full[g][b], 1);
@@ -274,68 +282,62 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
   if (warp < kIssuer) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegisters));
     // ---------------- queries, then softmax and ending: thread = query, group = every other tile ----------------
-    pdl_wait();
-    const float* q0 = p.q + static_cast<size_t>(token0) * p.q_width + p.q_off + head * (kDim + kRot);
-    // The rotated part first, then the rest, in pieces of eight values, all of a thread's reads in flight together.
-    {
-      float4 q[4][2], other[4][2], c[4][2], n[4][2];
-      const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // The queries come as they are, 32-bit rows of 192 values, where the keys will be; each thread then takes four pieces of
+    // eight rotated values and eight of the others into bfloat16.  The angles' tables are no kernel's result.
+    const int own_piece = tid & 7;
+    float4 c[4][2], n[4][2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = j * kSoftmaxThreads + tid, row = i >> 3, piece = i & 7;
-        q[j][0] = q[j][1] = other[j][0] = other[j][1] = c[j][0] = c[j][1] = n[j][0] = n[j][1] = none;
-        if (row < tokens) {
-          const float4* src = reinterpret_cast<const float4*>(q0 + row * p.q_width + kDim);
-          const size_t at = static_cast<size_t>(pos0 + row) * (kRot / 8);
-          const float4* cs = reinterpret_cast<const float4*>(p.cos_table) + at;
-          const float4* sn = reinterpret_cast<const float4*>(p.sin_table) + at;
-          q[j][0] = src[2 * piece], q[j][1] = src[2 * piece + 1];
-          if (p.pairing) {   // values half of the part apart turn together
-            other[j][0] = src[2 * (piece ^ 4)], other[j][1] = src[2 * (piece ^ 4) + 1];
-            c[j][0] = cs[2 * (piece & 3)], c[j][1] = cs[2 * (piece & 3) + 1];
-            n[j][0] = sn[2 * (piece & 3)], n[j][1] = sn[2 * (piece & 3) + 1];
-          } else {           // neighbours do
-            c[j][0] = cs[piece];
-            n[j][0] = sn[piece];
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = j * kSoftmaxThreads + tid, row = i >> 3, piece = i & 7;
-        uint4 to;
-        if (p.pairing) {
-          const float f = piece < 4 ? -1.0f : 1.0f;
-          to.x = packed_pair(q[j][0].x * c[j][0].x + f * (other[j][0].x * n[j][0].x), q[j][0].y * c[j][0].y + f * (other[j][0].y * n[j][0].y));
-          to.y = packed_pair(q[j][0].z * c[j][0].z + f * (other[j][0].z * n[j][0].z), q[j][0].w * c[j][0].w + f * (other[j][0].w * n[j][0].w));
-          to.z = packed_pair(q[j][1].x * c[j][1].x + f * (other[j][1].x * n[j][1].x), q[j][1].y * c[j][1].y + f * (other[j][1].y * n[j][1].y));
-          to.w = packed_pair(q[j][1].z * c[j][1].z + f * (other[j][1].z * n[j][1].z), q[j][1].w * c[j][1].w + f * (other[j][1].w * n[j][1].w));
-        } else {
-          to.x = packed_pair(q[j][0].x * c[j][0].x - q[j][0].y * n[j][0].x, q[j][0].y * c[j][0].x + q[j][0].x * n[j][0].x);
-          to.y = packed_pair(q[j][0].z * c[j][0].y - q[j][0].w * n[j][0].y, q[j][0].w * c[j][0].y + q[j][0].z * n[j][0].y);
-          to.z = packed_pair(q[j][1].x * c[j][0].z - q[j][1].y * n[j][0].z, q[j][1].y * c[j][0].z + q[j][1].x * n[j][0].z);
-          to.w = packed_pair(q[j][1].z * c[j][0].w - q[j][1].w * n[j][0].w, q[j][1].w * c[j][0].w + q[j][1].z * n[j][0].w);
-        }
-        *reinterpret_cast<uint4*>(queries + 2 * kQueryHalf + piece_offset(row, piece)) = to;
+    for (int j = 0; j < 4; ++j) {
+      const int row = (j * kSoftmaxThreads + tid) >> 3;
+      const size_t at = static_cast<size_t>(pos0 + min(row, tokens - 1)) * (kRot / 2);
+      const float4* cs = reinterpret_cast<const float4*>(p.cos_table + at);
+      const float4* sn = reinterpret_cast<const float4*>(p.sin_table + at);
+      if (p.pairing) {
+        c[j][0] = cs[2 * (own_piece & 3)], c[j][1] = cs[2 * (own_piece & 3) + 1];
+        n[j][0] = sn[2 * (own_piece & 3)], n[j][1] = sn[2 * (own_piece & 3) + 1];
+      } else {
+        c[j][0] = cs[own_piece], n[j][0] = sn[own_piece];
+        c[j][1] = n[j][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     }
-    {
-      float4 q[8][2];
+    pdl_wait();
+    if (tid == 0) {
+      expect_bytes(&s.raw, kQ * kRawPitch * 4);
+      load_box(keys, &query_map, &s.raw, p.q_off + head * (kDim + kRot), token0);
+    }
+    __syncwarp();
+    bar_wait<WAIT_EXPIRED>(&s.raw, 0, abort_flag, p.status);
+    const float* raw = reinterpret_cast<const float*>(keys);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int i = j * kSoftmaxThreads + tid, row = i >> 4, piece = i & 15;
-        q[j][0] = q[j][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (row < tokens) {
-          const float4* src = reinterpret_cast<const float4*>(q0 + row * p.q_width) + 2 * piece;
-          q[j][0] = src[0], q[j][1] = src[1];
+    for (int j = 0; j < 4; ++j) {
+      const int row = (j * kSoftmaxThreads + tid) >> 3, piece = own_piece;
+      uint4 to = make_uint4(0u, 0u, 0u, 0u);
+      if (row < tokens) {
+        const float4* src = reinterpret_cast<const float4*>(raw + row * kRawPitch + kDim);
+        const float4 q0 = src[2 * piece], q1 = src[2 * piece + 1];
+        if (p.pairing) {   // values half of the part apart turn together
+          const float4 o0 = src[2 * (piece ^ 4)], o1 = src[2 * (piece ^ 4) + 1];
+          const float f = piece < 4 ? -1.0f : 1.0f;
+          to.x = packed_pair(q0.x * c[j][0].x + f * (o0.x * n[j][0].x), q0.y * c[j][0].y + f * (o0.y * n[j][0].y));
+          to.y = packed_pair(q0.z * c[j][0].z + f * (o0.z * n[j][0].z), q0.w * c[j][0].w + f * (o0.w * n[j][0].w));
+          to.z = packed_pair(q1.x * c[j][1].x + f * (o1.x * n[j][1].x), q1.y * c[j][1].y + f * (o1.y * n[j][1].y));
+          to.w = packed_pair(q1.z * c[j][1].z + f * (o1.z * n[j][1].z), q1.w * c[j][1].w + f * (o1.w * n[j][1].w));
+        } else {           // neighbours do
+          to.x = packed_pair(q0.x * c[j][0].x - q0.y * n[j][0].x, q0.y * c[j][0].x + q0.x * n[j][0].x);
+          to.y = packed_pair(q0.z * c[j][0].y - q0.w * n[j][0].y, q0.w * c[j][0].y + q0.z * n[j][0].y);
+          to.z = packed_pair(q1.x * c[j][0].z - q1.y * n[j][0].z, q1.y * c[j][0].z + q1.x * n[j][0].z);
+          to.w = packed_pair(q1.z * c[j][0].w - q1.w * n[j][0].w, q1.w * c[j][0].w + q1.z * n[j][0].w);
         }
       }
+      *reinterpret_cast<uint4*>(queries + 2 * kQueryHalf + piece_offset(row, piece)) = to;
+    }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int i = j * kSoftmaxThreads + tid, row = i >> 4, piece = i & 15;
-        *reinterpret_cast<uint4*>(queries + (piece >> 3) * kQueryHalf + piece_offset(row, piece & 7)) =
-            make_uint4(packed_pair(q[j][0].x, q[j][0].y), packed_pair(q[j][0].z, q[j][0].w), packed_pair(q[j][1].x, q[j][1].y), packed_pair(q[j][1].z, q[j][1].w));
-      }
+    for (int j = 0; j < 8; ++j) {
+      const int i = j * kSoftmaxThreads + tid, row = i >> 4, piece = i & 15;
+      const float4* src = reinterpret_cast<const float4*>(raw + row * kRawPitch) + 2 * piece;
+      const float4 q0 = src[0], q1 = src[1];
+      *reinterpret_cast<uint4*>(queries + (piece >> 3) * kQueryHalf + piece_offset(row, piece & 7)) =
+          row < tokens ? make_uint4(packed_pair(q0.x, q0.y), packed_pair(q0.z, q0.w), packed_pair(q1.x, q1.y), packed_pair(q1.z, q1.w)) : make_uint4(0u, 0u, 0u, 0u);
     }
     fence_async();
     bar_arrive(&s.query);
@@ -394,18 +396,6 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
       bar_arrive(&s.weight[group][buffer]);
     }
     // ---------------- the two groups' folds are joined ----------------
-    // what the ending needs of the gate is asked for while the last products run: neighbouring threads read, and write, a row
-    const int piece = tid & 15;
-    float4 gate[8][2];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = (j * kSoftmaxThreads + tid) >> 4;
-      gate[j][0] = gate[j][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (p.gate != nullptr && r < tokens) {
-        const float4* z = reinterpret_cast<const float4*>(p.gate + static_cast<size_t>(token0 + r) * p.gate_width + head * kValues) + 2 * piece;
-        gate[j][0] = z[0], gate[j][1] = z[1];
-      }
-    }
     // (`done` would not do: the last scores tell only that the third product from the end is done, whose parity is the last's)
     if (group_tiles > 0) bar_wait<WAIT_EXPIRED>(&s.finished[group], 0, abort_flag, p.status);
     fence_after();
@@ -423,8 +413,8 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
     const float inverse = joint_sum > 0.0f ? 1.0f / joint_sum : 0.0f;
     const float own_factor = own_weight * inverse, other_factor = other_weight * inverse;
     const uint32_t other_o = lanes + kColsO + (group ^ 1) * 128;
-    // each group lays out half of the columns where the keys were (every product that read them is done)
-    float* staged = reinterpret_cast<float*>(keys);
+    // each group lays out half of the columns behind the gate, where keys were (every product that read them is done)
+    float* staged = reinterpret_cast<float*>(base + kGateBytes);
 #pragma unroll 1
     for (int c = group * 64; c < group * 64 + 64; c += 32) {
       uint32_t a[32], b[32];
@@ -441,7 +431,9 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
       for (int k = 0; k < 32; k += 4) *reinterpret_cast<float4*>(staged + row * kStagedPitch + c + k) = make_float4(y[k], y[k + 1], y[k + 2], y[k + 3]);
     }
     asm volatile("bar.sync 6, 256;" ::: "memory");
-    if (!*abort_flag) {
+    if (p.gate != nullptr) bar_wait<WAIT_EXPIRED>(&s.gate, 0, abort_flag, p.status);
+    if (!*abort_flag) {   // neighbouring threads write a row
+      const int piece = tid & 15;
       auto opened = [](float y, float z) { return y * __fdividef(1.0f, 1.0f + __expf(-z)); };
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -449,7 +441,8 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         const float4* from = reinterpret_cast<const float4*>(staged + r * kStagedPitch + piece * 8);
         float4 lo = from[0], hi = from[1];
         if (p.gate != nullptr) {
-          const float4 a = gate[j][0], b = gate[j][1];
+          const float4* z = reinterpret_cast<const float4*>(base) + r * (kValues / 4) + 2 * piece;
+          const float4 a = z[0], b = z[1];
           lo = make_float4(opened(lo.x, a.x), opened(lo.y, a.y), opened(lo.z, a.z), opened(lo.w, a.w));
           hi = make_float4(opened(hi.x, b.x), opened(hi.y, b.y), opened(hi.z, b.z), opened(hi.w, b.w));
         }
@@ -515,6 +508,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
     const int g = (warp - kLoader) >> 1, group_tiles = (num_tiles - g + 1) / 2;
     const bool brings_values = ((warp - kLoader) & 1) != 0;
     pdl_wait();
+    if (!brings_values) bar_wait<WAIT_EXPIRED>(&s.query, 0, abort_flag, p.status);   // the queries lay where the keys go
     for (int i = 0; i < group_tiles; ++i) {
       const int j = 2 * i + g, buffer = i & 1, row = run.row0 + (first_tile + j) * kKeys;
       uint8_t* tile = brings_values ? values + (2 * g + buffer) * kValueBytes : keys + (2 * g + buffer) * kKeyBytes;
@@ -543,6 +537,18 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         bar_arrive(&s.value_zeroed[g][buffer]);
       }
     }
+    // The gate's rows come where the queries and the first keys were, behind the last scores of both groups: the last softmax
+    // and product run meanwhile.  (Loaded by the ending's threads they held it up by 9,000 clocks.)
+    if (!brings_values && p.gate != nullptr) {
+      if (group_tiles > 0) bar_wait<WAIT_EXPIRED>(&s.key_empty[g][(group_tiles - 1) & 1], ((group_tiles - 1) >> 1) & 1, abort_flag, p.status);
+      if (lane == 0) bar_arrive(&s.scored);
+      if (g == 0) bar_wait<WAIT_EXPIRED>(&s.scored, 0, abort_flag, p.status);
+      if (g == 0 && lane == 0 && !*abort_flag) {
+        expect_bytes(&s.gate, kGateBytes);
+        load_box(base, &gate_map, &s.gate, head * kValues, token0);
+      }
+      __syncwarp();
+    }
   }
   fence_before();
   __syncthreads();
@@ -559,19 +565,21 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// [rows, columns] of bfloat16 in boxes of 64 rows x 64 columns, 128-byte swizzle
-inline int make_map(CUtensorMap* map, const void* base, int rows, int columns) {
+// [rows, columns] of bfloat16 in boxes of 64 rows x 64 columns, 128-byte swizzle; or of 32-bit numbers (queries, gate)
+// in boxes of 128 rows x `raw_columns`, as they are, rows `pitch` apart
+inline int make_map(CUtensorMap* map, const void* base, int rows, long long columns, int raw_columns = 0, long long pitch = 0) {
   void* entry = nullptr;
   cudaDriverEntryPointQueryResult result;
   if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &entry, cudaEnableDefault, &result) != cudaSuccess ||
       result != cudaDriverEntryPointSuccess || !entry)
     return VIPERA_NO_DRIVER_ENTRY;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(columns), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(columns) * 2};
-  cuuint32_t box[2] = {64, kKeys}, elem[2] = {1, 1};
+  const bool raw = raw_columns > 0;
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(raw ? pitch * 4 : columns * 2)};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(raw ? raw_columns : 64), static_cast<cuuint32_t>(raw ? kQ : kKeys)}, elem[2] = {1, 1};
   const CUresult r = reinterpret_cast<EncodeTiledFn>(entry)(
-      map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      map, raw ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, raw ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? VIPERA_OK : VIPERA_BAD_ARGUMENT;
 }
 
@@ -584,15 +592,19 @@ inline int launch(const Params& p, const void* expanded, int num_tokens, int sta
   if (p.row_capacity % kRunRows != 0 || p.rank % 8 != 0 || p.requests <= 0 || !p.status) return VIPERA_BAD_ARGUMENT;
   if (stage == 1)
     return vipera_launch(latent_gather_kernel, dim3(p.row_capacity / kGatherRows), dim3(kGatherThreads), 0, s, p);
-  CUtensorMap expanded_map, rot_map;
+  CUtensorMap expanded_map, rot_map, query_map, gate_map;
   int status = make_map(&expanded_map, expanded, p.row_capacity, 2 * p.heads * kDim);
   if (status == VIPERA_OK) status = make_map(&rot_map, p.rot_rows, p.row_capacity, kRot);
+  if (status == VIPERA_OK) status = make_map(&query_map, p.q, num_tokens, p.q_width, kRawPitch, p.q_width);
+  if (status == VIPERA_OK)   // (without a gate any valid map)
+    status = p.gate != nullptr ? make_map(&gate_map, p.gate, num_tokens, p.heads * kValues, kValues, p.gate_width)
+                               : make_map(&gate_map, p.rot_rows, p.row_capacity, kRot);
   if (status != VIPERA_OK) return status;
   static SharedMemoryOptIn opt_in;
   if ((status = opt_in.ask(reinterpret_cast<const void*>(latent_heads_kernel), kSharedBytes)) != 0) return status;
   // at most one partly filled tile per request beyond the full ones
   return vipera_launch(latent_heads_kernel, dim3(p.heads, (num_tokens + kQ - 1) / kQ + p.requests), dim3(kThreads), kSharedBytes, s,
-                       expanded_map, rot_map, p);
+                       expanded_map, rot_map, query_map, gate_map, p);
 }
 
 }  // namespace latent_heads
