@@ -96,7 +96,11 @@ struct GemmParams {
   // Grouped product (tokens on the 128-row side, whole tiles, blocks alone): W holds `groups`
   // matrices [N, K] one after the other, and the 128 tokens of tile tx use matrix tile_group[tx].
   // The table is written by a kernel ahead of this one, so no weight tile is fetched before it.
+  // tile_count: how many of the table's tiles there are (written like it); null: all of them.  A step's table is as long as
+  // its rows may need, every matrix's last tile partly filled; some 8 of 97 tiles (10,240 rows, 17 matrices) are not there,
+  // and computing them cost the mixture of [3584, 1536] and [1536, 1792] 234 us against 217.
   const int* tile_group;     // [tiles_x] or null
+  const int* tile_count;
   int group_stride;          // rows of W from one matrix to the next (N)
   const float* unit_limit;   // grouped, ACT_CLAMPED: [groups] the bound of each group's gated unit
   float unit_slope;          // and the slope inside its sigmoid
@@ -448,14 +452,18 @@ struct WorkLoop {
   const GemmParams& p;
   int item;
   long at, end;
-  int stride;
+  int stride, tiles_x;
   // `pair`: the two blocks of a cluster walk the same tiles
   __device__ __forceinline__ explicit WorkLoop(const GemmParams& params, bool pair = false)
-      : p(params), item(pair ? blockIdx.x >> 1 : blockIdx.x), at(0), end(0), stride(pair ? gridDim.x >> 1 : gridDim.x) {
+      : p(params), item(pair ? blockIdx.x >> 1 : blockIdx.x), at(0), end(0), stride(pair ? gridDim.x >> 1 : gridDim.x), tiles_x(params.tiles_x) {
     if (EVEN && p.even_shares) {
       at = share_begin(p, blockIdx.x, gridDim.x);
       end = share_begin(p, blockIdx.x + 1, gridDim.x);
     }
+  }
+  // behind pdl_wait: the work is that of the tiles there are
+  __device__ __forceinline__ void count_tiles() {
+    if (p.tile_count != nullptr) tiles_x = min(*p.tile_count, p.tiles_x);
   }
   __device__ __forceinline__ bool next(Piece& piece) {
     if (EVEN && p.even_shares) {
@@ -468,7 +476,7 @@ struct WorkLoop {
       at += piece.kb_end - piece.kb_begin;
       return true;
     }
-    if (item >= p.tiles_x * p.tiles_y * p.splits) return false;
+    if (item >= tiles_x * p.tiles_y * p.splits) return false;
     const int split = item % p.splits;
     piece.tile = item / p.splits;
     piece.kb_begin = split * p.k_blocks_per_split;
@@ -491,6 +499,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                               (static_cast<uint32_t>((PAIR ? 2 * kTileX : kTileX) >> 4) << 24);
   const uint32_t rank = PAIR ? cluster_rank() : 0u;   // 0: the block that issues the pair's products
   constexpr bool kWide = BN >= 128;                   // the forms for many tokens
+  constexpr bool kCounted = !SWAP && !PAIR && !EVEN;  // the forms that grouped products take
   constexpr bool kEven = EVEN;                        // the form that runs with even shares, an instance of its own
   static_assert(!EVEN || (!SWAP && BN >= 128 && !PAIR), "even shares: tokens on the 128-row side, wide tiles, blocks alone");
   extern __shared__ uint8_t smem_raw[];
@@ -566,10 +575,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       int stage = 0, issued = 0;
       uint32_t phase = 0;
       WorkLoop<kEven> work(p, PAIR);
+      if (kCounted) work.count_tiles();
       Piece piece;
       while (work.next(piece)) {
-        const int tx = PAIR ? 2 * (piece.tile % p.tiles_x) + static_cast<int>(rank) : piece.tile % p.tiles_x;
-        const int ty = piece.tile / p.tiles_x;
+        const int tx = PAIR ? 2 * (piece.tile % work.tiles_x) + static_cast<int>(rank) : piece.tile % work.tiles_x;
+        const int ty = piece.tile / work.tiles_x;
         const int group_row = (!SWAP && !PAIR && p.tile_group) ? p.tile_group[tx] * p.group_stride : 0;
         for (int kb = piece.kb_begin; kb < piece.kb_end; ++kb, ++issued) {
           if (issued % kProducers != mine) {
@@ -615,6 +625,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const uint32_t other_empty = PAIR ? in_block(smem_u32(&empty[0]), 1) : 0u;
       const uint32_t other_acc_full = PAIR ? in_block(smem_u32(&acc_full[0]), 1) : 0u;
       WorkLoop<kEven> work(p, PAIR);
+      if (kCounted && p.tile_count != nullptr) {
+        pdl_wait();
+        work.count_tiles();
+      }
       Piece piece;
       for (; work.next(piece); ++local) {
         const int kb_begin = piece.kb_begin, kb_end = piece.kb_end;
@@ -687,12 +701,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     pdl_wait();  // outputs, the residual stream, and the scratch belong to earlier kernels until now
     int local = 0;
     WorkLoop<kEven> work(p, PAIR);
+    if (kCounted) work.count_tiles();
     Piece piece;
     const uint32_t pair_acc_empty = PAIR ? in_block(smem_u32(&acc_empty[0]), 0) : 0u;
     for (; work.next(piece); ++local) {
       const int tile = piece.tile;
-      const int tx = PAIR ? 2 * (tile % p.tiles_x) + static_cast<int>(rank) : tile % p.tiles_x;
-      const int ty = tile / p.tiles_x;
+      const int tx = PAIR ? 2 * (tile % work.tiles_x) + static_cast<int>(rank) : tile % work.tiles_x;
+      const int ty = tile / work.tiles_x;
       const int acc = local & 1;
       // Even shares: a piece that starts inside a tile is a partial sum for another block; the
       // piece with the tile's first k-block that does not reach its last one waits for the blocks
@@ -1654,7 +1669,7 @@ static int launch_pairs(const CUtensorMap& map_x, const CUtensorMap& map_y, cons
 static int run_gemm(const void* A, const void* W, int T, int N, int K, int epilogue, const float* bias, void* out,
                     int out_dtype, float* resid, float* scratch, size_t scratch_bytes, int* status, void* stream,
                     const GemmParams* rope, int activation = ACT_SILU, const int* tile_group = nullptr, int groups = 1,
-                    const float* unit_limit = nullptr, float unit_slope = 0.0f) {
+                    const float* unit_limit = nullptr, float unit_slope = 0.0f, const int* tile_count = nullptr) {
   if (T <= 0) return VIPERA_OK;
   const bool grouped = tile_group != nullptr;
   if (grouped && (groups <= 0 || T % kTileX != 0 || rope != nullptr || epilogue == EPI_RESIDUAL)) return VIPERA_BAD_ARGUMENT;
@@ -1692,6 +1707,7 @@ static int run_gemm(const void* A, const void* W, int T, int N, int K, int epilo
   GemmParams p{};
   if (rope) p = *rope;
   p.tile_group = tile_group;
+  p.tile_count = tile_count;
   p.group_stride = N;
   p.unit_limit = unit_limit;
   p.unit_slope = unit_slope;
@@ -1806,13 +1822,13 @@ VIPERA_API int vipera_gemm_tc_act(const void* A, const void* W, int T, int N, in
 }
 
 // Grouped: W is [groups, N, K]; A is [T, K] with T a multiple of 128, and rows 128 * i .. 128 * i + 127
-// are multiplied by matrix tile_group[i] (a device table that a kernel ahead in the stream writes).
+// are multiplied by matrix tile_group[i] (a device table that a kernel ahead in the stream writes), where i < *tile_count (null: all).
 // Endings STORE and the gated unit; STORE into bfloat16 with activation ACT_RELU2 applies the square of
 // relu on the way out (a unit without a gate).  ACT_CLAMPED: the gated unit with the bound
 // unit_limit[tile_group[i]] (a device table) and `unit_slope`.
 VIPERA_API int vipera_gemm_tc_grouped(const void* A, const void* W, int T, int N, int K, int groups, const int* tile_group,
-                                      int epilogue, void* out, int out_dtype, int activation, const float* unit_limit,
-                                      float unit_slope, int* status, void* stream) {
+                                      const int* tile_count, int epilogue, void* out, int out_dtype, int activation,
+                                      const float* unit_limit, float unit_slope, int* status, void* stream) {
   if (epilogue != EPI_STORE && epilogue != EPI_SWIGLU) return VIPERA_BAD_ARGUMENT;
   if (activation == ACT_RELU2) {
     if (epilogue != EPI_STORE || out_dtype != VIPERA_BF16) return VIPERA_BAD_ARGUMENT;
@@ -1823,7 +1839,7 @@ VIPERA_API int vipera_gemm_tc_grouped(const void* A, const void* W, int T, int N
   }
   if (!tile_group) return VIPERA_BAD_ARGUMENT;
   return run_gemm(A, W, T, N, K, epilogue, nullptr, out, out_dtype, nullptr, nullptr, 0, status, stream, nullptr, activation,
-                  tile_group, groups, unit_limit, unit_slope);
+                  tile_group, groups, unit_limit, unit_slope, tile_count);
 }
 
 // What the q/k/v ending needs beside the product itself (mirrored by the caller).

@@ -2125,13 +2125,14 @@ def moe_scratch_words(tokens: int, top: int, experts: int) -> int:
 
 def gemm_tc_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, *, epilogue: int, out: torch.Tensor,
                     activation: int = ACT_SILU, unit_limit: Optional[torch.Tensor] = None, unit_slope: float = 0.0,
-                    what: str = "gemm_tc") -> None:
+                    what: str = "gemm_tc", tile_count: Optional[torch.Tensor] = None) -> None:
     """a[M, K] (M a multiple of 128) times one of the matrices w[G, N, K], transposed: rows 128 i ..
-    128 i + 127 use matrix tile_group[i] (int32, written on the device ahead of this call).
+    128 i + 127 use matrix tile_group[i] (int32, written on the device ahead of this call).  ``tile_count``
+    (int32, one number, written likewise): only that many of the table's tiles are computed.
     Endings: plain store, or the gated unit over interleaved gate and up rows (with ACT_CLAMPED each
     group's unit has the bound ``unit_limit[group]``, float32, and ``unit_slope``)."""
     fn = _function("gemm_tc", "vipera_gemm_tc_grouped",
-                   [_c_void, _c_void, _c_int, _c_int, _c_int, _c_int, _c_void, _c_int, _c_void, _c_int, _c_int, _c_void,
+                   [_c_void, _c_void, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int, _c_int, _c_void,
                     _c_float, _c_void, _c_void])
     if activation == ACT_CLAMPED and (unit_limit is None or unit_limit.numel() != w.shape[0]):
         raise InvalidArgumentError("gemm_tc_grouped: one bound per group")
@@ -2144,7 +2145,7 @@ def gemm_tc_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, 
         raise InvalidArgumentError(f"gemm_tc_grouped: out must be [{m}, {width}]")
     state = _tc_buffers(a.device, 0)
     _check(fn(_gpu(a, "a", torch.bfloat16), _gpu(w, "w", torch.bfloat16), m, n, k, groups,
-              _gpu(tile_group, "tile_group", torch.int32), epilogue, _gpu(out, "out"), dtype_code(out.dtype), int(activation),
+              _gpu(tile_group, "tile_group", torch.int32), _opt(tile_count, "tile_count", torch.int32), epilogue, _gpu(out, "out"), dtype_code(out.dtype), int(activation),
               _opt(unit_limit, "unit_limit", torch.float32), float(unit_slope),
               state["status"].data_ptr(), _stream()), what)
 
@@ -2238,13 +2239,14 @@ def moe(h: torch.Tensor, *, router: torch.Tensor, gate_up: torch.Tensor, down: t
     p.xs, p.ys = _gpu(xs, "xs"), _gpu(ys, "ys", torch.float32)
     _check(fn(ctypes.byref(p), dtype_code(h.dtype), _stream()), "moe", kernels=3)
     tile_expert = scratch[places + assignments + 1 + 3 * most:places + assignments + 1 + 3 * most + tiles]
+    tile_count = scratch[places + assignments:places + assignments + 1]
     xs_rows = xs.view(-1)[:capacity * hidden].view(capacity, hidden)
     act_rows = act.view(-1)[:capacity * ff].view(capacity, ff)
     ys_rows = ys.view(-1)[:capacity * hidden].view(capacity, hidden)
     gemm_tc_grouped(xs_rows, gate_up, tile_expert, epilogue=EPI_GATED if gated else EPI_STORE, out=act_rows,
                     activation=activation, unit_limit=unit_limit if activation == ACT_CLAMPED else None,
-                    unit_slope=unit_slope, what="moe")
-    gemm_tc_grouped(act_rows, down, tile_expert, epilogue=EPI_STORE, out=ys_rows, what="moe")
+                    unit_slope=unit_slope, what="moe", tile_count=tile_count)
+    gemm_tc_grouped(act_rows, down, tile_expert, epilogue=EPI_STORE, out=ys_rows, what="moe", tile_count=tile_count)
     if target is not None and target.data_ptr() % 16 == 0:
         total = _function("moe", "vipera_moe_sum", [ctypes.POINTER(_MoeParams), _c_void, _c_void])
         _check(total(ctypes.byref(p), _gpu(target, "target", torch.float32), _stream()), "moe")
