@@ -452,19 +452,18 @@ struct WorkLoop {
   const GemmParams& p;
   int item;
   long at, end;
-  int stride, tiles_x;
+  int stride, items;
   // `pair`: the two blocks of a cluster walk the same tiles
   __device__ __forceinline__ explicit WorkLoop(const GemmParams& params, bool pair = false)
-      : p(params), item(pair ? blockIdx.x >> 1 : blockIdx.x), at(0), end(0), stride(pair ? gridDim.x >> 1 : gridDim.x), tiles_x(params.tiles_x) {
+      : p(params), item(pair ? blockIdx.x >> 1 : blockIdx.x), at(0), end(0), stride(pair ? gridDim.x >> 1 : gridDim.x), items(params.tiles_x * params.tiles_y * params.splits) {
     if (EVEN && p.even_shares) {
       at = share_begin(p, blockIdx.x, gridDim.x);
       end = share_begin(p, blockIdx.x + 1, gridDim.x);
     }
   }
-  // behind pdl_wait: the work is that of the tiles there are
-  __device__ __forceinline__ void count_tiles() {
-    if (p.tile_count != nullptr) tiles_x = min(*p.tile_count, p.tiles_x);
-  }
+  // Counted tiles (a row of tiles after the other, so that a block finds its first tile without the count): behind pdl_wait,
+  // the work ends where they do.
+  __device__ __forceinline__ void end_at(int tile_count) { items = min(tile_count, p.tiles_x) * p.tiles_y; }
   __device__ __forceinline__ bool next(Piece& piece) {
     if (EVEN && p.even_shares) {
       if (at >= end) return false;
@@ -476,7 +475,7 @@ struct WorkLoop {
       at += piece.kb_end - piece.kb_begin;
       return true;
     }
-    if (item >= tiles_x * p.tiles_y * p.splits) return false;
+    if (item >= items) return false;
     const int split = item % p.splits;
     piece.tile = item / p.splits;
     piece.kb_begin = split * p.k_blocks_per_split;
@@ -486,6 +485,17 @@ struct WorkLoop {
     return true;
   }
 };
+
+// A tile's row and column of tiles; columns one after the other, or rows where the rows are counted on the device.
+template <bool COUNTED, bool PAIR>
+__device__ __forceinline__ void tile_place(const GemmParams& p, int tile, uint32_t rank, int& tx, int& ty) {
+  if (COUNTED && p.tile_count != nullptr) {
+    tx = tile / p.tiles_y, ty = tile % p.tiles_y;
+    return;
+  }
+  tx = PAIR ? 2 * (tile % p.tiles_x) + static_cast<int>(rank) : tile % p.tiles_x;
+  ty = tile / p.tiles_x;
+}
 
 template <int BN, bool SWAP, bool PAIR = false, bool EVEN = false, bool EXT = false>
 __global__ void __launch_bounds__(threads_for<BN>(), (BN >= 128 || VIPERA_SMALL_BUDGET > 110 ? 1 : 2))
@@ -575,12 +585,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       int stage = 0, issued = 0;
       uint32_t phase = 0;
       WorkLoop<kEven> work(p, PAIR);
-      if (kCounted) work.count_tiles();
+      int ahead = 0;   // the first tile's matrix, asked for together with the count
+      if (kCounted && p.tile_count != nullptr) {
+        ahead = p.tile_group[min(work.item / p.tiles_y, p.tiles_x - 1)];
+        work.end_at(*p.tile_count);
+      }
       Piece piece;
       while (work.next(piece)) {
-        const int tx = PAIR ? 2 * (piece.tile % work.tiles_x) + static_cast<int>(rank) : piece.tile % work.tiles_x;
-        const int ty = piece.tile / work.tiles_x;
-        const int group_row = (!SWAP && !PAIR && p.tile_group) ? p.tile_group[tx] * p.group_stride : 0;
+        int tx, ty;
+        tile_place<kCounted, PAIR>(p, piece.tile, rank, tx, ty);
+        const bool first_counted = kCounted && p.tile_count != nullptr && issued == 0;
+        const int group_row = first_counted ? ahead * p.group_stride : (!SWAP && !PAIR && p.tile_group) ? p.tile_group[tx] * p.group_stride : 0;
         for (int kb = piece.kb_begin; kb < piece.kb_end; ++kb, ++issued) {
           if (issued % kProducers != mine) {
             if (++stage == kStages) { stage = 0; phase ^= 1u; }
@@ -627,7 +642,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       WorkLoop<kEven> work(p, PAIR);
       if (kCounted && p.tile_count != nullptr) {
         pdl_wait();
-        work.count_tiles();
+        work.end_at(*p.tile_count);
       }
       Piece piece;
       for (; work.next(piece); ++local) {
@@ -701,13 +716,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     pdl_wait();  // outputs, the residual stream, and the scratch belong to earlier kernels until now
     int local = 0;
     WorkLoop<kEven> work(p, PAIR);
-    if (kCounted) work.count_tiles();
+    if (kCounted && p.tile_count != nullptr) work.end_at(*p.tile_count);
     Piece piece;
     const uint32_t pair_acc_empty = PAIR ? in_block(smem_u32(&acc_empty[0]), 0) : 0u;
     for (; work.next(piece); ++local) {
       const int tile = piece.tile;
-      const int tx = PAIR ? 2 * (tile % work.tiles_x) + static_cast<int>(rank) : tile % work.tiles_x;
-      const int ty = tile / work.tiles_x;
+      int tx, ty;
+      tile_place<kCounted, PAIR>(p, tile, rank, tx, ty);
       const int acc = local & 1;
       // Even shares: a piece that starts inside a tile is a partial sum for another block; the
       // piece with the tile's first k-block that does not reach its last one waits for the blocks
