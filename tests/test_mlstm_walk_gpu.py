@@ -84,3 +84,26 @@ def test_rule():
     assert walks(4, 128, 256, [65]) and not walks(4, 64, 128, [65])
     assert not walks(8, 256, 500, [2048]) and not walks(8, 256, 512, [2048], width=62) and not walks(8, 96, 512, [2048])
     assert not walks(8, 256, 512, [65] + [1] * 40)
+
+
+def test_the_plan_holds_the_scratch():
+    """Whatever step walks, its scratch fits what the memory plan counts for it: many short portions among them."""
+    from types import SimpleNamespace
+
+    from vipera_rs_b200.kernels import ops
+    from vipera_rs_b200.parts.mlstm import MLSTM
+
+    walked = 0
+    for heads, dim, vdim in ((8, 256, 512), (4, 128, 256), (4, 64, 128)):
+        part = SimpleNamespace(heads=heads, dim=dim, vdim=vdim, offsets=(0, 8, 16), AT_ONCE_FROM=256)
+        params = {"num_heads": heads, "head_dim": dim, "value_dim": vdim}
+        for entries in (1, 2, 3, 8, 9, 31, 32, 33, 40, 64, 255, 256, 341):
+            for tokens in (48, 96, 130, 200, 255, 300, 512, 1030, 2048):
+                ctx = SimpleNamespace(num_tokens=tokens, num_entries=entries, host_counts=[], max_count=tokens)
+                if entries > tokens or not MLSTM.walks(part, ctx, torch.zeros(1, 64)):
+                    continue
+                walked += 1
+                scratch = sum(size * dtype.itemsize for size, dtype in ops.mlstm_walk_scratch(heads, dim, vdim).values())
+                others = tokens * ((2 * heads * (dim + vdim) + 2 * heads) * 4 + heads * vdim * 6 + heads * (dim + 1) * 4)
+                assert (tokens // ops.MLSTM_CHUNK + entries) * scratch <= MLSTM.workspace_bytes(params, tokens, 2) - others
+    assert walked > 50

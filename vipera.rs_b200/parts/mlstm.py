@@ -29,6 +29,9 @@ from .base import FixedState, Mixer
 from .linear import Linear
 
 
+WALK_ENTRIES = 32   # most requests of a step that walks prepared chunks: each may end in a partly filled one, and memory is planned for them
+
+
 class MLSTM(Mixer):
     """params: hidden_size, num_heads, head_dim (size of q and k per head), value_dim, gate_cap,
     norm_eps (of the head norm) and, optionally, ``denominator_eps`` (default 1e-6) and
@@ -111,7 +114,7 @@ class MLSTM(Mixer):
         walk = 0
         if element_bytes == 2 and ops.mlstm_tc_takes(d, dv) and dv % 32 == 0:
             chunk = sum(size * dtype.itemsize for size, dtype in ops.mlstm_walk_scratch(heads, d, dv).values())
-            walk = (tokens // ops.MLSTM_CHUNK + 8) * chunk
+            walk = (tokens // ops.MLSTM_CHUNK + WALK_ENTRIES) * chunk
         return tokens * (width * 4 + heads * dv * (4 + element_bytes)) + tokens * heads * (d + 1) * 4 + walk
 
     def walks(self, ctx, proj) -> bool:
@@ -122,6 +125,8 @@ class MLSTM(Mixer):
         tokens 158 / 168, three requests of 1,024, 901 and 77 152 / 134.  Short steps, against the walk without preparation: 4
         heads of 256 x 512, 128 tokens 67 / 49; of 128 x 256 51 / 42; of 64 x 128, 65 tokens 39 / 38, 17 + 1 + 1 23 / 28."""
         tokens, entries = ctx.num_tokens, ctx.num_entries
+        if entries > WALK_ENTRIES:
+            return False
         if not ops.mlstm_walk_takes(proj, self.offsets, self.dim, self.vdim) or tokens < 6 * entries:
             return False
         if tokens < self.AT_ONCE_FROM:
