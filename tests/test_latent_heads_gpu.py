@@ -117,3 +117,71 @@ def test_rule():
         known, captured = step(counts, firsts), step(counts, firsts, host_counts=[])
         if part.expanded_rows(captured):
             assert 0 < part.expanded_rows(known) <= part.expanded_rows(captured)
+
+
+def _step(part, counts, firsts, page, rank, window=0, kept=None):
+    """The step's context and pages that hold `kept` (random latents where none are given)."""
+    from vipera_rs_b200.parts.base import PagedKVView, StepContext, Workspace
+
+    tokens, entries, longest = sum(counts), len(counts), max(c + f for c, f in zip(counts, firsts))
+    width = -(-longest // page)
+    table = torch.arange(entries * width).view(entries, width).to(torch.int32)
+    kept = kept or [(torch.randn(f, rank, device=DEV).bfloat16(), torch.randn(f, ROT, device=DEV).bfloat16()) for f in firsts]
+    k = torch.zeros(entries * width, page, 1, rank, device=DEV, dtype=torch.bfloat16)
+    v = torch.zeros(entries * width, page, 1, ROT, device=DEV, dtype=torch.bfloat16)
+    for e, (c, r) in enumerate(kept):
+        k.view(entries, width * page, rank)[e, :len(c)], v.view(entries, width * page, ROT)[e, :len(c)] = c, r
+    device = lambda values: torch.from_numpy(np.ascontiguousarray(values, dtype=np.int32)).to(DEV)  # noqa: E731
+    context = StepContext(
+        num_tokens=tokens, num_entries=entries, tokens=device(np.zeros(tokens)),
+        positions=device(np.concatenate([np.arange(f, f + c) for c, f in zip(counts, firsts)])),
+        token_entry=device(np.repeat(np.arange(entries), counts)), entry_starts=device(np.cumsum([0] + counts)), entry_pos0=device(firsts),
+        state_slots=device(np.arange(entries)), fresh=device(np.zeros(entries)), block_tables=[table.to(DEV)], logit_rows=None,
+        num_logit_rows=0, host_counts=counts, host_pos0=firsts, max_count=max(counts), max_kv_len=longest, all_single=False,
+        any_single=1 in counts, dtype=torch.bfloat16, workspace=Workspace(DEV))
+    part.prepare(4096)
+    return context, PagedKVView(0, k, v, page, window or None), kept
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(3, 512, 0, 16, "interleaved", False), (2, 256, 100, 7, "neox", True)])
+@pytest.mark.parametrize("token", [0, 1, 63, 64, 100, 127, 128, 200, 299])
+def test_tokens_that_are_not_finite(sizes, token):
+    """A token whose numbers are not finite shows in its own output and in those of the tokens that see it, nowhere else."""
+    heads, rank, window, page, style, gated = sizes
+    part, _ = _part(sizes, 5, DEV)
+    h = torch.randn(370, HIDDEN, device=DEV).bfloat16()
+    outs = []
+    for value in (None, float("nan"), float("inf")):
+        if value is not None:
+            h[token] = value
+        context, view, _ = _step(part, [300, 70], [0, 0], page, rank, window)
+        assert part.expanded_rows(context) > 0
+        out = torch.zeros(370, HIDDEN, device=DEV)
+        part.forward(context, h, out, view, True)
+        outs.append(out)
+    end = min(300, token + window) if window else 300
+    for out in outs[1:]:
+        assert torch.equal(out[:token], outs[0][:token]) and torch.equal(out[end:], outs[0][end:])
+        assert not torch.isfinite(out[token:end]).any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window", [0, 100])
+def test_values_that_are_not_finite(window):
+    """One value of a head is infinite for every token: it shows in that column of every token's heads, in no other column."""
+    sizes = (2, 256, window, 16, "interleaved", False)
+    mixed = []
+    for value in (None, float("inf")):
+        part, _ = _part(sizes, 7, DEV)
+        if value is not None:
+            part.up_kv[(2 + 1) * 128 + 5, 17] = value     # head 1, its value 5
+        torch.manual_seed(3)
+        h = torch.randn(333, HIDDEN, device=DEV).bfloat16()
+        context, view, _ = _step(part, [333], [40], 16, 256, window)
+        assert part.expanded_rows(context) > 0
+        part.forward(context, h, torch.zeros(333, HIDDEN, device=DEV), view, True)
+        mixed.append(context.workspace.get("latent.out", (333, 256), torch.bfloat16).clone())
+    columns = torch.arange(256, device=DEV) != 128 + 5
+    assert torch.equal(mixed[0][:, columns], mixed[1][:, columns])
+    assert not torch.isfinite(mixed[1][:, 128 + 5]).any()

@@ -21,6 +21,9 @@
 // which the exponentials are 512 and scaling the output to a new maximum some 400; tensor cores are busy a third of the time.
 // Measured: 2,048 tokens, 12 heads, rank 512, window 1,024: the mixer 287 -> 108 us; 1,748 tokens of four requests behind up
 // to 3,000, 32 heads, a gate: 663 -> 306 us (over the latents, latent_tc.cuh, before).
+// A value that is not finite shows in the outputs of the queries that see its key, and in no others: out of the tiles that some query
+// of a block sees and another does not, such values are taken before the product and given back at the end.  Looking through these
+// tiles costs 0.4 us of 112; with the product's own zeros times infinities up to 127 earlier tokens lost their outputs.
 // Every wait is bounded; one that runs out leaves a code in the status word.
 #pragma once
 
@@ -160,11 +163,14 @@ latent_gather_kernel(const Params p) {
   }
 }
 
+constexpr int kMostTakenOut = 6 * kKeys;
 struct Shared {
   // per group and, but for the output's, per buffer
-  uint64_t raw, query, scored, gate, key_full[2][2], key_empty[2][2], value_landed[2][2], value_zeroed[2][2], value_empty[2][2], score[2][2], weight[2][2], done[2], finished[2];
+  uint64_t raw, query, scored, gate, key_full[2][2], key_empty[2][2], value_landed[2][2], value_looked[2][2], value_empty[2][2], score[2][2], weight[2][2], done[2], finished[2];
   uint32_t tmem_base;
   int abort_flag;
+  int taken_out;
+  int taken_out_key[kMostTakenOut];
   Run run;
   int tile;
   float2 told[2][kQ];   // a group's maxima and sums, for the other
@@ -195,6 +201,54 @@ __device__ __forceinline__ uint32_t packed_pair(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&pair);
 }
 
+// Pairs of bfloat16 numbers times zero: what was not finite leaves a number that is none.
+__device__ __forceinline__ void times_zero(uint32_t& sum, const uint4& v) {
+  asm("fma.rn.bf16x2 %0, %1, %5, %0;\nfma.rn.bf16x2 %0, %2, %5, %0;\nfma.rn.bf16x2 %0, %3, %5, %0;\nfma.rn.bf16x2 %0, %4, %5, %0;"
+      : "+r"(sum) : "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(0u));
+}
+__device__ __forceinline__ uint32_t without_wrong(uint32_t pair) {
+  if ((pair & 0x7f80u) == 0x7f80u) pair &= 0xffff0000u;
+  if ((pair & 0x7f800000u) == 0x7f800000u) pair &= 0x0000ffffu;
+  return pair;
+}
+
+// Out of a tile of values [64 keys][128], its first key at position `key0`, go rows that no query of the block sees, whole, and of
+// the others what is not finite.
+__device__ __forceinline__ void take_out(Shared& s, uint8_t* tile, int lane, int key0, int first_key, int end_key) {
+  for (int r = lane; r < kKeys; r += 32) {
+    auto at = [&](int piece) { return reinterpret_cast<uint4*>(tile + (piece >> 3) * kHalf + piece_offset(r, piece & 7)); };
+    if (key0 + r < first_key || key0 + r >= end_key) {   // it may be anything
+#pragma unroll
+      for (int piece = 0; piece < 16; ++piece) *at(piece) = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    uint32_t sums[2] = {0u, 0u};
+#pragma unroll
+    for (int piece = 0; piece < 16; ++piece) times_zero(sums[piece & 1], *at(piece));
+    if (((sums[0] | sums[1]) & 0x7f807f80u) != 0u) {
+      for (int piece = 0; piece < 16; ++piece) {
+        const uint4 v = *at(piece);
+        *at(piece) = make_uint4(without_wrong(v.x), without_wrong(v.y), without_wrong(v.z), without_wrong(v.w));
+      }
+      const int place = atomicAdd(&s.taken_out, 1);
+      if (place < kMostTakenOut) s.taken_out_key[place] = key0 + r;
+    }
+  }
+}
+// A query's 64 outputs get back what was taken out of the values from column `column` on of the keys that it sees.
+__device__ __noinline__ void give_back(const Shared& s, const Params& p, const __nv_bfloat16* expanded, float* y, int column, int position) {
+  const int first = p.window > 0 ? max(0, position - p.window + 1) : 0;
+  for (int i = 0; i < min(s.taken_out, kMostTakenOut); ++i) {
+    const int key = s.taken_out_key[i];
+    if (key < first || key > position) continue;
+    const __nv_bfloat16* v = expanded + static_cast<size_t>(s.run.row0 + key - s.run.first_key) * (2 * p.heads * kDim) + p.heads * kValues + column;
+    for (int k = 0; k < 64; ++k) {
+      const float value = __bfloat162float(v[k]);
+      if (!isfinite(value)) y[k] += value;
+    }
+  }
+}
+
 // The largest of a row's 64 scores, three at a time.
 __device__ __forceinline__ float largest_of(const uint32_t (&v)[kKeys]) {
   float m[4];
@@ -219,7 +273,7 @@ __device__ __forceinline__ uint32_t weights_of(uint32_t a, uint32_t b, float sca
 
 __global__ void __launch_bounds__(kThreads, 1)
 latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __grid_constant__ CUtensorMap rot_map,
-                    const __grid_constant__ CUtensorMap query_map, const __grid_constant__ CUtensorMap gate_map, const Params p) {
+                    const __grid_constant__ CUtensorMap query_map, const __grid_constant__ CUtensorMap gate_map, const __nv_bfloat16* __restrict__ expanded, const Params p) {
   extern __shared__ uint8_t latent_heads_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(latent_heads_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* queries = base;                          // three halves
@@ -257,15 +311,15 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         bar_init(&s.key_full[g][b], 1);
         bar_init(&s.key_empty[g][b], 1);
         bar_init(&s.value_landed[g][b], 1);
-        bar_init(&s.value_zeroed[g][b], 32);
+        bar_init(&s.value_looked[g][b], 32);
         bar_init(&s.value_empty[g][b], 1);
         bar_init(&s.score[g][b], 1);
         bar_init(&s.weight[g][b], kGroupThreads);
       }
       bar_init(&s.done[g], 1);
-      bar_init(&s.finished[g], 1);
+      bar_init(&s.finished[g], 2);   // the last product's end, and its issuer's word that what was taken out stands written
     }
-    s.abort_flag = 0;
+    s.abort_flag = s.taken_out = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kIssuer) {
@@ -277,7 +331,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
   fence_after();
   const uint32_t tmem = s.tmem_base;
   // a value tile with rows that no query of the block may see: their weights are zero, but what they hold may be anything
-  auto ragged = [&](int j) { return key_base + j * kKeys < first_key || key_base + (j + 1) * kKeys > end_key; };
+  auto bounded = [&](int j) { const int key0 = key_base + j * kKeys; return key0 + kKeys - 1 > pos0 || (p.window > 0 && key0 < end_key - p.window); };
 
   if (warp < kIssuer) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegisters));
@@ -430,12 +484,14 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
 #pragma unroll
       for (int k = 0; k < 32; k += 4) *reinterpret_cast<float4*>(staged + row * kStagedPitch + c + k) = make_float4(y[k], y[k + 1], y[k + 2], y[k + 3]);
     }
+    if (s.taken_out > 0 && row < tokens) give_back(s, p, expanded, staged + row * kStagedPitch + group * 64, head * kValues + group * 64, pos0 + row);
     asm volatile("bar.sync 6, 256;" ::: "memory");
     if (p.gate != nullptr) bar_wait<WAIT_EXPIRED>(&s.gate, 0, abort_flag, p.status);
     if (!*abort_flag) {   // neighbouring threads write a row
       const int piece = tid & 15;
       auto opened = [](float y, float z) { return y * __fdividef(1.0f, 1.0f + __expf(-z)); };
-#pragma unroll
+      // (a row at a time: unrolled, this takes registers from the softmax above, 111.5 us for 108.3)
+#pragma unroll 1
       for (int j = 0; j < 8; ++j) {
         const int r = (j * kSoftmaxThreads + tid) >> 4;
         const float4* from = reinterpret_cast<const float4*>(staged + r * kStagedPitch + piece * 8);
@@ -461,7 +517,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
       constexpr uint32_t kOutputs = kCommon | (static_cast<uint32_t>(kValues >> 3) << 17) | (1u << 16);
       const uint32_t q_addr = shared_address(queries), k_addr = shared_address(keys + 2 * g * kKeyBytes), v_addr = shared_address(values + 2 * g * kValueBytes);
       const uint32_t s_tmem = tmem + kColsS + 2 * g * kKeys, o_tmem = tmem + kColsO + g * 128;
-      uint32_t zeroed[2] = {0, 0};   // ragged tiles so far, per buffer
+      uint32_t looked = 0;   // the bounded tiles' parities, a bit per buffer
       auto scores = [&](int i) {
         const uint32_t buffer = i & 1;
         bar_wait<WAIT_EXPIRED>(&s.key_full[g][buffer], (i >> 1) & 1, abort_flag, p.status);
@@ -482,9 +538,9 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
       if (group_tiles > 1) scores(1);
       for (int i = 0; i < group_tiles; ++i) {
         const uint32_t buffer = i & 1;
-        if (ragged(2 * i + g)) {
-          bar_wait<WAIT_EXPIRED>(&s.value_zeroed[g][buffer], zeroed[buffer] & 1, abort_flag, p.status);
-          ++zeroed[buffer];
+        if (bounded(2 * i + g)) {
+          bar_wait<WAIT_EXPIRED>(&s.value_looked[g][buffer], (looked >> buffer) & 1, abort_flag, p.status);
+          looked ^= 1u << buffer;
         } else {
           bar_wait<WAIT_EXPIRED>(&s.value_landed[g][buffer], (i >> 1) & 1, abort_flag, p.status);
         }
@@ -494,7 +550,10 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
         for (int k = 0; k < kKeys / 16; ++k)
           mma_tensor(o_tmem, s_tmem + buffer * kKeys + 8 * k, descriptor(v_addr + buffer * kValueBytes + k * 2048, true), kOutputs, (i > 0 || k > 0) ? 1u : 0u);
         commit(&s.done[g]);
-        if (i + 1 == group_tiles) commit(&s.finished[g]);
+        if (i + 1 == group_tiles) {
+          commit(&s.finished[g]);
+          if (lane == 0) bar_arrive(&s.finished[g]);
+        }
         commit(&s.value_empty[g][buffer]);
         if (i + 2 < group_tiles) {
           bar_wait<WAIT_EXPIRED>(&s.done[g], i & 1, abort_flag, p.status);   // (it reads the weights from the scores' columns)
@@ -509,32 +568,29 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap expanded_map, const __gr
     const bool brings_values = ((warp - kLoader) & 1) != 0;
     pdl_wait();
     if (!brings_values) bar_wait<WAIT_EXPIRED>(&s.query, 0, abort_flag, p.status);   // the queries lay where the keys go
-    for (int i = 0; i < group_tiles; ++i) {
-      const int j = 2 * i + g, buffer = i & 1, row = run.row0 + (first_tile + j) * kKeys;
-      uint8_t* tile = brings_values ? values + (2 * g + buffer) * kValueBytes : keys + (2 * g + buffer) * kKeyBytes;
-      if (i > 1)
-        bar_wait<WAIT_EXPIRED>(brings_values ? &s.value_empty[g][buffer] : &s.key_empty[g][buffer], ((i >> 1) - 1) & 1, abort_flag, p.status);
-      if (__any_sync(0xffffffffu, *abort_flag)) break;   // (what is in flight is waited for below)
-      if (lane == 0) {
-        uint64_t* full = brings_values ? &s.value_landed[g][buffer] : &s.key_full[g][buffer];
-        const int column = brings_values ? (p.heads + head) * kValues : head * kDim;
-        expect_bytes(full, brings_values ? kValueBytes : kKeyBytes);
-        for (int h = 0; h < 2; ++h) load_box(tile + h * kHalf, &expanded_map, full, column + 64 * h, row);
-        if (!brings_values) load_box(tile + 2 * kHalf, &rot_map, full, 0, row);
-      }
-      __syncwarp();
-      if (brings_values && ragged(j)) {
-        bar_wait<WAIT_EXPIRED>(&s.value_landed[g][buffer], (i >> 1) & 1, abort_flag, p.status);
-        for (int r = lane; r < kKeys; r += 32) {
-          const int key = key_base + j * kKeys + r;
-          if (key < first_key || key >= end_key) {
-#pragma unroll
-            for (int piece = 0; piece < 16; ++piece)
-              *reinterpret_cast<uint4*>(tile + (piece >> 3) * kHalf + piece_offset(r, piece & 7)) = make_uint4(0, 0, 0, 0);
-          }
+    // (a bounded tile's values are looked through behind the request for the next tile)
+    for (int i = 0; i <= group_tiles; ++i) {
+      if (i < group_tiles) {
+        const int j = 2 * i + g, buffer = i & 1, row = run.row0 + (first_tile + j) * kKeys;
+        uint8_t* tile = brings_values ? values + (2 * g + buffer) * kValueBytes : keys + (2 * g + buffer) * kKeyBytes;
+        if (i > 1)
+          bar_wait<WAIT_EXPIRED>(brings_values ? &s.value_empty[g][buffer] : &s.key_empty[g][buffer], ((i >> 1) - 1) & 1, abort_flag, p.status);
+        if (__any_sync(0xffffffffu, *abort_flag)) break;   // (what is in flight is waited for below)
+        if (lane == 0) {
+          uint64_t* full = brings_values ? &s.value_landed[g][buffer] : &s.key_full[g][buffer];
+          const int column = brings_values ? (p.heads + head) * kValues : head * kDim;
+          expect_bytes(full, brings_values ? kValueBytes : kKeyBytes);
+          for (int h = 0; h < 2; ++h) load_box(tile + h * kHalf, &expanded_map, full, column + 64 * h, row);
+          if (!brings_values) load_box(tile + 2 * kHalf, &rot_map, full, 0, row);
         }
+        __syncwarp();
+      }
+      const int before = i - 1, j = 2 * before + g, buffer = before & 1;
+      if (brings_values && before >= 0 && bounded(j)) {
+        bar_wait<WAIT_EXPIRED>(&s.value_landed[g][buffer], (before >> 1) & 1, abort_flag, p.status);
+        take_out(s, values + (2 * g + buffer) * kValueBytes, lane, key_base + j * kKeys, first_key, end_key);
         fence_async();
-        bar_arrive(&s.value_zeroed[g][buffer]);
+        bar_arrive(&s.value_looked[g][buffer]);
       }
     }
     // The gate's rows come where the queries and the first keys were, behind the last scores of both groups: the last softmax
@@ -604,7 +660,7 @@ inline int launch(const Params& p, const void* expanded, int num_tokens, int sta
   if ((status = opt_in.ask(reinterpret_cast<const void*>(latent_heads_kernel), kSharedBytes)) != 0) return status;
   // at most one partly filled tile per request beyond the full ones
   return vipera_launch(latent_heads_kernel, dim3(p.heads, (num_tokens + kQ - 1) / kQ + p.requests), dim3(kThreads), kSharedBytes, s,
-                       expanded_map, rot_map, query_map, gate_map, p);
+                       expanded_map, rot_map, query_map, gate_map, static_cast<const __nv_bfloat16*>(expanded), p);
 }
 
 }  // namespace latent_heads
