@@ -185,3 +185,84 @@ def test_values_that_are_not_finite(window):
     columns = torch.arange(256, device=DEV) != 128 + 5
     assert torch.equal(mixed[0][:, columns], mixed[1][:, columns])
     assert not torch.isfinite(mixed[1][:, 128 + 5]).any()
+
+
+def _folder(monkeypatch, window):
+    """A one-layer model of such heads, its scales such that attention outweighs the tokens' own rows, and sharp enough to show."""
+    import nuvezen_cases as cases
+
+    name = f"heads_of_128_{window}"
+    layer = cases.latent(heads=3, dim=DIM, rot_dim=ROT, vdim=VDIM, rank=256, q_rank=96, window=window, base=10000.0, scale=192 ** -0.5)
+    monkeypatch.setitem(cases.CONFIGS, name, cases.config([layer], width=256, vocab=300, eps=1e-5))
+    monkeypatch.setitem(cases.RULES, "attending", {".ls1": (0.0, 4.0), ".mix.uq": 5.0, ".mix.dkv": 4.0, ".mix.uk": 8.0, ".mix.uv": 8.0, ".mix.o": 8.0})
+    return cases, cases.folder(name, "bfloat16", 7, "attending")
+
+
+# (requests, tokens each brings) step by step: paddings of 81, 62 and 54 tokens; the second and third behind histories, a lone token among them
+STEPS_OF_A_RUN = [([0, 1], [200, 103]), ([0, 1, 2], [100, 1, 221]), ([2, 3, 4, 0], [64, 64, 64, 10])]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window", [0, 150])
+def test_captured_steps(window, monkeypatch):
+    """Steps through the runner, padded to their size class and replayed from a graph, whose rows follow from the step's own requests."""
+    from vipera_rs_b200.cache import CachePools
+    from vipera_rs_b200.engine import ModelRunner, StepInput
+    from vipera_rs_b200.engine.loader import load_model
+    from vipera_rs_b200.kernels import ops
+
+    cases, path = _folder(monkeypatch, window)
+    model = load_model(path, "bfloat16", DEV)
+    pools = CachePools(model.cache_requests, page_size=16, num_pages=100, num_state_slots=8, dtype=torch.bfloat16, device=torch.device(DEV))
+    runner, taken, real = ModelRunner(model, pools, max_model_len=1024), [], ops.latent_heads
+    monkeypatch.setattr(ops, "latent_heads", lambda *args, **named: taken.append(named["rows"].shape[0]) or real(*args, **named))
+    rng = np.random.RandomState(11)
+    tokens = {request: rng.randint(0, 300, 400).astype(np.int32) for request in range(5)}
+    done = dict.fromkeys(tokens, 0)
+    for requests, counts in STEPS_OF_A_RUN:
+        for request, count in zip(requests, counts):
+            if done[request] == 0:
+                pools.manager.open(request)
+            pools.manager.reserve(request, done[request] + count)
+            pools.manager.commit(request, done[request])
+        step = StepInput(requests=requests, counts=counts, pos0=[done[r] for r in requests], fresh=[int(done[r] == 0) for r in requests],
+                         tokens=np.concatenate([tokens[r][done[r]:done[r] + c] for r, c in zip(requests, counts)]),
+                         logit_rows=np.arange(sum(counts), dtype=np.int32))
+        before = len(taken)
+        got = [runner.run(step).double().cpu() for _ in range(2)]
+        assert len(taken) == before + 2 and taken[-1] in (512, 1024, 2048)     # a warm-up and a capture; the second run replays
+        assert torch.equal(got[0], got[1])
+        ops.check_kernel_status(DEV)
+        at = 0
+        for request, count in zip(requests, counts):
+            want = torch.from_numpy(np.asarray(cases.plain_logits(path, tokens[request][:done[request] + count].tolist())))[done[request]:]
+            # bfloat16 operands of seven products in a row, the rows' norms between them
+            assert float((got[0][at:at + count] - want).norm() / want.norm()) < 4e-2, (requests, counts, request)
+            at += count
+            done[request] += count
+    assert runner.eager_steps == 0 and len(runner._step_graphs) == len(STEPS_OF_A_RUN)
+
+
+def test_rows_of_captured_steps():
+    """A captured step's rows hold every request's, its padding's too; they are not what a size class leaves room for."""
+    from types import SimpleNamespace
+
+    part, _ = _part((3, 512, 0, 16, "interleaved", True), 0, "cpu")
+    windowed, _ = _part((3, 512, 1024, 16, "interleaved", True), 0, "cpu")
+
+    def rows(counts, firsts, own=part):
+        return own.step_forms(np.array(counts), np.array(firsts)).get(own._form_name(), 0)
+
+    assert rows([64] * 15 + [64], [0] * 16) == 2048             # fifteen prompts of 64 and their padding
+    assert rows([500] * 4 + [48], [0] * 5) == 4096
+    assert rows([1200, 1, 437, 110, 300], [0, 700, 64, 3000, 0]) == 8192
+    assert rows([2048], [0]) == 2048 and rows([1030, 506], [0, 0]) == 2048
+    assert rows([512], [7000]) == 8192 and rows([512], [7000], windowed) == 2048
+    assert rows([512, 8, 1], [0, 0, 20000]) == 0                # more rows than are planned for
+    assert rows([64] + [1] * 10, [0] + [2000] * 10) == 0 and rows([63], [0]) == 0
+    # a captured step whose requests nobody named expands all its bound allows: no more rows than it brings tokens
+    step = dict(host_counts=[], host_pos0=[], dtype=torch.bfloat16, all_single=False, extras={"graph": True})
+    assert part.expanded_rows(SimpleNamespace(num_tokens=1024, num_entries=16, max_kv_len=1024, **step)) == 0
+    assert part.expanded_rows(SimpleNamespace(num_tokens=2048, num_entries=1, max_kv_len=2048, **step)) == 2048
+    step["extras"] = {"graph": True, "forms": part.step_forms(np.array([1030, 506]), np.array([0, 0]))}
+    assert part.expanded_rows(SimpleNamespace(num_tokens=1536, num_entries=2, max_kv_len=4096, **step)) == 2048

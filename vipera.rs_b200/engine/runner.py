@@ -271,15 +271,24 @@ class ModelRunner:
         # whether the split-key attention runs beside the flash kernel is part of the class: some
         # entry (the padding entry included) brings exactly one token
         any_single = 1 in step.counts or bucket - total == 1
-        key = (bucket, entry_bucket, row_bucket, widths, any_single)
+        # and so are forms that follow from the requests themselves, which a class only bounds
+        forms = self._step_forms(step, bucket - total)
+        key = (bucket, entry_bucket, row_bucket, widths, any_single, tuple(sorted(forms.items())))
         graph = self._step_graphs.get(key)
         if graph is not None and graph.stale():
             graph = None
         if graph is None:
             if len(self._step_graphs) >= self.max_kept_graphs:
                 self._step_graphs.pop(next(iter(self._step_graphs)))
-            graph = self._step_graphs[key] = _StepGraph(self, bucket, entry_bucket, row_bucket, widths, any_single)
+            graph = self._step_graphs[key] = _StepGraph(self, bucket, entry_bucket, row_bucket, widths, any_single, forms)
         return graph
+
+    def _step_forms(self, step: StepInput, spare: int) -> dict:
+        asked = getattr(self.model, "step_forms", None)
+        if asked is None:
+            return {}
+        padding = [spare] if spare else []   # the padding tokens' entry begins at position 0
+        return asked(np.asarray(list(step.counts) + padding, dtype=np.int64), np.asarray(list(step.pos0) + [0] * len(padding), dtype=np.int64))
 
     # ------------------------------------------------------------------------------
     # decode steps through CUDA graphs
@@ -455,8 +464,9 @@ class _StepGraph:
     only the group's scratch page (a page no request ever holds), so what they compute lands
     nowhere; entries beyond that bring no tokens; spare wanted rows repeat the first."""
 
-    def __init__(self, runner: ModelRunner, tokens: int, entries: int, rows: int, widths, any_single: bool):
+    def __init__(self, runner: ModelRunner, tokens: int, entries: int, rows: int, widths, any_single: bool, forms: dict):
         self._runner = weakref.ref(runner)   # the runner owns its graphs, not the other way round
+        self.forms = forms
         self.tokens, self.entries, self.rows = int(tokens), int(entries), int(rows)
         self.any_single = bool(any_single)
         self.widths = [int(w) for w in widths]
@@ -540,7 +550,7 @@ class _StepGraph:
             host_counts=[], host_pos0=[], max_count=t,
             max_kv_len=min(w * runner._page_sizes[g] for g, w in enumerate(self.widths)) if self.widths else 0,
             all_single=False, any_single=self.any_single, dtype=runner.model.dtype, workspace=runner.workspace,
-            logits_all_rows=False, extras={"graph": True})
+            logits_all_rows=False, extras={"graph": True, "forms": self.forms})
 
     def run(self, step: StepInput) -> Optional[torch.Tensor]:
         from ..kernels import ops

@@ -218,6 +218,13 @@ class Part:
         tokens (for the memory plan; parts of one kind share their buffers between layers)."""
         return 0
 
+    def step_forms(self, counts, firsts) -> Dict[str, int]:
+        """What this part's launches in a captured step follow from beside the step's size class (its bounds on tokens, entries
+        and history): name -> number, from the step's own requests (tokens each brings, position it begins at; the entry that
+        pads the step among them).  Steps share a captured graph where the numbers agree; forward() finds them in
+        ``ctx.extras["forms"]``."""
+        return {}
+
 
 class Norm(Part):
     def forward(self, ctx: StepContext, x: torch.Tensor, out: torch.Tensor,

@@ -23,6 +23,7 @@ block, and a step of few tokens cuts its keys between blocks.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ..config.registry import MIXERS, POSITION_ENCODINGS
@@ -42,6 +43,11 @@ EXPANDED_FROM = 64
 EXPANDED_SHARE = 1.4    # (query, key) pairs per row, at least: 32 heads, 64 + 1 + 1 behind 0, 2,000, 2,000 has 1.4 and 191 / 117
 EXPANDED_ROWS = 16384   # most rows of keys; memory is planned for them
 HEAD_MAJOR_FROM = 64   # tokens of a step from which the up products run head by head on the tensor cores
+
+
+def _whole_runs(keys):
+    """Rows of a request's run of keys."""
+    return -(-keys // ops.LATENT_HEADS_ROWS) * ops.LATENT_HEADS_ROWS
 
 
 class LatentAttention(Mixer):
@@ -149,19 +155,34 @@ class LatentAttention(Mixer):
         128 per pair."""
         if not self.expands or ctx.all_single or ctx.dtype != torch.bfloat16 or ctx.num_tokens < EXPANDED_FROM:
             return 0
-        reach = self.window if self.window else 1 << 30
-        block = ops.LATENT_HEADS_ROWS
         if ctx.host_counts:
-            rows, pairs = 0, 0.0
-            for count, first in zip(ctx.host_counts, ctx.host_pos0):
-                kept = min(first, reach - 1)
-                rows += -(-(kept + count) // block) * block
-                pairs += count * min(kept + 0.5 * count, reach)
-        else:   # a captured step: any request may have the longest history, and the tokens may all be one request's own
+            rows, pairs = self._rows_and_pairs(np.asarray(ctx.host_counts, dtype=np.int64), np.asarray(ctx.host_pos0, dtype=np.int64))
+        elif self._form_name() in (forms := getattr(ctx, "extras", {}).get("forms", {})):
+            return forms[self._form_name()]
+        else:
+            # Requests that nobody named: any may have the longest history, and all rows that this takes are expanded, whether keys
+            # are there or not, instead of the two products over the step's tokens that cost as much per token as a row does here.
+            reach = self.window if self.window else 1 << 30
             longest = min(max(int(ctx.max_kv_len), 1), reach - 1 + ctx.num_tokens)
-            rows = ctx.num_entries * (-(-longest // block) * block)
-            pairs = 0.5 * ctx.num_tokens * min(ctx.num_tokens / ctx.num_entries, reach)
+            rows = ctx.num_entries * _whole_runs(longest)
+            pairs = min(0.5 * ctx.num_tokens * min(ctx.num_tokens / ctx.num_entries, reach), EXPANDED_SHARE * ctx.num_tokens)
         return rows if rows <= EXPANDED_ROWS and pairs >= EXPANDED_SHARE * rows else 0
+
+    def _rows_and_pairs(self, counts, firsts):
+        reach = self.window if self.window else 1 << 30
+        kept = np.minimum(firsts, reach - 1)
+        return int(_whole_runs(kept + counts).sum()), float((counts * np.minimum(kept + 0.5 * counts, reach)).sum())
+
+    def _form_name(self):
+        return f"latent.expanded.{self.window}"
+
+    def step_forms(self, counts, firsts):
+        # a captured step's rows: the requests' own, up to the next power of two, so that few graphs serve all histories
+        if not self.expands or int(counts.sum()) < EXPANDED_FROM:
+            return {}
+        rows, pairs = self._rows_and_pairs(counts, firsts)
+        rows = 1 << (rows - 1).bit_length()
+        return {self._form_name(): rows if rows <= EXPANDED_ROWS and pairs >= EXPANDED_SHARE * rows else 0}
 
     def prepare(self, max_positions: int) -> None:
         self.position.prepare(max_positions)

@@ -16,7 +16,7 @@ from ..config.spec import ModelSpec
 from ..errors import InternalError, InvalidArgumentError
 from ..kernels import ops
 from ..weights import Schema, TensorSpec, WeightSource, check_source, to_run_dtype
-from .base import StepContext
+from .base import Part, StepContext
 from .block import PendingJoin
 from .linear import Linear, NormedInput
 
@@ -52,6 +52,7 @@ class DecoderModel:
 
         embedding = fetch([spec.embedding_name])[spec.embedding_name]
         self.embedding = embedding.to(device=self.device, dtype=dtype).contiguous()
+        self._forming = None
         self.blocks = []
         for layer in spec.layers:
             block_cls = BLOCKS.find(layer.block)
@@ -100,6 +101,16 @@ class DecoderModel:
                 if not getattr(part, "graph_safe", True):
                     return False
         return True
+
+    def step_forms(self, counts, firsts) -> Dict[str, int]:
+        """What the parts' launches in a captured step follow from beside its size class (Part.step_forms)."""
+        if self._forming is None:   # one part of each kind and description: the others answer alike
+            self._forming = list({(type(part), repr(part.params)): part for block in self.blocks for part in block.parts()
+                                  if getattr(type(part), "step_forms", Part.step_forms) is not Part.step_forms}.values())
+        forms: Dict[str, int] = {}
+        for part in self._forming:
+            forms.update(part.step_forms(counts, firsts))
+        return forms
 
     def kernel_families(self) -> List[str]:
         names = ["rowwise", *self.head.kernel_families()]

@@ -79,6 +79,12 @@ class ParallelMixers(Mixer):
             if prepare is not None:
                 prepare(max_positions)
 
+    def step_forms(self, counts, firsts):
+        forms = {}
+        for _, branch in self.branches:
+            forms.update(branch.step_forms(counts, firsts))
+        return forms
+
     @classmethod
     def cache_request_for(cls, params):
         return CacheBundle.of(**{name: kind.cache_request_for(branch_params)
