@@ -266,3 +266,14 @@ def test_rows_of_captured_steps():
     assert part.expanded_rows(SimpleNamespace(num_tokens=2048, num_entries=1, max_kv_len=2048, **step)) == 2048
     step["extras"] = {"graph": True, "forms": part.step_forms(np.array([1030, 506]), np.array([0, 0]))}
     assert part.expanded_rows(SimpleNamespace(num_tokens=1536, num_entries=2, max_kv_len=4096, **step)) == 2048
+
+
+def test_plan():
+    """The memory plan counts the rows of expanded keys and values for runs that expand them."""
+    from vipera_rs_b200.parts.latent import EXPANDED_ROWS, LatentAttention
+
+    sizes = {"num_heads": 32, "kv_rank": 512, "rot_dim": 64, "head_dim": 128, "value_dim": 128}
+    bytes_of = lambda element, **other: LatentAttention.workspace_bytes(dict(sizes, **other), 2048, element)  # noqa: E731
+    mixed = 2048 * 32 * 128                     # the heads' outputs are in the run's type; the rest is alike
+    assert bytes_of(4) - bytes_of(2) == mixed * 2 - EXPANDED_ROWS * (32 * 256 + 512 + 64) * 2
+    assert bytes_of(4, rot_dim=32) - bytes_of(2, rot_dim=32) == mixed * 2

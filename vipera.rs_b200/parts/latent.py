@@ -198,7 +198,7 @@ class LatentAttention(Mixer):
         # (the splits of a step of few tokens: at most some 600 blocks of 16 rows more than the step's own)
         padded = tokens + 127
         head_major = heads * padded * (params["head_dim"] * 2 + rank * 6 + params["value_dim"] * 4) + tokens * heads * r * 4 + 4096
-        if params["head_dim"] == 128 and r == 64 and params["value_dim"] == 128:
+        if element_bytes == 2 and params["head_dim"] == 128 and r == 64 and params["value_dim"] == 128:   # (32-bit runs never expand)
             head_major += EXPANDED_ROWS * (heads * 256 + rank + r) * 2
         return (tokens * (width * 4 + heads * (2 * rank + r) * 4 + heads * params["value_dim"] * element_bytes)
                 + 16 * (rank + 2) * 4 * 1300 + head_major)
