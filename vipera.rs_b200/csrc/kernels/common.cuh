@@ -56,12 +56,18 @@ __device__ __forceinline__ float gate_activation(float z, int activation) {
   return z / (1.0f + expf(-z));
 }
 
-// 1 / (1 + e^-z) for a result that is stored as T: where that is bfloat16 (2^-9) by the approximate exponential and quotient,
-// some 2^-21 off, in a third of the instructions.
+// 1 / (1 + e^-z) without a branch, so that neighbouring values' chains overlap: the approximate quotient and one step of Newton's
+// method, r + r (1 - d r), the denominator scaled so that the largest one has a quotient too.  As far from 64 bits as the plain
+// expression, 3.5 times 2^-24 at most (by the approximate exponential 64 times at z = -80, and 0 below -87.3).
+__device__ __forceinline__ float sigmoid(float z) {
+  const float d = (1.0f + expf(-z)) * 0x1p-64f, near = __fdividef(1.0f, d), inverse = fmaf(near, fmaf(-d, near, 1.0f), near);
+  return d == INFINITY ? 0.0f : inverse * 0x1p-64f;
+}
+// z / (1 + e^-z) for a result that is stored as T: a rounding more where that is bfloat16.
 template <typename T>
-__device__ __forceinline__ float sigmoid_for(float z) {
-  if constexpr (sizeof(T) == 2) return __fdividef(1.0f, 1.0f + __expf(-z));
-  return 1.0f / (1.0f + expf(-z));
+__device__ __forceinline__ float silu_for(float z) {
+  if constexpr (sizeof(T) == 2) return z * sigmoid(z);
+  return z / (1.0f + expf(-z));
 }
 // Four neighbours of a row of T.
 template <typename T>

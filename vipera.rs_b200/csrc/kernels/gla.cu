@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(128) gla_finish_kernel(const GlaParams p) {
   const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off + head * p.vdim;
   TO* out = static_cast<TO*>(p.out) + base;
   auto ending = [&](float o, float inverse, float g, int e) {
-    out[e] = from_float<TO>(o * inverse * p.norm_weight[e] * (g * sigmoid_for<TO>(g)) * p.out_scale);
+    out[e] = from_float<TO>(o * inverse * p.norm_weight[e] * silu_for<TO>(g) * p.out_scale);
   };
   float squares = 0.0f;
   if (p.shares == 1 && p.vdim <= 32 * kFinishKept) {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(128) gla_finish_kernel(const GlaParams p) {
         const int e = (lane + 32 * j) * 4;
         if (e >= p.vdim) break;
         const float4 w = *reinterpret_cast<const float4*>(p.norm_weight + e);
-        auto gated = [&](float v, float weight, float z) { return v * inverse * weight * (z * sigmoid_for<TO>(z)) * p.out_scale; };
+        auto gated = [&](float v, float weight, float z) { return v * inverse * weight * silu_for<TO>(z) * p.out_scale; };
         store_four_as<TO>(out + e, gated(o[j].x, w.x, g[j].x), gated(o[j].y, w.y, g[j].y), gated(o[j].z, w.z, g[j].z), gated(o[j].w, w.w, g[j].w));
       }
       return;

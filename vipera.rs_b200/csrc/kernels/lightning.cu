@@ -280,8 +280,8 @@ lightning_finish_kernel(LightningParams p) {
       const int i = (threadIdx.x + 256 * j) * 4;
       if (i >= width) break;
       const float4 w = *reinterpret_cast<const float4*>(p.norm_weight + i);
-      store_four_as<TO>(out + i, o[j].x * inverse * w.x * sigmoid_for<TO>(g[j].x), o[j].y * inverse * w.y * sigmoid_for<TO>(g[j].y),
-                        o[j].z * inverse * w.z * sigmoid_for<TO>(g[j].z), o[j].w * inverse * w.w * sigmoid_for<TO>(g[j].w));
+      store_four_as<TO>(out + i, o[j].x * inverse * w.x * sigmoid(g[j].x), o[j].y * inverse * w.y * sigmoid(g[j].y),
+                        o[j].z * inverse * w.z * sigmoid(g[j].z), o[j].w * inverse * w.w * sigmoid(g[j].w));
     }
     return;
   }
@@ -290,7 +290,7 @@ lightning_finish_kernel(LightningParams p) {
   const float inverse = 1.0f / sqrtf(block_sum(sum, scratch) / static_cast<float>(width) + p.eps);
   TO* out = static_cast<TO*>(p.out) + static_cast<size_t>(t) * width;
   for (int i = threadIdx.x; i < width; i += blockDim.x)
-    out[i] = from_float<TO>(raw[i] * inverse * p.norm_weight[i] * sigmoid_for<TO>(gate[i]));
+    out[i] = from_float<TO>(raw[i] * inverse * p.norm_weight[i] * sigmoid(gate[i]));
 }
 
 static int launch_carry(const LightningParams& p, cudaStream_t s) {

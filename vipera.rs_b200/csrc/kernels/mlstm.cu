@@ -1283,12 +1283,12 @@ mlstm_finish_kernel(const MlstmParams p, int num_tokens, const float* __restrict
     read(w, c, scale);
     T y[kWidth];
 #pragma unroll
-    for (int j = 0; j < kWidth; ++j) y[j] = from_float<T>(mine[i][j] * inverse * scale[j] * sigmoid_for<T>(gates[i][j]));
+    for (int j = 0; j < kWidth; ++j) y[j] = from_float<T>(mine[i][j] * inverse * scale[j] * sigmoid(gates[i][j]));
     if constexpr (!FOURS) dst[c] = y[0];
     else if constexpr (sizeof(T) == 2) *reinterpret_cast<uint2*>(dst + c) = *reinterpret_cast<const uint2*>(y);
     else *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(y);
   }
-  for (int c = 512 + lane; c < dv; c += 32) dst[c] = from_float<T>(o[c] * inverse * w[c] * sigmoid_for<T>(gate[c]));
+  for (int c = 512 + lane; c < dv; c += 32) dst[c] = from_float<T>(o[c] * inverse * w[c] * sigmoid(gate[c]));
   const int e = token_entry[t];
   if (t == p.entry_starts[e + 1] - 1) {
     float* state = p.state + static_cast<long long>(p.state_slots[e]) * p.state_stride;
