@@ -1205,19 +1205,14 @@ mlstm_decode_kernel(const MlstmParams p) {
 
 template <int D>
 static int launch_walk(const MlstmParams& p, cudaStream_t s) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t error = cudaFuncSetAttribute(mlstm_prepare_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(PrepareLayout<D>::kBytes));
-    if (error == cudaSuccess)
-      error = cudaFuncSetAttribute(mlstm_walk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, WalkLayout<D>::kBytes);
-    if (error != cudaSuccess) return static_cast<int>(error);
-    configured = true;
-  }
+  static SharedMemoryOptIn opt_in_prepare, opt_in_walk;
+  int status = opt_in_prepare.ask(reinterpret_cast<const void*>(mlstm_prepare_kernel<D>), static_cast<int>(PrepareLayout<D>::kBytes));
+  if (status == 0) status = opt_in_walk.ask(reinterpret_cast<const void*>(mlstm_walk_kernel<D>), WalkLayout<D>::kBytes);
+  if (status != 0) return status;
   const WalkBuffers buffers{static_cast<__nv_bfloat16*>(p.walk_q), static_cast<__nv_bfloat16*>(p.walk_k), static_cast<__nv_bfloat16*>(p.walk_w),
                             static_cast<__nv_bfloat16*>(p.walk_v), p.walk_token, p.walk_factors, p.status};
   const dim3 jobs(p.heads, p.max_jobs);
-  int status = vipera_launch(mlstm_prepare_kernel<D>, jobs, kTcThreads, PrepareLayout<D>::kBytes, s, p, buffers);
+  status = vipera_launch(mlstm_prepare_kernel<D>, jobs, kTcThreads, PrepareLayout<D>::kBytes, s, p, buffers);
   if (status == 0) status = vipera_launch(mlstm_nm_kernel, dim3(p.heads, p.num_entries), 256, 0, s, p);
   if (status == 0) status = vipera_launch(mlstm_factors_kernel<D>, dim3(p.heads, p.max_jobs, (p.vdim + kFactorCols - 1) / kFactorCols), 256, 0, s, p, buffers);
   if (status == 0)
