@@ -37,3 +37,10 @@ def test_rows_alone_and_together(n, k, ending):
         want = z + (1.0 if ending == "residual" else 0.0)
     # chains of K / 128 products a lane: 2^-24 times the root of their number, and the factors around
     assert float((alone.double() - want).norm() / want.norm()) < 2e-6
+
+
+@pytest.mark.parametrize("n,k", [(4097, 2100), (9001, 1000), (2049, 3076), (2049, 2052), (14209, 1028)])
+@pytest.mark.parametrize("ending", ["store", "gated"])
+def test_members_of_enough_runs(n, k, ending):
+    """Four, two and eight blocks of a cluster on either side of three runs a block, and four rows on eight."""
+    test_rows_alone_and_together(n, k, ending)

@@ -273,6 +273,11 @@ constexpr int kFewStages = 3;   // runs of a warp's ring
 constexpr int kFewRun = 128;    // values of K
 constexpr int kFewSplit = 8;    // most members
 constexpr long long kSharedFrom = 4000000;   // numbers of W
+// Runs of a member, below which the cluster's barriers and a run of A that is asked for behind the wait are not made up for, by
+// more than four rows and by up to four.  8 rows, inputs out of L2, us in warps / shared: 2,048 x 2,048 (two runs) 6.5 / 7.8, 8,000 x
+// 512 (two) 6.4 / 7.5, 3,072 x 2,048 (two) 12.4 / 13.3, 9,728 x 896 (three and a half) 18.1 / 15.7, 1,024 x 4,096 (four) 9.8 / 8.2.
+// 4 rows: 16,384 x 256 (two) 4.6 / 5.0, 32,000 x 896 (seven) 21.8 / 22.1, 17,920 x 1,536 (twelve) 19.6 / 18.8.
+constexpr int kSharedRuns = 3, kSharedRunsFour = 8;
 
 // The lanes' sums of N values: at each step a lane keeps one half of the values it holds and hands over the other, until
 // it holds one or two; then every lane holds the same value's.  Returns the first value a lane ends with, and how many.
@@ -567,8 +572,9 @@ static int launch_few(const GemmArgs& p, cudaStream_t s) {
   if (p.M == 1) return launch_few_rows<1>(p, members, s);
   if (p.M == 2) return launch_few_rows<2>(p, members, s);
   const bool large = static_cast<long long>(p.N) * p.K >= kSharedFrom;
-  if (p.M <= 4) return members == 1 && large ? launch_few_shared<4>(p, members, s) : launch_few_rows<4>(p, members, s);
-  return large ? launch_few_shared<8>(p, members, s) : launch_few_rows<8>(p, members, s);
+  const int runs = p.K / (kFewRun * members);
+  if (p.M <= 4) return members == 1 && large && runs >= kSharedRunsFour ? launch_few_shared<4>(p, members, s) : launch_few_rows<4>(p, members, s);
+  return large && (members == 1 || runs >= kSharedRuns) ? launch_few_shared<8>(p, members, s) : launch_few_rows<8>(p, members, s);
 }
 
 template <typename TA, typename TW, typename T, bool DIRECT, bool CLUSTER>
