@@ -745,12 +745,15 @@ static int launch_split(const AttentionParams& p, int clusters, cudaStream_t s) 
 // Among how many blocks a tile's keys are cut: 1, 2 or 4, by the longest of what a block walks and what all of them cost a
 // multiprocessor, in microseconds: a tile of 64 keys `tile`, a block's start and ending `start`, joining 4.  The keys are those the
 // block table, a window or a chunk leaves room for; several requests see half of them on average (the longest history may be
-// a lone token's, whose launch is another), and below 128 tokens of several requests it may be a lone token's alone.  1 / 2 / 4
+// a lone token's, whose launch is another), and below 128 tokens of several requests it may be a lone token's alone.  `longest`: the
+// keys of the longest of the requests that bring several tokens, where the caller knows (0: not): short requests in a wide table
+// have none to share (eight portions of 60 tokens, room for 512, a 32-bit step of four layers: 1,220 us shared, 1,142 not).  1 / 2 / 4
 // blocks: 14 heads of 64 on 2, 200 tokens 28 / 25 / 21 us, 800 106 / 75 / 85, 2,048 299 / 292 / 342, 800 under a window of 256 55 / 60 / 72,
 // 100 behind 1,000 119 / 68 / 52; 12 heads of 128 on 2, 1,024 tokens of three requests 206 / 138 / 146, 100 behind 3,000 556 / 285 /
 // 190; 4 heads of 256 on 1, 800 tokens 245 / 146 / 109; two tiles of keys: 65 tokens, 14 heads of 64 14.8 / 17.2.
-static int tile_members(const AttentionParams& p, int dp, int requests) {
+static int tile_members(const AttentionParams& p, int dp, int requests, int longest) {
   long long most = static_cast<long long>(p.table_width) * p.page_size;
+  if (longest > 0) most = std::min<long long>(most, longest);
   if (p.window > 0) most = std::min<long long>(most, static_cast<long long>(p.window) + kTileRows + p.keep_first);
   if (p.chunk > 0) most = std::min<long long>(most, p.chunk);
   const long long walked = (most + kTileKeys - 1) / kTileKeys;
@@ -775,7 +778,7 @@ static int tile_members(const AttentionParams& p, int dp, int requests) {
 // histories in a tile's rows that they do not fill, behind the tile's other requests: they go to the split form, a launch
 // of their own (1,024 tokens, one of them alone behind 900 keys: 270 us in the tiles alone, 133 + 21 us).
 template <typename T, int DP, bool VEC>
-static int launch_attention(const AttentionParams& asked, int requests, cudaStream_t s) {
+static int launch_attention(const AttentionParams& asked, int requests, int longest, cudaStream_t s) {
   AttentionParams p = asked;
   if (warps_win(p, DP, VEC, sizeof(T) == 2, requests))
     return vipera_launch(attention_warp_kernel<T, VEC>, dim3(p.num_tokens, (p.num_heads + kWarpsPerBlock - 1) / kWarpsPerBlock),
@@ -789,7 +792,7 @@ static int launch_attention(const AttentionParams& asked, int requests, cudaStre
   static SharedMemoryOptIn opt_in, opt_in_join;
   constexpr int kBytes = static_cast<int>(sizeof(TileShared<DP>));
   const dim3 grid(p.num_heads, (p.num_tokens + kTileRows - 1) / kTileRows);
-  const int members = tile_members(p, DP, requests);
+  const int members = tile_members(p, DP, requests, longest);
   if (members == 1) {
     const int opted = opt_in.ask(reinterpret_cast<const void*>(attention_tile_kernel<T, DP, VEC, false>), kBytes);
     return opted ? opted : vipera_launch(attention_tile_kernel<T, DP, VEC, false>, grid, dim3(kTileThreads), kBytes, s, p, 1);
@@ -799,14 +802,14 @@ static int launch_attention(const AttentionParams& asked, int requests, cudaStre
 }
 
 template <typename T>
-static int launch_sizes(const AttentionParams& p, int requests, cudaStream_t s) {
+static int launch_sizes(const AttentionParams& p, int requests, int longest, cudaStream_t s) {
   constexpr int kPiece = 16 / static_cast<int>(sizeof(T));
   const bool vec = p.head_dim % kPiece == 0 && p.value_dim % kPiece == 0 &&
                    ((reinterpret_cast<uintptr_t>(p.k_pool) | reinterpret_cast<uintptr_t>(p.v_pool)) & 15) == 0;
   const int largest = p.head_dim > p.value_dim ? p.head_dim : p.value_dim;
-  if (largest <= 64) return vec ? launch_attention<T, 64, true>(p, requests, s) : launch_attention<T, 64, false>(p, requests, s);
-  if (largest <= 128) return vec ? launch_attention<T, 128, true>(p, requests, s) : launch_attention<T, 128, false>(p, requests, s);
-  return vec ? launch_attention<T, 256, true>(p, requests, s) : launch_attention<T, 256, false>(p, requests, s);
+  if (largest <= 64) return vec ? launch_attention<T, 64, true>(p, requests, longest, s) : launch_attention<T, 64, false>(p, requests, longest, s);
+  if (largest <= 128) return vec ? launch_attention<T, 128, true>(p, requests, longest, s) : launch_attention<T, 128, false>(p, requests, longest, s);
+  return vec ? launch_attention<T, 256, true>(p, requests, longest, s) : launch_attention<T, 256, false>(p, requests, longest, s);
 }
 
 // q is [tokens, heads, d] and out [tokens, heads, value_dim]; the key pool is
@@ -824,7 +827,7 @@ VIPERA_API int vipera_attention_step(const void* q, void* out, int dtype, const 
                                       int table_width, int page_size, int num_tokens, int num_heads,
                                       int num_kv_heads, int head_dim, int value_dim, float scale, int window,
                                       int keep_first, int sink, int chunk, float out_scale, const float* sink_values,
-                                      const float* gate, long long gate_stride, int gate_per_head, int requests, void* stream) {
+                                      const float* gate, long long gate_stride, int gate_per_head, int requests, int longest, void* stream) {
   if (num_tokens <= 0) return VIPERA_OK;
   if (chunk < 0 || (chunk > 0 && window > 0)) return VIPERA_BAD_ARGUMENT;
   if (head_dim <= 0 || head_dim > kMaxHeadDim) return VIPERA_BAD_SHAPE;
@@ -836,8 +839,8 @@ VIPERA_API int vipera_attention_step(const void* q, void* out, int dtype, const 
                           num_kv_heads, head_dim, value_dim, scale, window, keep_first, sink, chunk, out_scale, sink_values, gate,
                           gate_stride, gate_per_head, 0};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == VIPERA_F32) return launch_sizes<float>(p, requests, s);
-  if (dtype == VIPERA_BF16) return launch_sizes<__nv_bfloat16>(p, requests, s);
+  if (dtype == VIPERA_F32) return launch_sizes<float>(p, requests, longest, s);
+  if (dtype == VIPERA_BF16) return launch_sizes<__nv_bfloat16>(p, requests, longest, s);
   return VIPERA_BAD_DTYPE;
 }
 

@@ -529,7 +529,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: 
               num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
               value_dim: Optional[int] = None, keep_first: int = 0, sink: bool = False, chunk: int = 0,
               out_scale: float = 1.0, sink_values: Optional[torch.Tensor] = None,
-              gate: Optional[torch.Tensor] = None, gate_offset: int = 0, gate_per_head: bool = False) -> None:
+              gate: Optional[torch.Tensor] = None, gate_offset: int = 0, gate_per_head: bool = False, longest: int = 0) -> None:
     """Causal grouped-query attention of every token of the step over its request's pages.
     ``value_dim``: a value row's size (default d); ``keep_first``: with a window, that many
     first keys stay visible; ``sink``: one is added to the softmax's denominator; ``chunk``:
@@ -537,11 +537,12 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: 
     (chunks counted from position 0); ``out_scale`` multiplies the output.  ``sink_values``
     float32 [heads]: exp(sink_h) joins head h's denominator instead of one.  ``gate`` float32
     [tokens, width]: the output is multiplied by the sigmoid of the heads * value_dim values that
-    start at column ``gate_offset`` of the token's row (``gate_per_head``: of heads values, one for a whole head)."""
+    start at column ``gate_offset`` of the token's row (``gate_per_head``: of heads values, one for a whole head).
+    ``longest``: no request that brings several tokens sees more keys (0: not known); it decides how they are shared, no more."""
     fn = _function("attention", "vipera_attention_step",
                    [_c_void, _c_void, _c_int, _c_void, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_int,
                     _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void,
-                    _c_void, ctypes.c_longlong, _c_int, _c_int, _c_void])
+                    _c_void, ctypes.c_longlong, _c_int, _c_int, _c_int, _c_void])
     if chunk and window:
         raise InvalidArgumentError("attention: a mask is a window or chunks, not both")
     count = q.shape[0]
@@ -567,7 +568,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: 
               num_heads, num_kv_heads, head_dim, value_dim, float(scale), int(window or 0),
               int(keep_first or 0) if window else 0, 1 if sink else 0, int(chunk or 0), float(out_scale),
               _opt(sink_values, "sink_values", torch.float32), gate_pointer, gate_stride, int(bool(gate_per_head)),
-              block_table.shape[0], _stream()), "attention", kernels=2 if count > 64 and block_table.shape[0] > 1 else 1)
+              block_table.shape[0], int(longest), _stream()), "attention", kernels=2 if count > 64 and block_table.shape[0] > 1 else 1)
 
 
 # ----------------------------------------------------------------------------------------

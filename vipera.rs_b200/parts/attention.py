@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import os
 
+import numpy as np
 import torch
 
 from ..config.registry import MIXERS, POSITION_ENCODINGS
@@ -279,6 +280,21 @@ class GQAttention(Mixer):
         # (and the rows it leaves where an arrangement takes rows)
         return tokens * ((q_width + params["num_heads"] * dv) * element_bytes + qkv_width * 4 + params["hidden_size"] * 4)
 
+    def _general(self, dtype) -> bool:
+        """Whether steps run the general kernel, whatever they bring (an output gate or sinks may send others there too)."""
+        return self.talk is None and (dtype != torch.bfloat16 or self.head_dim not in ops.MMA_HEAD_DIMS or
+                                      self.value_dim != self.head_dim or self.out_scale != 1.0)
+
+    @staticmethod
+    def _longest(counts, firsts) -> int:
+        """Keys of the longest request that brings several tokens, up to the next power of two (one for all steps alike)."""
+        most = int(np.where(counts > 1, firsts + counts, 1).max())
+        return max(1 << (most - 1).bit_length(), 64)
+
+    def step_forms(self, counts, firsts):
+        # few tokens take forms that no request's length decides
+        return {"attention.longest": self._longest(counts, firsts)} if self._general(self.dtype) and int(counts.sum()) > 64 else {}
+
     def _output(self, ctx, mixed, residual):
         """The output product: added into the stream, or left as rows where there is none."""
         if residual is None:
@@ -459,11 +475,15 @@ class GQAttention(Mixer):
                                          window=window, chunk=chunk, num_splits=splits, scratch=scratch,
                                          entry_starts=ctx.entry_starts, **kept)
             return
+        if ctx.host_counts:
+            longest = self._longest(np.asarray(ctx.host_counts, dtype=np.int64), np.asarray(ctx.host_pos0, dtype=np.int64))
+        else:
+            longest = ctx.extras.get("forms", {}).get("attention.longest", 0)
         ops.attention(q, mixed, cache.k, cache.v, token_seq=ctx.token_entry, positions=ctx.positions,
                       block_table=table, num_heads=heads, num_kv_heads=kv_heads, head_dim=d,
                       scale=self.scale, window=window, value_dim=self.value_dim, keep_first=self.keep_first,
                       sink=self.sink, chunk=self.chunk, out_scale=self.out_scale, sink_values=self.sink_values,
-                      gate=gate, gate_offset=self.gate_offset, gate_per_head=self.gate_per_head)
+                      gate=gate, gate_offset=self.gate_offset, gate_per_head=self.gate_per_head, longest=longest)
 
 
 MIXERS.register("gqa_attention", GQAttention)
