@@ -767,7 +767,7 @@ static int tile_members(const AttentionParams& p, int dp, int requests, int long
   int members = 1;
   for (int m = 1; m <= kMostMembers; m *= 2) {
     const double longest = start + tile * in_tile * ((walked + m - 1) / m);
-    const double all = blocks * (m * start + in_tile * seen / kTileKeys * tile) / 148;
+    const double all = blocks * (m * start + in_tile * seen / kTileKeys * tile) / multiprocessors();
     const double cost = (m > 1 ? 4.0 : 0.0) + std::max(longest, all);
     if (m == 1 || cost < best) best = cost, members = m;
   }

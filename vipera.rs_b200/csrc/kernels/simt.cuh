@@ -45,6 +45,17 @@ struct SharedMemoryOptIn {
   }
 };
 
+// Multiprocessors of the current device, asked for once per device.
+static inline int multiprocessors() {
+  static std::atomic<int> counts[64];
+  int device = 0, count = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return 148;
+  if (device < 64 && (count = counts[device].load(std::memory_order_relaxed)) > 0) return count;
+  if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count <= 0) return 148;
+  if (device < 64) counts[device].store(count, std::memory_order_relaxed);
+  return count;
+}
+
 // Launch `kernel` as vipera_launch does; `cluster` > 1: in clusters of that many blocks along x.
 template <typename... KernelArgs, typename... Args>
 static inline int launch_in_clusters(void (*kernel)(KernelArgs...), int cluster, dim3 grid, dim3 block, size_t shared_bytes,

@@ -134,7 +134,8 @@ class MLSTM(Mixer):
         chunks = -(-max(ctx.host_counts or [ctx.max_count]) // ops.MLSTM_CHUNK)
         blocks = (tokens / ops.MLSTM_CHUNK + 0.5 * entries) * self.heads * (self.vdim // 32)
         states = (tokens // ops.MLSTM_CHUNK + entries) * self.heads * self.dim * self.vdim * 4e-6
-        return 30.0 + 2.0 * max(chunks, blocks / 148) < 4.0 + 2.1 * states
+        sms = ops.sm_count(proj.device) if proj.is_cuda else 148
+        return 30.0 + 2.0 * max(chunks, blocks / sms) < 4.0 + 2.1 * states
 
     def forward(self, ctx, h, residual, cache, writes_cache):
         count = ctx.num_tokens
