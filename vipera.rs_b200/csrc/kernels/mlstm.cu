@@ -1223,28 +1223,31 @@ static int launch_walk(const MlstmParams& p, cudaStream_t s) {
 // ---------------------------------------------------------------------------------------
 // the ending: head norm, scale, output gate; and the new n and m into the state
 // ---------------------------------------------------------------------------------------
-// A warp per (token, head).  out[t, h*dv + c] = o / rms(o) * weight[h*dv + c] * sigmoid(g[t, h*dv + c]).  Values come four
-// at a time where rows start on 16 bytes (FOURS), and up to 512 of them stay in registers between the two passes.
-// What bounds it: memory.  2,048 tokens, 8 heads of 512: 24 us (a block per (token, head), a value at a time: 27).
-constexpr int kFinishWarps = 8;
+// LANES threads per (token, head), which keep KEPT times four values each (FOURS: rows that start on 16 bytes) or KEPT values.
+// out[t, h*dv + c] = o / rms(o) * weight[h*dv + c] * sigmoid(g[t, h*dv + c]).
+// What bounds it: one trip to memory where rows are few, so that a row has as many threads as take four values each.  The mixer, 8
+// heads of 512, a token: 24.1 us (a warp per (token, head) 27.2), 2,048 tokens 333 (336).
+constexpr int kFinishThreads = 256;
 
-template <typename T, bool FOURS>
-__global__ void __launch_bounds__(kFinishWarps * 32)
+template <typename T, int LANES, int KEPT, bool FOURS>
+__global__ void __launch_bounds__(kFinishThreads)
 mlstm_finish_kernel(const MlstmParams p, int num_tokens, const float* __restrict__ weight, float eps, T* __restrict__ out,
                     const int* __restrict__ token_entry) {
+  __shared__ float sums[kFinishThreads / 32];
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long long item = static_cast<long long>(blockIdx.x) * kFinishWarps + (threadIdx.x >> 5);
-  if (item >= static_cast<long long>(num_tokens) * p.heads) return;
-  const int t = static_cast<int>(item / p.heads), h = static_cast<int>(item % p.heads);
-  const int dv = p.vdim, d = p.dim;
-  const float* o = p.o_raw + static_cast<size_t>(item) * dv;
-  const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off + h * dv;
-  const float* w = weight + h * dv;
-  T* dst = out + static_cast<size_t>(item) * dv;
-  constexpr int kWidth = FOURS ? 4 : 1, kKept = 16 / kWidth;   // values a thread takes at a time, and how often
-  float mine[kKept][kWidth], gates[kKept][kWidth];
+  constexpr int kRows = kFinishThreads / LANES;
+  const int lane = threadIdx.x % LANES;
+  const long long item = static_cast<long long>(blockIdx.x) * kRows + threadIdx.x / LANES;
+  const bool valid = item < static_cast<long long>(num_tokens) * p.heads;
+  const int t = valid ? static_cast<int>(item / p.heads) : 0, h = valid ? static_cast<int>(item % p.heads) : 0;
+  const int dv = valid ? p.vdim : 0, d = p.dim;
+  const float* o = p.o_raw + (static_cast<size_t>(t) * p.heads + h) * p.vdim;
+  const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off + h * p.vdim;
+  const float* w = weight + h * p.vdim;
+  T* dst = out + (static_cast<size_t>(t) * p.heads + h) * p.vdim;
+  constexpr int kWidth = FOURS ? 4 : 1;   // values a thread takes at a time
+  float mine[KEPT][kWidth], gates[KEPT][kWidth], scale[KEPT][kWidth];
   auto read = [&](const float* from, int c, float (&to)[kWidth]) {
     if constexpr (FOURS) {
       const float4 v = *reinterpret_cast<const float4*>(from + c);
@@ -1255,54 +1258,71 @@ mlstm_finish_kernel(const MlstmParams p, int num_tokens, const float* __restrict
   };
   float squares = 0.0f;
 #pragma unroll
-  for (int i = 0; i < kKept; ++i) {
-    const int c = (i * 32 + lane) * kWidth;
+  for (int i = 0; i < KEPT; ++i) {
+    const int c = (i * LANES + lane) * kWidth;
 #pragma unroll
-    for (int j = 0; j < kWidth; ++j) mine[i][j] = gates[i][j] = 0.0f;
+    for (int j = 0; j < kWidth; ++j) mine[i][j] = gates[i][j] = scale[i][j] = 0.0f;
     if (c < dv) {
       read(o, c, mine[i]);
       read(gate, c, gates[i]);
+      read(w, c, scale[i]);
     }
   }
 #pragma unroll
-  for (int i = 0; i < kKept; ++i)
+  for (int i = 0; i < KEPT; ++i)
 #pragma unroll
     for (int j = 0; j < kWidth; ++j) squares = fmaf(mine[i][j], mine[i][j], squares);
-  for (int c = 512 + lane; c < dv; c += 32) squares = fmaf(o[c], o[c], squares);
-  const float inverse = rsqrtf(warp_sum(squares) / static_cast<float>(dv) + eps);
+  constexpr int kHeld = KEPT * LANES * kWidth;
+  for (int c = kHeld + lane; c < dv; c += LANES) squares = fmaf(o[c], o[c], squares);
+  squares = warp_sum(squares);
+  if constexpr (LANES > 32) {
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = squares;
+    __syncthreads();
+    squares = 0.0f;
 #pragma unroll
-  for (int i = 0; i < kKept; ++i) {
-    const int c = (i * 32 + lane) * kWidth;
-    if (c >= dv) continue;
-    float scale[kWidth];
-    read(w, c, scale);
-    T y[kWidth];
-#pragma unroll
-    for (int j = 0; j < kWidth; ++j) y[j] = from_float<T>(mine[i][j] * inverse * scale[j] * sigmoid(gates[i][j]));
-    if constexpr (!FOURS) dst[c] = y[0];
-    else if constexpr (sizeof(T) == 2) *reinterpret_cast<uint2*>(dst + c) = *reinterpret_cast<const uint2*>(y);
-    else *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(y);
+    for (int i = 0; i < LANES / 32; ++i) squares += sums[threadIdx.x / LANES * (LANES / 32) + i];
   }
-  for (int c = 512 + lane; c < dv; c += 32) dst[c] = from_float<T>(o[c] * inverse * w[c] * sigmoid(gate[c]));
+  if (!valid) return;
+  const float inverse = rsqrtf(squares / static_cast<float>(dv) + eps);
+#pragma unroll
+  for (int i = 0; i < KEPT; ++i) {
+    const int c = (i * LANES + lane) * kWidth;
+    if (c >= dv) continue;
+    float y[kWidth];
+#pragma unroll
+    for (int j = 0; j < kWidth; ++j) y[j] = mine[i][j] * inverse * scale[i][j] * sigmoid(gates[i][j]);
+    if constexpr (FOURS) store_four_as<T>(dst + c, y[0], y[1], y[2], y[3]);
+    else dst[c] = from_float<T>(y[0]);
+  }
+  for (int c = kHeld + lane; c < dv; c += LANES) dst[c] = from_float<T>(o[c] * inverse * w[c] * sigmoid(gate[c]));
   const int e = token_entry[t];
   if (t == p.entry_starts[e + 1] - 1) {
     float* state = p.state + static_cast<long long>(p.state_slots[e]) * p.state_stride;
     float* n_state = state + static_cast<size_t>(p.heads) * d * dv + static_cast<size_t>(h) * d;
     float* m_state = state + static_cast<size_t>(p.heads) * d * (dv + 1) + h;
     const float* scratch = p.nm_scratch + (static_cast<size_t>(e) * p.heads + h) * (d + 1);
-    for (int dd = lane; dd < d; dd += 32) n_state[dd] = scratch[dd];
+#pragma unroll 4
+    for (int dd = lane; dd < d; dd += LANES) n_state[dd] = scratch[dd];
     if (lane == 0) m_state[0] = scratch[d];
   }
+}
+
+template <typename T, int LANES, int KEPT, bool FOURS>
+static int launch_finish_lanes(const MlstmParams& p, int num_tokens, const float* weight, float eps, T* out, const int* token_entry, cudaStream_t s) {
+  const long long rows = static_cast<long long>(num_tokens) * p.heads;
+  constexpr int kRows = kFinishThreads / LANES;
+  return vipera_launch(mlstm_finish_kernel<T, LANES, KEPT, FOURS>, dim3(static_cast<unsigned>((rows + kRows - 1) / kRows)), kFinishThreads, 0, s, p, num_tokens,
+                       weight, eps, out, token_entry);
 }
 
 template <typename T>
 static int launch_finish(const MlstmParams& p, int num_tokens, const float* weight, float eps, T* out, const int* token_entry, cudaStream_t s) {
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.o_raw) | reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(out);
   const bool fours = (bases & 15) == 0 && p.vdim % 4 == 0 && p.proj_width % 4 == 0 && p.g_off % 4 == 0;
-  const long long warps = static_cast<long long>(num_tokens) * p.heads;
-  const dim3 grid(static_cast<unsigned>((warps + kFinishWarps - 1) / kFinishWarps));
-  return fours ? vipera_launch(mlstm_finish_kernel<T, true>, grid, kFinishWarps * 32, 0, s, p, num_tokens, weight, eps, out, token_entry)
-               : vipera_launch(mlstm_finish_kernel<T, false>, grid, kFinishWarps * 32, 0, s, p, num_tokens, weight, eps, out, token_entry);
+  if (!fours) return launch_finish_lanes<T, 128, 4, false>(p, num_tokens, weight, eps, out, token_entry, s);
+  if (p.vdim <= 128) return launch_finish_lanes<T, 32, 1, true>(p, num_tokens, weight, eps, out, token_entry, s);
+  if (p.vdim <= 256) return launch_finish_lanes<T, 64, 1, true>(p, num_tokens, weight, eps, out, token_entry, s);
+  return launch_finish_lanes<T, 128, 1, true>(p, num_tokens, weight, eps, out, token_entry, s);
 }
 
 static size_t chunk_shared_bytes(int d, int tile) {
