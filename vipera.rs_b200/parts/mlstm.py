@@ -29,7 +29,7 @@ from .base import FixedState, Mixer
 from .linear import Linear
 
 
-WALK_ENTRIES = 32   # most requests of a step that walks prepared chunks: each may end in a partly filled one, and memory is planned for them
+WALK_ENTRIES = 64   # most requests of a step that walks prepared chunks: each may end in a partly filled one, and memory is planned for them
 
 
 class MLSTM(Mixer):
@@ -130,7 +130,7 @@ class MLSTM(Mixer):
         if not ops.mlstm_walk_takes(proj, self.offsets, self.dim, self.vdim) or tokens < 6 * entries:
             return False
         if tokens < self.AT_ONCE_FROM:
-            return self.dim >= 128 or tokens >= 128
+            return tokens > ops.MLSTM_CHUNK if self.dim >= 128 else tokens >= 128
         chunks = -(-max(ctx.host_counts or [ctx.max_count]) // ops.MLSTM_CHUNK)
         blocks = (tokens / ops.MLSTM_CHUNK + 0.5 * entries) * self.heads * (self.vdim // 32)
         states = (tokens // ops.MLSTM_CHUNK + entries) * self.heads * self.dim * self.vdim * 4e-6
