@@ -199,47 +199,72 @@ lightning_scan_kernel(LightningParams p) {
   }
 }
 
-// A thread N neighbouring values of a head's state and entry (two where rows are whole 8-byte pieces): the entry's chunks in a
-// row.  What bounds it: the chunks' states, read and written.  2,048 tokens, 6 heads of 128 x 256, the mixer by 1, 2 and 4
-// values a thread: 164.4, 160.0 and 163.0 us.
-template <int N>
-__global__ void __launch_bounds__(128)
+// A thread N neighbouring values of a head's state and entry (where rows are whole pieces of N): the entry's chunks in a row,
+// `AHEAD` of them asked for together, then walked in order.  What bounds it: the chunks' states, read and written; the powers of
+// lambda, which every thread computed for itself, were most of its instructions (28 us of ten requests of 100 tokens, 6 heads of
+// 128 x 256, where the bytes are 6; two values and sixteen ahead with them 46).  The mixer, cold, us by one value and eight ahead, each
+// with its powers / two and sixteen / four and four: 6 heads of 128 x 256, 2,048 tokens 156.6 / 148.5 / 156.5, 1,030 124.0 / 123.2 /
+// 127.9, ten requests of 100 119.9 / 130.7 / 124.6, twenty of 20 124 / 117 / 106, forty of 50 276 / 206 / 177; of 64 x 128, three of 700
+// 132 / 128 / 122, eight of 256 114 / 124 / 122.  So requests of few chunks take four and four.
+constexpr int kCarryThreads = 128;
+constexpr int kCarryShort = 12;   // chunks of a request on average, up to which it takes four values and four ahead
+
+template <int N, int AHEAD>
+__global__ void __launch_bounds__(kCarryThreads)
 lightning_carry_kernel(LightningParams p) {
+  // lambda^kChunk of each head of the block's values, and what the request's last chunk leaves: by repeated multiplication, the same
+  // way the scan applies it, a thread a head (each of the block's threads for itself they were most of this kernel's instructions)
+  __shared__ float whole[kCarryThreads * N + 2], ends_with[kCarryThreads * N + 2];
+  __shared__ int first_job;
   pdl_launch_dependents();
   pdl_wait();
-  const int entry = blockIdx.y;
-  const size_t state_size = static_cast<size_t>(p.heads) * p.d * p.dv;
-  const size_t element = (static_cast<size_t>(blockIdx.x) * 128 + threadIdx.x) * N;
-  if (element >= state_size) return;
+  const int entry = blockIdx.y, head_size = p.d * p.dv;
+  const size_t state_size = static_cast<size_t>(p.heads) * head_size, first = static_cast<size_t>(blockIdx.x) * (kCarryThreads * N);
+  const size_t element = first + threadIdx.x * N;
   const int start = p.entry_starts[entry], stop = p.entry_starts[entry + 1];
   if (stop <= start) return;
-  int job = 0;
-  for (int e = 0; e < entry; ++e) job += (p.entry_starts[e + 1] - p.entry_starts[e] + kChunk - 1) / kChunk;
-  const float lambda = p.decay[element / (static_cast<size_t>(p.d) * p.dv)];
+  const int head0 = static_cast<int>(first / head_size), heads = min(p.heads - head0, static_cast<int>((first % head_size + kCarryThreads * N - 1) / head_size) + 1);
+  if (threadIdx.x >= kCarryThreads - 32) {
+    const int lane = threadIdx.x & 31;
+    int jobs = 0;
+    for (int e = lane; e < entry; e += 32) jobs += (p.entry_starts[e + 1] - p.entry_starts[e] + kChunk - 1) / kChunk;
+    jobs = __reduce_add_sync(0xffffffffu, jobs);
+    if (lane == 0) first_job = jobs;
+  }
+  for (int i = threadIdx.x; i < heads; i += kCarryThreads) {
+    const float lambda = p.decay[head0 + i];
+    const int tail = (stop - start - 1) % kChunk + 1;
+    float power = 1.0f, ends = 1.0f;
+#pragma unroll
+    for (int k = 1; k <= kChunk; ++k) {
+      power *= lambda;
+      if (k == tail) ends = power;
+    }
+    whole[i] = power;
+    ends_with[i] = ends;
+  }
   struct alignas(4 * N) Values { float v[N]; };
+  const bool valid = element < state_size;
   Values* own = reinterpret_cast<Values*>(p.state + static_cast<size_t>(p.state_slots[entry]) * state_size + element);
   Values s{};
-  if (!p.fresh[entry]) s = *own;
-  // sixteen chunks at a time: their endings are asked for together, then walked in order
-  constexpr int kAhead = 16;
-  float whole = 1.0f;   // lambda^kChunk by repeated multiplication, the same way the scan applies it
-  for (int i = 0; i < kChunk; ++i) whole *= lambda;
-  for (int begin = start; begin < stop; begin += kAhead * kChunk, job += kAhead) {
-    Values ending[kAhead];
+  if (valid && !p.fresh[entry]) s = *own;
+  __syncthreads();
+  if (!valid) return;
+  const int at = static_cast<int>(static_cast<unsigned>(element) / static_cast<unsigned>(head_size)) - head0;   // (a state of 4 G elements does not exist)
+  const float factor = whole[at], last_factor = ends_with[at];
+  Values* states = reinterpret_cast<Values*>(p.chunk_state + static_cast<size_t>(first_job) * state_size + element);
+  const size_t step = state_size / N;   // (a row of the state is whole pieces)
+  const int chunks = (stop - start + kChunk - 1) / kChunk;
+  for (int c0 = 0; c0 < chunks; c0 += AHEAD, states += AHEAD * step) {
+    Values ending[AHEAD];
 #pragma unroll
-    for (int c = 0; c < kAhead; ++c)
-      if (begin + c * kChunk < stop) ending[c] = *reinterpret_cast<const Values*>(p.chunk_state + static_cast<size_t>(job + c) * state_size + element);
+    for (int c = 0; c < AHEAD; ++c)
+      if (c0 + c < chunks) ending[c] = states[c * step];
 #pragma unroll
-    for (int c = 0; c < kAhead; ++c) {
-      const int first = begin + c * kChunk;
-      if (first >= stop) break;
-      const int length = min(kChunk, stop - first);
-      *reinterpret_cast<Values*>(p.chunk_state + static_cast<size_t>(job + c) * state_size + element) = s;
-      float power = whole;
-      if (length < kChunk) {
-        power = 1.0f;
-        for (int i = 0; i < length; ++i) power *= lambda;
-      }
+    for (int c = 0; c < AHEAD; ++c) {
+      if (c0 + c >= chunks) break;
+      states[c * step] = s;
+      const float power = c0 + c + 1 < chunks ? factor : last_factor;
 #pragma unroll
       for (int j = 0; j < N; ++j) s.v[j] = fmaf(power, s.v[j], ending[c].v[j]);
     }
@@ -248,9 +273,11 @@ lightning_carry_kernel(LightningParams p) {
 }
 
 // The norm over the concatenated heads, the norm's weight and the output gate; a block per token.  What bounds it: memory.
-constexpr int kFinishKept = 4;   // pieces of a row a thread keeps
+// KEPT: pieces of four values a thread keeps of a row (0: rows that are read again, a value at a time).  Narrow rows take blocks of no
+// more threads than they have pieces: 2,048 rows of 768 values 6.5 us, by 256 threads of four pieces 8.4, a value at a time 10.8.
+constexpr int kFinishKept = 4;
 
-template <typename TO>
+template <typename TO, int KEPT>
 __global__ void __launch_bounds__(256)
 lightning_finish_kernel(LightningParams p) {
   __shared__ float scratch[32];
@@ -260,44 +287,58 @@ lightning_finish_kernel(LightningParams p) {
   const int width = p.heads * p.dv;
   const float* raw = p.raw + static_cast<size_t>(t) * width;
   const float* gate = p.proj + static_cast<size_t>(t) * p.proj_width + p.g_off;
-  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.raw) | reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.norm_weight) | reinterpret_cast<uintptr_t>(p.out);
-  if (width <= 4 * kFinishKept * 256 && width % 4 == 0 && p.proj_width % 4 == 0 && p.g_off % 4 == 0 && (bases & 15) == 0) {
+  if constexpr (KEPT > 0) {
     // rows of whole 16-byte pieces that fit the block's registers: read once, all of it at the same time
-    float4 o[kFinishKept], g[kFinishKept];
+    float4 o[KEPT], g[KEPT];
     float sum = 0.0f;
 #pragma unroll
-    for (int j = 0; j < kFinishKept; ++j) {
-      const int i = (threadIdx.x + 256 * j) * 4;
+    for (int j = 0; j < KEPT; ++j) {
+      const int i = (threadIdx.x + blockDim.x * j) * 4;
       o[j] = g[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (i < width) o[j] = *reinterpret_cast<const float4*>(raw + i), g[j] = *reinterpret_cast<const float4*>(gate + i);
     }
 #pragma unroll
-    for (int j = 0; j < kFinishKept; ++j) sum += o[j].x * o[j].x + o[j].y * o[j].y + o[j].z * o[j].z + o[j].w * o[j].w;
+    for (int j = 0; j < KEPT; ++j) sum += o[j].x * o[j].x + o[j].y * o[j].y + o[j].z * o[j].z + o[j].w * o[j].w;
     const float inverse = 1.0f / sqrtf(block_sum(sum, scratch) / static_cast<float>(width) + p.eps);
     TO* out = static_cast<TO*>(p.out) + static_cast<size_t>(t) * width;
 #pragma unroll
-    for (int j = 0; j < kFinishKept; ++j) {
-      const int i = (threadIdx.x + 256 * j) * 4;
+    for (int j = 0; j < KEPT; ++j) {
+      const int i = (threadIdx.x + blockDim.x * j) * 4;
       if (i >= width) break;
       const float4 w = *reinterpret_cast<const float4*>(p.norm_weight + i);
       store_four_as<TO>(out + i, o[j].x * inverse * w.x * sigmoid(g[j].x), o[j].y * inverse * w.y * sigmoid(g[j].y),
                         o[j].z * inverse * w.z * sigmoid(g[j].z), o[j].w * inverse * w.w * sigmoid(g[j].w));
     }
-    return;
+  } else {
+    float sum = 0.0f;
+    for (int i = threadIdx.x; i < width; i += blockDim.x) sum += raw[i] * raw[i];
+    const float inverse = 1.0f / sqrtf(block_sum(sum, scratch) / static_cast<float>(width) + p.eps);
+    TO* out = static_cast<TO*>(p.out) + static_cast<size_t>(t) * width;
+    for (int i = threadIdx.x; i < width; i += blockDim.x)
+      out[i] = from_float<TO>(raw[i] * inverse * p.norm_weight[i] * sigmoid(gate[i]));
   }
-  float sum = 0.0f;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) sum += raw[i] * raw[i];
-  const float inverse = 1.0f / sqrtf(block_sum(sum, scratch) / static_cast<float>(width) + p.eps);
-  TO* out = static_cast<TO*>(p.out) + static_cast<size_t>(t) * width;
-  for (int i = threadIdx.x; i < width; i += blockDim.x)
-    out[i] = from_float<TO>(raw[i] * inverse * p.norm_weight[i] * sigmoid(gate[i]));
 }
 
+template <typename TO>
+static int launch_finish(const LightningParams& p, cudaStream_t s) {
+  const int width = p.heads * p.dv, pieces = (width + 3) / 4;
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.raw) | reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.norm_weight) | reinterpret_cast<uintptr_t>(p.out);
+  if (pieces > kFinishKept * 256 || width % 4 || p.proj_width % 4 || p.g_off % 4 || (bases & 15))
+    return vipera_launch(lightning_finish_kernel<TO, 0>, p.num_tokens, 256, 0, s, p);
+  const int threads = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
+  if (pieces <= 256) return vipera_launch(lightning_finish_kernel<TO, 1>, p.num_tokens, threads, 0, s, p);
+  return vipera_launch(lightning_finish_kernel<TO, kFinishKept>, p.num_tokens, threads, 0, s, p);
+}
+
+template <int N, int AHEAD>
+static int launch_carry_as(const LightningParams& p, cudaStream_t s) {
+  const size_t threads = static_cast<size_t>(p.heads) * p.d * p.dv / N;
+  return vipera_launch(lightning_carry_kernel<N, AHEAD>, dim3(static_cast<unsigned>((threads + kCarryThreads - 1) / kCarryThreads), p.num_entries), kCarryThreads, 0, s, p);
+}
 static int launch_carry(const LightningParams& p, cudaStream_t s) {
-  const bool pairs = p.dv % 2 == 0 && ((reinterpret_cast<uintptr_t>(p.state) | reinterpret_cast<uintptr_t>(p.chunk_state)) & 7) == 0;
-  const size_t threads = static_cast<size_t>(p.heads) * p.d * p.dv / (pairs ? 2 : 1);
-  const dim3 grid(static_cast<unsigned>((threads + 127) / 128), p.num_entries);
-  return pairs ? vipera_launch(lightning_carry_kernel<2>, grid, 128, 0, s, p) : vipera_launch(lightning_carry_kernel<1>, grid, 128, 0, s, p);
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(p.state) | reinterpret_cast<uintptr_t>(p.chunk_state);
+  if (p.dv % 4 == 0 && (bases & 15) == 0 && p.num_tokens <= static_cast<long long>(kCarryShort) * kChunk * p.num_entries) return launch_carry_as<4, 4>(p, s);
+  return p.dv % 2 == 0 && (bases & 7) == 0 ? launch_carry_as<2, 16>(p, s) : launch_carry_as<1, 16>(p, s);
 }
 
 template <int RPT>
@@ -345,8 +386,8 @@ VIPERA_API int vipera_lightning(const LightningParams* params, int out_dtype, vo
   else if (p.d <= 128) status = launch_scans<32>(p, chunked, s);
   else status = launch_scans<64>(p, chunked, s);
   if (status) return status;
-  if (out_dtype == VIPERA_F32) return vipera_launch(lightning_finish_kernel<float>, p.num_tokens, 256, 0, s, p);
-  if (out_dtype == VIPERA_BF16) return vipera_launch(lightning_finish_kernel<__nv_bfloat16>, p.num_tokens, 256, 0, s, p);
+  if (out_dtype == VIPERA_F32) return launch_finish<float>(p, s);
+  if (out_dtype == VIPERA_BF16) return launch_finish<__nv_bfloat16>(p, s);
   return VIPERA_BAD_DTYPE;
 }
 
