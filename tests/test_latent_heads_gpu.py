@@ -187,6 +187,53 @@ def test_values_that_are_not_finite(window):
     assert not torch.isfinite(mixed[1][:, 128 + 5]).any()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("own_cache", [True, False])
+def test_query_latents_and_shared_pages(gated, own_cache):
+    """Queries that come through a latent (a buffer of their own, the gate in another), and a layer that reads another's pages."""
+    from vipera_rs_b200.kernels import ops
+
+    heads, rank, q_rank, counts, firsts = 3, 256, 96, [150, 1, 200], [70, 40, 0]
+    parts, weights = [], []
+    for index in range(1 if own_cache else 2):
+        writer = index == 0
+        part, w = _part((heads, rank, 0, 16, "interleaved", gated), index, DEV)
+        params = dict(part.params, q_rank=q_rank, own_cache=writer)
+        schema = type(part).schema(params, "p")
+        for name, std in (("p.dq.weight", 0.06), ("p.uq.weight", 0.1)):
+            w[name] = (torch.randn(*schema[name].shape, device=DEV) * std).bfloat16()
+        w["p.dq.norm.weight"] = torch.randn(q_rank, device=DEV) * 0.1 + 1.0
+        parts.append(type(part)(params, "p", {name: w[name] for name in schema}, torch.bfloat16, DEV))
+        weights.append(w)
+    h = torch.randn(sum(counts), HIDDEN, device=DEV).bfloat16()
+    context, view, kept = _step(parts[-1], counts, firsts, 16, rank)
+    parts[0].prepare(4096)
+    for part in parts:
+        assert part.expanded_rows(context) > 0
+        out = torch.zeros(len(h), HIDDEN, device=DEV)
+        part.forward(context, h, out, view, part.own_cache)
+    torch.cuda.synchronize()
+    ops.check_kernel_status(DEV)
+    wide = {name: t.double() for name, t in weights[-1].items()}
+    for name in ("p.dkv.weight", "p.dkv.norm.weight"):
+        wide[name] = weights[0][name].double()
+    # the restatement's queries are a product of its rows: the query latents stand beside them
+    low = h.double() @ wide["p.dq.weight"].T
+    low = low / torch.sqrt((low * low).mean(-1, keepdim=True) + 1e-6) * wide["p.dq.norm.weight"]
+    rows, zeros = torch.cat([h.double(), low], dim=1), lambda n, m: torch.zeros(n, m, dtype=torch.float64, device=DEV)  # noqa: E731
+    wide["p.q.weight"] = torch.cat([zeros(heads * (DIM + ROT), HIDDEN), wide["p.uq.weight"]], dim=1)
+    wide["p.dkv.weight"] = torch.cat([wide["p.dkv.weight"], zeros(rank + ROT, q_rank)], dim=1)
+    eye = dict(wide, **{"p.o.weight": torch.eye(heads * VDIM, dtype=torch.float64, device=DEV)})
+    want = _plain(eye, rows, kept, counts, firsts, heads, DIM, ROT, rank, VDIM, 0, False)
+    if gated:
+        want = want * torch.sigmoid(h.double() @ wide["p.g.weight"].T)
+    want = want @ wide["p.o.weight"].T
+    # bfloat16 operands of six products in a row: 2^-9 each and a little
+    assert float((out.double() - want).norm() / want.norm()) < 1e-2
+    assert float(((out.double() - want).norm(dim=1) / want.norm(dim=1)).max()) < 4e-2
+
+
 def _folder(monkeypatch, window):
     """A one-layer model of such heads, its scales such that attention outweighs the tokens' own rows, and sharp enough to show."""
     import nuvezen_cases as cases
