@@ -82,7 +82,7 @@ class ParallelMixers(Mixer):
     def step_forms(self, counts, firsts):
         forms = {}
         for _, branch in self.branches:
-            forms.update(branch.step_forms(counts, firsts))
+            forms.update(getattr(branch, "step_forms", lambda *_: {})(counts, firsts))
         return forms
 
     @classmethod
