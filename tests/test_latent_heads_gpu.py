@@ -169,22 +169,22 @@ def test_tokens_that_are_not_finite(sizes, token):
 @pytest.mark.gpu
 @pytest.mark.parametrize("window", [0, 100])
 def test_values_that_are_not_finite(window):
-    """One value of a head is infinite for every token: it shows in that column of every token's heads, in no other column."""
+    """Two values of a head are infinite for every token: they show in those columns of every token's heads, in no other column."""
     sizes = (2, 256, window, 16, "interleaved", False)
     mixed = []
     for value in (None, float("inf")):
         part, _ = _part(sizes, 7, DEV)
         if value is not None:
-            part.up_kv[(2 + 1) * 128 + 5, 17] = value     # head 1, its value 5
+            part.up_kv[(2 + 1) * 128 + 5, 17], part.up_kv[(2 + 1) * 128 + 100, 30] = value, -value     # head 1, its values 5 and 100
         torch.manual_seed(3)
         h = torch.randn(333, HIDDEN, device=DEV).bfloat16()
         context, view, _ = _step(part, [333], [40], 16, 256, window)
         assert part.expanded_rows(context) > 0
         part.forward(context, h, torch.zeros(333, HIDDEN, device=DEV), view, True)
         mixed.append(context.workspace.get("latent.out", (333, 256), torch.bfloat16).clone())
-    columns = torch.arange(256, device=DEV) != 128 + 5
+    columns = (torch.arange(256, device=DEV) != 128 + 5) & (torch.arange(256, device=DEV) != 128 + 100)
     assert torch.equal(mixed[0][:, columns], mixed[1][:, columns])
-    assert not torch.isfinite(mixed[1][:, 128 + 5]).any()
+    assert not torch.isfinite(mixed[1][:, ~columns]).any()
 
 
 @pytest.mark.gpu

@@ -132,3 +132,10 @@ def test_values_that_are_not_finite(kind, dim, vdim, token):
         outs.append(out)
     for out in outs[1:]:
         assert torch.equal(out[:token], outs[0][:token]) and not torch.isfinite(out[token:]).any()
+
+
+@pytest.mark.parametrize("dim,vdim", [(4, 4), (18, 30), (70, 36), (30, 7)])
+def test_requests_of_many_chunks(dim, vdim):
+    """The carry's forms for requests of many chunks (rows of whole pairs and not), beside one that ends within its first."""
+    test_decays_per_head([850, 3], dim, vdim)
+    test_decays_per_head([1700, 1], dim, vdim)

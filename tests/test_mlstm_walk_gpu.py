@@ -107,3 +107,10 @@ def test_the_plan_holds_the_scratch():
                 others = tokens * ((2 * heads * (dim + vdim) + 2 * heads) * 4 + heads * vdim * 6 + heads * (dim + 1) * 4)
                 assert (tokens // ops.MLSTM_CHUNK + entries) * scratch <= MLSTM.workspace_bytes(params, tokens, 2) - others
     assert walked > 50
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("steps", [[[65, 1, 64, 3, 130, 1, 20], [2, 64, 1, 1, 66, 128, 9]], [[5] * 40]])
+def test_walk_of_many_requests(steps):
+    """More requests than a handful, lone tokens among them: their chunks lie one request after another."""
+    test_walk(steps, (2, 128, 64))
