@@ -20,7 +20,8 @@
 // What bounds it: a block's start (set-up, queries: some 8 K clocks) and its softmax, 2.4 K clocks per 64 keys and group, of
 // which the exponentials are 512 and scaling the output to a new maximum some 400; tensor cores are busy a third of the time.
 // Measured: 2,048 tokens, 12 heads, rank 512, window 1,024: the mixer 287 -> 108 us; 1,748 tokens of four requests behind up
-// to 3,000, 32 heads, a gate: 663 -> 306 us (over the latents, latent_tc.cuh, before).
+// to 3,000, 32 heads, a gate: 663 -> 306 us (over the latents, latent_tc.cuh, before; the same inputs again, in L2: with inputs
+// that change 290 -> 113 and 668 -> 352).
 // A value that is not finite shows in the outputs of the queries that see its key, and in no others: out of the tiles that some query
 // of a block sees and another does not, such values are taken before the product and given back at the end.  Looking through these
 // tiles costs 0.4 us of 112; with the product's own zeros times infinities up to 127 earlier tokens lost their outputs.

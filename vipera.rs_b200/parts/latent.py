@@ -35,10 +35,12 @@ from .linear import Linear
 
 
 # Where every head's keys and values are expanded for a step (csrc/kernels/latent_heads.cuh), us of the mixer over the latents
-# and expanded.  From 64 tokens on it is the faster one in all of 100 steps of 8 to 32 heads, ranks 256 and 512, behind up to
+# and expanded (the same inputs again, in L2).  From 64 tokens on it is the faster one in all of 100 steps of 8 to 32 heads, ranks 256 and 512, behind up to
 # 7,000 tokens: 12 heads, a prompt of 2,048 under a window of 1,024: 287 / 108; 32 heads, 1,748 tokens of four requests behind
 # up to 3,000: 663 / 306; closest where few heads walk many keys, 8 heads, 64 behind 7,000: 182 / 161.  Below, few heads lose:
-# 8 heads, 32 and 48 behind 3,000: 71 / 89 and 85 / 90; 12 heads of rank 256, a prompt of 32: 37 / 41.
+# 8 heads, 32 and 48 behind 3,000: 71 / 89 and 85 / 90; 12 heads of rank 256, a prompt of 32: 37 / 41.  Captured steps of one such
+# layer, of 2,048, whose rows are a power of two: 12 heads, fifteen prompts of 64 142 / 109, 512 tokens beside eight single ones behind
+# 1,000 480 / 164; 32 heads, four prompts of 500 487 / 218, the four requests above 1,146 / 275.
 EXPANDED_FROM = 64
 EXPANDED_SHARE = 1.4    # (query, key) pairs per row, at least: 32 heads, 64 + 1 + 1 behind 0, 2,000, 2,000 has 1.4 and 191 / 117
 EXPANDED_ROWS = 16384   # most rows of keys; memory is planned for them

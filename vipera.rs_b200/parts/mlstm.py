@@ -120,10 +120,11 @@ class MLSTM(Mixer):
     def walks(self, ctx, proj) -> bool:
         """Whether a step's portions walk chunks that were prepared ahead (csrc/kernels/mlstm_walk.cuh).  Such a walk takes 30 us
         and 2.0 us per chunk of the longest request, or of all blocks where they are more than the multiprocessors; all chunks
-        at once (long steps) take 2.1 us per megabyte of states at the chunks' starts.  us of the mixer at once / walking: 8 heads
-        of 256 x 512, 2,048 tokens 511 / 332, 512 tokens 154 / 129; 4 heads, 512 tokens 73 / 77; 8 heads of 128 x 256, 2,048
-        tokens 158 / 168, three requests of 1,024, 901 and 77 152 / 134.  Short steps, against the walk without preparation: 4
-        heads of 256 x 512, 128 tokens 67 / 49; of 128 x 256 51 / 42; of 64 x 128, 65 tokens 39 / 38, 17 + 1 + 1 23 / 28."""
+        at once (long steps) take 2.1 us per megabyte of states at the chunks' starts.  us of the mixer at once / walking (the same
+        inputs again, in L2; the first with inputs that change 533 / 369): 8 heads of 256 x 512, 2,048 tokens 511 / 332, 512 tokens
+        154 / 129; 4 heads, 512 tokens 73 / 77; 8 heads of 128 x 256, 2,048 tokens 158 / 168, three requests of 1,024, 901 and 77 152 /
+        134.  Short steps, against the walk without preparation: 4 heads of 256 x 512, 128 tokens 67 / 49; of 128 x 256 51 / 42, 64
+        tokens 33.3 / 35.8; of 64 x 128, 65 tokens 39 / 38, 17 + 1 + 1 23 / 28."""
         tokens, entries = ctx.num_tokens, ctx.num_entries
         if entries > WALK_ENTRIES:
             return False
