@@ -97,8 +97,9 @@ struct GemmParams {
   // matrices [N, K] one after the other, and the 128 tokens of tile tx use matrix tile_group[tx].
   // The table is written by a kernel ahead of this one, so no weight tile is fetched before it.
   // tile_count: how many of the table's tiles there are (written like it); null: all of them.  A step's table is as long as
-  // its rows may need, every matrix's last tile partly filled; some 8 of 97 tiles (10,240 rows, 17 matrices) are not there,
-  // and computing them cost the mixture of [3584, 1536] and [1536, 1792] 234 us against 217.
+  // its rows may need, every matrix's last tile partly filled; some 8 of 97 tiles (10,240 rows, 17 matrices) are not there.
+  // Counted tiles run a row of tiles after the other: neighbouring blocks read one matrix together.  2,048 tokens, 4 of 16 units
+  // of [3584, 1536] and [1536, 1792] and a shared one, the mixture with cold weights: 230 us not counted, 218 counted column by column, 208 so.
   const int* tile_group;     // [tiles_x] or null
   const int* tile_count;
   int group_stride;          // rows of W from one matrix to the next (N)
